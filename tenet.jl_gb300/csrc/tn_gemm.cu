@@ -7,7 +7,10 @@
 // the bound for this kernel, so the design goal is to keep every SM's DFMA units fed:
 // register tiles of 4×4 (or 2×2 for small grids) complex accumulators per thread,
 // A/B tiles staged through shared memory, and a tile size chosen so the grid covers
-// all 152 SMs even for the small bond-dimension GEMMs of an MPS sweep.
+// all 152 SMs even for the small bond-dimension GEMMs of an MPS sweep (k_gemm_fine below
+// is the kernel for grids that 64×64 tiles leave partly idle).
+#include <cooperative_groups.h>
+
 #include "tn_internal.cuh"
 
 namespace {
@@ -125,6 +128,149 @@ tn_status_t launch(tn_ctx* ctx, char opa, char opb, int64_t m, int64_t n, int64_
   return TN_OK;
 }
 
+// Fine-grained GEMM: one output per thread and K group, tiles of BM·BN ≤ 64 outputs.
+//
+// Bound: the FP64 pipe retires 2 DFMA per clock and SM (64 clocks per warp instruction,
+// measured), so a 32×32 tile with k = 64 holds one SM for 70 µs while the chip's rate for the
+// whole 64×128×64 product is 4 µs: what counts for an MPS-sized product is that every SM has
+// work.  8×8 tiles keep 128 of 152 SMs busy there; operand traffic (32 bytes per 4 DFMA)
+// stays two orders below the L2 rate.  Measured (GB300): the overlap of two L = 64, χ = 256 MPS
+// (256×512×256 and 256×256×512 products) 49.2 → 27.8 ms, 24.7 ms being the FP64 pipe's time;
+// a served burst of 64 queries (L ≤ 48, χ ≤ 128) 18.9 → 7.5 ms; one two-site DMRG sweep
+// (L = 24, χ = 32) 297 → 258 ms.  K goes in stages of 32 prefetched to registers, split
+// over KS thread groups inside the CTA and over a cluster of CS CTAs (summed through
+// distributed shared memory) when the columns alone leave SMs idle.
+//
+// The sum over k is the same sequence for every tile shape: 16 interleaved accumulators
+// (k mod 16) per cluster rank, added in a fixed order, and CS depends on n and k only.  A
+// row of C is therefore bit-identical whatever number of rows it is computed with, as long
+// as this kernel serves both products.
+constexpr int kFineBK = 32, kFineAcc = 16, kFineThreads = 256;
+
+template <typename T, int BM, int BN>
+__global__ void __launch_bounds__(kFineThreads)
+    k_gemm_fine(char opa, char opb, int64_t m, int64_t n, int64_t k, cx<T> alpha, const cx<T>* __restrict__ A, int64_t lda,
+                int64_t sA, const cx<T>* __restrict__ B, int64_t ldb, int64_t sB, cx<T> beta, cx<T>* __restrict__ C,
+                int64_t ldc, int64_t sC, int64_t batch, int CS) {
+  namespace cg = cooperative_groups;
+  constexpr int KS = kFineThreads / (BM * BN), NA = kFineAcc / KS;
+  constexpr int LA = (BM * kFineBK + kFineThreads - 1) / kFineThreads, LB = (BN * kFineBK + kFineThreads - 1) / kFineThreads;
+  static_assert(KS * NA == kFineAcc, "accumulators must divide among the K groups");
+  __shared__ cx<T> As[kFineBK][BM + 1];
+  __shared__ cx<T> Bs[kFineBK][BN + 1];
+  __shared__ cx<T> part[kFineAcc][BM * BN];
+  __shared__ cx<T> total[BM * BN];
+  const int tid = threadIdx.x, out = tid % (BM * BN), kg = tid / (BM * BN);
+  const int ti = out % BM, tj = out / BM;
+  const int rank = (int)(blockIdx.x % (unsigned)CS);
+  const int64_t i0 = (int64_t)(blockIdx.x / (unsigned)CS) * BM, j0 = (int64_t)blockIdx.y * BN;
+  // this rank's part of K, a whole number of stages
+  const int64_t stages = (k + kFineBK - 1) / kFineBK, per = (stages + CS - 1) / CS;
+  const int64_t kb = min((int64_t)rank * per * kFineBK, k), ke = min((int64_t)(rank + 1) * per * kFineBK, k);
+  for (int64_t bz = blockIdx.z; bz < batch; bz += gridDim.z) {
+    const cx<T>* Ab = A + bz * sA;
+    const cx<T>* Bb = B + bz * sB;
+    cx<T> acc[NA], ra[LA], rb[LB];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) acc[a] = mkcx<T>(0, 0);
+    auto fetch = [&](int64_t p0) {
+#pragma unroll
+      for (int u = 0; u < LA; ++u) {
+        const int t = tid + u * kFineThreads;
+        const int ii = opa == 'N' ? t % BM : t / kFineBK, pp = opa == 'N' ? t / BM : t % kFineBK;
+        ra[u] = (t < BM * kFineBK && i0 + ii < m && p0 + pp < ke) ? load_op(Ab, lda, opa, i0 + ii, p0 + pp) : mkcx<T>(0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < LB; ++u) {
+        const int t = tid + u * kFineThreads;
+        const int pp = opb == 'N' ? t % kFineBK : t / BN, jj = opb == 'N' ? t / kFineBK : t % BN;
+        rb[u] = (t < BN * kFineBK && p0 + pp < ke && j0 + jj < n) ? load_op(Bb, ldb, opb, p0 + pp, j0 + jj) : mkcx<T>(0, 0);
+      }
+    };
+    if (kb < ke) fetch(kb);
+    for (int64_t p0 = kb; p0 < ke; p0 += kFineBK) {
+#pragma unroll
+      for (int u = 0; u < LA; ++u) {
+        const int t = tid + u * kFineThreads;
+        if (t < BM * kFineBK) As[opa == 'N' ? t / BM : t % kFineBK][opa == 'N' ? t % BM : t / kFineBK] = ra[u];
+      }
+#pragma unroll
+      for (int u = 0; u < LB; ++u) {
+        const int t = tid + u * kFineThreads;
+        if (t < BN * kFineBK) Bs[opb == 'N' ? t % kFineBK : t / BN][opb == 'N' ? t / kFineBK : t % BN] = rb[u];
+      }
+      __syncthreads();
+      if (p0 + kFineBK < ke) fetch(p0 + kFineBK);
+      const int kk = (int)min((int64_t)kFineBK, ke - p0);
+      // k = p0 + pp + a·KS + kg: accumulator (k mod 16) = a·KS + kg
+#pragma unroll
+      for (int pp = 0; pp < kFineBK; pp += kFineAcc)
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+          const int q = pp + a * KS + kg;
+          if (q < kk) cfma(acc[a], As[q][ti], Bs[q][tj]);
+        }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int a = 0; a < NA; ++a) part[a * KS + kg][out] = acc[a];
+    __syncthreads();
+    cx<T> v = mkcx<T>(0, 0);
+    if (tid < BM * BN) {
+      v = part[0][tid];
+#pragma unroll
+      for (int g = 1; g < kFineAcc; ++g) v = v + part[g][tid];
+    }
+    if (CS > 1) {
+      cg::cluster_group cl = cg::this_cluster();
+      if (tid < BM * BN) total[tid] = v;
+      cl.sync();
+      if (rank == 0 && tid < BM * BN)
+        for (int c = 1; c < CS; ++c) v = v + cl.map_shared_rank(total, c)[tid];
+      cl.sync();
+    }
+    const int64_t gi = i0 + tid % BM, gj = j0 + tid / BM;
+    if (rank == 0 && tid < BM * BN && gi < m && gj < n) {
+      cx<T>* dst = C + bz * sC + gi + gj * ldc;
+      cx<T> r = alpha * v;
+      if (!(beta.x == T(0) && beta.y == T(0))) r = r + beta * *dst;
+      *dst = r;
+    }
+    __syncthreads();
+  }
+}
+
+template <typename T, int BM, int BN>
+tn_status_t launch_fine(tn_ctx* ctx, char opa, char opb, int64_t m, int64_t n, int64_t k, cx<T> alpha, const cx<T>* A,
+                        int64_t lda, int64_t sA, const cx<T>* B, int64_t ldb, int64_t sB, cx<T> beta, cx<T>* C,
+                        int64_t ldc, int64_t sC, int64_t batch) {
+  // K split over a cluster while the 8-wide column tiles leave SMs idle and a rank keeps a
+  // whole stage: a function of n and k only (see the kernel)
+  int CS = 1;
+  while (CS < 8 && (int64_t)cdiv(n, 8) * CS * 2 <= ctx->num_sms && k >= (int64_t)kFineBK * CS * 2) CS *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cdiv(m, BM) * (unsigned)CS, cdiv(n, BN), (unsigned)(batch < 65535 ? batch : 65535));
+  cfg.blockDim = dim3(kFineThreads);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)CS;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const int slot = sizeof(T) == 8 ? prof_begin(ctx) : -1;
+  TN_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_gemm_fine<T, BM, BN>, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB,
+                                        beta, C, ldc, sC, batch, CS));
+  TN_LAUNCHED(ctx);
+  if (slot >= 0) {
+    const bool b0 = beta.x == T(0) && beta.y == T(0);
+    prof_end(ctx, slot, TN_PROF_GEMM_F64, 1, 8.0 * m * n * k * batch,
+             sizeof(cx<T>) * ((double)m * k + (double)k * n + (double)m * n * (b0 ? 1 : 2)) * batch);
+  }
+  return TN_OK;
+}
+
 // C(i, j) = conj(C(j, i)) for i > j (n × n, batched)
 template <typename T>
 __global__ void k_mirror_lower(int64_t n, cx<T>* C, int64_t ldc, int64_t sC, int64_t batch) {
@@ -143,8 +289,26 @@ tn_status_t gemm_cx(tn_ctx* ctx, char opa, char opb, int64_t m, int64_t n, int64
                     const cx<T>* A, int64_t lda, int64_t sA, const cx<T>* B, int64_t ldb,
                     int64_t sB, cx<T> beta, cx<T>* C, int64_t ldc, int64_t sC, int64_t batch) {
   if (m == 0 || n == 0 || batch == 0) return TN_OK;
-  if (k == 0) {
-    // C = beta C: run the kernel with an empty reduction
+  // Which kernel: the SM with the most tiles sets the time, (tiles per SM) × (outputs per
+  // tile) in units of k/2 clocks per output.  64×64 tiles reuse operands best and are kept
+  // where their last wave is nearly full; 8×8 tiles (5 % overhead assumed) elsewhere.
+  // FP32 has 64 times the lanes, so there the small tiles only pay where 32×32 tiles leave
+  // three quarters of the SMs idle.
+  const int64_t sms = ctx->num_sms;
+  const int64_t tiles64 = (int64_t)cdiv(m, 64) * cdiv(n, 64) * batch, tiles32 = (int64_t)cdiv(m, 32) * cdiv(n, 32) * batch;
+  const int64_t bm = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : 8, bn = bm < 8 ? 16 : 8;
+  const int64_t tiles_f = (int64_t)cdiv(m, bm) * cdiv(n, bn) * batch;
+  const bool fits = cdiv(n, bn) <= 65535u && (int64_t)cdiv(m, bm) * 8 <= 0x7fffffff;
+  const bool fine = sizeof(T) == 8 ? cdiv(tiles64, sms) * 4096.0 > cdiv(tiles_f, sms) * (double)(bm * bn) * 1.05
+                                   : 4 * tiles32 <= sms;
+  if (fine && fits) {
+    if (bm == 1)
+      return launch_fine<T, 1, 16>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+    if (bm == 2)
+      return launch_fine<T, 2, 16>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+    if (bm == 4)
+      return launch_fine<T, 4, 16>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+    return launch_fine<T, 8, 8>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
   }
   // a few rows against wide operands (batched amplitudes, environment rows): row tiles
   // of 8 / 16 so the DFMA work is not spent on padding
@@ -152,8 +316,7 @@ tn_status_t gemm_cx(tn_ctx* ctx, char opa, char opb, int64_t m, int64_t n, int64
     return launch<T, 8, 32, 8, 1, 1>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
   if (m <= 16 && n >= 64)
     return launch<T, 16, 32, 8, 2, 1>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
-  int64_t tiles64 = (int64_t)cdiv(m, 64) * cdiv(n, 64) * batch;
-  if (tiles64 >= ctx->num_sms)
+  if (tiles64 >= sms)
     return launch<T, 64, 64, 8, 4, 4>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C,
                                       ldc, sC, batch);
   return launch<T, 32, 32, 8, 2, 2>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C,
