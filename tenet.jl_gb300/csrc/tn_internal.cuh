@@ -337,6 +337,20 @@ tn_status_t svd_tall_cx(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>* A, int64
                         int64_t sA, cx<T>* U, int64_t sU, double* S, int64_t sS, cx<T>* V,
                         int64_t sV, int64_t batch, int* sweeps_out);
 
+// persistent FP64 one-sided Jacobi of a list of matrices (tn_jacobi.cu): W m × n dense
+// (m ≥ n, m ≤ 512), V n × n dense or null, nrm n doubles
+struct JacobiMat {
+  cxd* W;
+  cxd* V;
+  double* nrm;
+  int m, n;
+};
+bool jacobi_pairs_fits(int64_t m, int64_t n);
+size_t jacobi_pairs_workspace(int64_t m, int64_t n, int64_t count, int64_t ctas, bool with_v);
+tn_status_t jacobi_pairs_resident(tn_ctx* ctx, int64_t m, bool with_v, int64_t* out);
+tn_status_t jacobi_pairs(tn_ctx* ctx, const std::vector<JacobiMat>& mats, bool v_given, int max_sweeps, int* sweeps_out,
+                         bool* noconv_out);
+
 // mixed precision SVD (C64 data): FP32 Jacobi pre-pass + FP64 polish.  keep > 0 (V null
 // only): only the `keep` largest triplets are wanted; the rest of U and S is approximate.
 size_t svd_mixed_workspace(int64_t m, int64_t n, int64_t batch);

@@ -19,8 +19,6 @@
 // The complex 2×2 rotation: with γ = |γ|e^{iφ}, ζ = (β−α)/(2|γ|),
 // t = sgn(ζ)/(|ζ|+√(1+ζ²)), c = 1/√(1+t²), s = c·t:
 //   w_i' = c·w_i − s·e^{−iφ}·w_j,   w_j' = s·e^{iφ}·w_i + c·w_j.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <mutex>
 
@@ -33,6 +31,7 @@ namespace {
 // matrices take 40-60 sweeps
 constexpr int kMaxSweeps = 80;
 constexpr size_t kSmemMax = 200 * 1024;
+constexpr int64_t kPairsMinN = 8;  // fewest columns for the column-pair kernel
 
 template <typename T>
 __host__ __device__ inline T jacobi_tol(int64_t m) {
@@ -137,52 +136,6 @@ __device__ __forceinline__ RotC<T> make_rot_c(T alpha, T beta, cx<T> g, T tol, T
   return R;
 }
 
-// The rotation for the latency-bound small-matrix kernels: the same angle as make_rot_c
-// from fewer long-latency operations on the one thread that forms it (1/|γ| once, no
-// monitor ratio: another thread derives that off the critical path).
-template <typename T>
-__device__ __forceinline__ RotC<T> make_rot_lean(T alpha, T beta, cx<T> g, T tol, T negl) {
-  RotC<T> R;
-  R.c = T(1);
-  R.tag = T(0);
-  R.se = mkcx<T>(0, 0);
-  R.apply = 0;
-  R.ratio = 0.f;
-  const T fl = negl > JacobiFloor<T>::value ? negl : JacobiFloor<T>::value;
-  if (!(alpha > fl) || !(beta > fl)) return R;
-  T ag;
-  const T ab = alpha * beta;
-  if (ab > JacobiFloor<T>::value) {
-    const T ag2 = abs2(g);
-    if (!(ag2 > tol * tol * ab && ag2 > T(0))) return R;
-    ag = sqrt(ag2);
-  } else {
-    ag = hypot(g.x, g.y);
-    if (!(ag > tol * (sqrt(alpha) * sqrt(beta)) && ag > T(0))) return R;
-  }
-  const T inv_ag = T(1) / ag;
-  const T zeta = (beta - alpha) * (T(0.5) * inv_ag);
-  const T t = (zeta >= T(0) ? T(1) : T(-1)) / (fabs(zeta) + sqrt(T(1) + zeta * zeta));
-  if (t == T(0)) return R;
-  const T c = T(1) / sqrt(T(1) + t * t);
-  const T sn = c * t * inv_ag;
-  R.apply = 1;
-  R.c = c;
-  R.tag = t * ag;
-  R.se = mkcx<T>(sn * g.x, sn * g.y);
-  return R;
-}
-
-// the convergence monitor of a pair, as make_rot_c computes it
-template <typename T>
-__device__ __forceinline__ float rot_ratio(T alpha, T beta, cx<T> g, T negl) {
-  const T fl = negl > JacobiFloor<T>::value ? negl : JacobiFloor<T>::value;
-  if (!(alpha > fl) || !(beta > fl)) return 0.f;
-  const T ab = alpha * beta;
-  if (ab > JacobiFloor<T>::value) return sqrtf((float)(abs2(g) / ab));
-  return (float)(hypot(g.x, g.y) / (sqrt(alpha) * sqrt(beta)));
-}
-
 template <typename T>
 __device__ __forceinline__ void rot_apply_c(T c, cx<T> se, cx<T>& wi, cx<T>& wj) {
   // wi' = c wi − conj(se) wj ; wj' = se wi + c wj
@@ -198,27 +151,15 @@ __device__ __forceinline__ void rot_apply_c(T c, cx<T> se, cx<T>& wi, cx<T>& wj)
 // use the cached norms nrm[], updated analytically (α' = α − t|γ|, β' = β + t|γ|) and
 // recomputed exactly at the start of every sweep (FP64).  V may be null (no
 // accumulation: the caller recovers Vh from U and A).
-// The rotation of columns (i, j) of matrix b by one CTA (shared by the per-round kernel
-// and the persistent cooperative one).  nmat: matrices in the batch (‖W_b‖²_F sits at
+// The rotation of columns (i, j) of matrix b by one CTA.  nmat: matrices in the batch (‖W_b‖²_F sits at
 // nrm[n·nmat + b]); counters: rotations of matrix b at cnt[b], the largest off-diagonal
 // ratio (float bits) at ratio[b].
-// LAT (cached norms, no truncation flags): the latency-bound form for the dataflow
-// kernel — the cached norms and ‖A‖²_F are fetched with the columns, thread 0 forms only
-// the rotation (make_rot_lean), and thread 32 updates the norms and counters.
-template <typename T, int NT, int R, bool EXACT, bool LAT = false, bool PV = false>
+template <typename T, int NT, int R, bool EXACT, bool PV = false>
 __device__ __forceinline__ void jacobi_pair(int64_t m, int64_t n, int64_t b, int i, int j, cx<T>* W, int64_t sW,
                                             cx<T>* V, int64_t sV, T* nrm, int64_t nmat, int* cnt, int* ratio, T tol,
                                             const unsigned char* __restrict__ tail) {
-  static_assert(!(LAT && EXACT), "the latency form uses cached norms");
-  static_assert(!LAT || NT > 32, "the latency form needs a second warp");
   // both columns ranked below the kept set: their mutual orthogonality is never used
-  if (!LAT && tail && tail[b * n + i] && tail[b * n + j]) return;
-  T pre_al = 0, pre_be = 0, pre_f = 0;
-  if (LAT && threadIdx.x == 0) {
-    pre_al = nrm[b * n + i];
-    pre_be = nrm[b * n + j];
-    pre_f = nrm[n * nmat + b];
-  }
+  if (tail && tail[b * n + i] && tail[b * n + j]) return;
   cx<T>* wi = W + b * sW + (int64_t)i * m;
   cx<T>* wj = W + b * sW + (int64_t)j * m;
   constexpr int NW = NT / 32;
@@ -269,42 +210,7 @@ __device__ __forceinline__ void jacobi_pair(int64_t m, int64_t n, int64_t b, int
   // part) and hands (c, s·e^{iφ}) to the block through shared memory
   __shared__ T s_rot[3];
   __shared__ int s_apply;
-  if (LAT) {
-    __shared__ T s_mon[6];
-    if (threadIdx.x == 0) {
-      g = mkcx<T>(0, 0);
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        g.x += red[w][0];
-        g.y += red[w][1];
-      }
-      const T negl = jacobi_eps<T>() * jacobi_eps<T>() * pre_f;
-      const RotC<T> Rt = make_rot_lean(pre_al, pre_be, g, tol, negl);
-      s_apply = Rt.apply;
-      s_rot[0] = Rt.c;
-      s_rot[1] = Rt.se.x;
-      s_rot[2] = Rt.se.y;
-      s_mon[0] = pre_al;
-      s_mon[1] = pre_be;
-      s_mon[2] = g.x;
-      s_mon[3] = g.y;
-      s_mon[4] = negl;
-      s_mon[5] = Rt.tag;
-    }
-    __syncthreads();
-    const int apply = s_apply;
-    if (threadIdx.x == 32) {
-      const T al2 = s_mon[0], be2 = s_mon[1];
-      if (al2 > T(0) && be2 > T(0))
-        atomicMax(&ratio[b], __float_as_int(rot_ratio(al2, be2, mkcx<T>(s_mon[2], s_mon[3]), s_mon[4])));
-      if (apply) {
-        atomicAdd(&cnt[b], 1);
-        nrm[b * n + i] = al2 - s_mon[5];
-        nrm[b * n + j] = be2 + s_mon[5];
-      }
-    }
-    if (!apply) return;
-  } else if (threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     g = mkcx<T>(0, 0);
     al = 0;
     be = 0;
@@ -344,10 +250,8 @@ __device__ __forceinline__ void jacobi_pair(int64_t m, int64_t n, int64_t b, int
       s_rot[2] = Rt.se.y;
     }
   }
-  if (!LAT) {
-    __syncthreads();
-    if (!s_apply) return;
-  }
+  __syncthreads();
+  if (!s_apply) return;
   const T c = s_rot[0];
   const cx<T> se = mkcx<T>(s_rot[1], s_rot[2]);
 #pragma unroll
@@ -388,7 +292,7 @@ __global__ void __launch_bounds__(NT)
   int i, j;
   rr_pair(N, r, blockIdx.x, i, j);
   if (j >= n) return;
-  jacobi_pair<T, NT, R, EXACT, false, PV>(m, n, b, i, j, W, sW, V, sV, nrm, gridDim.y, rotated, rotated + gridDim.y,
+  jacobi_pair<T, NT, R, EXACT, PV>(m, n, b, i, j, W, sW, V, sV, nrm, gridDim.y, rotated, rotated + gridDim.y,
                                           tol, tail);
 }
 
@@ -563,224 +467,6 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   if (t == 0) {
     if (s_cnt) atomicAdd(&cnt[b], s_cnt);
     if (s_ratio) atomicMax(&cnt[nmat + b], s_ratio);
-  }
-}
-
-// Persistent one-sided Jacobi for small matrices, where a round is far too little work to
-// hide a launch: one cooperative launch runs every sweep of every matrix.  Rounds are
-// separated by grid-wide barriers (all CTAs co-resident by construction of the cooperative
-// launch); the exact column norms, ‖W‖²_F and the convergence test of each sweep are done
-// on the device, so there is no host round trip until the end.  Every loop is bounded by
-// max_sweeps.  ctl (ints, zeroed by the caller): [0, 2B) and [2B, 4B) the rotation
-// counters / largest ratios of even and odd sweeps; [4B] any matrix still active; [4B+1]
-// sweeps run; [4B+2 …] worst ratio (float bits) and its rotation count per sweep (≤ 64).
-constexpr int kCoopDiag = 64;
-template <typename T, int NT, int R>
-__global__ void __launch_bounds__(NT)
-    k_jacobi_coop(int64_t m, int64_t n, int N, cx<T>* W, cx<T>* V, T* nrm, int* active, int* ctl, int64_t batch, T tol,
-                  int max_sweeps, float stop_ratio) {
-  namespace cg = cooperative_groups;
-  cg::grid_group grid = cg::this_grid();
-  __shared__ T red[NT / 32];
-  const int64_t G = gridDim.x, g = blockIdx.x;
-  const int64_t pairs = N / 2, items = pairs * batch;
-  const int64_t sW = m * n, sV = n * n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int* any = ctl + 4 * batch;
-  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
-    int* cnt = ctl + (sweep & 1) * 2 * batch;
-    int* rat = cnt + batch;
-    // exact column norms, one warp per column (as k_col_norms)
-    for (int64_t col = g * (NT / 32) + warp; col < n * batch; col += G * (NT / 32)) {
-      const int64_t b = col / n, c = col % n;
-      if (!active[b]) continue;
-      const cx<T>* w = W + b * sW + c * m;
-      T sq = 0;
-      for (int64_t t = lane; t < m; t += 32) sq += abs2(w[t]);
-      sq = warp_sum(sq);
-      if (lane == 0) nrm[col] = sq;
-    }
-    grid.sync();
-    // ‖W_b‖²_F, one CTA per matrix
-    for (int64_t b = g; b < batch; b += G) {
-      if (!active[b]) continue;
-      T f = 0;
-      for (int64_t c = threadIdx.x; c < n; c += NT) f += nrm[b * n + c];
-      f = warp_sum(f);
-      if (lane == 0) red[warp] = f;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        T a = 0;
-        for (int w = 0; w < NT / 32; ++w) a += red[w];
-        nrm[n * batch + b] = a;
-      }
-      __syncthreads();
-    }
-    grid.sync();
-    for (int r = 0; r < N - 1; ++r) {
-      for (int64_t it = g; it < items; it += G) {
-        const int64_t b = it / pairs;
-        if (!active[b]) continue;
-        int i, j;
-        rr_pair(N, r, (int)(it % pairs), i, j);
-        if (j >= n) continue;
-        jacobi_pair<T, NT, R, false>(m, n, b, i, j, W, sW, V, sV, nrm, batch, cnt, rat, tol, nullptr);
-        __syncthreads();
-      }
-      // the other parity's counters were last read before this sweep began
-      if (r == 0 && g == 0)
-        for (int64_t t = threadIdx.x; t < 2 * batch; t += NT) ctl[((sweep + 1) & 1) * 2 * batch + t] = 0;
-      grid.sync();
-    }
-    if (g == 0 && threadIdx.x == 0) {
-      int n_act = 0, worst_rot = 0;
-      float worst = 0.f;
-      for (int64_t b = 0; b < batch; ++b) {
-        if (!active[b]) continue;
-        const float rt = __int_as_float(rat[b]);
-        if (rt > worst) {
-          worst = rt;
-          worst_rot = cnt[b];
-        }
-        const int a = cnt[b] > 0 && rt > stop_ratio;
-        active[b] = a;
-        n_act += a;
-      }
-      *any = n_act;
-      ctl[4 * batch + 1] = sweep + 1;
-      if (sweep < kCoopDiag) {
-        ctl[4 * batch + 2 + sweep] = __float_as_int(worst);
-        ctl[4 * batch + 2 + kCoopDiag + sweep] = worst_rot;
-      }
-    }
-    grid.sync();
-    if (*any == 0) break;
-  }
-}
-
-// The same iteration with the per-round grid barrier replaced by dataflow: in the circle
-// ordering a column held by slot k in round r was held in round r−1 by the slot
-// rr_holder(N, r−1, column), so a CTA (one per pair slot and matrix) waits only for the
-// two CTAs that last wrote its columns.  Each CTA publishes the round it finished
-// (release at GPU scope after its writes) and polls its two predecessors (acquire);
-// grid barriers remain only at sweep boundaries (norm refresh, stop test).  A poll that
-// exceeds kFlowSpinLimit iterations sets the error word and moves on, so every CTA still
-// reaches every barrier and the launch ends; the host reports the error.
-constexpr long long kFlowSpinLimit = 1ll << 24;
-
-__device__ __forceinline__ int rr_holder(int N, int r, int c) {
-  if (c == N - 1 || c == r % (N - 1)) return 0;
-  const int a = ((c - r) % (N - 1) + (N - 1)) % (N - 1);
-  if (a >= 1 && a <= N / 2 - 1) return a;
-  return ((r - c) % (N - 1) + (N - 1)) % (N - 1);
-}
-
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-template <typename T, int NT, int R>
-__global__ void __launch_bounds__(NT)
-    k_jacobi_flow(int64_t m, int64_t n, int N, cx<T>* W, cx<T>* V, T* nrm, int* active, int* ctl, int* done,
-                  int64_t batch, T tol, int max_sweeps, float stop_ratio) {
-  namespace cg = cooperative_groups;
-  cg::grid_group grid = cg::this_grid();
-  __shared__ T red[NT / 32];
-  const int64_t G = gridDim.x, g = blockIdx.x;
-  const int64_t pairs = N / 2;
-  const int64_t b = g / pairs;
-  const int k = (int)(g % pairs);
-  const int64_t sW = m * n, sV = n * n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int* any = ctl + 4 * batch;
-  int* err = ctl + 4 * batch + 2 + 2 * kCoopDiag;
-  int* done_b = done + b * pairs;
-  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
-    int* cnt = ctl + (sweep & 1) * 2 * batch;
-    int* rat = cnt + batch;
-    for (int64_t col = g * (NT / 32) + warp; col < n * batch; col += G * (NT / 32)) {
-      const int64_t bb = col / n, c = col % n;
-      if (!active[bb]) continue;
-      const cx<T>* w = W + bb * sW + c * m;
-      T sq = 0;
-      for (int64_t t = lane; t < m; t += 32) sq += abs2(w[t]);
-      sq = warp_sum(sq);
-      if (lane == 0) nrm[col] = sq;
-    }
-    grid.sync();
-    for (int64_t bb = g; bb < batch; bb += G) {
-      if (!active[bb]) continue;
-      T f = 0;
-      for (int64_t c = threadIdx.x; c < n; c += NT) f += nrm[bb * n + c];
-      f = warp_sum(f);
-      if (lane == 0) red[warp] = f;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        T a = 0;
-        for (int w = 0; w < NT / 32; ++w) a += red[w];
-        nrm[n * batch + bb] = a;
-      }
-      __syncthreads();
-    }
-    grid.sync();
-    if (g == 0)  // the other parity's counters were last read before this sweep began
-      for (int64_t t = threadIdx.x; t < 2 * batch; t += NT) ctl[((sweep + 1) & 1) * 2 * batch + t] = 0;
-    if (active[b]) {
-      for (int r = 0; r < N - 1; ++r) {
-        int i, j;
-        rr_pair(N, r, k, i, j);
-        if (r > 0) {
-          if (threadIdx.x == 0) {
-            const int want = sweep * N + r;  // published by a holder when it finished round r−1
-            const int h1 = rr_holder(N, r - 1, i), h2 = rr_holder(N, r - 1, j);
-            long long spins = 0;
-            while (ld_acquire_gpu(&done_b[h1]) < want || ld_acquire_gpu(&done_b[h2]) < want) {
-              if (++spins > kFlowSpinLimit) {
-                atomicExch(err, 1);
-                break;
-              }
-            }
-            __threadfence();
-          }
-          __syncthreads();
-        }
-        if (j < n) jacobi_pair<T, NT, R, false, true>(m, n, b, i, j, W, sW, V, sV, nrm, batch, cnt, rat, tol, nullptr);
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) st_release_gpu(&done_b[k], sweep * N + r + 1);
-      }
-    }
-    grid.sync();
-    if (g == 0 && threadIdx.x == 0) {
-      int n_act = 0, worst_rot = 0;
-      float worst = 0.f;
-      const int failed = *err;
-      for (int64_t bb = 0; bb < batch; ++bb) {
-        if (!active[bb]) continue;
-        const float rt = __int_as_float(rat[bb]);
-        if (rt > worst) {
-          worst = rt;
-          worst_rot = cnt[bb];
-        }
-        const int a = !failed && cnt[bb] > 0 && rt > stop_ratio;
-        active[bb] = a;
-        n_act += a;
-      }
-      *any = n_act;
-      ctl[4 * batch + 1] = sweep + 1;
-      if (sweep < kCoopDiag) {
-        ctl[4 * batch + 2 + sweep] = __float_as_int(worst);
-        ctl[4 * batch + 2 + kCoopDiag + sweep] = worst_rot;
-      }
-    }
-    grid.sync();
-    if (*any == 0) break;
   }
 }
 
@@ -1027,7 +713,8 @@ template <typename T>
 size_t svd_workspace(int64_t m, int64_t n, int64_t batch) {
   return ws_round(sizeof(cx<T>) * (size_t)(m * n * batch)) + ws_round(sizeof(cx<T>) * (size_t)(n * n * batch)) +
          ws_round(sizeof(int) * (size_t)(n * batch)) + ws_round(sizeof(int) * (size_t)(batch + 1)) +
-         ws_round(sizeof(int) * (size_t)(2 * batch + 2)) + ws_round(sizeof(T) * (size_t)((n + 1) * batch));
+         ws_round(sizeof(int) * (size_t)(2 * batch + 2)) + ws_round(sizeof(T) * (size_t)((n + 1) * batch)) +
+         (sizeof(T) == 8 && jacobi_pairs_fits(m, n) ? jacobi_pairs_workspace(m, n, batch, (n + 1) / 2 * batch, true) : 0);
 }
 template size_t svd_workspace<double>(int64_t, int64_t, int64_t);
 template size_t svd_workspace<float>(int64_t, int64_t, int64_t);
@@ -1101,57 +788,18 @@ static tn_status_t launch_step(tn_ctx* ctx, int64_t m, int64_t n, int N, int r, 
   return TN_OK;
 }
 
-// matrices with at most this many columns take the persistent cooperative path
-constexpr int64_t kCoopMaxN = 256;
-
-// the whole Jacobi iteration of a small FP64 batch in one cooperative launch
-template <typename T>
-static tn_status_t jacobi_coop(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T>* V, int64_t batch, int* active,
-                               T* nrm, int max_sweeps, int* sweeps_out, bool* noconv_out) {
-  constexpr int NT = 128, R = 4;  // m ≤ 512
-  const int N = (int)(n + (n & 1));
-  const int64_t items = (int64_t)(N / 2) * batch;
-  int per_sm = 0;
-  TN_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_jacobi_coop<T, NT, R>, NT, 0));
-  int per_sm_flow = 0;
-  TN_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_flow, k_jacobi_flow<T, NT, R>, NT, 0));
-  // dataflow rounds need one resident CTA per pair slot and matrix
-  const bool flow = items <= (int64_t)std::max(per_sm_flow, 0) * ctx->num_sms;
-  const int64_t G = flow ? items : std::min<int64_t>(items, (int64_t)std::max(per_sm, 1) * ctx->num_sms);
-  const size_t nhdr = (size_t)(4 * batch + 2 + 2 * kCoopDiag + 1);
-  const size_t nctl = nhdr + (flow ? (size_t)items : 0);
-  int* ctl = nullptr;
-  TN_RETURN_IF(ctx_flags(ctx, nctl, &ctl));
-  TN_CHECK_CUDA(ctx, cudaMemsetAsync(ctl, 0, sizeof(int) * nctl, ctx->stream));
-  std::vector<int> h_act(batch, 1);
-  TN_CHECK_CUDA(ctx, cudaMemcpyAsync(active, h_act.data(), sizeof(int) * batch, cudaMemcpyHostToDevice, ctx->stream));
-  const T tol = jacobi_tol<T>(m);
-  const float stop_ratio = (float)sqrt((double)tol * 1e-1);
-  int64_t bt = batch;
-  if (flow) {
-    int* done = ctl + nhdr;
-    void* args[] = {&m, &n, (void*)&N, &W, &V, &nrm, &active, &ctl, &done, &bt, (void*)&tol, &max_sweeps,
-                    (void*)&stop_ratio};
-    TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k_jacobi_flow<T, NT, R>, dim3((unsigned)G), dim3(NT),
-                                                   args, 0, ctx->stream));
-  } else {
-    void* args[] = {&m, &n, (void*)&N, &W, &V, &nrm, &active, &ctl, &bt, (void*)&tol, &max_sweeps, (void*)&stop_ratio};
-    TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k_jacobi_coop<T, NT, R>, dim3((unsigned)G), dim3(NT),
-                                                   args, 0, ctx->stream));
-  }
-  TN_LAUNCHED(ctx);
-  std::vector<int> h(nctl);
-  TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h.data(), ctl, sizeof(int) * nctl, cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  const int sweeps = h[4 * batch + 1];
-  for (int k = 0; k < kCoopDiag && k < 64; ++k) {
-    memcpy(&ctx->sweep_ratio[k], &h[4 * batch + 2 + k], sizeof(float));
-    ctx->sweep_rotations[k] = h[4 * batch + 2 + kCoopDiag + k];
-  }
-  *sweeps_out = sweeps;
-  *noconv_out = h[4 * batch] > 0;
-  if (h[4 * batch + 2 + 2 * kCoopDiag])
-    return tn_set_error(ctx, TN_ECUDA, "svd: a dataflow wait of the Jacobi rounds exceeded its limit");
+// Which FP64 kernel a batch takes (no truncation flags): the persistent column-pair kernel
+// spreads every matrix over n/2 SMs; one CTA per matrix in shared memory is left for matrices
+// of a few columns, where the launch is the time, and for batches of so many small matrices
+// that they fill the chip twice over with one SM each.
+static tn_status_t jacobi_takes_pairs(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch, bool* out) {
+  *out = false;
+  if (!jacobi_pairs_fits(m, n) || n < kPairsMinN) return TN_OK;
+  int64_t resident = 0;
+  TN_RETURN_IF(jacobi_pairs_resident(ctx, m, true, &resident));
+  if ((n + 1) / 2 > resident) return TN_OK;
+  const bool in_smem = sizeof(cxd) * (size_t)(m * n + n * n) <= kSmemMax && n <= 256;
+  *out = !(in_smem && (n + 1) / 2 * batch > 2 * resident && batch >= 2 * ctx->num_sms);
   return TN_OK;
 }
 
@@ -1185,7 +833,14 @@ static tn_status_t jacobi_core(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T
   int sweeps = 0;
   bool noconv = false;
   const size_t smem_need = sizeof(cx<T>) * (size_t)(m * n + n * n);
-  if (V && smem_need <= kSmemMax && n <= 256) {
+  bool pairs_kernel = false;
+  if (sizeof(T) == 8 && !tail && min_rot_frac <= 0.0) TN_RETURN_IF(jacobi_takes_pairs(ctx, m, n, batch, &pairs_kernel));
+  if (pairs_kernel) {
+    std::vector<JacobiMat> mats((size_t)batch);
+    for (int64_t b = 0; b < batch; ++b)
+      mats[b] = {(cxd*)W + b * m * n, V ? (cxd*)V + b * n * n : nullptr, (double*)nrm + b * n, (int)m, (int)n};
+    TN_RETURN_IF(jacobi_pairs(ctx, mats, v_given, max_sweeps, &sweeps, &noconv));
+  } else if (V && smem_need <= kSmemMax && n <= 256) {
     TN_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_jacobi_smem<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     int threads = n >= 32 ? 512 : 128;
     k_jacobi_smem<T><<<gy, threads, smem_need, ctx->stream>>>(m, n, W, m * n, V, n * n, rotated, tol, max_sweeps,
@@ -1196,13 +851,6 @@ static tn_status_t jacobi_core(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T
     TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     for (int64_t b = 0; b < batch; ++b) noconv |= st[b] != 0;
     sweeps = -1;
-  } else if (sizeof(T) == 8 && !tail && min_rot_frac <= 0.0 && m <= 512 && n <= kCoopMaxN) {
-    if (V && !v_given) {
-      int64_t blocks = std::min<int64_t>((n * n + 255) / 256, 2048);
-      k_identity<T><<<dim3((unsigned)blocks, gy), 256, 0, ctx->stream>>>(n, V, n * n, batch);
-      TN_LAUNCHED(ctx);
-    }
-    TN_RETURN_IF(jacobi_coop<T>(ctx, m, n, W, V, batch, active, nrm, max_sweeps, &sweeps, &noconv));
   } else {
     if (V && !v_given) {
       int64_t blocks = std::min<int64_t>((n * n + 255) / 256, 2048);
@@ -1717,6 +1365,7 @@ size_t svd_mixed_workspace(int64_t m, int64_t n, int64_t batch) {
   s += ws_round((size_t)(n * batch));                     // tail flags
   s += ws_round(sizeof(cxd) * (size_t)(n * n * batch));  // R / E of the refinement
   s += ws_round((size_t)(n * batch)) + ws_round(sizeof(int) * (size_t)(5 * batch + 4));  // cluster marks, stats
+  if (jacobi_pairs_fits(m, n)) s += jacobi_pairs_workspace(m, n, batch, (n + 1) / 2 * batch, true);
   return s;
 }
 
@@ -2025,13 +1674,11 @@ tn_status_t svd_left(tn_ctx* ctx, tn_precision_t prec, int64_t m, int64_t n, con
                                                                                          batch);
     TN_LAUNCHED(ctx);
   }
-  // the one-CTA shared-memory kernel needs V resident; the large path runs without it
-  // small matrices: one CTA per matrix in shared memory when there are many of them; a
-  // few (a DMRG or TEBD pair, one MPS) take the persistent cooperative sweeps instead,
-  // which spread each round's pairs over many SMs (one SM's FP64 rate serialises a whole
-  // SVD; no right vectors are needed here)
-  const bool coop = m <= 512 && n <= kCoopMaxN;
-  const bool small = sizeof(cxd) * (size_t)(m * n + n * n) <= kSmemMax && n <= 256 && !(coop && batch < 32);
+  // no right vectors are needed here; only the one-CTA shared-memory kernel, which keeps V
+  // resident, takes them
+  bool pairs_kernel = false;
+  TN_RETURN_IF(jacobi_takes_pairs(ctx, m, n, batch, &pairs_kernel));
+  const bool small = !pairs_kernel && sizeof(cxd) * (size_t)(m * n + n * n) <= kSmemMax && n <= 256;
   bool noconv = false;
   ctx->last_sweeps_fp32 = 0;
   TN_RETURN_IF(jacobi_core<double>(ctx, m, n, W, small ? V : nullptr, batch, false, active, rotated, nrm, kMaxSweeps,
