@@ -55,8 +55,23 @@ void ws_overflow(tn_ctx* ctx, size_t need) {
   std::abort();
 }
 
+constexpr size_t kPinnedBytes = 1 << 16;
+
+tn_status_t wait_error_word(tn_ctx* ctx, int** out) {
+  *out = reinterpret_cast<int*>(static_cast<char*>(ctx->pinned) + kPinnedBytes) - 1;  // (unified addressing)
+  return TN_OK;
+}
+
+tn_status_t wait_error_check(tn_ctx* ctx) {
+  volatile int* w = reinterpret_cast<int*>(static_cast<char*>(ctx->pinned) + kPinnedBytes) - 1;
+  if (*w == 0) return TN_OK;
+  *w = 0;
+  return tn_set_error(ctx, TN_ETIMEOUT, "a wait between the blocks of a factorisation exceeded its limit");
+}
+
 tn_status_t ws_reserve(tn_ctx* ctx, size_t bytes) {
   ctx->ws_top = 0;
+  TN_RETURN_IF(wait_error_check(ctx));
   if (bytes <= ctx->ws_cap) return TN_OK;
   // growth: the stream must be idle before the old arena is released
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -121,12 +136,13 @@ tn_status_t tn_create(tn_ctx** out, int device) {
     return tn_set_error(nullptr, TN_ECUDA, "stream create: %s", cudaGetErrorString(e));
   }
   ctx->stream = ctx->own_stream;
-  e = cudaMallocHost(&ctx->pinned, 1 << 16);
+  e = cudaMallocHost(&ctx->pinned, kPinnedBytes);
   if (e != cudaSuccess) {
     cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return tn_set_error(nullptr, TN_ECUDA, "pinned alloc: %s", cudaGetErrorString(e));
   }
+  memset(ctx->pinned, 0, kPinnedBytes);
   *out = ctx;
   return TN_OK;
 }
@@ -173,7 +189,7 @@ void* tn_get_stream(tn_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 tn_status_t tn_sync(tn_ctx* ctx) {
   if (!ctx) return TN_EINVAL;
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return TN_OK;
+  return wait_error_check(ctx);
 }
 
 tn_status_t tn_alloc(tn_ctx* ctx, size_t bytes, void** dptr) {
@@ -200,7 +216,7 @@ tn_status_t tn_memcpy_d2h(tn_ctx* ctx, void* dst, const void* src, size_t bytes)
   TN_ARG(ctx, dst && src, "tn_memcpy_d2h: null pointer");
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return TN_OK;
+  return wait_error_check(ctx);
 }
 
 tn_status_t tn_memcpy_d2d(tn_ctx* ctx, void* dst, const void* src, size_t bytes) {

@@ -154,7 +154,7 @@ struct tn_ctx {
   char* ws = nullptr;
   size_t ws_cap = 0;
   size_t ws_top = 0;
-  // small pinned host buffer for scalar read-backs
+  // small pinned host buffer for scalar read-backs (its last int: wait_error_word)
   void* pinned = nullptr;
   int* d_flags = nullptr;  // device status / convergence words
   size_t flags_cap = 0;
@@ -210,6 +210,11 @@ struct tn_ctx {
   bool autotune = false;
   std::unordered_map<std::string, std::pair<int, int>> tuning;
 };
+// a word of page-locked host memory that kernels of this context set when a bounded wait ran
+// out (kernels whose callers do not synchronise); wait_error_check reports and clears it.
+// It is looked at by every workspace reservation and every read-back to the host.
+tn_status_t wait_error_word(tn_ctx* ctx, int** out);
+tn_status_t wait_error_check(tn_ctx* ctx);
 void ctx_release(tn_ctx* ctx);  // frees the context (called when refs drop to 0)
 
 // ---------------------------------------------------------------------------------
@@ -328,6 +333,19 @@ size_t qr_workspace(int64_t m, int64_t n, int64_t batch);
 template <typename T>
 tn_status_t qr_cx(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>* A, int64_t lda, int64_t sA,
                   cx<T>* Q, int64_t sQ, cx<T>* R, int64_t sR, int64_t batch);
+
+// thin QR with one CTA per column (tn_qr_cols.cu): Q m × k (ld m) or null, R k × n (ld k)
+struct QrMat {
+  const cxd* A;
+  cxd *Q, *R;
+  int64_t lda;
+  int m, n;
+};
+size_t qr_cols_workspace(int64_t m, int64_t n, int64_t count);
+tn_status_t qr_cols_takes(tn_ctx* ctx, int64_t m, int64_t columns, bool* out);
+tn_status_t qr_cols(tn_ctx* ctx, const std::vector<QrMat>& mats);
+tn_status_t qr_cols_batch(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda, int64_t sA, cxd* Q, int64_t sQ,
+                          cxd* R, int64_t sR, int64_t batch);
 
 template <typename T>
 size_t svd_workspace(int64_t m, int64_t n, int64_t batch);

@@ -479,6 +479,7 @@ tn_status_t overlap_impl(const tn_mps* a, const tn_mps* b, double* h_out) {
   TN_CHECK_CUDA(ctx, cudaMemcpy2DAsync(h_out, sizeof(cxd), F, env * sizeof(cxd), sizeof(cxd), B, cudaMemcpyDeviceToHost,
                                        ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(wait_error_check(ctx));
   return TN_OK;
 }
 
@@ -684,6 +685,7 @@ tn_status_t tn_mps_get_instance_site(const tn_mps* p, int32_t b, int32_t i, void
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h, p->site[i] + (size_t)b * p->cap[i], sizeof(cxd) * sz(p, i),
                                      cudaMemcpyDeviceToHost, ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(wait_error_check(ctx));
   return TN_OK;
 }
 
@@ -712,6 +714,7 @@ tn_status_t tn_mps_get_instance_sites(const tn_mps* p, int32_t b, void* const* h
     TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h[i - 1], p->site[i] + (size_t)b * p->cap[i], sizeof(cxd) * sz(p, i),
                                        cudaMemcpyDeviceToHost, ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(wait_error_check(ctx));
   return TN_OK;
 }
 
@@ -924,6 +927,7 @@ tn_status_t tn_mps_amplitude(const tn_mps* p, const void* h_vectors, double* h_o
   TN_CHECK_CUDA(ctx, cudaMemcpy2DAsync(h_out, sizeof(cxd), e, ve * sizeof(cxd), sizeof(cxd), B, cudaMemcpyDeviceToHost,
                                        ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(wait_error_check(ctx));
   return TN_OK;
 }
 
@@ -1036,6 +1040,7 @@ tn_status_t tn_mps_sample(tn_mps* p, int32_t instance, int64_t nshots, const dou
   }
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h_out, O, sizeof(int32_t) * nshots * L, cudaMemcpyDeviceToHost, ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(wait_error_check(ctx));
   return TN_OK;
 }
 

@@ -198,6 +198,7 @@ tn_status_t sumsq(tn_ctx* ctx, int64_t n, const E* x, double* h_out) {
   double* hp = reinterpret_cast<double*>(ctx->pinned);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(hp, partial + nb, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(wait_error_check(ctx));
   *h_out = hp[0];
   return TN_OK;
 }
@@ -214,6 +215,7 @@ tn_status_t rank_select_batched(tn_ctx* ctx, double* S, int64_t k, int64_t sS, i
   int* hp = reinterpret_cast<int*>(ctx->pinned);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(hp, flags, sizeof(int) * batch, cudaMemcpyDeviceToHost, ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(wait_error_check(ctx));
   int64_t r = 0;
   bool uneven = false;
   for (int64_t b = 0; b < batch; ++b) {
@@ -434,6 +436,7 @@ tn_status_t norms_batched(tn_ctx* ctx, bool complex_data, int64_t n, const void*
   TN_LAUNCHED(ctx);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h_out, d, sizeof(double) * batch, cudaMemcpyDeviceToHost, ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(wait_error_check(ctx));
   for (int64_t b = 0; b < batch; ++b) h_out[b] = sqrt(h_out[b]);
   return TN_OK;
 }
@@ -478,6 +481,7 @@ tn_status_t zdotc_batched(tn_ctx* ctx, int64_t n, const cxd* x, int64_t sx, cons
   TN_LAUNCHED(ctx);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h_out, d, 2 * sizeof(double) * batch, cudaMemcpyDeviceToHost, ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(wait_error_check(ctx));
   return TN_OK;
 }
 

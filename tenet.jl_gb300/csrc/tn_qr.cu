@@ -248,7 +248,9 @@ size_t qr_workspace(int64_t m, int64_t n, int64_t batch) {
   size_t tm = ws_round(sizeof(cx<T>) * (size_t)((npan + 1) * nb * nb * batch + 1));
   // the autotuner's private copy of A (Q may alias A)
   size_t a0 = ws_round(sizeof(cx<T>) * (size_t)(m * n * batch));
-  return w + tau + tm + a0;
+  const size_t blocked = w + tau + tm + a0;
+  // (the one-CTA-per-column kernel runs instead of the blocked one, never beside it)
+  return sizeof(T) == 8 ? std::max(blocked, qr_cols_workspace(m, n, batch)) : blocked;
 }
 template size_t qr_workspace<double>(int64_t, int64_t, int64_t);
 template size_t qr_workspace<float>(int64_t, int64_t, int64_t);
@@ -316,6 +318,31 @@ tn_status_t qr_run(tn_ctx* ctx, int nb, int slab, int64_t m, int64_t n, const cx
 
 }  // namespace
 
+// Whether [a, a + na) and [b, b + nb) share bytes
+static bool ranges_meet(const void* a, size_t na, const void* b, size_t nb) {
+  const char *x = (const char*)a, *y = (const char*)b;
+  return x < y + nb && y < x + na;
+}
+
+// Which kernel: one CTA per column (tn_qr_cols.cu) while all columns of all matrices are
+// resident at once, the blocked panels below beyond that (rows > 512, or batches that fill
+// the FP64 pipe with panels of different matrices) and for shapes whose launch configuration
+// the caller set (tn_tuning_load).  Measured, one matrix, blocked / columns: QRCOLS_NUMBERS
+// A column's CTA reads it before anything is written only if no other CTA's output lies
+// there, so Q or R over A is left to the blocked kernel (which factors a copy) unless Q is
+// exactly A.
+static tn_status_t qr_takes_columns(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda, int64_t sA, const cxd* Q,
+                                    int64_t sQ, const cxd* R, int64_t sR, int64_t batch, bool* out) {
+  *out = false;
+  const int64_t k = std::min(m, n);
+  const size_t ba = sizeof(cxd) * (size_t)((batch - 1) * sA + lda * n), bq = sizeof(cxd) * (size_t)((batch - 1) * sQ + m * k),
+               br = sizeof(cxd) * (size_t)((batch - 1) * sR + k * n);
+  const bool in_place = Q == A && lda == m && (batch == 1 || sA == sQ);
+  if (ranges_meet(R, br, A, ba) || (!in_place && ranges_meet(Q, bq, A, ba))) return TN_OK;
+  if (batch > 1 && (sA < 0 || sQ < 0 || sR < 0)) return TN_OK;
+  return qr_cols_takes(ctx, m, n * batch, out);
+}
+
 // Panel width and slab width come from the context's tuning table, keyed by the shape
 // (m, n and a batch bucket).  With autotuning on, the first call of an unseen shape
 // times every candidate (panel 4/8/16/32 that fits shared memory × slab 1/2/4) with
@@ -330,14 +357,28 @@ tn_status_t qr_cx(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>* A, int64_t lda
   if (sizeof(cx<T>) * (size_t)m * 1 > kPanelSmemMax)
     return tn_set_error(ctx, TN_EUNSUPPORTED, "qr: m=%lld too large for the panel kernel", (long long)m);
   const int64_t npan_max = (k + nb_max - 1) / nb_max;
-  cx<T>* W = ws_take<cx<T>>(ctx, (size_t)(m * n * batch));
-  cx<T>* tau = ws_take<cx<T>>(ctx, (size_t)(k * batch + 1));
-  cx<T>* Tm = ws_take<cx<T>>(ctx, (size_t)((npan_max + 1) * nb_max * nb_max * batch + 1));
-  TN_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_qr_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemMax));
   const int bb = batch <= 1 ? 1 : batch <= 4 ? 4 : batch <= 16 ? 16 : 64;
   char key[96];
   snprintf(key, sizeof(key), "qr%zu:%lld:%lld:%d", sizeof(T), (long long)m, (long long)n, bb);
   auto it = ctx->tuning.find(key);
+  const double kk = (double)k, f = 4.0 * (2.0 * m * kk * kk - 2.0 / 3.0 * kk * kk * kk);
+  if constexpr (sizeof(T) == 8) {
+    bool columns = false;
+    if (it == ctx->tuning.end())
+      TN_RETURN_IF(qr_takes_columns(ctx, m, n, A, lda, sA, Q, sQ, R, sR, batch, &columns));
+    if (columns) {
+      const int slot = prof_begin(ctx);
+      TN_RETURN_IF(qr_cols_batch(ctx, m, n, A, lda, sA, Q, sQ, R, sR, batch));
+      if (slot >= 0)
+        prof_end(ctx, slot, TN_PROF_QR, 1, 2.0 * f * batch,
+                 sizeof(cx<T>) * ((double)m * n + (double)m * k + (double)k * n) * batch);
+      return TN_OK;
+    }
+  }
+  cx<T>* W = ws_take<cx<T>>(ctx, (size_t)(m * n * batch));
+  cx<T>* tau = ws_take<cx<T>>(ctx, (size_t)(k * batch + 1));
+  cx<T>* Tm = ws_take<cx<T>>(ctx, (size_t)((npan_max + 1) * nb_max * nb_max * batch + 1));
+  TN_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_qr_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemMax));
   int nb = std::min(8, nb_max), slab = 2;
   if (it != ctx->tuning.end()) {
     nb = std::min(it->second.first, nb_max);
@@ -388,7 +429,6 @@ tn_status_t qr_cx(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>* A, int64_t lda
   TN_RETURN_IF(qr_run<T>(ctx, nb, slab, m, n, A, lda, sA, Q, sQ, R, sR, batch, W, tau, Tm));
   if (slot >= 0) {
     // geqrf + forming Q: 2 × 4·(2mk² − ⅔k³)·… (LAWN 41, ×4 complex); A read, Q and R written
-    const double kk = (double)k, f = 4.0 * (2.0 * m * kk * kk - 2.0 / 3.0 * kk * kk * kk);
     prof_end(ctx, slot, TN_PROF_QR, ctx->launches - l0, 2.0 * f * batch,
              sizeof(cx<T>) * ((double)m * n + (double)m * k + (double)k * n) * batch);
   }

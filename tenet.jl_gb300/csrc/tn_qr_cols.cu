@@ -1,0 +1,323 @@
+// K3b — thin QR of few matrices, complex FP64: one CTA per column, reflectors handed on as
+// flagged packets.
+//
+// What bounds it.  The FP64 pipe retires 2 DFMA per clock and SM, so a panel factored by one
+// CTA (k_qr_panel) runs at 1/152 of the chip and a bond-sized QR is a chain of such panels:
+// 128×64 took 795 µs where the chip's FP64 rate for it is 7 µs.  The chain that cannot be
+// avoided is one step per column: reflector j in, inner product with column j+1, update,
+// norm, reflector j+1 out.  Here every column has its own CTA and stays in registers:
+//  * the entries below the diagonal of an updated column are its reflector as they are
+//    (u = x − β e₁ is not normalised; H = I − κ u uᴴ), so they are sent at once, and the
+//    receivers form uᴴc while the sender still reduces ‖x‖² and forms β and κ;
+//  * entries travel as packets of two 64-bit words with 32 data bits and a flag each, polled
+//    by the receivers directly: no fence, no barrier between CTAs, and they stay in place as
+//    the stored reflectors;
+//  * column q of Q = H₀…H_{k−1} needs reflectors q…0 only, all known when column q is done,
+//    so its CTA forms it right away, while later columns are still being factored.
+// Reflectors and signs are LAPACK's (H = I − τ v vᴴ, v₁ = 1, τ v vᴴ = κ u uᴴ, R_jj real with
+// the sign opposite to Re x₁).  Every wait is bounded: a CTA whose wait ran out records an
+// error and leaves.
+#include <algorithm>
+
+#include "tn_internal.cuh"
+
+namespace {
+
+constexpr int kNT = 128;
+constexpr long long kSpinLimit = 1ll << 22;
+
+struct QMat {
+  const cxd* A;
+  cxd *Q, *R;       // Q m × k (ld m), R k × n (ld k)
+  ulonglong2* box;  // k reflectors × (2m + 4) packets
+  int64_t lda;
+  int m, n, k, cta0;
+};
+
+__device__ __forceinline__ void put(ulonglong2* p, double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v), f = 1ull << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"((b & 0xffffffffull) | f), "l"((b >> 32) | f)
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 get_raw(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool arrived(ulonglong2 v) { return (v.x >> 32) != 0 && (v.y >> 32) != 0; }
+__device__ __forceinline__ double value_of(ulonglong2 v) {
+  return __longlong_as_double((long long)((v.x & 0xffffffffull) | (v.y << 32)));
+}
+
+// Σ over the warp of (a, b): lanes 0-15 end with Σa, lanes 16-31 with Σb
+__device__ __forceinline__ double warp_sum2(double a, double b, int lane) {
+  double keep = (lane & 16) ? b : a;
+  const double send = (lane & 16) ? a : b;
+  keep += __shfl_xor_sync(0xffffffffu, send, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) keep += __shfl_xor_sync(0xffffffffu, keep, o);
+  return keep;
+}
+
+// a batch of equal matrices: the first one and the strides to the next
+struct QBatch {
+  QMat first;
+  int64_t sA, sQ, sR, sBox;
+};
+
+// mats/owner: the list form (owner[CTA] = its matrix); null: the batch form
+template <int R>
+__global__ void __launch_bounds__(kNT, 4)
+    k_qr_cols(QBatch batch, const QMat* __restrict__ mats, const int* __restrict__ owner, int* err) {
+  QMat M;
+  if (mats) {
+    M = mats[owner[blockIdx.x]];
+  } else {
+    M = batch.first;
+    const int b = (int)blockIdx.x / M.n;
+    M.A += b * batch.sA;
+    if (M.Q) M.Q += b * batch.sQ;
+    M.R += b * batch.sR;
+    M.box += b * batch.sBox;
+    M.cta0 = b * M.n;
+  }
+  const int m = M.m, k = M.k, col = (int)blockIdx.x - M.cta0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = lane >> 4;
+  const int64_t stride = 2 * (int64_t)m + 4;
+  __shared__ double red[2][4][2];
+  __shared__ double s_row[2][2];  // this column's entry in the pivot row
+  __shared__ int s_fail;
+  if (tid == 0) s_fail = 0;
+  cxd x[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const int t = tid + q * kNT;
+    x[q] = t < m ? M.A[(int64_t)col * M.lda + t] : mkcx(0.0, 0.0);
+  }
+  int buf = 0;
+  // x ← (I − f-form of reflector j) x: rows > j of u from the packets, u₁ and conj(κ) from the
+  // scalar packets; adj: the factorisation's Hᴴ, otherwise H
+  auto reflect = [&](int j, bool adj) -> bool {
+    const ulonglong2* b = M.box + (int64_t)j * stride;
+    cxd u[R];
+    long long spins = 0;
+    bool ok;
+    do {
+      ok = true;
+      ulonglong2 p[2 * R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int t = tid + q * kNT;
+        if (t > j && t < m) {
+          p[2 * q] = get_raw(b + t);
+          p[2 * q + 1] = get_raw(b + m + t);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int t = tid + q * kNT;
+        u[q] = mkcx(0.0, 0.0);
+        if (t > j && t < m) {
+          ok = ok && arrived(p[2 * q]) && arrived(p[2 * q + 1]);
+          u[q] = mkcx(value_of(p[2 * q]), value_of(p[2 * q + 1]));
+        }
+      }
+      // a column far from its turn leaves the memory to the ones whose turn it is
+      if (!ok && adj && col > j + 8) __nanosleep(64);
+    } while (!ok && ++spins < kSpinLimit);
+    double wx = 0, wy = 0;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      wx = fma(u[q].x, x[q].x, fma(u[q].y, x[q].y, wx));
+      wy = fma(u[q].x, x[q].y, fma(-u[q].y, x[q].x, wy));
+      if (tid + q * kNT == j) {
+        s_row[buf][0] = x[q].x;
+        s_row[buf][1] = x[q].y;
+      }
+    }
+    const double s = warp_sum2(wx, wy, lane);
+    if ((lane & 15) == 0) red[buf][warp][half] = s;
+    ulonglong2 p0, p1, p2, p3;
+    do {
+      p0 = get_raw(b + 2 * m);
+      p1 = get_raw(b + 2 * m + 1);
+      p2 = get_raw(b + 2 * m + 2);
+      p3 = get_raw(b + 2 * m + 3);
+      ok = ok && arrived(p0) && arrived(p1) && arrived(p2) && arrived(p3);
+      if (ok) break;
+      ok = true;
+      if (adj && col > j + 8) __nanosleep(64);
+    } while (++spins < kSpinLimit);
+    if (spins >= kSpinLimit) {
+      atomicExch(err, 1);
+      s_fail = 1;
+    }
+    __syncthreads();
+    if (s_fail) return false;
+    double d = red[buf][lane & 3][half];
+    d += __shfl_xor_sync(0xffffffffu, d, 1);
+    d += __shfl_xor_sync(0xffffffffu, d, 2);
+    const double ux = value_of(p0), uy = value_of(p1), kx = value_of(p2), ky = adj ? value_of(p3) : -value_of(p3);
+    // w = uᴴx + conj(u₁)·x_j, f = κ'·w (κ' = conj(κ) for Hᴴ): Re in lanes 0-15, Im in 16-31
+    const double cx_ = s_row[buf][0], cy_ = s_row[buf][1];
+    const double w = fma(ux, half ? cy_ : cx_, fma(uy, half ? -cx_ : cy_, d));
+    const double wo = __shfl_xor_sync(0xffffffffu, w, 16);
+    const double f = fma(kx, w, (half ? ky : -ky) * wo);
+    const double fx = __shfl_sync(0xffffffffu, f, 0), fy = __shfl_sync(0xffffffffu, f, 16);
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const cxd v = tid + q * kNT == j ? mkcx(ux, uy) : u[q];
+      x[q].x = fma(-fx, v.x, fma(fy, v.y, x[q].x));
+      x[q].y = fma(-fx, v.y, fma(-fy, v.x, x[q].y));
+    }
+    buf ^= 1;
+    return true;
+  };
+
+  const int steps = min(col, k);
+  for (int j = 0; j < steps; ++j)
+    if (!reflect(j, true)) return;
+  if (col < k) {
+    // this column's reflector: the entries below the pivot go out first
+    ulonglong2* b = M.box + (int64_t)col * stride;
+    double s2 = 0;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int t = tid + q * kNT;
+      if (t > col && t < m) {
+        put(b + t, x[q].x);
+        put(b + m + t, x[q].y);
+        s2 = fma(x[q].x, x[q].x, fma(x[q].y, x[q].y, s2));
+      }
+      if (t == col) {
+        s_row[buf][0] = x[q].x;
+        s_row[buf][1] = x[q].y;
+      }
+    }
+    s2 = warp_sum(s2);
+    if (lane == 0) red[buf][warp][0] = s2;
+    __syncthreads();
+    s2 = red[buf][lane & 3][0];
+    s2 += __shfl_xor_sync(0xffffffffu, s2, 1);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, 2);
+    const double ax = s_row[buf][0], ay = s_row[buf][1];
+    buf ^= 1;
+    double beta = ax, ux = 0, uy = 0, kx = 0, ky = 0;
+    if (!(s2 == 0.0 && ay == 0.0)) {
+      // β = −sgn(Re α)·‖x‖, u₁ = α − β, conj(κ) = −1/(β·u₁) = −(conj(u₁)/|u₁|²)/β
+      const double nrm = sqrt(fma(ax, ax, fma(ay, ay, s2)));
+      beta = ax >= 0.0 ? -nrm : nrm;
+      ux = ax - beta;
+      uy = ay;
+      const double inv2 = 1.0 / fma(ux, ux, uy * uy), invb = -1.0 / beta;
+      kx = (ux * inv2) * invb;
+      ky = (-uy * inv2) * invb;
+    }
+    if (tid < 4) put(b + 2 * m + tid, tid == 0 ? ux : (tid == 1 ? uy : (tid == 2 ? kx : ky)));
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+      if (tid + q * kNT == col) x[q] = mkcx(beta, 0.0);
+  }
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const int t = tid + q * kNT;
+    if (t < k) M.R[(int64_t)col * k + t] = t <= col ? x[q] : mkcx(0.0, 0.0);
+  }
+  if (col >= k || !M.Q) return;
+#pragma unroll
+  for (int q = 0; q < R; ++q) x[q] = mkcx(tid + q * kNT == col ? 1.0 : 0.0, 0.0);
+  for (int j = col; j >= 0; --j)
+    if (!reflect(j, false)) return;
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const int t = tid + q * kNT;
+    if (t < m) M.Q[(int64_t)col * m + t] = x[q];
+  }
+}
+
+const void* kernel_for(int64_t m) {
+  return m <= kNT ? (const void*)k_qr_cols<1> : (m <= 2 * kNT ? (const void*)k_qr_cols<2> : (const void*)k_qr_cols<4>);
+}
+
+size_t boxes_bytes(int64_t m, int64_t k) { return (size_t)k * (size_t)(2 * m + 4) * sizeof(ulonglong2); }
+
+}  // namespace
+
+size_t qr_cols_workspace(int64_t m, int64_t n, int64_t count) {
+  return ws_round((size_t)count * boxes_bytes(m, std::min(m, n)) + 256) +
+         ws_round((size_t)count * (sizeof(QMat) + sizeof(int) * (size_t)n) + 256);
+}
+
+// whether the one-CTA-per-column kernel takes these matrices: rows in the registers of one
+// CTA, and every column of every matrix resident at once
+tn_status_t qr_cols_takes(tn_ctx* ctx, int64_t m, int64_t columns, bool* out) {
+  static int per_sm[3] = {};
+  *out = false;
+  if (m > 4 * kNT) return TN_OK;
+  int& p = per_sm[m <= kNT ? 0 : (m <= 2 * kNT ? 1 : 2)];
+  int q = p;
+  if (q == 0) {
+    TN_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, kernel_for(m), kNT, 0));
+    p = q;
+  }
+  *out = columns <= (int64_t)q * ctx->num_sms;
+  return TN_OK;
+}
+
+// thin QR of every matrix of the list (one launch; the caller asked qr_cols_takes with the
+// sum of their columns); Q null: R only
+tn_status_t qr_cols(tn_ctx* ctx, const std::vector<QrMat>& mats) {
+  if (mats.empty()) return TN_OK;
+  size_t boxes = 0;
+  int64_t ctas = 0, mmax = 1;
+  for (const QrMat& q : mats) {
+    boxes += boxes_bytes(q.m, std::min(q.m, q.n));
+    ctas += q.n;
+    mmax = std::max<int64_t>(mmax, q.m);
+  }
+  char* box = ws_take<char>(ctx, boxes + 256);
+  TN_CHECK_CUDA(ctx, cudaMemsetAsync(box, 0, boxes, ctx->stream));
+  const size_t owner_at = sizeof(QMat) * mats.size();
+  char* table = ws_take<char>(ctx, owner_at + sizeof(int) * (size_t)ctas);
+  std::vector<char> host(owner_at + sizeof(int) * (size_t)ctas, 0);
+  QMat* hm = reinterpret_cast<QMat*>(host.data());
+  int* ho = reinterpret_cast<int*>(host.data() + owner_at);
+  int cta = 0;
+  for (size_t q = 0; q < mats.size(); ++q) {
+    const QrMat& s = mats[q];
+    const int k = std::min(s.m, s.n);
+    hm[q] = QMat{s.A, s.Q, s.R, reinterpret_cast<ulonglong2*>(box), s.lda, s.m, s.n, k, cta};
+    box += boxes_bytes(s.m, k);
+    for (int c = 0; c < s.n; ++c) ho[cta++] = (int)q;
+  }
+  TN_CHECK_CUDA(ctx, cudaMemcpyAsync(table, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream));
+  const QMat* dm = reinterpret_cast<const QMat*>(table);
+  const int* down = reinterpret_cast<const int*>(table + owner_at);
+  QBatch none = {};
+  int* err = nullptr;
+  TN_RETURN_IF(wait_error_word(ctx, &err));
+  void* args[] = {&none, &dm, &down, &err};
+  TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel(kernel_for(mmax), dim3((unsigned)ctas), dim3(kNT), args, 0, ctx->stream));
+  TN_LAUNCHED(ctx);
+  return TN_OK;
+}
+
+// the same for a batch of equal matrices at fixed strides
+tn_status_t qr_cols_batch(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda, int64_t sA, cxd* Q, int64_t sQ,
+                          cxd* R, int64_t sR, int64_t batch) {
+  const int64_t k = std::min(m, n);
+  const size_t one = boxes_bytes(m, k);
+  char* box = ws_take<char>(ctx, one * (size_t)batch);
+  TN_CHECK_CUDA(ctx, cudaMemsetAsync(box, 0, one * (size_t)batch, ctx->stream));
+  QBatch b = {QMat{A, Q, R, reinterpret_cast<ulonglong2*>(box), lda, (int)m, (int)n, (int)k, 0}, sA, sQ, sR,
+              (int64_t)(one / sizeof(ulonglong2))};
+  const QMat* dm = nullptr;
+  const int* down = nullptr;
+  int* err = nullptr;
+  TN_RETURN_IF(wait_error_word(ctx, &err));
+  void* args[] = {&b, &dm, &down, &err};
+  TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel(kernel_for(m), dim3((unsigned)(n * batch)), dim3(kNT), args, 0,
+                                                 ctx->stream));
+  TN_LAUNCHED(ctx);
+  return TN_OK;
+}

@@ -1,0 +1,82 @@
+"""QR with one CTA per column (k_qr_cols) at the edges of its rows per thread, for tall, square
+and wide matrices, batches, rank deficiency and in-place calls, against LAPACK.
+
+Tolerances: Householder QR is backward stable, ‖QR − A‖ and ‖QᴴQ − I‖ are a small multiple of
+√(m·k)·u with u = 1.1e-16; 1e-13 covers m = 512.  Q and R themselves follow LAPACK's sign
+convention and agree with it to κ(A)·√(m·k)·u, κ ≤ 1e3 here for the tall Gaussian matrices.
+"""
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import tenetgb
+
+    return tenetgb.Context(0)
+
+
+def _qr(ctx, A, in_place=False, lda_pad=0):
+    import tenetgb
+
+    batch, m, n = A.shape
+    k, lda = min(m, n), m + lda_pad
+    store = np.zeros((batch, n, lda), complex)
+    store[:, :, :m] = A.transpose(0, 2, 1)
+    dA = tenetgb.DeviceTensor.from_numpy(ctx, store.reshape(-1), ["x"])
+    dQ = dA if in_place else tenetgb.DeviceTensor.from_numpy(ctx, np.full(batch * m * k, np.nan + 0j), ["x"])
+    dR = tenetgb.DeviceTensor.from_numpy(ctx, np.full(batch * k * n, np.nan + 0j), ["x"])
+    sQ = lda * n if in_place else m * k
+    ctx.check(ctx.lib.tn_qr_thin(ctx.h, 3, 0, m, n, C.c_void_p(dA.ptr), lda, lda * n, C.c_void_p(dQ.ptr), sQ,
+                                 C.c_void_p(dR.ptr), k * n, batch))
+    q, r = dQ.numpy(), dR.numpy()
+    Q = np.stack([q[b * sQ: b * sQ + m * k].reshape((m, k), order="F") for b in range(batch)])
+    return Q, r.reshape(batch, n, k).transpose(0, 2, 1)
+
+
+def _check(A, Q, R, lapack=True):
+    for a, q, r in zip(A, Q, R):
+        scale = max(np.linalg.norm(a), 1e-300)
+        assert np.linalg.norm(q @ r - a) <= 1e-13 * scale
+        assert np.abs(q.conj().T @ q - np.eye(q.shape[1])).max() <= 1e-13
+        assert (np.tril(r, -1) == 0).all() and (np.diagonal(r).imag == 0).all()
+        if lapack:
+            q0, r0 = np.linalg.qr(a)
+            assert np.abs(q - q0).max() <= 1e-10 and np.abs(r - r0).max() <= 1e-10 * scale
+
+
+@pytest.mark.parametrize("m,n,batch", [
+    (1, 1, 1), (2, 1, 3), (2, 2, 1), (127, 5, 1), (128, 64, 2), (129, 40, 1), (256, 31, 1), (257, 33, 1), (512, 200, 1),
+    (37, 90, 2), (128, 128, 1), (5, 300, 1), (300, 300, 1), (16, 8, 40), (513, 20, 1),
+])
+def test_columns_qr_matches_lapack(ctx, m, n, batch):
+    rng = np.random.default_rng(m * 1000 + n)
+    A = rng.standard_normal((batch, m, n)) + 1j * rng.standard_normal((batch, m, n))
+    Q, R = _qr(ctx, A)
+    _check(A, Q, R, lapack=m != n)
+
+
+@pytest.mark.parametrize("m,n,batch,pad", [(64, 32, 2, 0), (200, 200, 1, 0), (30, 80, 2, 0), (64, 32, 2, 7)])
+def test_columns_qr_in_place(ctx, m, n, batch, pad):
+    rng = np.random.default_rng(m + n)
+    A = rng.standard_normal((batch, m, n)) + 1j * rng.standard_normal((batch, m, n))
+    Q, R = _qr(ctx, A, in_place=True, lda_pad=pad)
+    _check(A, Q, R, lapack=m != n)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-120, 1e120])
+def test_columns_qr_of_special_matrices(ctx, scale):
+    """A zero column, repeated columns, a real matrix, an upper triangular one; tiny and huge entries."""
+    rng = np.random.default_rng(5)
+    g = rng.standard_normal((60, 24)) + 1j * rng.standard_normal((60, 24))
+    zero, twice = g.copy(), g.copy()
+    zero[:, 3] = 0
+    twice[:, 9] = twice[:, 2]
+    A = scale * np.stack([zero, twice, g.real + 0j, np.triu(g)])
+    Q, R = _qr(ctx, A)
+    _check(A, Q, R, lapack=False)
