@@ -334,18 +334,13 @@ template <typename T>
 tn_status_t qr_cx(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>* A, int64_t lda, int64_t sA,
                   cx<T>* Q, int64_t sQ, cx<T>* R, int64_t sR, int64_t batch);
 
-// thin QR with one CTA per column (tn_qr_cols.cu): Q m × k (ld m) or null, R k × n (ld k)
-struct QrMat {
-  const cxd* A;
-  cxd *Q, *R;
-  int64_t lda;
-  int m, n;
-};
-size_t qr_cols_workspace(int64_t m, int64_t n, int64_t count);
+// thin QR with one CTA per column (tn_qr_cols.cu): of op(A)·Π, Q m × k (ld m) or null, R k × n
+// (ld k) or its adjoint (ld n)
+size_t qr_cols_workspace(int64_t m, int64_t n, int64_t batch);
 tn_status_t qr_cols_takes(tn_ctx* ctx, int64_t m, int64_t columns, bool* out);
-tn_status_t qr_cols(tn_ctx* ctx, const std::vector<QrMat>& mats);
 tn_status_t qr_cols_batch(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda, int64_t sA, cxd* Q, int64_t sQ,
-                          cxd* R, int64_t sR, int64_t batch);
+                          cxd* R, int64_t sR, int64_t batch, const int* perm = nullptr, bool adj_in = false,
+                          bool adj_r = false);
 
 template <typename T>
 size_t svd_workspace(int64_t m, int64_t n, int64_t batch);

@@ -30,8 +30,10 @@ struct QMat {
   const cxd* A;
   cxd *Q, *R;       // Q m × k (ld m), R k × n (ld k)
   ulonglong2* box;  // k reflectors × (2m + 4) packets
+  const int* perm;  // column c of the factored matrix is column perm[c] of op(A); null: c
   int64_t lda;
-  int m, n, k, cta0;
+  int m, n, k, cta0;  // m × n: the factored matrix
+  int adj;            // bit 0: op(A) = Aᴴ (A n × m); bit 1: Rᴴ (n × k, ld n) is stored for R
 };
 
 __device__ __forceinline__ void put(ulonglong2* p, double v) {
@@ -65,20 +67,16 @@ struct QBatch {
   int64_t sA, sQ, sR, sBox;
 };
 
-// mats/owner: the list form (owner[CTA] = its matrix); null: the batch form
 template <int R>
-__global__ void __launch_bounds__(kNT, 4)
-    k_qr_cols(QBatch batch, const QMat* __restrict__ mats, const int* __restrict__ owner, int* err) {
-  QMat M;
-  if (mats) {
-    M = mats[owner[blockIdx.x]];
-  } else {
-    M = batch.first;
+__global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
+  QMat M = batch.first;
+  {
     const int b = (int)blockIdx.x / M.n;
     M.A += b * batch.sA;
     if (M.Q) M.Q += b * batch.sQ;
     M.R += b * batch.sR;
     M.box += b * batch.sBox;
+    if (M.perm) M.perm += b * M.n;
     M.cta0 = b * M.n;
   }
   const int m = M.m, k = M.k, col = (int)blockIdx.x - M.cta0;
@@ -89,10 +87,12 @@ __global__ void __launch_bounds__(kNT, 4)
   __shared__ int s_fail;
   if (tid == 0) s_fail = 0;
   cxd x[R];
+  const int64_t src = M.perm ? M.perm[col] : col;
 #pragma unroll
   for (int q = 0; q < R; ++q) {
-    const int t = tid + q * kNT;
-    x[q] = t < m ? M.A[(int64_t)col * M.lda + t] : mkcx(0.0, 0.0);
+    const int64_t t = tid + q * kNT;
+    x[q] = mkcx(0.0, 0.0);
+    if (t < m) x[q] = (M.adj & 1) ? conjg(M.A[src + t * M.lda]) : M.A[src * M.lda + t];
   }
   int buf = 0;
   // x ← (I − f-form of reflector j) x: rows > j of u from the packets, u₁ and conj(κ) from the
@@ -221,7 +221,12 @@ __global__ void __launch_bounds__(kNT, 4)
 #pragma unroll
   for (int q = 0; q < R; ++q) {
     const int t = tid + q * kNT;
-    if (t < k) M.R[(int64_t)col * k + t] = t <= col ? x[q] : mkcx(0.0, 0.0);
+    if (t >= k) continue;
+    const cxd v = t <= col ? x[q] : mkcx(0.0, 0.0);
+    if (M.adj & 2)
+      M.R[(int64_t)t * M.n + col] = conjg(v);
+    else
+      M.R[(int64_t)col * k + t] = v;
   }
   if (col >= k || !M.Q) return;
 #pragma unroll
@@ -243,9 +248,8 @@ size_t boxes_bytes(int64_t m, int64_t k) { return (size_t)k * (size_t)(2 * m + 4
 
 }  // namespace
 
-size_t qr_cols_workspace(int64_t m, int64_t n, int64_t count) {
-  return ws_round((size_t)count * boxes_bytes(m, std::min(m, n)) + 256) +
-         ws_round((size_t)count * (sizeof(QMat) + sizeof(int) * (size_t)n) + 256);
+size_t qr_cols_workspace(int64_t m, int64_t n, int64_t batch) {
+  return ws_round((size_t)batch * boxes_bytes(m, std::min(m, n)));
 }
 
 // whether the one-CTA-per-column kernel takes these matrices: rows in the registers of one
@@ -264,58 +268,20 @@ tn_status_t qr_cols_takes(tn_ctx* ctx, int64_t m, int64_t columns, bool* out) {
   return TN_OK;
 }
 
-// thin QR of every matrix of the list (one launch; the caller asked qr_cols_takes with the
-// sum of their columns); Q null: R only
-tn_status_t qr_cols(tn_ctx* ctx, const std::vector<QrMat>& mats) {
-  if (mats.empty()) return TN_OK;
-  size_t boxes = 0;
-  int64_t ctas = 0, mmax = 1;
-  for (const QrMat& q : mats) {
-    boxes += boxes_bytes(q.m, std::min(q.m, q.n));
-    ctas += q.n;
-    mmax = std::max<int64_t>(mmax, q.m);
-  }
-  char* box = ws_take<char>(ctx, boxes + 256);
-  TN_CHECK_CUDA(ctx, cudaMemsetAsync(box, 0, boxes, ctx->stream));
-  const size_t owner_at = sizeof(QMat) * mats.size();
-  char* table = ws_take<char>(ctx, owner_at + sizeof(int) * (size_t)ctas);
-  std::vector<char> host(owner_at + sizeof(int) * (size_t)ctas, 0);
-  QMat* hm = reinterpret_cast<QMat*>(host.data());
-  int* ho = reinterpret_cast<int*>(host.data() + owner_at);
-  int cta = 0;
-  for (size_t q = 0; q < mats.size(); ++q) {
-    const QrMat& s = mats[q];
-    const int k = std::min(s.m, s.n);
-    hm[q] = QMat{s.A, s.Q, s.R, reinterpret_cast<ulonglong2*>(box), s.lda, s.m, s.n, k, cta};
-    box += boxes_bytes(s.m, k);
-    for (int c = 0; c < s.n; ++c) ho[cta++] = (int)q;
-  }
-  TN_CHECK_CUDA(ctx, cudaMemcpyAsync(table, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream));
-  const QMat* dm = reinterpret_cast<const QMat*>(table);
-  const int* down = reinterpret_cast<const int*>(table + owner_at);
-  QBatch none = {};
-  int* err = nullptr;
-  TN_RETURN_IF(wait_error_word(ctx, &err));
-  void* args[] = {&none, &dm, &down, &err};
-  TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel(kernel_for(mmax), dim3((unsigned)ctas), dim3(kNT), args, 0, ctx->stream));
-  TN_LAUNCHED(ctx);
-  return TN_OK;
-}
-
-// the same for a batch of equal matrices at fixed strides
+// thin QR of a batch of m × n matrices op(A)·Π (the caller asked qr_cols_takes with n·batch).
+// Q null: not formed.  perm (n per matrix): the column order Π, null for none.
 tn_status_t qr_cols_batch(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda, int64_t sA, cxd* Q, int64_t sQ,
-                          cxd* R, int64_t sR, int64_t batch) {
+                          cxd* R, int64_t sR, int64_t batch, const int* perm, bool adj_in, bool adj_r) {
   const int64_t k = std::min(m, n);
   const size_t one = boxes_bytes(m, k);
   char* box = ws_take<char>(ctx, one * (size_t)batch);
   TN_CHECK_CUDA(ctx, cudaMemsetAsync(box, 0, one * (size_t)batch, ctx->stream));
-  QBatch b = {QMat{A, Q, R, reinterpret_cast<ulonglong2*>(box), lda, (int)m, (int)n, (int)k, 0}, sA, sQ, sR,
-              (int64_t)(one / sizeof(ulonglong2))};
-  const QMat* dm = nullptr;
-  const int* down = nullptr;
+  QBatch b = {QMat{A, Q, R, reinterpret_cast<ulonglong2*>(box), perm, lda, (int)m, (int)n, (int)k, 0,
+                   (adj_in ? 1 : 0) + (adj_r ? 2 : 0)},
+              sA, sQ, sR, (int64_t)(one / sizeof(ulonglong2))};
   int* err = nullptr;
   TN_RETURN_IF(wait_error_word(ctx, &err));
-  void* args[] = {&b, &dm, &down, &err};
+  void* args[] = {&b, &err};
   TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel(kernel_for(m), dim3((unsigned)(n * batch)), dim3(kNT), args, 0,
                                                  ctx->stream));
   TN_LAUNCHED(ctx);
