@@ -359,8 +359,8 @@ struct JacobiMat {
   int m, n;
 };
 bool jacobi_pairs_fits(int64_t m, int64_t n);
-size_t jacobi_pairs_workspace(int64_t m, int64_t n, int64_t count, int64_t ctas, bool with_v);
-tn_status_t jacobi_pairs_resident(tn_ctx* ctx, int64_t m, bool with_v, int64_t* out);
+size_t jacobi_pairs_workspace(int64_t m, int64_t n, int64_t count, bool with_v);
+tn_status_t jacobi_pairs_resident(tn_ctx* ctx, int64_t m, int64_t* out);
 tn_status_t jacobi_pairs(tn_ctx* ctx, const std::vector<JacobiMat>& mats, bool v_given, int max_sweeps, int* sweeps_out,
                          bool* noconv_out);
 

@@ -790,7 +790,7 @@ size_t svd_workspace(int64_t m, int64_t n, int64_t batch) {
          ws_round(sizeof(int) * (size_t)(n * batch)) + ws_round(sizeof(int) * (size_t)(batch + 1)) +
          ws_round(sizeof(int) * (size_t)(2 * batch + 2)) + ws_round(sizeof(T) * (size_t)((n + 1) * batch)) +
          (sizeof(T) == 8 && jacobi_pairs_fits(m, n)
-              ? jacobi_pairs_workspace(m, n, batch, (n + 1) / 2 * batch, true) + svd_ordered_workspace(m, n, batch)
+              ? jacobi_pairs_workspace(m, n, batch, true) + svd_ordered_workspace(m, n, batch)
               : 0);
 }
 template size_t svd_workspace<double>(int64_t, int64_t, int64_t);
@@ -869,12 +869,12 @@ static tn_status_t launch_step(tn_ctx* ctx, int64_t m, int64_t n, int N, int r, 
 // spreads every matrix over n/2 SMs; one CTA per matrix in shared memory is left for matrices
 // of a few columns, where the launch is the time, and for batches of so many small matrices
 // that they fill the chip twice over with one SM each.
-static tn_status_t jacobi_takes_pairs(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch, bool* out) {
+static tn_status_t jacobi_takes_pairs(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch, bool with_v, bool* out) {
   *out = false;
   if (!jacobi_pairs_fits(m, n) || n < kPairsMinN) return TN_OK;
   int64_t resident = 0;
-  TN_RETURN_IF(jacobi_pairs_resident(ctx, m, true, &resident));
-  if ((n + 1) / 2 > resident) return TN_OK;
+  TN_RETURN_IF(jacobi_pairs_resident(ctx, m, &resident));
+  if ((n + 1) / 2 * (with_v ? 2 : 1) > resident) return TN_OK;
   const bool in_smem = sizeof(cxd) * (size_t)(m * n + n * n) <= kSmemMax && n <= 256;
   *out = !(in_smem && (n + 1) / 2 * batch > 2 * resident && batch >= 2 * ctx->num_sms);
   return TN_OK;
@@ -911,7 +911,7 @@ static tn_status_t jacobi_core(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T
   bool noconv = false;
   const size_t smem_need = sizeof(cx<T>) * (size_t)(m * n + n * n);
   bool pairs_kernel = false;
-  if (sizeof(T) == 8 && !tail && min_rot_frac <= 0.0) TN_RETURN_IF(jacobi_takes_pairs(ctx, m, n, batch, &pairs_kernel));
+  if (sizeof(T) == 8 && !tail && min_rot_frac <= 0.0) TN_RETURN_IF(jacobi_takes_pairs(ctx, m, n, batch, V != nullptr, &pairs_kernel));
   if (pairs_kernel) {
     std::vector<JacobiMat> mats((size_t)batch);
     for (int64_t b = 0; b < batch; ++b)
@@ -1101,11 +1101,11 @@ static tn_status_t jacobi_finalize(tn_ctx* ctx, int64_t m, int64_t n, const cx<T
 // ---------------------------------------------------------------------------------
 constexpr int64_t kOrderedMinN = 24;  // below this the QR costs more than the sweeps it saves
 
-static tn_status_t svd_takes_ordered(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch, bool* out) {
+static tn_status_t svd_takes_ordered(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch, bool with_v, bool* out) {
   *out = false;
   if (n < kOrderedMinN) return TN_OK;
   bool pairs = false;
-  TN_RETURN_IF(jacobi_takes_pairs(ctx, m, n, batch, &pairs));
+  TN_RETURN_IF(jacobi_takes_pairs(ctx, m, n, batch, with_v || m > n, &pairs));
   if (pairs) TN_RETURN_IF(qr_cols_takes(ctx, m, n * batch, out));
   return TN_OK;
 }
@@ -1167,7 +1167,7 @@ static tn_status_t svd_tall_impl(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>*
   T* nrm = ws_take<T>(ctx, (size_t)((n + 1) * batch));  // column norms, then ‖W_b‖²_F
   if constexpr (sizeof(T) == 8) {
     bool ordered = false, nc = false;
-    TN_RETURN_IF(svd_takes_ordered(ctx, m, n, batch, &ordered));
+    TN_RETURN_IF(svd_takes_ordered(ctx, m, n, batch, Vo != nullptr, &ordered));
     if (ordered) {
       ctx->last_sweeps_fp32 = 0;
       TN_RETURN_IF(svd_ordered(ctx, m, n, A, lda, sA, U, sU, S, sS, Vo, sVo, vh, batch, W, V, order, nrm, sweeps_out, &nc));
@@ -1515,7 +1515,7 @@ size_t svd_mixed_workspace(int64_t m, int64_t n, int64_t batch) {
   s += ws_round((size_t)(n * batch));                     // tail flags
   s += ws_round(sizeof(cxd) * (size_t)(n * n * batch));  // R / E of the refinement
   s += ws_round((size_t)(n * batch)) + ws_round(sizeof(int) * (size_t)(5 * batch + 4));  // cluster marks, stats
-  if (jacobi_pairs_fits(m, n)) s += jacobi_pairs_workspace(m, n, batch, (n + 1) / 2 * batch, true);
+  if (jacobi_pairs_fits(m, n)) s += jacobi_pairs_workspace(m, n, batch, true);
   return s;
 }
 
@@ -1819,7 +1819,7 @@ tn_status_t svd_left(tn_ctx* ctx, tn_precision_t prec, int64_t m, int64_t n, con
   int* rotated = ws_take<int>(ctx, (size_t)(2 * batch + 2));
   double* nrm = ws_take<double>(ctx, (size_t)((n + 1) * batch));
   bool ordered = false;
-  TN_RETURN_IF(svd_takes_ordered(ctx, m, n, batch, &ordered));
+  TN_RETURN_IF(svd_takes_ordered(ctx, m, n, batch, false, &ordered));
   if (ordered) {
     bool nc = false;
     ctx->last_sweeps_fp32 = 0;
@@ -1836,7 +1836,7 @@ tn_status_t svd_left(tn_ctx* ctx, tn_precision_t prec, int64_t m, int64_t n, con
   // no right vectors are needed here; only the one-CTA shared-memory kernel, which keeps V
   // resident, takes them
   bool pairs_kernel = false;
-  TN_RETURN_IF(jacobi_takes_pairs(ctx, m, n, batch, &pairs_kernel));
+  TN_RETURN_IF(jacobi_takes_pairs(ctx, m, n, batch, false, &pairs_kernel));
   const bool small = !pairs_kernel && sizeof(cxd) * (size_t)(m * n + n * n) <= kSmemMax && n <= 256;
   bool noconv = false;
   ctx->last_sweeps_fp32 = 0;
