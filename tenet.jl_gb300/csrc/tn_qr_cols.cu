@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     double wx = 0, wy = 0;
 #pragma unroll
     for (int q = 0; q < R; ++q) {
+      if ((q + 1) * kNT <= j) continue;  // rows above the pivot: u = 0
       wx = fma(u[q].x, x[q].x, fma(u[q].y, x[q].y, wx));
       wy = fma(u[q].x, x[q].y, fma(-u[q].y, x[q].x, wy));
       if (tid + q * kNT == j) {
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     const double fx = __shfl_sync(0xffffffffu, f, 0), fy = __shfl_sync(0xffffffffu, f, 16);
 #pragma unroll
     for (int q = 0; q < R; ++q) {
+      if ((q + 1) * kNT <= j) continue;
       const cxd v = tid + q * kNT == j ? mkcx(ux, uy) : u[q];
       x[q].x = fma(-fx, v.x, fma(fy, v.y, x[q].x));
       x[q].y = fma(-fx, v.y, fma(-fy, v.x, x[q].y));
@@ -205,11 +207,15 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     double beta = ax, ux = 0, uy = 0, kx = 0, ky = 0;
     if (!(s2 == 0.0 && ay == 0.0)) {
       // β = −sgn(Re α)·‖x‖, u₁ = α − β, conj(κ) = −1/(β·u₁) = −(conj(u₁)/|u₁|²)/β
-      const double nrm = sqrt(fma(ax, ax, fma(ay, ay, s2)));
+      // (‖x‖ and 1/‖x‖ from one reciprocal square root, ‖x‖ corrected by its residual: a square
+      // root and a division are 580 clocks each)
+      const double n2 = fma(ax, ax, fma(ay, ay, s2)), rs = rsqrt(n2);
+      double nrm = n2 * rs;
+      nrm = fma(fma(-nrm, nrm, n2), 0.5 * rs, nrm);
       beta = ax >= 0.0 ? -nrm : nrm;
       ux = ax - beta;
       uy = ay;
-      const double inv2 = 1.0 / fma(ux, ux, uy * uy), invb = -1.0 / beta;
+      const double inv2 = 1.0 / fma(ux, ux, uy * uy), invb = ax >= 0.0 ? rs : -rs;
       kx = (ux * inv2) * invb;
       ky = (-uy * inv2) * invb;
     }
