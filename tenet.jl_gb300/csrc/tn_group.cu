@@ -669,19 +669,10 @@ tn_status_t g_qr(tn_ctx* ctx, const std::vector<QrD>& h) {
   return TN_OK;
 }
 
-// U (r leading columns) and Σ of every W (m ≥ n) by grouped one-sided Jacobi sweeps
-tn_status_t g_svd_left(tn_ctx* ctx, std::vector<JacD>& h, int* active, int* rotated) {
-  if (h.empty()) return TN_OK;
+// the sweeps by grouped launches, one per round (rows > 512)
+tn_status_t g_sweeps_by_rounds(tn_ctx* ctx, const std::vector<JacD>& h, JacD* d, int64_t mmax, int64_t Nmax, int* active,
+                               int* rotated) {
   const int P = (int)h.size();
-  int64_t mmax = 1, Nmax = 2;
-  for (auto& j : h) {
-    j.N = (int)(j.n + (j.n & 1));
-    mmax = std::max(mmax, j.m);
-    Nmax = std::max<int64_t>(Nmax, j.N);
-  }
-  if (mmax > 4096) return tn_set_error(ctx, TN_EUNSUPPORTED, "group svd: more than 4096 rows");
-  JacD* d = nullptr;
-  TN_RETURN_IF(upload(ctx, h, &d));
   std::vector<int> h_act(P, 1), h_rot(2 * P);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(active, h_act.data(), sizeof(int) * P, cudaMemcpyHostToDevice, ctx->stream));
   const double stop_ratio = sqrt(4.0 * sqrt((double)mmax) * 2.220446049250313e-16 * 1e-2);
@@ -732,6 +723,38 @@ tn_status_t g_svd_left(tn_ctx* ctx, std::vector<JacD>& h, int* active, int* rota
     TN_CHECK_CUDA(ctx, cudaMemcpyAsync(active, h_act.data(), sizeof(int) * P, cudaMemcpyHostToDevice, ctx->stream));
   }
   if (n_active > 0) return tn_set_error(ctx, TN_ENOCONV, "group svd: no convergence within 40 sweeps");
+  return TN_OK;
+}
+
+// U (r leading columns) and Σ of every W by one-sided Jacobi sweeps: the persistent
+// column-pair kernel while a column's rows fit one CTA (every matrix then stops at its own
+// convergence; measured GROUP_NUMBERS), one grouped launch per round beyond
+tn_status_t g_svd_left(tn_ctx* ctx, std::vector<JacD>& h, int* active, int* rotated) {
+  if (h.empty()) return TN_OK;
+  const int P = (int)h.size();
+  int64_t mmax = 1, Nmax = 2;
+  for (auto& j : h) {
+    j.N = (int)(j.n + (j.n & 1));
+    mmax = std::max(mmax, j.m);
+    Nmax = std::max<int64_t>(Nmax, j.N);
+  }
+  if (mmax > 4096) return tn_set_error(ctx, TN_EUNSUPPORTED, "group svd: more than 4096 rows");
+  JacD* d = nullptr;
+  TN_RETURN_IF(upload(ctx, h, &d));
+  int64_t resident = 0;
+  TN_RETURN_IF(jacobi_pairs_resident(ctx, mmax, &resident));
+  if (mmax <= 512 && Nmax / 2 <= resident) {
+    std::vector<JacobiMat> mats;
+    for (auto& j : h) mats.push_back({j.W, nullptr, j.nrm, (int)j.m, (int)j.n});
+    // like sizes together: a launch lasts as long as its slowest matrix
+    std::stable_sort(mats.begin(), mats.end(), [](const JacobiMat& a, const JacobiMat& b) { return a.n > b.n; });
+    int sweeps = 0;
+    bool noconv = false;
+    TN_RETURN_IF(jacobi_pairs(ctx, mats, false, 80, &sweeps, &noconv));
+    if (noconv) return tn_set_error(ctx, TN_ENOCONV, "group svd: no convergence within 80 sweeps");
+  } else {
+    TN_RETURN_IF(g_sweeps_by_rounds(ctx, h, d, mmax, Nmax, active, rotated));
+  }
   int P2 = 1;
   int64_t nmax = 1;
   for (auto& j : h) nmax = std::max(nmax, j.n);
@@ -982,6 +1005,12 @@ tn_status_t tn_group_canonize_compress_norm(tn_group* g, const int64_t* maxdim, 
     if (ids.empty()) continue;
     const int P = (int)ids.size();
     size_t need = table_bytes(ids.size()) + al256(sizeof(int) * (size_t)(3 * P + 4));
+    int64_t mmax = 1, nmax = 1;
+    for (int b : ids) {
+      mmax = std::max(mmax, g->bond[b][k - 1] * d);
+      nmax = std::max(nmax, g->bond[b][k]);
+    }
+    if (mmax <= 512) need += jacobi_pairs_workspace(mmax, nmax, P, false);
     for (int b : ids) {
       const int64_t m = g->bond[b][k - 1] * d, n = g->bond[b][k], n2 = d * g->bond[b][k + 1];
       const int64_t r = std::min<int64_t>(maxdim[b], std::min(m, n));
