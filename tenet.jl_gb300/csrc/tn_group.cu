@@ -728,7 +728,7 @@ tn_status_t g_sweeps_by_rounds(tn_ctx* ctx, const std::vector<JacD>& h, JacD* d,
 
 // U (r leading columns) and Σ of every W by one-sided Jacobi sweeps: the persistent
 // column-pair kernel while a column's rows fit one CTA (every matrix then stops at its own
-// convergence; measured GROUP_NUMBERS), one grouped launch per round beyond
+// convergence; measured 16 MPS of χ ≤ 72: 124 → 64 ms, 24 of χ ≤ 512: 571 → 469 ms), one grouped launch per round beyond
 tn_status_t g_svd_left(tn_ctx* ctx, std::vector<JacD>& h, int* active, int* rotated) {
   if (h.empty()) return TN_OK;
   const int P = (int)h.size();

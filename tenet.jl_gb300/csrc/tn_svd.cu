@@ -297,10 +297,10 @@ __global__ void __launch_bounds__(NT)
 }
 
 // ---------------------------------------------------------------------------------
-// Block round of the FP32 pre-pass (m, n ≤ NT): the n columns form blocks of 8; the blocks
+// Block round of the FP32 pre-pass (m, n ≤ 2·NT): the n columns form blocks of 8; the blocks
 // play a round-robin tournament (NB − 1 outer rounds per sweep, one launch each), and the
-// CTA of block pair (P, Q) of matrix b holds the 16 columns of W and V in registers — one
-// row per thread — while it visits the 64 cross pairs (P_i, Q_k) in 8 inner rounds of 8
+// CTA of block pair (P, Q) of matrix b holds the 16 columns of W and V in registers — two
+// rows per thread — while it visits the 64 cross pairs (P_i, Q_k) in 8 inner rounds of 8
 // disjoint pairs; in outer round 0 every block first visits its own 28 pairs (7 inner
 // rounds over P and Q together).  Every column pair is visited once per sweep, as in the
 // column-pair rounds, but W and V cross L2 once per outer round instead of once per pair
@@ -328,9 +328,9 @@ __device__ __forceinline__ void transpose_stage(float* v, int lane) {
 // rotate slots 0..6 by one, so after r rotations slot s holds original column (s + r) mod 7
 // (slot 7 stays); cross rounds pair P slot k with Q slot k and then rotate the Q slots, so
 // Q slot k holds original column (k + r) mod 8.  Seven (eight) rotations restore the order.
-template <int OFF, int LEN>
-__device__ __forceinline__ void rotate_slots(cxf* a) {
-  const cxf t = a[OFF];
+template <int OFF, int LEN, typename C>
+__device__ __forceinline__ void rotate_slots(C* a) {
+  const C t = a[OFF];
 #pragma unroll
   for (int q = 0; q < LEN - 1; ++q) a[OFF + q] = a[OFF + q + 1];
   a[OFF + LEN - 1] = t;
@@ -342,8 +342,48 @@ __host__ __device__ constexpr int blk_slot_orig(bool intra, int r, int slot) {
   return intra ? ((slot & 7) < 7 ? ((slot & 7) + r) % 7 : 7) + (slot & 8) : (slot < 8 ? slot : 8 + ((slot - 8) + r) % 8);
 }
 
+// Two rows per thread, packed: one fma.rn.f32x2 carries the same operation of both rows, so a
+// round takes half the instructions (the round is issue-bound).
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// a column's two rows in one thread: (re, re') and (im, im')
+struct Col2 {
+  f2 x, y;
+};
+// the constants of one rotation, each twice: c, sx, −sx, sy, −sy
+struct __align__(16) Rot2 {
+  f2 c, sx, nsx, sy, nsy, pad;
+};
+// wi' = c·wi − conj(se)·wj, wj' = se·wi + c·wj
+__device__ __forceinline__ void rot_apply_2(const Rot2& q, Col2& wi, Col2& wj) {
+  const f2 ax = f2_fma(q.c, wi.x, f2_fma(q.nsx, wj.x, f2_mul(q.nsy, wj.y)));
+  const f2 ay = f2_fma(q.c, wi.y, f2_fma(q.nsx, wj.y, f2_mul(q.sy, wj.x)));
+  const f2 bx = f2_fma(q.c, wj.x, f2_fma(q.sx, wi.x, f2_mul(q.nsy, wi.y)));
+  const f2 by = f2_fma(q.c, wj.y, f2_fma(q.sx, wi.y, f2_mul(q.sy, wi.x)));
+  wi.x = ax;
+  wi.y = ay;
+  wj.x = bx;
+  wj.y = by;
+}
+
+// NT threads, rows t and t + NT of W and V
 template <int NT>
-__global__ void __launch_bounds__(NT, 512 / NT)
+__global__ void __launch_bounds__(NT, 256 / NT)
     k_jacobi_block_f32(int64_t m, int64_t n, int NB, int R, cxf* __restrict__ W, cxf* __restrict__ V,
                        const float* __restrict__ nrm, const int* __restrict__ active, int* __restrict__ cnt, float tol,
                        const unsigned char* __restrict__ tail) {
@@ -355,6 +395,7 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   __shared__ int s_col[NC];
   __shared__ unsigned char s_tail[NC];
   __shared__ float red[2][NW][32];
+  __shared__ Rot2 s_rot[NW][8];
   __shared__ int s_cnt, s_ratio;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   if (t < NC) {
@@ -369,29 +410,47 @@ __global__ void __launch_bounds__(NT, 512 / NT)
   __syncthreads();
   cxf* Wb = W + b * m * n;
   cxf* Vb = V + b * n * n;
-  cxf w[NC], v[NC];
+  Col2 w[NC], v[NC];
+  const cxf zero = mkcx<float>(0.f, 0.f);
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int col = s_col[c];
-    w[c] = (col >= 0 && t < m) ? Wb[(int64_t)col * m + t] : mkcx<float>(0.f, 0.f);
-    v[c] = (col >= 0 && t < n) ? Vb[(int64_t)col * n + t] : mkcx<float>(0.f, 0.f);
+    const cxf a0 = (col >= 0 && t < m) ? Wb[(int64_t)col * m + t] : zero;
+    const cxf a1 = (col >= 0 && t + NT < m) ? Wb[(int64_t)col * m + t + NT] : zero;
+    const cxf b0 = (col >= 0 && t < n) ? Vb[(int64_t)col * n + t] : zero;
+    const cxf b1 = (col >= 0 && t + NT < n) ? Vb[(int64_t)col * n + t + NT] : zero;
+    w[c].x = f2_pack(a0.x, a1.x);
+    w[c].y = f2_pack(a0.y, a1.y);
+    v[c].x = f2_pack(b0.x, b1.x);
+    v[c].y = f2_pack(b0.y, b1.y);
   }
   const float negl = jacobi_eps<float>() * jacobi_eps<float>() * nrm[n * nmat + b];
+  const f2 minus = f2_pack(-1.f, -1.f);
 
   // one inner round over 8 disjoint pairs (column slots i_k, j_k, compile-time after
   // unrolling).  One barrier per round: every warp sums the per-warp partials itself (in
   // the same order, so all warps form bit-identical rotations) from a double-buffered
-  // table, and lanes 4k hand pair k's rotation to the other lanes by shuffles.
+  // table, and lane 4k leaves pair k's rotation in its warp's shared slots, from where the
+  // packed constants are read as they are.
   int rb = 0;
   auto round = [&](const bool intra, const int r) {
     float val[32];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const cxf x = w[blk_slot_i(intra, k)], y = w[blk_slot_j(intra, k)];
-      val[4 * k + 0] = x.x * x.x + x.y * x.y;
-      val[4 * k + 1] = y.x * y.x + y.y * y.y;
-      val[4 * k + 2] = x.x * y.x + x.y * y.y;
-      val[4 * k + 3] = x.x * y.y - x.y * y.x;
+      const Col2 x = w[blk_slot_i(intra, k)], y = w[blk_slot_j(intra, k)];
+      const f2 al = f2_fma(x.x, x.x, f2_mul(x.y, x.y));
+      const f2 be = f2_fma(y.x, y.x, f2_mul(y.y, y.y));
+      const f2 gx = f2_fma(x.x, y.x, f2_mul(x.y, y.y));
+      const f2 gy = f2_fma(x.x, y.y, f2_mul(f2_mul(x.y, minus), y.x));
+      float a, c;
+      f2_unpack(al, a, c);
+      val[4 * k + 0] = a + c;
+      f2_unpack(be, a, c);
+      val[4 * k + 1] = a + c;
+      f2_unpack(gx, a, c);
+      val[4 * k + 2] = a + c;
+      f2_unpack(gy, a, c);
+      val[4 * k + 3] = a + c;
     }
     transpose_stage<16>(val, lane);
     transpose_stage<8>(val, lane);
@@ -408,7 +467,6 @@ __global__ void __launch_bounds__(NT, 512 / NT)
     const float al = __shfl_sync(0xffffffffu, tot, base);
     const float be = __shfl_sync(0xffffffffu, tot, base + 1);
     const cxf g = mkcx<float>(__shfl_sync(0xffffffffu, tot, base + 2), __shfl_sync(0xffffffffu, tot, base + 3));
-    float rc = 1.f, rsx = 0.f, rsy = 0.f;
     int app = 0;
     if ((lane & 3) == 0) {
       const int k = lane >> 2;  // lane-dependent: the original columns at run time
@@ -422,24 +480,29 @@ __global__ void __launch_bounds__(NT, 512 / NT)
           if (!(monitor > tol)) Rt.apply = 0;
         }
         app = Rt.apply;
-        rc = Rt.c;
-        rsx = Rt.se.x;
-        rsy = Rt.se.y;
+        Rot2& o = s_rot[warp][k];
+        o.c = f2_pack(Rt.c, Rt.c);
+        o.sx = f2_pack(Rt.se.x, Rt.se.x);
+        o.nsx = f2_pack(-Rt.se.x, -Rt.se.x);
+        o.sy = f2_pack(Rt.se.y, Rt.se.y);
+        o.nsy = f2_pack(-Rt.se.y, -Rt.se.y);
         if (warp == 0) {
           if (al > 0.f && be > 0.f) atomicMax(&s_ratio, __float_as_int(monitor));
           if (app) atomicAdd(&s_cnt, 1);
         }
       }
     }
+    const unsigned who = __ballot_sync(0xffffffffu, app);  // (also orders the shared slots in the warp)
+    __syncwarp();
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      if (__shfl_sync(0xffffffffu, app, 4 * k)) {
-        const float c = __shfl_sync(0xffffffffu, rc, 4 * k);
-        const cxf se = mkcx<float>(__shfl_sync(0xffffffffu, rsx, 4 * k), __shfl_sync(0xffffffffu, rsy, 4 * k));
-        rot_apply_c(c, se, w[blk_slot_i(intra, k)], w[blk_slot_j(intra, k)]);
-        rot_apply_c(c, se, v[blk_slot_i(intra, k)], v[blk_slot_j(intra, k)]);
+      if (who >> (4 * k) & 1u) {
+        const Rot2 q = s_rot[warp][k];
+        rot_apply_2(q, w[blk_slot_i(intra, k)], w[blk_slot_j(intra, k)]);
+        rot_apply_2(q, v[blk_slot_i(intra, k)], v[blk_slot_j(intra, k)]);
       }
     }
+    __syncwarp();
   };
   if (R == 0) {
 #pragma unroll 1
@@ -461,8 +524,16 @@ __global__ void __launch_bounds__(NT, 512 / NT)
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int col = s_col[c];
-    if (col >= 0 && t < m) Wb[(int64_t)col * m + t] = w[c];
-    if (col >= 0 && t < n) Vb[(int64_t)col * n + t] = v[c];
+    if (col < 0) continue;
+    cxf a0, a1;
+    f2_unpack(w[c].x, a0.x, a1.x);
+    f2_unpack(w[c].y, a0.y, a1.y);
+    if (t < m) Wb[(int64_t)col * m + t] = a0;
+    if (t + NT < m) Wb[(int64_t)col * m + t + NT] = a1;
+    f2_unpack(v[c].x, a0.x, a1.x);
+    f2_unpack(v[c].y, a0.y, a1.y);
+    if (t < n) Vb[(int64_t)col * n + t] = a0;
+    if (t + NT < n) Vb[(int64_t)col * n + t + NT] = a1;
   }
   if (t == 0) {
     if (s_cnt) atomicAdd(&cnt[b], s_cnt);
@@ -970,11 +1041,11 @@ static tn_status_t jacobi_core(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T
           const dim3 grid((unsigned)(NB / 2), gy);
           for (int r = 0; r < NB - 1; ++r) {
             if (m <= 128 && n <= 128)
-              k_jacobi_block_f32<128><<<grid, 128, 0, ctx->stream>>>(m, n, NB, r, W, V, nrm, active, rotated, tol, tail);
+              k_jacobi_block_f32<64><<<grid, 64, 0, ctx->stream>>>(m, n, NB, r, W, V, nrm, active, rotated, tol, tail);
             else if (m <= 256 && n <= 256)
-              k_jacobi_block_f32<256><<<grid, 256, 0, ctx->stream>>>(m, n, NB, r, W, V, nrm, active, rotated, tol, tail);
+              k_jacobi_block_f32<128><<<grid, 128, 0, ctx->stream>>>(m, n, NB, r, W, V, nrm, active, rotated, tol, tail);
             else
-              k_jacobi_block_f32<512><<<grid, 512, 0, ctx->stream>>>(m, n, NB, r, W, V, nrm, active, rotated, tol, tail);
+              k_jacobi_block_f32<256><<<grid, 256, 0, ctx->stream>>>(m, n, NB, r, W, V, nrm, active, rotated, tol, tail);
             TN_LAUNCHED(ctx);
           }
         }
