@@ -364,6 +364,12 @@ tn_status_t jacobi_pairs_resident(tn_ctx* ctx, int64_t m, int64_t* out);
 tn_status_t jacobi_pairs(tn_ctx* ctx, const std::vector<JacobiMat>& mats, bool v_given, int max_sweeps, int* sweeps_out,
                          bool* noconv_out);
 
+// block round of the mixed SVD's FP32 pre-pass on the tensor pipe (tn_jacobi_tc.cu)
+bool jacobi_block_tc_fits(int64_t m, int64_t n);
+tn_status_t jacobi_block_tc(tn_ctx* ctx, cudaStream_t stream, int64_t m, int64_t n, int NB, int r, cxf* W, cxf* V,
+                            const float* nrm, const int* active, int* rotated, float tol, int64_t batch,
+                            const unsigned char* tail);
+
 // mixed precision SVD (C64 data): FP32 Jacobi pre-pass + FP64 polish.  keep > 0 (V null
 // only): only the `keep` largest triplets are wanted; the rest of U and S is approximate.
 size_t svd_mixed_workspace(int64_t m, int64_t n, int64_t batch);

@@ -15,8 +15,8 @@
 //    the rotation itself from the same numbers;
 //  * the rotation's angle and phase come from FP32 (4 approximate MUFU operations instead of
 //    6 FP64 divisions and roots) and are made unitary to FP64 by one scaling (unit_rotation):
-//    the angle's 1e-7 relative error leaves 1e-7 of the coupling, which the next sweep
-//    removes, while W, V and the inner products stay FP64 throughout;
+//    the angle's 1e-7 relative error leaves 1e-7 of the coupling, which a later sweep
+//    removes (the stop test counts on it), while W, V and the inner products stay FP64;
 //  * V has CTAs of its own, which get each rotation as packets from the CTA that formed it, so
 //    its half of the FP64 work is off the chain and on other SMs;
 //  * the column norms (cached as unevaluated FP32 sums, updated by t|γ|, recomputed exactly in
@@ -310,8 +310,13 @@ __global__ void __launch_bounds__(kNT, 4)
   static_assert(!SPLIT || R == 1, "two threads per row cover 64 rows");
   const Mat M = mats[owner[blockIdx.x]];
   const int m = M.m, n = M.n, N = M.N, pairs = N / 2;
-  const double tol = tol_rel * sqrt((double)(m > 1 ? m : 1));
-  const float tol2 = (float)(tol * tol), stop_ratio = (float)sqrt(tol * 0.1);
+  // A pair above 2u is rotated (the angle's FP32 error leaves couplings of 1e-7 of what they
+  // were: none of those above rounding are left standing), and the sweeps end after one whose
+  // largest ratio was at most stop_ratio, so that what it left, by either rule (its square or
+  // 1e-7 of it), is below rounding
+  constexpr float kTwoU = 2.220446e-16f;
+  const float tol2 = kTwoU * kTwoU;
+  const float stop_ratio = (float)fmin(sqrt(tol_rel * sqrt((double)(m > 1 ? m : 1)) * 0.1), 1e-9);
   if ((int)blockIdx.x - M.cta0 >= pairs) {
     v_role<R, SPLIT>(M, (int)blockIdx.x - M.cta0 - pairs, v_given, max_sweeps, stop_ratio, err);
     return;

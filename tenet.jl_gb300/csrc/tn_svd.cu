@@ -31,6 +31,7 @@ namespace {
 // matrices take 40-60 sweeps
 constexpr int kMaxSweeps = 80;
 constexpr size_t kSmemMax = 200 * 1024;
+constexpr int64_t kTensorMinN = 128;  // fewest columns for the tensor-pipe block round
 constexpr int64_t kPairsMinN = 8;  // fewest columns for the column-pair kernel
 
 template <typename T>
@@ -971,7 +972,7 @@ template <typename T>
 static tn_status_t jacobi_core(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T>* V, int64_t batch, bool v_given,
                                int* active, int* rotated, T* nrm, int max_sweeps, int* sweeps_out, bool* noconv_out,
                                unsigned char* tail = nullptr, int64_t keep = 0, bool tail_preset = false,
-                               double min_rot_frac = 0.0, bool tail_fixed = false) {
+                               double min_rot_frac = 0.0, bool tail_fixed = false, bool tensor = false) {
   if (!(tail && keep > 0 && keep < n && n <= 4096)) {
     tail = nullptr;
     keep = 0;
@@ -1008,9 +1009,12 @@ static tn_status_t jacobi_core(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T
     std::vector<int> h_act(batch, 1), h_rot(2 * batch);
     TN_CHECK_CUDA(ctx, cudaMemcpyAsync(active, h_act.data(), sizeof(int) * batch, cudaMemcpyHostToDevice, ctx->stream));
     const int N = (int)(n + (n & 1));
-    // FP32 with V and m, n ≤ 512: block rounds (16 columns per CTA in registers)
+    // FP32 with V and m, n ≤ 512: block rounds, 16 columns per CTA in registers, or 32 columns
+    // per CTA on the tensor pipe (`tensor`: a pre-pass whose residue an FP64 stage removes)
     const bool blocked = sizeof(T) == 4 && V && m <= 512 && n <= 512 && n >= 32;
-    const int NB0 = (int)((n + 7) / 8), NB = NB0 + (NB0 & 1);
+    const bool on_tensor = blocked && tensor && n >= kTensorMinN && jacobi_block_tc_fits(m, n);
+    const int bw = on_tensor ? 16 : 8;
+    const int NB0 = (int)((n + bw - 1) / bw), NB = NB0 + (NB0 & 1);
     const int rounds = blocked ? NB - 1 : N - 1;
     // A sweep whose largest off-diagonal ratio is ρ leaves ~ρ² for the next one
     // (one-sided Jacobi converges quadratically); when ρ² is below tol/10 the next
@@ -1018,8 +1022,8 @@ static tn_status_t jacobi_core(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T
     const double stop_ratio = sqrt((double)tol * 1e-1);
     // graph for one sweep
     char key[256];
-    snprintf(key, sizeof(key), "jac%zu:%lld:%lld:%lld:%p:%p:%p:%p:%p:%p", sizeof(T), (long long)m, (long long)n,
-             (long long)batch, (void*)W, (void*)V, (void*)nrm, (void*)active, (void*)rotated, (void*)tail);
+    snprintf(key, sizeof(key), "jac%zu%s:%lld:%lld:%lld:%p:%p:%p:%p:%p:%p", sizeof(T), on_tensor ? "t" : "",
+             (long long)m, (long long)n, (long long)batch, (void*)W, (void*)V, (void*)nrm, (void*)active, (void*)rotated, (void*)tail);
     cudaGraphExec_t ge = nullptr;
     auto it = ctx->graphs.find(key);
     if (it != ctx->graphs.end()) {
@@ -1039,7 +1043,11 @@ static tn_status_t jacobi_core(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T
       if constexpr (sizeof(T) == 4) {
         if (blocked) {
           const dim3 grid((unsigned)(NB / 2), gy);
-          for (int r = 0; r < NB - 1; ++r) {
+          for (int r = 0; r < NB - 1 && st == TN_OK; ++r) {
+            if (on_tensor) {
+              st = jacobi_block_tc(ctx, ctx->stream, m, n, NB, r, W, V, nrm, active, rotated, tol, batch, tail);
+              continue;
+            }
             if (m <= 128 && n <= 128)
               k_jacobi_block_f32<64><<<grid, 64, 0, ctx->stream>>>(m, n, NB, r, W, V, nrm, active, rotated, tol, tail);
             else if (m <= 256 && n <= 256)
@@ -1284,10 +1292,26 @@ __global__ void k_d2f(int64_t count, const cxd* __restrict__ a, int64_t lda, int
     b[t] = mkcx<float>((float)v.x, (float)v.y);
   }
 }
-__global__ void k_f2d(int64_t count, const cxf* __restrict__ a, cxd* __restrict__ b) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < count; t += (int64_t)gridDim.x * blockDim.x) {
-    cxf v = a[t];
-    b[t] = mkcx<double>(v.x, v.y);
+// b = a in FP64 with every column (n rows) scaled to unit length: the pre-pass's rounding moves
+// the lengths of V's columns most (TF32 products accumulate towards zero), and what the FP64
+// stages do about V's unitarity is a series in its deviation.  The scaled entries are rounded
+// to FP32 again: products of 24-bit entries are exact in the split-BF16 GEMM that forms VᴴV.
+// One warp per column.
+__global__ void k_lift_unit(int64_t n, int64_t columns, const cxf* __restrict__ a, cxd* __restrict__ b) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w < columns; w += warps) {
+    double s = 0.0;
+    for (int64_t t = lane; t < n; t += 32) {
+      const cxf v = a[w * n + t];
+      s = fma((double)v.x, (double)v.x, fma((double)v.y, (double)v.y, s));
+    }
+    s = warp_sum(s);
+    const double f = s > 0.0 ? rsqrt(s) : 1.0;
+    for (int64_t t = lane; t < n; t += 32) {
+      const cxf v = a[w * n + t];
+      b[w * n + t] = mkcx<double>((double)(float)(f * v.x), (double)(float)(f * v.y));
+    }
   }
 }
 
@@ -1354,7 +1378,7 @@ inline double refine_noise(int slices) { return std::max(kRefineNoise, 32.0 * sl
 inline double refine_gapmin(double noise) { return std::max(kRefineGapMin, 1e4 * noise); }
 constexpr float kRefineStop = 1e-8f;
 constexpr double kRefineNormMax = 0.5;  // ‖E‖_F above which the first-order steps diverge
-constexpr int kRefineMaxIter = 6;
+constexpr int kRefineMaxIter = 7;
 
 __global__ void k_set_identity_cxd(int64_t n, int64_t batch, cxd* X) {
   const int64_t total = n * n * batch;
@@ -1633,7 +1657,7 @@ tn_status_t svd_tall_mixed(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int6
   // FP32 pre-pass, stopped once a sweep rotates ≤ 5 % of the pairs (the FP64 phase removes
   // the residue)
   TN_RETURN_IF(jacobi_core<float>(ctx, m, n, W32, V32, batch, false, active, rotated, nrm32, kMaxSweeps, nullptr, &noconv,
-                                  (keep_m > 0 && keep_m < n) ? tail : nullptr, keep_m, false, 0.05));
+                                  (keep_m > 0 && keep_m < n) ? tail : nullptr, keep_m, false, 0.05, false, true));
   if (keep_m > 0 && keep_m < n) {
     // rank the columns by their FP32 norms (the pre-pass left them nearly orthogonal)
     int64_t nb = std::min<int64_t>((n * batch * 32 + 255) / 256, (int64_t)ctx->num_sms * 8);
@@ -1642,9 +1666,7 @@ tn_status_t svd_tall_mixed(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int6
     TN_RETURN_IF(update_tail_flags<float>(ctx, n, batch, nrm32, keep_m, tail));
   }
   {
-    int64_t cnt = n * n * batch;
-    int64_t blocks = std::min<int64_t>((cnt + 255) / 256, 4096);
-    k_f2d<<<(unsigned)blocks, 256, 0, ctx->stream>>>(cnt, V32, V64);
+    k_lift_unit<<<cdiv(n * batch, 8), 256, 0, ctx->stream>>>(n, n * batch, V32, V64);
     TN_LAUNCHED(ctx);
   }
   if (keep_m > 0 && keep_m < n) {
@@ -1729,7 +1751,7 @@ tn_status_t svd_tall_mixed(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int6
       // outside the quadratic regime (a basis the FP32 pre-pass could not resolve, e.g.
       // values below ~1e-7 of the largest inside the kept set): the first-order steps
       // would not converge, so the FP64 sweeps take over from the pre-pass basis
-      if (!finite || enorm > kRefineNormMax || rmax > 0.25f || (it >= 3 && emax > 1e-3f)) {
+      if (!finite || enorm > kRefineNormMax || rmax > 0.25f || (it >= 4 && emax > 1e-3f)) {
         diverged = true;
         break;
       }
@@ -1763,8 +1785,7 @@ tn_status_t svd_tall_mixed(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int6
     if (!converged) {
       if (diverged) {
         // back to the pre-pass basis
-        const int64_t cnt = n * n * batch;
-        k_f2d<<<(unsigned)std::min<int64_t>((cnt + 255) / 256, 4096), 256, 0, ctx->stream>>>(cnt, V32, V64);
+        k_lift_unit<<<cdiv(n * batch, 8), 256, 0, ctx->stream>>>(n, n * batch, V32, V64);
         TN_LAUNCHED(ctx);
       }
       // restore V's unitarity (V ← V + V·R/2, quadratic: the pre-pass leaves R ~ 1e-4)
