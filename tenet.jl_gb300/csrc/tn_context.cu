@@ -20,16 +20,56 @@ tn_status_t tn_set_error(tn_ctx* ctx, tn_status_t st, const char* fmt, ...) {
   return st;
 }
 
+// most bytes of freed blocks a context keeps
+constexpr size_t kPoolBytes = size_t(4) << 30;
+
+namespace {
+
+// gives pooled blocks back to the driver, oldest first, until at most `keep` bytes are pooled
+cudaError_t pool_shrink(tn_ctx* ctx, size_t keep) {
+  while (ctx->pool_bytes > keep && !ctx->pool.empty()) {
+    auto oldest = ctx->pool.begin();
+    for (auto it = ctx->pool.begin(); it != ctx->pool.end(); ++it)
+      if (it->second.age < oldest->second.age) oldest = it;
+    void* p = oldest->second.p;
+    ctx->pool_bytes -= oldest->first;
+    ctx->pool.erase(oldest);
+    ctx->capacity.erase(p);
+    const cudaError_t e = cudaFree(p);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace
+
 tn_status_t tn_dev_alloc(tn_ctx* ctx, size_t bytes, void** p) {
   if (bytes == 0) bytes = 256;
   if (ctx->budget && ctx->in_use + bytes > ctx->budget)
     return tn_set_error(ctx, TN_ENOMEM, "HBM budget exceeded: %zu in use + %zu > %zu",
                         ctx->in_use, bytes, ctx->budget);
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return tn_set_error(ctx, TN_ENOMEM, "cudaMalloc(%zu) failed: %s", bytes,
-                        cudaGetErrorString(e));
+  // the smallest pooled block that holds it with at most a quarter to spare
+  auto it = ctx->pool.lower_bound(bytes);
+  if (it != ctx->pool.end() && it->first <= bytes + bytes / 4 + 4096 &&
+      (!ctx->budget || ctx->in_use + ctx->pool_bytes <= ctx->budget)) {
+    *p = it->second.p;
+    ctx->pool_bytes -= it->first;
+    ctx->pool.erase(it);
+  } else {
+    if (ctx->budget && ctx->in_use + ctx->pool_bytes + bytes > ctx->budget)
+      TN_CHECK_CUDA(ctx, pool_shrink(ctx, ctx->budget - ctx->in_use - bytes));
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess && !ctx->pool.empty()) {
+      cudaGetLastError();
+      TN_CHECK_CUDA(ctx, pool_shrink(ctx, 0));
+      e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return tn_set_error(ctx, TN_ENOMEM, "cudaMalloc(%zu) failed: %s", bytes,
+                          cudaGetErrorString(e));
+    }
+    ctx->capacity[*p] = bytes;
   }
   ctx->allocs[*p] = bytes;
   ctx->in_use += bytes;
@@ -43,7 +83,23 @@ tn_status_t tn_dev_free(tn_ctx* ctx, void* p) {
     return tn_set_error(ctx, TN_EINVAL, "tn_free: pointer %p not allocated by this context", p);
   ctx->in_use -= it->second;
   ctx->allocs.erase(it);
-  TN_CHECK_CUDA(ctx, cudaFree(p));
+  const size_t cap = ctx->capacity[p];
+  {
+    int current = ctx->device;
+    cudaGetDevice(&current);
+    if (current != ctx->device) cudaSetDevice(ctx->device);
+    const cudaError_t e = cudaDeviceSynchronize();
+    if (current != ctx->device) cudaSetDevice(current);
+    TN_CHECK_CUDA(ctx, e);
+  }
+  if (cap > kPoolBytes) {
+    ctx->capacity.erase(p);
+    TN_CHECK_CUDA(ctx, cudaFree(p));
+    return TN_OK;
+  }
+  ctx->pool.emplace(cap, tn_ctx::pool_block{p, ctx->pool_age++});
+  ctx->pool_bytes += cap;
+  TN_CHECK_CUDA(ctx, pool_shrink(ctx, kPoolBytes));
   return TN_OK;
 }
 
@@ -159,7 +215,9 @@ void ctx_release(tn_ctx* ctx) {
     cudaEventDestroy(r.b);
   }
   for (cudaEvent_t e : ctx->prof_pool) cudaEventDestroy(e);
-  for (auto& kv : ctx->allocs) cudaFree(kv.first);
+  for (auto& kv : ctx->capacity) cudaFree(kv.first);  // live and pooled blocks
+  ctx->capacity.clear();
+  ctx->pool.clear();
   ctx->allocs.clear();
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
@@ -229,6 +287,7 @@ tn_status_t tn_memcpy_d2d(tn_ctx* ctx, void* dst, const void* src, size_t bytes)
 tn_status_t tn_set_hbm_budget(tn_ctx* ctx, size_t bytes) {
   if (!ctx) return TN_EINVAL;
   ctx->budget = bytes;
+  if (bytes) TN_CHECK_CUDA(ctx, pool_shrink(ctx, bytes > ctx->in_use ? bytes - ctx->in_use : 0));
   return TN_OK;
 }
 

@@ -72,7 +72,7 @@ def test_mixed_svd(ctx, m, n, batch):
     _check(A, *_svd(ctx, A, 1), 1e-12)
 
 
-@pytest.mark.parametrize("m,n", [(64, 64), (100, 60), (200, 200)])
+@pytest.mark.parametrize("m,n", [(32, 32), (100, 40)])
 @pytest.mark.parametrize("scale", [1.0, 1e-130, 1e130])
 def test_columns_of_different_scale(ctx, m, n, scale):
     """A·D with D over twelve decades, unsorted: one-sided Jacobi finds the small values to their
