@@ -23,6 +23,33 @@ int find(const int32_t* modes, int r, int32_t m) {
   return -1;
 }
 
+// The index formed by `modes` of t (first fastest) as a two-level view of t's memory; false
+// when its modes fuse into more than two runs.
+bool index_view(const tn_tensor* t, const std::vector<int>& modes, IndexView* out) {
+  int64_t stride[TN_MAX_RANK], s = 1;
+  for (int i = 0; i < t->rank; ++i) {
+    stride[i] = s;
+    s *= t->dims[i];
+  }
+  int64_t ext[2] = {1, 1}, str[2] = {1, 0};
+  int runs = 0;
+  for (int i : modes) {
+    if (t->dims[i] == 1) continue;
+    if (runs > 0 && stride[i] == str[runs - 1] * ext[runs - 1]) {
+      ext[runs - 1] *= t->dims[i];
+      continue;
+    }
+    if (runs == 2) return false;
+    ext[runs] = t->dims[i];
+    str[runs++] = stride[i];
+  }
+  if (runs == 2 && ext[0] * ext[1] > 0x7fffffff) return false;
+  out->extent = ext[0];
+  out->inner = str[0];
+  out->outer = runs == 2 ? str[1] : 0;
+  return true;
+}
+
 bool is_identity(const std::vector<int32_t>& p) {
   for (size_t i = 0; i < p.size(); ++i)
     if (p[i] != (int32_t)i) return false;
@@ -116,6 +143,18 @@ extern "C" tn_status_t tn_contract(tn_ctx* ctx, tn_dtype_t dtype, tn_precision_t
   std::vector<int32_t> pc(c->rank);
   for (int i = 0; i < c->rank; ++i) pc[i] = find(out_modes.data(), (int)out_modes.size(), c->modes[i]);
   const bool perm_c = !is_identity(pc);
+  // ComplexF32 products with tall outputs read their operands in place where the modes fuse into
+  // two runs each (a boundary tensor absorbing the next site of a lattice), without a permuted
+  // copy
+  if (dtype == TN_C32 && prec == TN_PREC_NATIVE && h == 1 && !perm_c && gemm_f32_views_pays(ctx, m, n, 1)) {
+    GemmView va, vb;
+    va.conj = vb.conj = false;
+    if (index_view(a, M, &va.row) && index_view(a, K, &va.col) && index_view(b, Kb, &vb.row) && index_view(b, N, &vb.col)) {
+      TN_RETURN_IF(ws_reserve(ctx, 0));
+      return gemm_f32_views(ctx, m, n, k, mkcx(1.0f, 0.0f), (const cxf*)a->data, va, 0, (const cxf*)b->data, vb, 0,
+                            mkcx(0.0f, 0.0f), (cxf*)c->data, std::max<int64_t>(m, 1), 0, 1);
+    }
+  }
   size_t need = 0;
   if (perm_a) need += ws_round(es * (size_t)(m * k * h));
   if (perm_b) need += ws_round(es * (size_t)(k * n * h));

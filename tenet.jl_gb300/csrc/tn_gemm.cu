@@ -310,6 +310,11 @@ tn_status_t gemm_cx(tn_ctx* ctx, char opa, char opb, int64_t m, int64_t n, int64
       return launch_fine<T, 4, 16>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
     return launch_fine<T, 8, 8>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
   }
+  if constexpr (sizeof(T) == 4) {
+    if (gemm_f32_views_pays(ctx, m, n, batch))
+      return gemm_f32_views(ctx, m, n, k, alpha, A, matrix_view(opa, lda), sA, B, matrix_view(opb, ldb), sB, beta, C, ldc,
+                            sC, batch);
+  }
   // a few rows against wide operands (batched amplitudes, environment rows): row tiles
   // of 8 / 16 so the DFMA work is not spent on padding
   if (m <= 8 && n >= 64)

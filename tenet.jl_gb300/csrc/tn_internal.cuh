@@ -326,6 +326,29 @@ tn_status_t gemm_cx(tn_ctx* ctx, char opa, char opb, int64_t m, int64_t n, int64
                     int64_t ldb, int64_t sB, cx<T> beta, cx<T>* C, int64_t ldc, int64_t sC,
                     int64_t batch);
 
+// an index i of a strided operand: offset (i mod extent)·inner + (i / extent)·outer, or i·inner
+// when outer is 0
+struct IndexView {
+  int64_t extent, inner, outer;
+};
+struct GemmView {
+  IndexView row, col;
+  bool conj;
+};
+// ComplexF32 GEMM on the FP32 pipe through views (tn_gemm_f32.cu)
+bool gemm_f32_views_pays(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch);
+tn_status_t gemm_f32_views(tn_ctx* ctx, int64_t m, int64_t n, int64_t k, cxf alpha, const cxf* A, const GemmView& va,
+                           int64_t sA, const cxf* B, const GemmView& vb, int64_t sB, cxf beta, cxf* C, int64_t ldc,
+                           int64_t sC, int64_t batch);
+// op(X) of a column-major matrix as a view
+inline GemmView matrix_view(char op, int64_t ld) {
+  GemmView v;
+  v.row = {0, op == 'N' ? 1 : ld, 0};
+  v.col = {0, op == 'N' ? ld : 1, 0};
+  v.conj = op == 'C';
+  return v;
+}
+
 // C = Aᴴ A (A k × n, C n × n Hermitian), batched
 template <typename T>
 tn_status_t herk_cx(tn_ctx* ctx, int64_t n, int64_t k, const cx<T>* A, int64_t lda, int64_t sA, cx<T>* C, int64_t ldc,
