@@ -146,13 +146,21 @@ extern "C" tn_status_t tn_contract(tn_ctx* ctx, tn_dtype_t dtype, tn_precision_t
   // ComplexF32 products with tall outputs read their operands in place where the modes fuse into
   // two runs each (a boundary tensor absorbing the next site of a lattice), without a permuted
   // copy
-  if (dtype == TN_C32 && prec == TN_PREC_NATIVE && h == 1 && !perm_c && gemm_f32_views_pays(ctx, m, n, 1)) {
+  if (dtype == TN_C32 && h == 1 && !perm_c) {
     GemmView va, vb;
     va.conj = vb.conj = false;
-    if (index_view(a, M, &va.row) && index_view(a, K, &va.col) && index_view(b, Kb, &vb.row) && index_view(b, N, &vb.col)) {
+    const bool views =
+        index_view(a, M, &va.row) && index_view(a, K, &va.col) && index_view(b, Kb, &vb.row) && index_view(b, N, &vb.col);
+    const bool tensor = gemm_on_tensor_pipe(dtype, prec, m, n, k);
+    if (views && !tensor && gemm_f32_views_pays(ctx, m, n, 1)) {
       TN_RETURN_IF(ws_reserve(ctx, 0));
       return gemm_f32_views(ctx, m, n, k, mkcx(1.0f, 0.0f), (const cxf*)a->data, va, 0, (const cxf*)b->data, vb, 0,
                             mkcx(0.0f, 0.0f), (cxf*)c->data, std::max<int64_t>(m, 1), 0, 1);
+    }
+    if (views && tensor && tc_gemm_tall_fits(ctx, m, n, k, va)) {
+      TN_RETURN_IF(ws_reserve(ctx, 0));
+      return tc_gemm_tall(ctx, prec == TN_PREC_TF32 ? 1 : 3, m, n, k, 1.0f, (const cxf*)a->data, va, (const cxf*)b->data, vb,
+                          0.0f, (cxf*)c->data, std::max<int64_t>(m, 1));
     }
   }
   size_t need = 0;

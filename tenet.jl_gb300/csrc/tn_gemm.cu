@@ -431,12 +431,12 @@ static bool valid_op(char c) { return c == 'N' || c == 'T' || c == 'C'; }
 // The tensor path pays an operand-preparation pass (split + 4M expansion) and 128×128
 // tiles; skinny GEMMs (any of m, n < 64 or k < 32) are HBM-bound and stay on the FP32
 // CUDA cores, which are also the more accurate choice.
-static bool use_tensor_path(tn_dtype_t dt, tn_precision_t prec, int64_t m, int64_t n, int64_t k) {
+bool gemm_on_tensor_pipe(tn_dtype_t dt, tn_precision_t prec, int64_t m, int64_t n, int64_t k) {
   return (dt == TN_C32 || dt == TN_F32) && prec != TN_PREC_NATIVE && m >= 64 && n >= 64 && k >= 32;
 }
 
 size_t gemm_any_workspace(tn_dtype_t dt, tn_precision_t prec, int64_t m, int64_t n, int64_t k) {
-  if (use_tensor_path(dt, prec, m, n, k)) return tc_gemm_workspace(dt == TN_C32, prec == TN_PREC_TF32 ? 1 : 3, m, n, k);
+  if (gemm_on_tensor_pipe(dt, prec, m, n, k)) return tc_gemm_workspace(dt == TN_C32, prec == TN_PREC_TF32 ? 1 : 3, m, n, k);
   return 0;
 }
 
@@ -444,13 +444,20 @@ tn_status_t gemm_any(tn_ctx* ctx, tn_dtype_t dtype, tn_precision_t prec, char op
                      int64_t k, const double* alpha, const void* A, int64_t lda, int64_t strideA, const void* B,
                      int64_t ldb, int64_t strideB, const double* beta, void* C, int64_t ldc, int64_t strideC,
                      int64_t batch) {
-  const bool tc = use_tensor_path(dtype, prec, m, n, k);
+  const bool tc = gemm_on_tensor_pipe(dtype, prec, m, n, k);
   if (tc) {
     if (dtype == TN_C32 && (alpha[1] != 0.0 || beta[1] != 0.0))
       return tn_set_error(ctx, TN_EUNSUPPORTED, "tensor-core GEMM: complex alpha/beta not supported");
     const int passes = prec == TN_PREC_TF32 ? 1 : 3;
     const size_t es = dtype == TN_C32 ? 8 : 4;
     const size_t top = ctx->ws_top;
+    const GemmView va = matrix_view(opa, lda), vb = matrix_view(opb, ldb);
+    if (dtype == TN_C32 && tc_gemm_tall_fits(ctx, m, n, k, va)) {
+      for (int64_t b = 0; b < batch; ++b)
+        TN_RETURN_IF(tc_gemm_tall(ctx, passes, m, n, k, (float)alpha[0], (const cxf*)A + b * strideA, va,
+                                  (const cxf*)B + b * strideB, vb, (float)beta[0], (cxf*)C + b * strideC, ldc));
+      return TN_OK;
+    }
     for (int64_t b = 0; b < batch; ++b) {
       ctx->ws_top = top;
       TN_RETURN_IF(tc_gemm(ctx, dtype == TN_C32, passes, opa, opb, m, n, k, (float)alpha[0],

@@ -25,6 +25,7 @@
 // word, skips the remaining work, and still releases its TMEM.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "tn_internal.cuh"
@@ -225,6 +226,247 @@ __global__ void __launch_bounds__(128, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tcols) : "memory");
+}
+
+// ---------------------------------------------------------------------------------
+// tall complex products with a short contraction (k ≤ 64): C[m, n] = α Σ_k A[m, k]·B[k, n] + β C
+//
+// Bound: HBM.  The general path expands A fourfold (the 4M form's two row blocks, hi and lo)
+// in a pass of its own and reads it back; for a lattice's boundary tensor (2²⁴ entries, k = n =
+// 64) that is 1 GB beside the product's own 0.27 GB.  Here A is read once, through a strided
+// view, and split on the way into shared memory; the real form doubles B's columns instead
+// of A's rows:  [Re C | Im C] = [Re A | Im A] · [[Br, Bi], [−Bi, Br]].
+// A CTA keeps its 64 columns of B (128 real ones, hi and lo, 128 KB) for all its row tiles.
+// 8 producer warps load 128 rows × 16 k (two stages ahead in registers), split them and write
+// the K-major 128-byte-swizzled tiles of a two-slot ring; one thread issues tcgen05.mma
+// (M = 128, N = 128, K = 8: hi·hi in one TMEM accumulator, lo·hi and hi·lo in another, as the
+// general kernel); 4 epilogue warps drain one pair of accumulators while the next fills.
+// Every mbarrier wait is bounded (error word, the remaining work is skipped, TMEM released).
+// ---------------------------------------------------------------------------------
+constexpr int TALL_KT = 4;                       // K tiles of 16 complex (32 real) entries
+constexpr int TALL_THREADS = 13 * 32;            // 8 producer, 4 epilogue, 1 issuing warp
+constexpr int TALL_TILE = 128 * 128;             // bytes of a 128-row tile
+constexpr int TALL_SMEM = 2 * TALL_KT * TALL_TILE + 2 * 2 * TALL_TILE + 1024 + 256;
+constexpr long long kTallSpin = 1ll << 24;
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool tall_wait(uint64_t* bar, uint32_t parity, int* err);
+// one lane waits for its warp, so that the warp's lanes go on or give up together
+__device__ __forceinline__ bool tall_wait_warp(uint64_t* bar, uint32_t parity, int* err) {
+  int ok = 1;
+  if ((threadIdx.x & 31) == 0) ok = tall_wait(bar, parity, err);
+  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+__device__ __forceinline__ bool tall_wait(uint64_t* bar, uint32_t parity, int* err) {
+  for (long long i = 0; i < kTallSpin; ++i)
+    if (mbar_try_wait(bar, parity)) return true;
+  atomicExch(err, 1);
+  return false;
+}
+// x rounded to the nearest TF32 value, ties away from zero
+__device__ __forceinline__ float to_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return __uint_as_float(r);
+}
+// byte offset of element (row, j) of a K-major tile of 32 floats per row, 128-byte swizzle
+__device__ __forceinline__ uint32_t tall_at(int row, int j) {
+  return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((j * 4) ^ ((row & 7) << 4)));
+}
+__device__ __forceinline__ int64_t view_offset(const IndexView& v, int64_t i) {
+  if (v.outer == 0) return i * v.inner;
+  const unsigned n = (unsigned)v.extent, q = (unsigned)i / n;
+  return (int64_t)((unsigned)i - q * n) * v.inner + (int64_t)q * v.outer;
+}
+constexpr uint32_t kIdescTall = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+__device__ __forceinline__ void mma_tall(uint32_t d, uint64_t a, uint64_t b, uint32_t accum) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+               "l"(a), "l"(b), "r"(kIdescTall), "r"(accum)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+  uint32_t r[16];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+}
+
+// grid: (CTAs per column block, column blocks of 64)
+__global__ void __launch_bounds__(TALL_THREADS, 1)
+    k_gemm_tf32_tall(int64_t m, int64_t n, int k, int passes, const cxf* __restrict__ A, GemmView va, const cxf* __restrict__ B,
+                     GemmView vb, float alpha, float beta, cxf* __restrict__ C, int64_t ldc, int* err) {
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t base_u = smem_u32(smem_raw);
+  unsigned char* smem = smem_raw + ((1024 - (base_u & 1023)) & 1023);
+  unsigned char* sB = smem;                                    // hi: KT tiles, lo: KT tiles
+  unsigned char* sA = smem + 2 * TALL_KT * TALL_TILE;          // 2 slots × (hi, lo)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sA + 4 * TALL_TILE);
+  uint64_t *full = bars, *empty = bars + 2, *tfull = bars + 4, *tempty = bars + 6;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 8);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t j0 = (int64_t)blockIdx.y * 64, tiles = (m + 127) / 128;
+  const int KT = (k + 15) / 16;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 32) {
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&full[s], 8);
+      mbar_init(&empty[s], 1);
+      mbar_init(&tfull[s], 1);
+      mbar_init(&tempty[s], 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // B's real form, rows c (Re C) and 64 + c (Im C); K tile t holds Re then Im of entries 16t…16t+15
+  for (int e = tid; e < KT * 16 * 64; e += TALL_THREADS) {
+    const int c = e & 63, kk = e >> 6;
+    cxf b = mkcx<float>(0.f, 0.f);
+    if (kk < k && j0 + c < n) b = B[view_offset(vb.row, kk) + view_offset(vb.col, j0 + c)];
+    if (vb.conj) b.y = -b.y;
+    const float v[4] = {b.x, -b.y, b.y, b.x};  // (Re row, Re k), (Re row, Im k), (Im row, Re k), (Im row, Im k)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t at = (uint32_t)(kk >> 4) * TALL_TILE + tall_at(c + (q >> 1) * 64, (kk & 15) + (q & 1) * 16);
+      const float h = to_tf32(v[q]);
+      *reinterpret_cast<float*>(sB + at) = h;
+      *reinterpret_cast<float*>(sB + TALL_KT * TALL_TILE + at) = v[q] - h;
+    }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tslot;
+
+  if (warp < 8) {
+    // producers: thread = (row of the tile, 8 of the stage's 16 entries)
+    const int row = tid & 127, hf = tid >> 7;
+    const int64_t stages = tiles > (int64_t)blockIdx.x ? ((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x) * KT : 0;
+    cxf r[2][8];
+    auto fetch = [&](int64_t st, cxf* v) {
+      const int64_t i = (blockIdx.x + (st / KT) * gridDim.x) * 128 + row;
+      const int k0 = (int)(st % KT) * 16 + hf * 8;
+      const cxf* p = A + (i < m ? view_offset(va.row, i) : 0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        v[j] = (i < m && k0 + j < k) ? p[view_offset(va.col, k0 + j)] : mkcx<float>(0.f, 0.f);
+    };
+    if (stages > 0) fetch(0, r[0]);
+    if (stages > 1) fetch(1, r[1]);
+    bool ok = true;
+    for (int64_t st = 0; st < stages && ok; st += 2) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (st + u >= stages) break;
+        const int64_t g = st + u;
+        const int slot = u;  // g mod 2
+        if (g >= 2 && !(ok = tall_wait_warp(&empty[slot], (uint32_t)(((g >> 1) & 1) ^ 1), err))) break;
+        unsigned char* hi = sA + slot * 2 * TALL_TILE;
+        unsigned char* lo = hi + TALL_TILE;
+#pragma unroll
+        for (int part = 0; part < 2; ++part)
+#pragma unroll
+          for (int q = 0; q < 8; q += 4) {
+            float x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = part ? (va.conj ? -r[u][q + j].y : r[u][q + j].y) : r[u][q + j].x;
+            const uint32_t at = tall_at(row, part * 16 + hf * 8 + q);
+            const float4 h = make_float4(to_tf32(x[0]), to_tf32(x[1]), to_tf32(x[2]), to_tf32(x[3]));
+            *reinterpret_cast<float4*>(hi + at) = h;
+            if (passes > 1) *reinterpret_cast<float4*>(lo + at) = make_float4(x[0] - h.x, x[1] - h.y, x[2] - h.z, x[3] - h.w);
+          }
+        if (g + 2 < stages) fetch(g + 2, r[u]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[slot]);
+      }
+    }
+  } else if (warp == 12) {
+    if (lane == 0) {
+      int64_t g = 0, it = 0;
+      bool ok = true;
+      for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++it) {
+        const int ab = (int)(it & 1);
+        if (it >= 2 && !(ok = tall_wait(&tempty[ab], (uint32_t)(((it >> 1) & 1) ^ 1), err))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t d = tmem + (uint32_t)(ab * 256);
+        for (int kt = 0; kt < KT; ++kt, ++g) {
+          const int slot = (int)(g & 1);
+          if (!(ok = tall_wait(&full[slot], (uint32_t)((g >> 1) & 1), err))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint64_t ah = sdesc(sA + slot * 2 * TALL_TILE), al = sdesc(sA + slot * 2 * TALL_TILE + TALL_TILE);
+          const uint64_t bh = sdesc(sB + kt * TALL_TILE), bl = sdesc(sB + (TALL_KT + kt) * TALL_TILE);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) mma_tall(d, ah + 2 * q, bh + 2 * q, (kt > 0 || q > 0) ? 1u : 0u);
+          if (passes > 1) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) mma_tall(d + 128, al + 2 * q, bh + 2 * q, (kt > 0 || q > 0) ? 1u : 0u);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) mma_tall(d + 128, ah + 2 * q, bl + 2 * q, 1u);
+          }
+          mma_commit(&empty[slot]);
+        }
+        if (ok) mma_commit(&tfull[ab]);
+      }
+    }
+  } else {
+    // epilogue: warps 8-11, TMEM lanes 32·(warp mod 4)…
+    const uint32_t tl = (uint32_t)((warp & 3) * 32) << 16;
+    int64_t it = 0;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+      const int ab = (int)(it & 1);
+      if (!tall_wait_warp(&tfull[ab], (uint32_t)((it >> 1) & 1), err)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int64_t i = tile * 128 + (warp & 3) * 32 + lane;
+      const uint32_t d = tmem + tl + (uint32_t)(ab * 256);
+#pragma unroll 1
+      for (int c0 = 0; c0 < 64; c0 += 16) {
+        if (j0 + c0 >= n) break;
+        float re[16], im[16];
+        tmem_ld16(d + c0, re);
+        tmem_ld16(d + 64 + c0, im);
+        if (passes > 1) {
+          float q[16];
+          tmem_ld16(d + 128 + c0, q);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) re[j] += q[j];
+          tmem_ld16(d + 192 + c0, q);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) im[j] += q[j];
+        }
+        if (i < m) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (j0 + c0 + j >= n) break;
+            cxf* dst = C + i + (j0 + c0 + j) * ldc;
+            cxf v = mkcx<float>(alpha * re[j], alpha * im[j]);
+            if (beta != 0.f) {
+              v.x += beta * dst->x;
+              v.y += beta * dst->y;
+            }
+            *dst = v;
+          }
+        }
+        __syncwarp();
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[ab]);
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
 // ---------------------------------------------------------------------------------
@@ -449,5 +691,26 @@ tn_status_t tc_gemm(tn_ctx* ctx, bool complex_in, int passes, char opa, char opb
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(hp, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (hp[0]) return tn_set_error(ctx, TN_ETIMEOUT, "tc_gemm: a pipeline wait timed out");
+  return TN_OK;
+}
+
+// Tall products with k ≤ 64 whose rows are contiguous in A: at least one 128-row tile per SM for
+// every column block of 64, and enough contraction and columns that the tensor pipe pays
+// (the general path's own bounds).
+bool tc_gemm_tall_fits(tn_ctx* ctx, int64_t m, int64_t n, int64_t k, const GemmView& va) {
+  return k >= 32 && k <= 16 * TALL_KT && n >= 48 && va.row.inner == 1 &&
+         (va.row.outer == 0 || va.row.extent >= 32) && (m + 127) / 128 * ((n + 63) / 64) >= ctx->num_sms && (n + 63) / 64 <= 65535;
+}
+
+tn_status_t tc_gemm_tall(tn_ctx* ctx, int passes, int64_t m, int64_t n, int64_t k, float alpha, const cxf* A,
+                         const GemmView& va, const cxf* B, const GemmView& vb, float beta, cxf* C, int64_t ldc) {
+  int* err = nullptr;
+  TN_RETURN_IF(wait_error_word(ctx, &err));
+  const int64_t blocks = (n + 63) / 64, tiles = (m + 127) / 128;
+  const int64_t gx = std::min<int64_t>(tiles, std::max<int64_t>(1, ctx->num_sms / blocks));
+  TN_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tf32_tall, cudaFuncAttributeMaxDynamicSharedMemorySize, TALL_SMEM));
+  k_gemm_tf32_tall<<<dim3((unsigned)gx, (unsigned)blocks), TALL_THREADS, TALL_SMEM, ctx->stream>>>(
+      m, n, (int)k, passes, A, va, B, vb, alpha, beta, C, ldc, err);
+  TN_LAUNCHED(ctx);
   return TN_OK;
 }

@@ -340,6 +340,12 @@ bool gemm_f32_views_pays(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch);
 tn_status_t gemm_f32_views(tn_ctx* ctx, int64_t m, int64_t n, int64_t k, cxf alpha, const cxf* A, const GemmView& va,
                            int64_t sA, const cxf* B, const GemmView& vb, int64_t sB, cxf beta, cxf* C, int64_t ldc,
                            int64_t sC, int64_t batch);
+// whether gemm_any takes a 32-bit product to the TF32 tensor pipe
+bool gemm_on_tensor_pipe(tn_dtype_t dt, tn_precision_t prec, int64_t m, int64_t n, int64_t k);
+// tall ComplexF32 products with a short contraction on the TF32 tensor pipe (tn_gemm_tc.cu)
+bool tc_gemm_tall_fits(tn_ctx* ctx, int64_t m, int64_t n, int64_t k, const GemmView& va);
+tn_status_t tc_gemm_tall(tn_ctx* ctx, int passes, int64_t m, int64_t n, int64_t k, float alpha, const cxf* A,
+                         const GemmView& va, const cxf* B, const GemmView& vb, float beta, cxf* C, int64_t ldc);
 // op(X) of a column-major matrix as a view
 inline GemmView matrix_view(char op, int64_t ld) {
   GemmView v;

@@ -45,3 +45,27 @@ def test_contraction_through_views(la, da, lb, db, con, precision):
     u = 2.0**-24
     rel = {"native": 2 * (4 * k + 8) * u, "mixed": 16 * 2 * (4 * k + 8) * u, "tf32": 2.0**-9 + 2 * (4 * k + 8) * u}[precision]
     assert (np.abs(got.numpy() - ref) <= rel * mag).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(20000, 64, 64), (19457, 49, 49), (30000, 100, 33), (9800, 130, 40), (128 * 152, 64, 32)])
+@pytest.mark.parametrize("precision", ["mixed", "tf32"])
+def test_tall_tensor_pipe_products(m, n, k, precision):
+    """The tall TF32 kernel at ragged rows, columns and contraction lengths, with alpha and beta."""
+    import ctypes as C
+
+    import tenetgb
+
+    ctx = tenetgb.default_context()
+    rng = np.random.default_rng(m + n + k)
+    g = lambda *s: (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)
+    A, B, C0 = g(m, k), g(n, k), g(m, n)
+    dA, dB, dC = (tenetgb.DeviceTensor.from_numpy(ctx, x) for x in (A, B, C0))
+    al, be = (C.c_double * 2)(0.5, 0), (C.c_double * 2)(-0.25, 0)
+    code = tenetgb.core.precision_code(precision)
+    ctx.check(ctx.lib.tn_gemm(ctx.h, 2, code, b"N", b"C", m, n, k, al, C.c_void_p(dA.ptr), m, 0, C.c_void_p(dB.ptr), n, 0, be,
+                              C.c_void_p(dC.ptr), m, 0, 1))
+    ref = 0.5 * A.astype(complex) @ B.astype(complex).conj().T - 0.25 * C0
+    mag = 0.5 * np.abs(A).astype(float) @ np.abs(B).astype(float).T + 0.25 * np.abs(C0)
+    u = 2.0**-24
+    rel = {"mixed": 32 * (4 * k + 8) * u, "tf32": 2.0**-9 + 2 * (4 * k + 8) * u}[precision]
+    assert (np.abs(dC.numpy() - ref) <= rel * mag).all()
