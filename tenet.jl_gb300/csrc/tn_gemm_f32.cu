@@ -5,7 +5,8 @@
 //
 // Bound: FP32 issue.  A 64×64 tile with 4×4 outputs per thread (k_gemm_cx) spends as many
 // instructions on shared-memory loads and scalar FMAs as the pipe has slots; here a thread
-// holds 8×4 outputs of a 128×64 tile, rows in pairs, so one fma.rn.f32x2 does two rows, operands
+// holds 8×8 outputs of a 128×64 tile (with 8×4 the shared-memory loads took as long as the
+// FMAs), rows in pairs, so one fma.rn.f32x2 does two rows, operands
 // sit in shared memory as the instruction wants them (A split into Re and Im planes, B's
 // parts doubled), and the next stage of K is fetched to registers under the current one.
 // A view maps an index to an offset by two levels (inner extent, inner and outer stride), so
@@ -32,7 +33,8 @@ __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
   return r;
 }
 
-constexpr int BM = 128, BN = 64, BK = 8, NT = 256;
+constexpr int BM = 128, BN = 64, BK = 8, NT = 128;
+constexpr int LA = BM * BK / NT, LB = BN * BK / NT;  // entries a thread stages
 
 __device__ __forceinline__ int64_t at(const IndexView& v, int64_t i) {
   if (v.outer == 0) return i * v.inner;
@@ -46,55 +48,55 @@ __global__ void __launch_bounds__(NT, 2)
                      int64_t sC, int64_t batch) {
   __shared__ __align__(16) float Ar[2][BK][BM], Ai[2][BK][BM];
   __shared__ float4 Bs[2][BK][BN];  // (Re, Re, Im, Im)
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
   const int64_t i0 = (int64_t)blockIdx.x * BM, j0 = (int64_t)blockIdx.y * BN;
   // staging: along the index that is contiguous in memory
   const bool a_rows = va.row.inner == 1, b_cols = vb.col.inner == 1 && vb.row.inner != 1;
   for (int64_t bz = blockIdx.z; bz < batch; bz += gridDim.z) {
     const cxf* Ab = A + bz * sA;
     const cxf* Bb = B + bz * sB;
-    int ai[4], ap[4], bp[2], bj[2];
-    int64_t ao[4], bo[2];
+    int64_t ao[LA], bo[LB];
+    auto a_i = [&](int u) { return a_rows ? tid : tid / BK + u * (NT / BK); };
+    auto a_p = [&](int u) { return a_rows ? u : tid % BK; };
+    auto b_j = [&](int u) { return b_cols ? tid % BN : tid / BK + u * (NT / BK); };
+    auto b_p = [&](int u) { return b_cols ? tid / BN + u * (NT / BN) : tid % BK; };
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int t = tid + u * NT;
-      ai[u] = a_rows ? t % BM : t / BK;
-      ap[u] = a_rows ? t / BM : t % BK;
-      ao[u] = i0 + ai[u] < m ? at(va.row, i0 + ai[u]) : -1;
-    }
+    for (int u = 0; u < LA; ++u) ao[u] = i0 + a_i(u) < m ? at(va.row, i0 + a_i(u)) : -1;  // (one value when a_rows)
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int t = tid + u * NT;
-      bj[u] = b_cols ? t % BN : t / BK;
-      bp[u] = b_cols ? t / BN : t % BK;
-      bo[u] = j0 + bj[u] < n ? at(vb.col, j0 + bj[u]) : -1;
-    }
-    cxf ra[4], rb[2];
+    for (int u = 0; u < LB; ++u) bo[u] = j0 + b_j(u) < n ? at(vb.col, j0 + b_j(u)) : -1;
+    cxf ra[LA], rb[LB];
     auto fetch = [&](int64_t p0) {
+      if (a_rows) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        ra[u] = (ao[u] >= 0 && p0 + ap[u] < k) ? Ab[ao[u] + at(va.col, p0 + ap[u])] : mkcx<float>(0.f, 0.f);
+        for (int u = 0; u < LA; ++u)
+          ra[u] = (ao[0] >= 0 && p0 + u < k) ? Ab[ao[0] + at(va.col, p0 + u)] : mkcx<float>(0.f, 0.f);
+      } else {
+        const bool in = p0 + a_p(0) < k;
+        const int64_t o = in ? at(va.col, p0 + a_p(0)) : 0;
 #pragma unroll
-      for (int u = 0; u < 2; ++u)
-        rb[u] = (bo[u] >= 0 && p0 + bp[u] < k) ? Bb[bo[u] + at(vb.row, p0 + bp[u])] : mkcx<float>(0.f, 0.f);
+        for (int u = 0; u < LA; ++u) ra[u] = (in && ao[u] >= 0) ? Ab[ao[u] + o] : mkcx<float>(0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < LB; ++u)
+        rb[u] = (bo[u] >= 0 && p0 + b_p(u) < k) ? Bb[bo[u] + at(vb.row, p0 + b_p(u))] : mkcx<float>(0.f, 0.f);
     };
     auto stage = [&](int s) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        Ar[s][ap[u]][ai[u]] = ra[u].x;
-        Ai[s][ap[u]][ai[u]] = va.conj ? -ra[u].y : ra[u].y;
+      for (int u = 0; u < LA; ++u) {
+        Ar[s][a_p(u)][a_i(u)] = ra[u].x;
+        Ai[s][a_p(u)][a_i(u)] = va.conj ? -ra[u].y : ra[u].y;
       }
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < LB; ++u) {
         const float y = vb.conj ? -rb[u].y : rb[u].y;
-        Bs[s][bp[u]][bj[u]] = make_float4(rb[u].x, rb[u].x, y, y);
+        Bs[s][b_p(u)][b_j(u)] = make_float4(rb[u].x, rb[u].x, y, y);
       }
     };
-    f2 re[4][4], im[4][4];  // [row pair][column]
+    f2 re[4][8], im[4][8];  // [row pair][column]
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) re[r][c] = im[r][c] = 0ull;
+      for (int c = 0; c < 8; ++c) re[r][c] = im[r][c] = 0ull;
     if (k > 0) {
       fetch(0);
       stage(0);
@@ -120,8 +122,8 @@ __global__ void __launch_bounds__(NT, 2)
 #pragma unroll
         for (int r = 0; r < 4; ++r) an[r] = ay[r] ^ 0x8000000080000000ull;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float4 b = Bs[s][pp][tx + 16 * c];
+        for (int c = 0; c < 8; ++c) {
+          const float4 b = Bs[s][pp][tx + 8 * c];
           const f2 br = f2_pack(b.x, b.y), bi = f2_pack(b.z, b.w);
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
@@ -138,8 +140,8 @@ __global__ void __launch_bounds__(NT, 2)
     const bool beta0 = beta.x == 0.f && beta.y == 0.f;
     cxf* Cb = C + bz * sC;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int64_t gj = j0 + tx + 16 * c;
+    for (int c = 0; c < 8; ++c) {
+      const int64_t gj = j0 + tx + 8 * c;
       if (gj >= n) continue;
 #pragma unroll
       for (int r = 0; r < 4; ++r) {

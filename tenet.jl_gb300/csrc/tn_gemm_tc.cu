@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(128, 1)
 // view, and split on the way into shared memory; the real form doubles B's columns instead
 // of A's rows:  [Re C | Im C] = [Re A | Im A] · [[Br, Bi], [−Bi, Br]].
 // A CTA keeps its 64 columns of B (128 real ones, hi and lo, 128 KB) for all its row tiles.
-// 8 producer warps load 128 rows × 16 k (two stages ahead in registers), split them and write
+// 8 producer warps load 128 rows × 16 k (four stages ahead in registers), split them and write
 // the K-major 128-byte-swizzled tiles of a two-slot ring; one thread issues tcgen05.mma
 // (M = 128, N = 128, K = 8: hi·hi in one TMEM accumulator, lo·hi and hi·lo in another, as the
 // general kernel); 4 epilogue warps drain one pair of accumulators while the next fills.
@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(TALL_THREADS, 1)
     k_gemm_tf32_tall(int64_t m, int64_t n, int k, int passes, const cxf* __restrict__ A, GemmView va, const cxf* __restrict__ B,
                      GemmView vb, float alpha, float beta, cxf* __restrict__ C, int64_t ldc, int* err) {
   extern __shared__ unsigned char smem_raw[];
+  __shared__ int64_t s_koff[16 * TALL_KT];
   const uint32_t base_u = smem_u32(smem_raw);
   unsigned char* smem = smem_raw + ((1024 - (base_u & 1023)) & 1023);
   unsigned char* sB = smem;                                    // hi: KT tiles, lo: KT tiles
@@ -325,6 +326,7 @@ __global__ void __launch_bounds__(TALL_THREADS, 1)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  for (int kk = tid; kk < k; kk += TALL_THREADS) s_koff[kk] = view_offset(va.col, kk);
   // B's real form, rows c (Re C) and 64 + c (Im C); K tile t holds Re then Im of entries 16t…16t+15
   for (int e = tid; e < KT * 16 * 64; e += TALL_THREADS) {
     const int c = e & 63, kk = e >> 6;
@@ -350,24 +352,30 @@ __global__ void __launch_bounds__(TALL_THREADS, 1)
     // producers: thread = (row of the tile, 8 of the stage's 16 entries)
     const int row = tid & 127, hf = tid >> 7;
     const int64_t stages = tiles > (int64_t)blockIdx.x ? ((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x) * KT : 0;
-    cxf r[2][8];
-    auto fetch = [&](int64_t st, cxf* v) {
-      const int64_t i = (blockIdx.x + (st / KT) * gridDim.x) * 128 + row;
-      const int k0 = (int)(st % KT) * 16 + hf * 8;
-      const cxf* p = A + (i < m ? view_offset(va.row, i) : 0);
+    cxf r[4][8];  // stages in flight
+    int64_t ftile = blockIdx.x;  // the next stage to fetch: its tile, row pointer and K tile
+    int fkt = 0;
+    const cxf* fp = nullptr;
+    auto fetch = [&](cxf* v) {
+      if (fkt == 0) fp = ftile * 128 + row < m ? A + view_offset(va.row, ftile * 128 + row) : nullptr;
+      const int k0 = fkt * 16 + hf * 8;
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        v[j] = (i < m && k0 + j < k) ? p[view_offset(va.col, k0 + j)] : mkcx<float>(0.f, 0.f);
+      for (int j = 0; j < 8; ++j) v[j] = (fp && k0 + j < k) ? fp[s_koff[k0 + j]] : mkcx<float>(0.f, 0.f);
+      if (++fkt == KT) {
+        fkt = 0;
+        ftile += gridDim.x;
+      }
     };
-    if (stages > 0) fetch(0, r[0]);
-    if (stages > 1) fetch(1, r[1]);
-    bool ok = true;
-    for (int64_t st = 0; st < stages && ok; st += 2) {
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < 4; ++u)
+      if (u < stages) fetch(r[u]);
+    bool ok = true;
+    for (int64_t st = 0; st < stages && ok; st += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
         if (st + u >= stages) break;
         const int64_t g = st + u;
-        const int slot = u;  // g mod 2
+        const int slot = u & 1;  // g mod 2
         if (g >= 2 && !(ok = tall_wait_warp(&empty[slot], (uint32_t)(((g >> 1) & 1) ^ 1), err))) break;
         unsigned char* hi = sA + slot * 2 * TALL_TILE;
         unsigned char* lo = hi + TALL_TILE;
@@ -383,7 +391,7 @@ __global__ void __launch_bounds__(TALL_THREADS, 1)
             *reinterpret_cast<float4*>(hi + at) = h;
             if (passes > 1) *reinterpret_cast<float4*>(lo + at) = make_float4(x[0] - h.x, x[1] - h.y, x[2] - h.z, x[3] - h.w);
           }
-        if (g + 2 < stages) fetch(g + 2, r[u]);
+        if (g + 4 < stages) fetch(r[u]);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(&full[slot]);
