@@ -16,7 +16,7 @@
 //   1-site  y = Heff x:  T1 = Lcᴴ x  →  T2 = fiber(T1, Wp_i)  →  y = T2 · R_i
 //   2-site  y = Heff θ:  T1 = Lcᴴ θ  →  fiber(Wp_j)  →  fiber(Wp_{j+1})  →  y = T3 · R_{j+1}
 //
-// The Lanczos scalars stay on the device: one block per instance orthogonalises the new
+// The Lanczos scalars stay on the device: one cluster per instance orthogonalises the new
 // vector (two Gram–Schmidt passes against the basis), one thread per instance
 // diagonalises the tridiagonal matrix (cyclic Jacobi) and decides convergence / restart,
 // and an element-wise kernel forms the Ritz vector.  An eigensolve is therefore a fixed
@@ -27,12 +27,14 @@
 #include <cstdlib>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "tn_mps_internal.cuh"
 
 namespace {
 
 constexpr int kLzMax = 16;   // Krylov basis + residual slot
-constexpr int kFiberP = 16;  // fiber kernel: inputs per output kept in registers
+constexpr int kFiberP = 16;  // most inputs per output of the fibre kernel
 const cxd kOne = {1.0, 0.0};
 const cxd kZero = {0.0, 0.0};
 
@@ -100,22 +102,54 @@ __global__ void __launch_bounds__(kLzThreads) k_lz_start(int64_t N, const double
 
 // Lanczos step k: w = H v_k has been formed in W.  α_k, β_k, v_{k+1} = r / β_k with r = w
 // orthogonalised against v_0..v_k (two classical Gram–Schmidt passes).
-// KM ≥ k+1 dot products are accumulated in registers; NT threads per block
-template <int KM, int NT>
-__global__ void __launch_bounds__(NT) k_lz_orth(int64_t N, int k, double2* __restrict__ V, int64_t sV, int64_t slot,
-                                                double2* __restrict__ W, int64_t sW, LzState* st, double tol) {
-  __shared__ double red[32];
-  __shared__ double cs[2 * KM];
-  const int b = blockIdx.x;
-  if (st[b].done || st[b].frozen || st[b].K != k) return;
+//
+// Bound: FP64.  16(k+1) + 4 DFMA per entry on one SM (2 per clock) took 72 µs for 4096 entries;
+// a cluster of CTAs per instance shares them (≤ 16 SMs, 16 µs), with the sums exchanged through
+// distributed shared memory: four cluster barriers in all.  KM ≥ k+1 dot products are
+// accumulated in registers; two sums share one butterfly (Re in one half warp, Im in the
+// other).  Every CTA adds the ranks' partial sums in rank order, so all hold the same bits.
+constexpr int kOrthThreads = 128;
+template <int KM>
+__global__ void __launch_bounds__(kOrthThreads)
+    k_lz_orth(int64_t N, int k, double2* __restrict__ V, int64_t sV, int64_t slot, double2* __restrict__ W, int64_t sW,
+              LzState* st, double tol, int CS) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  constexpr int NW = kOrthThreads / 32;
+  __shared__ double part[NW][2 * KM];   // per warp
+  __shared__ double mine[3][2 * KM];    // this CTA's sums: pass 0, pass 1, the norm
+  __shared__ double cs[2 * KM];         // the cluster's
+  const int b = blockIdx.x / CS, rank = blockIdx.x % CS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // (the cluster leaves together: its CTAs read the same state, written only at the end)
+  const bool skip = st[b].done || st[b].frozen || st[b].K != k;
+  if (skip) return;
   double2* v = V + b * sV;
   double2* w = W + b * sW;
+  // `vals` sums of the CTA are in mine[step]: the cluster's go to cs
+  auto cluster_sum = [&](int step, int vals) {
+    __syncthreads();
+    for (int q = threadIdx.x; q < vals; q += kOrthThreads) {
+      double s = part[0][q];
+#pragma unroll
+      for (int u = 1; u < NW; ++u) s += part[u][q];
+      mine[step][q] = s;
+    }
+    cluster.sync();
+    for (int q = warp; q < vals; q += NW) {
+      double s = lane < CS ? cluster.map_shared_rank(&mine[step][0], lane)[q] : 0.0;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) cs[q] = s;
+    }
+    __syncthreads();
+  };
+  const int64_t first = rank * (int64_t)kOrthThreads + threadIdx.x, step = (int64_t)CS * kOrthThreads;
   double alpha = 0.0;
   for (int pass = 0; pass < 2; ++pass) {
     double cr[KM], ci[KM];
 #pragma unroll
     for (int j = 0; j < KM; ++j) cr[j] = ci[j] = 0.0;
-    for (int64_t t = threadIdx.x; t < N; t += NT) {
+    for (int64_t t = first; t < N; t += step) {
       const double2 y = w[t];
 #pragma unroll
       for (int j = 0; j < KM; ++j)
@@ -128,37 +162,38 @@ __global__ void __launch_bounds__(NT) k_lz_orth(int64_t N, int k, double2* __res
 #pragma unroll
     for (int j = 0; j < KM; ++j)
       if (j <= k) {
-        const double r = block_sum<NT>(cr[j], red);
-        const double i = block_sum<NT>(ci[j], red);
-        if (threadIdx.x == 0) {
-          cs[2 * j] = r;
-          cs[2 * j + 1] = i;
-        }
+        double s = lane < 16 ? cr[j] : ci[j];
+        s += __shfl_xor_sync(0xffffffffu, lane < 16 ? ci[j] : cr[j], 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if ((lane & 15) == 0) part[warp][2 * j + (lane >> 4)] = s;
       }
-    __syncthreads();
+    cluster_sum(pass, 2 * (k + 1));
     alpha += cs[2 * k];
-    for (int64_t t = threadIdx.x; t < N; t += NT) {
+    for (int64_t t = first; t < N; t += step) {
       double2 y = w[t];
       for (int j = 0; j <= k; ++j) {
         const double2 q = v[j * slot + t];
         const double a = cs[2 * j], c = cs[2 * j + 1];
-        y.x -= a * q.x - c * q.y;
-        y.y -= a * q.y + c * q.x;
+        y.x = fma(-a, q.x, fma(c, q.y, y.x));
+        y.y = fma(-a, q.y, fma(-c, q.x, y.y));
       }
       w[t] = y;
     }
-    __syncthreads();
   }
   double s = 0.0;
-  for (int64_t t = threadIdx.x; t < N; t += NT) s += w[t].x * w[t].x + w[t].y * w[t].y;
-  s = block_sum<NT>(s, red);
-  const double beta = sqrt(s);
+  for (int64_t t = first; t < N; t += step) s = fma(w[t].x, w[t].x, fma(w[t].y, w[t].y, s));
+  s = warp_sum(s);
+  __syncthreads();
+  if (lane == 0) part[warp][0] = s;
+  cluster_sum(2, 1);
+  const double beta = sqrt(cs[0]);
   if (beta > tol) {
     const double inv = 1.0 / beta;
-    for (int64_t t = threadIdx.x; t < N; t += NT)
-      v[(k + 1) * slot + t] = make_double2(w[t].x * inv, w[t].y * inv);
+    for (int64_t t = first; t < N; t += step) v[(k + 1) * slot + t] = make_double2(w[t].x * inv, w[t].y * inv);
   }
-  if (threadIdx.x == 0) {
+  cluster.sync();  // no CTA leaves while another may read its sums; the state is written last
+  if (rank == 0 && threadIdx.x == 0) {
     LzState& S = st[b];
     S.alpha[k] = alpha;
     S.beta[k] = beta;
@@ -280,7 +315,10 @@ __global__ void k_lz_combine(int64_t N, double2* __restrict__ V, int64_t sV, int
 }
 
 // out[b][x + X(q + Q j)] = Σ_p in[b][x + X(p + P j)] · M[b][p + P q]
-__global__ void k_fiber(int64_t X, int P, int Q, int64_t J, const cxd* __restrict__ in, int64_t sIn,
+// One thread per output entry, 64 to a block: the FP64 pipe takes 64 clocks per warp
+// instruction, so the P·Q products of a fibre are worth spreading over SMs (χ = 32: a thread per
+// fibre filled 8 SMs, 30 µs a launch; now 6.6) and the P reads that Q threads share stay in L1.
+__global__ void __launch_bounds__(64) k_fiber(int64_t X, int P, int Q, int64_t J, const cxd* __restrict__ in, int64_t sIn,
                         const cxd* __restrict__ M, int64_t sM, cxd* __restrict__ out, int64_t sOut) {
   extern __shared__ cxd Ms[];
   const int b = blockIdx.y;
@@ -288,20 +326,16 @@ __global__ void k_fiber(int64_t X, int P, int Q, int64_t J, const cxd* __restric
   __syncthreads();
   const cxd* ib = in + b * sIn;
   cxd* ob = out + b * sOut;
-  const int64_t total = X * J;
+  const int64_t total = X * Q * J;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t x = t % X, j = t / X;
-    cxd v[kFiberP];
-#pragma unroll
-    for (int p = 0; p < kFiberP; ++p)
-      if (p < P) v[p] = ib[x + X * (p + (int64_t)P * j)];
-    for (int q = 0; q < Q; ++q) {
-      cxd acc = mkcx(0.0, 0.0);
-#pragma unroll
-      for (int p = 0; p < kFiberP; ++p)
-        if (p < P) cfma(acc, v[p], Ms[p + P * q]);
-      ob[x + X * (q + (int64_t)Q * j)] = acc;
-    }
+    const int64_t x = t % X, r = t / X, j = r / Q;
+    const int q = (int)(r - j * Q);
+    const cxd* src = ib + x + X * P * j;
+    const cxd* mq = Ms + P * q;
+    cxd acc = mkcx(0.0, 0.0);
+#pragma unroll 4
+    for (int p = 0; p < P; ++p) cfma(acc, src[X * p], mq[p]);
+    ob[t] = acc;
   }
 }
 
@@ -412,8 +446,9 @@ tn_status_t fiber(Dmrg& D, int64_t X, int64_t P, int64_t Q, int64_t J, const cxd
                   int64_t sM, cxd* out, int64_t sOut) {
   tn_ctx* ctx = D.ctx;
   if (P <= kFiberP && P * Q <= 3072) {
-    dim3 grid(grid_for(ctx, X * J, 256), (unsigned)D.B);
-    k_fiber<<<grid, 256, sizeof(cxd) * P * Q, ctx->stream>>>(X, (int)P, (int)Q, J, in, sIn, M, sM, out, sOut);
+    dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * 32, (X * Q * J + 63) / 64)),
+              (unsigned)D.B);
+    k_fiber<<<grid, 64, sizeof(cxd) * P * Q, ctx->stream>>>(X, (int)P, (int)Q, J, in, sIn, M, sM, out, sOut);
     TN_LAUNCHED(ctx);
     return TN_OK;
   }
@@ -484,6 +519,31 @@ tn_status_t matvec(Dmrg& D, int nsite, int i, int k) {
                          wr * chr, D.eS[i + 1], kZero, D.Wv, chl * d * d, D.Nmax, D.B);
 }
 
+// one Lanczos orthogonalisation: as many CTAs per instance (a power of two, at most the 16 of
+// the largest cluster) as the vector and the chip have use for
+template <int KM>
+tn_status_t lz_orth(Dmrg& D, int64_t N, int k) {
+  tn_ctx* ctx = D.ctx;
+  int CS = 1;
+  while (CS < 16 && N > (int64_t)CS * kOrthThreads && 2 * CS * D.B <= ctx->num_sms) CS *= 2;
+  TN_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_lz_orth<KM>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(D.B * CS));
+  cfg.blockDim = dim3(kOrthThreads);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)CS;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  TN_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_lz_orth<KM>, N, k, (double2*)D.V, D.sV, D.Nmax, (double2*)D.Wv, D.Nmax, D.st,
+                                        D.tol, CS));
+  TN_LAUNCHED(ctx);
+  return TN_OK;
+}
+
 // restarted Lanczos from x0 (instance stride sx0, N elements); the Ritz vector ends in slot 0
 tn_status_t eigsolve(Dmrg& D, int nsite, int i, int64_t N, const cxd* x0, int64_t sx0) {
   tn_ctx* ctx = D.ctx;
@@ -493,15 +553,11 @@ tn_status_t eigsolve(Dmrg& D, int nsite, int i, int64_t N, const cxd* x0, int64_
     for (int k = it == 1 ? 0 : 1; k < D.kdim; ++k) {
       TN_RETURN_IF(matvec(D, nsite, i, k));
       if (k < 4)
-        k_lz_orth<4, 1024><<<D.B, 1024, 0, ctx->stream>>>(N, k, (double2*)D.V, D.sV, D.Nmax, (double2*)D.Wv, D.Nmax,
-                                                           D.st, D.tol);
+        TN_RETURN_IF(lz_orth<4>(D, N, k));
       else if (k < 8)
-        k_lz_orth<8, 512><<<D.B, 512, 0, ctx->stream>>>(N, k, (double2*)D.V, D.sV, D.Nmax, (double2*)D.Wv, D.Nmax,
-                                                         D.st, D.tol);
+        TN_RETURN_IF(lz_orth<8>(D, N, k));
       else
-        k_lz_orth<kLzMax, 256><<<D.B, 256, 0, ctx->stream>>>(N, k, (double2*)D.V, D.sV, D.Nmax, (double2*)D.Wv,
-                                                              D.Nmax, D.st, D.tol);
-      TN_LAUNCHED(ctx);
+        TN_RETURN_IF(lz_orth<kLzMax>(D, N, k));
     }
     k_lz_ritz<<<cdiv(D.B, 32), 32, 0, ctx->stream>>>(D.B, D.kdim, D.maxiter, D.tol, D.st);
     TN_LAUNCHED(ctx);
