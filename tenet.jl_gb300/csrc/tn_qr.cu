@@ -327,7 +327,9 @@ static bool ranges_meet(const void* a, size_t na, const void* b, size_t nb) {
 // Which kernel: one CTA per column (tn_qr_cols.cu) while all columns of all matrices are
 // resident at once, the blocked panels below beyond that (rows > 512, or batches that fill
 // the FP64 pipe with panels of different matrices) and for shapes whose launch configuration
-// the caller set (tn_tuning_load).  Measured, one matrix, blocked / columns: QRCOLS_NUMBERS
+// the caller set (tn_tuning_load).  Measured, one matrix, blocked /
+// columns, µs: 64×64 630 / 174, 128×128 1420 / 394, 256×256 3345 / 1158, 512×256 5728 / 1510,
+// 512×512 9634 / 4000.
 // A column's CTA reads it before anything is written only if no other CTA's output lies
 // there, so Q or R over A is left to the blocked kernel (which factors a copy) unless Q is
 // exactly A.

@@ -12,8 +12,15 @@
 //  * entries travel as packets of two 64-bit words with 32 data bits and a flag each, polled
 //    by the receivers directly: no fence, no barrier between CTAs, and they stay in place as
 //    the stored reflectors;
-//  * column q of Q = H₀…H_{k−1} needs reflectors q…0 only, all known when column q is done,
-//    so its CTA forms it right away, while later columns are still being factored.
+//  * Q is formed in one of two ways.  With CTAs to spare, m more of them carry the rows: row i
+//    of Q is (Qᴴeᵢ)ᴴ, the reflectors applied to eᵢ in the order in which they appear, so Q is
+//    ready one step after R (64×64 255 → 174 µs, 128×128 498 → 394).  At more than two CTAs
+//    an SM the FP64 pipe is what they wait for (256×256 1158 → 1400, 512×64 361 → 521), and
+//    column q of Q = H₀…H_{k−1}, which needs reflectors q…0 only, is formed by its column's CTA
+//    as soon as column q is done, with half the products.
+//  * u₁ is sent before κ, so that the receivers' wᴴ = uᴴc is complete when κ arrives.
+// A step takes 2.3 µs with a column per SM: a packet's 0.4 µs, two reductions of 0.4 µs, the
+// scalars of 0.5 µs and the updates, in FP64 operations of 64 clocks' latency each.
 // Reflectors and signs are LAPACK's (H = I − τ v vᴴ, v₁ = 1, τ v vᴴ = κ u uᴴ, R_jj real with
 // the sign opposite to Re x₁).  Every wait is bounded: a CTA whose wait ran out records an
 // error and leaves.
@@ -25,6 +32,9 @@ namespace {
 
 constexpr int kNT = 128;
 constexpr long long kSpinLimit = 1ll << 22;
+// A column or row far from its turn leaves the memory to the ones whose turn it is: asleep for
+// 1 µs between looks at a packet (a step is 2.3 µs) instead of 64 ns, 128 × 128 took 398 µs, not 443.
+constexpr unsigned kFarSleep = 1000;
 
 struct QMat {
   const cxd* A;
@@ -32,7 +42,8 @@ struct QMat {
   ulonglong2* box;  // k reflectors × (2m + 4) packets
   const int* perm;  // column c of the factored matrix is column perm[c] of op(A); null: c
   int64_t lda;
-  int m, n, k, cta0;  // m × n: the factored matrix
+  int m, n, k;        // m × n: the factored matrix
+  int rows;           // CTAs that form rows of Q (m or 0)
   int adj;            // bit 0: op(A) = Aᴴ (A n × m); bit 1: Rᴴ (n × k, ld n) is stored for R
 };
 
@@ -49,6 +60,33 @@ __device__ __forceinline__ ulonglong2 get_raw(const ulonglong2* p) {
 __device__ __forceinline__ bool arrived(ulonglong2 v) { return (v.x >> 32) != 0 && (v.y >> 32) != 0; }
 __device__ __forceinline__ double value_of(ulonglong2 v) {
   return __longlong_as_double((long long)((v.x & 0xffffffffull) | (v.y << 32)));
+}
+
+// ‖x‖ = √n2, 1/‖x‖ and, by reciprocal(), 1/|u₁|²: the hardware's approximations (some 20 bits)
+// and one step of third order, y ← y + y·e(1/2 + 3e/8) with e = 1 − n2·y² and
+// y ← y + y·e(1 + e) with e = 1 − x·y, which leaves an error of order e³.  They are in the chain
+// of every step; CUDA's rsqrt and divide, of up to 600 clocks each, take the arguments outside
+// the range where the approximations are normal numbers.
+constexpr double kNormLo = 1e-280, kNormHi = 1e280;
+__device__ __forceinline__ void norm_of(double n2, double* nrm, double* inv) {
+  if (n2 > kNormLo && n2 < kNormHi) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(n2));
+    const double t = n2 * y, e = fma(-t, y, 1.0), p = fma(0.375, e, 0.5);
+    *nrm = fma(t * e, p, t);
+    *inv = fma(y * e, p, y);
+  } else {
+    const double rs = rsqrt(n2), r = n2 * rs;
+    *nrm = fma(fma(-r, r, n2), 0.5 * rs, r);
+    *inv = rs;
+  }
+}
+__device__ __forceinline__ double reciprocal(double x) {
+  if (!(x > kNormLo && x < kNormHi)) return 1.0 / x;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
 // Σ over the warp of (a, b): lanes 0-15 end with Σa, lanes 16-31 with Σb
@@ -70,16 +108,18 @@ struct QBatch {
 template <int R>
 __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
   QMat M = batch.first;
+  int b;
   {
-    const int b = (int)blockIdx.x / M.n;
+    b = (int)blockIdx.x / (M.n + M.rows);
     M.A += b * batch.sA;
     if (M.Q) M.Q += b * batch.sQ;
     M.R += b * batch.sR;
     M.box += b * batch.sBox;
     if (M.perm) M.perm += b * M.n;
-    M.cta0 = b * M.n;
   }
-  const int m = M.m, k = M.k, col = (int)blockIdx.x - M.cta0;
+  const int m = M.m, k = M.k, index = (int)blockIdx.x - b * (M.n + M.rows);
+  const bool row = index >= M.n;         // a CTA that forms a row of Q
+  const int col = row ? m + k : index;  // (rows wait for all reflectors)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = lane >> 4;
   const int64_t stride = 2 * (int64_t)m + 4;
   __shared__ double red[2][4][2];
@@ -87,12 +127,12 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
   __shared__ int s_fail;
   if (tid == 0) s_fail = 0;
   cxd x[R];
-  const int64_t src = M.perm ? M.perm[col] : col;
+  const int64_t src = row ? 0 : (M.perm ? M.perm[col] : col);
 #pragma unroll
   for (int q = 0; q < R; ++q) {
     const int64_t t = tid + q * kNT;
-    x[q] = mkcx(0.0, 0.0);
-    if (t < m) x[q] = (M.adj & 1) ? conjg(M.A[src + t * M.lda]) : M.A[src * M.lda + t];
+    x[q] = mkcx(row && t == index - M.n ? 1.0 : 0.0, 0.0);
+    if (!row && t < m) x[q] = (M.adj & 1) ? conjg(M.A[src + t * M.lda]) : M.A[src * M.lda + t];
   }
   int buf = 0;
   // x ← (I − f-form of reflector j) x: rows > j of u from the packets, u₁ and conj(κ) from the
@@ -102,9 +142,14 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     cxd u[R];
     long long spins = 0;
     bool ok;
+    ulonglong2 p0, p1, p2, p3;
     do {
       ok = true;
       ulonglong2 p[2 * R];
+      p0 = get_raw(b + 2 * m);
+      p1 = get_raw(b + 2 * m + 1);
+      p2 = get_raw(b + 2 * m + 2);
+      p3 = get_raw(b + 2 * m + 3);
 #pragma unroll
       for (int q = 0; q < R; ++q) {
         const int t = tid + q * kNT;
@@ -122,8 +167,7 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
           u[q] = mkcx(value_of(p[2 * q]), value_of(p[2 * q + 1]));
         }
       }
-      // a column far from its turn leaves the memory to the ones whose turn it is
-      if (!ok && adj && col > j + 8) __nanosleep(64);
+      if (!ok && adj && col > j + 8) __nanosleep(kFarSleep);
     } while (!ok && ++spins < kSpinLimit);
     double wx = 0, wy = 0;
 #pragma unroll
@@ -138,17 +182,14 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     }
     const double s = warp_sum2(wx, wy, lane);
     if ((lane & 15) == 0) red[buf][warp][half] = s;
-    ulonglong2 p0, p1, p2, p3;
-    do {
+    const bool far = adj && col > j + 8;
+    while (!(arrived(p0) && arrived(p1)) && ++spins < kSpinLimit) {
+      if (far) __nanosleep(kFarSleep);
       p0 = get_raw(b + 2 * m);
       p1 = get_raw(b + 2 * m + 1);
       p2 = get_raw(b + 2 * m + 2);
       p3 = get_raw(b + 2 * m + 3);
-      ok = ok && arrived(p0) && arrived(p1) && arrived(p2) && arrived(p3);
-      if (ok) break;
-      ok = true;
-      if (adj && col > j + 8) __nanosleep(64);
-    } while (++spins < kSpinLimit);
+    }
     if (spins >= kSpinLimit) {
       atomicExch(err, 1);
       s_fail = 1;
@@ -158,10 +199,19 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     double d = red[buf][lane & 3][half];
     d += __shfl_xor_sync(0xffffffffu, d, 1);
     d += __shfl_xor_sync(0xffffffffu, d, 2);
-    const double ux = value_of(p0), uy = value_of(p1), kx = value_of(p2), ky = adj ? value_of(p3) : -value_of(p3);
+    const double ux = value_of(p0), uy = value_of(p1);
     // w = uᴴx + conj(u₁)·x_j, f = κ'·w (κ' = conj(κ) for Hᴴ): Re in lanes 0-15, Im in 16-31
     const double cx_ = s_row[buf][0], cy_ = s_row[buf][1];
     const double w = fma(ux, half ? cy_ : cx_, fma(uy, half ? -cx_ : cy_, d));
+    while (!(arrived(p2) && arrived(p3)) && ++spins < kSpinLimit) {
+      p2 = get_raw(b + 2 * m + 2);
+      p3 = get_raw(b + 2 * m + 3);
+    }
+    if (spins >= kSpinLimit) {  // (seen after the next reflector's barrier)
+      atomicExch(err, 1);
+      s_fail = 1;
+    }
+    const double kx = value_of(p2), ky = adj ? value_of(p3) : -value_of(p3);
     const double wo = __shfl_xor_sync(0xffffffffu, w, 16);
     const double f = fma(kx, w, (half ? ky : -ky) * wo);
     const double fx = __shfl_sync(0xffffffffu, f, 0), fy = __shfl_sync(0xffffffffu, f, 16);
@@ -179,6 +229,15 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
   const int steps = min(col, k);
   for (int j = 0; j < steps; ++j)
     if (!reflect(j, true)) return;
+  if (row) {
+    // x = Qᴴ e_i: row i of Q is its conjugate
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int t = tid + q * kNT;
+      if (t < k) M.Q[(int64_t)t * m + index - M.n] = conjg(x[q]);
+    }
+    return;
+  }
   if (col < k) {
     // this column's reflector: the entries below the pivot go out first
     ulonglong2* b = M.box + (int64_t)col * stride;
@@ -207,19 +266,20 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     double beta = ax, ux = 0, uy = 0, kx = 0, ky = 0;
     if (!(s2 == 0.0 && ay == 0.0)) {
       // β = −sgn(Re α)·‖x‖, u₁ = α − β, conj(κ) = −1/(β·u₁) = −(conj(u₁)/|u₁|²)/β
-      // (‖x‖ and 1/‖x‖ from one reciprocal square root, ‖x‖ corrected by its residual: a square
-      // root and a division are 580 clocks each)
-      const double n2 = fma(ax, ax, fma(ay, ay, s2)), rs = rsqrt(n2);
-      double nrm = n2 * rs;
-      nrm = fma(fma(-nrm, nrm, n2), 0.5 * rs, nrm);
+      const double n2 = fma(ax, ax, fma(ay, ay, s2));
+      double nrm, rs;
+      norm_of(n2, &nrm, &rs);
       beta = ax >= 0.0 ? -nrm : nrm;
       ux = ax - beta;
       uy = ay;
-      const double inv2 = 1.0 / fma(ux, ux, uy * uy), invb = ax >= 0.0 ? rs : -rs;
+      if (tid < 2) put(b + 2 * m + tid, tid == 0 ? ux : uy);  // κ follows
+      const double inv2 = reciprocal(fma(ux, ux, uy * uy)), invb = ax >= 0.0 ? rs : -rs;
       kx = (ux * inv2) * invb;
       ky = (-uy * inv2) * invb;
+    } else if (tid < 2) {
+      put(b + 2 * m + tid, 0.0);
     }
-    if (tid < 4) put(b + 2 * m + tid, tid == 0 ? ux : (tid == 1 ? uy : (tid == 2 ? kx : ky)));
+    if (tid < 2) put(b + 2 * m + 2 + tid, tid == 0 ? kx : ky);
 #pragma unroll
     for (int q = 0; q < R; ++q)
       if (tid + q * kNT == col) x[q] = mkcx(beta, 0.0);
@@ -234,7 +294,7 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     else
       M.R[(int64_t)col * k + t] = v;
   }
-  if (col >= k || !M.Q) return;
+  if (col >= k || !M.Q || M.rows) return;
 #pragma unroll
   for (int q = 0; q < R; ++q) x[q] = mkcx(tid + q * kNT == col ? 1.0 : 0.0, 0.0);
   for (int j = col; j >= 0; --j)
@@ -282,13 +342,14 @@ tn_status_t qr_cols_batch(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64
   const size_t one = boxes_bytes(m, k);
   char* box = ws_take<char>(ctx, one * (size_t)batch);
   TN_CHECK_CUDA(ctx, cudaMemsetAsync(box, 0, one * (size_t)batch, ctx->stream));
-  QBatch b = {QMat{A, Q, R, reinterpret_cast<ulonglong2*>(box), perm, lda, (int)m, (int)n, (int)k, 0,
+  const int64_t rows = Q && (n + m) * batch <= 2 * (int64_t)ctx->num_sms ? m : 0;
+  QBatch b = {QMat{A, Q, R, reinterpret_cast<ulonglong2*>(box), perm, lda, (int)m, (int)n, (int)k, (int)rows,
                    (adj_in ? 1 : 0) + (adj_r ? 2 : 0)},
               sA, sQ, sR, (int64_t)(one / sizeof(ulonglong2))};
   int* err = nullptr;
   TN_RETURN_IF(wait_error_word(ctx, &err));
   void* args[] = {&b, &err};
-  TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel(kernel_for(m), dim3((unsigned)(n * batch)), dim3(kNT), args, 0,
+  TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel(kernel_for(m), dim3((unsigned)((n + rows) * batch)), dim3(kNT), args, 0,
                                                  ctx->stream));
   TN_LAUNCHED(ctx);
   return TN_OK;

@@ -1,4 +1,4 @@
-"""QR with one CTA per column (k_qr_cols) at the edges of its rows per thread, for tall, square
+"""QR with one CTA per column (k_qr_cols), with and without CTAs for the rows of Q, at the edges of its rows per thread, for tall, square
 and wide matrices, batches, rank deficiency and in-place calls, against LAPACK.
 
 Tolerances: Householder QR is backward stable, ‖QR − A‖ and ‖QᴴQ − I‖ are a small multiple of
@@ -53,6 +53,7 @@ def _check(A, Q, R, lapack=True):
 @pytest.mark.parametrize("m,n,batch", [
     (1, 1, 1), (2, 1, 3), (2, 2, 1), (127, 5, 1), (128, 64, 2), (129, 40, 1), (256, 31, 1), (257, 33, 1), (512, 200, 1),
     (37, 90, 2), (128, 128, 1), (5, 300, 1), (300, 300, 1), (16, 8, 40), (513, 20, 1),
+    (152, 152, 1), (153, 152, 1), (19, 19, 8), (19, 20, 8), (300, 4, 1), (300, 5, 1),
 ])
 def test_columns_qr_matches_lapack(ctx, m, n, batch):
     rng = np.random.default_rng(m * 1000 + n)
