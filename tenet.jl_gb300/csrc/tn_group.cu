@@ -44,12 +44,14 @@ struct GemmD {
   int opa, opb;  // 'N' / 'C'
 };
 struct QrD {
+  cxd* A;  // the site: m × n, or (adjoint) the n × m matrix whose adjoint is factored; becomes Q, or Qᴴ
   cxd* W;  // m × n work (ld m), factored in place
   cxd* tau;
   cxd* T;  // npan · nb · nb
   cxd* Q;  // m × n (ld m)
   cxd* R;  // n × n (ld n)
   int64_t m, n;
+  bool adjoint;
 };
 struct JacD {
   cxd* W;  // m × n (ld m)
@@ -616,11 +618,15 @@ tn_status_t g_copy(tn_ctx* ctx, const std::vector<CopyD>& h) {
 
 tn_status_t g_gemm(tn_ctx* ctx, const std::vector<GemmD>& h) {
   if (h.empty()) return TN_OK;
-  // 64×64 tiles when the group fills the GPU twice over with them, else 32×32
-  int64_t t64 = 0;
-  for (auto& g : h) t64 += ((g.m + 63) / 64) * ((g.n + 63) / 64);
-  const bool big = t64 >= 2 * (int64_t)ctx->num_sms;
-  const int BM = big ? 64 : 32;
+  // 64×64 tiles when the group fills the GPU twice over with them, 32×32 from four to an SM, else
+  // 16×16: a 32×32 tile of k = 72 is 77 µs of an SM's FP64 pipe, and the launch lasts as long as the
+  // SM with one more tile than the others
+  int64_t t64 = 0, t32 = 0;
+  for (auto& g : h) {
+    t64 += ((g.m + 63) / 64) * ((g.n + 63) / 64);
+    t32 += ((g.m + 31) / 32) * ((g.n + 31) / 32);
+  }
+  const int BM = t64 >= 2 * (int64_t)ctx->num_sms ? 64 : (t32 >= 4 * (int64_t)ctx->num_sms ? 32 : 16);
   std::vector<int64_t> start(h.size() + 1, 0);
   for (size_t b = 0; b < h.size(); ++b) start[b + 1] = start[b] + ((h[b].m + BM - 1) / BM) * ((h[b].n + BM - 1) / BM);
   GemmD* d = nullptr;
@@ -630,17 +636,54 @@ tn_status_t g_gemm(tn_ctx* ctx, const std::vector<GemmD>& h) {
   const int64_t tiles = start.back();
   if (tiles <= 0) return TN_OK;
   if (tiles > 0x7fffffffll) return tn_set_error(ctx, TN_EUNSUPPORTED, "group gemm: too many tiles");
-  if (big)
+  if (BM == 64)
     k_g_gemm<64, 64, 8, 4, 4><<<(unsigned)tiles, 256, 0, ctx->stream>>>(d, st, (int)h.size());
-  else
+  else if (BM == 32)
     k_g_gemm<32, 32, 8, 2, 2><<<(unsigned)tiles, 256, 0, ctx->stream>>>(d, st, (int)h.size());
+  else
+    k_g_gemm<16, 16, 16, 1, 2><<<(unsigned)tiles, 128, 0, ctx->stream>>>(d, st, (int)h.size());
   TN_LAUNCHED(ctx);
   return TN_OK;
 }
 
-// QR of every W (m ≥ n), Q and R written to the descriptor's buffers
-tn_status_t g_qr(tn_ctx* ctx, const std::vector<QrD>& h) {
+size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
+
+// scratch of one instance's QR in either form
+size_t qr_need(int64_t m, int64_t n, bool columns) {
+  if (columns) return al256(sizeof(cxd) * (size_t)n * (size_t)(2 * m + 4)) + al256(sizeof(int) * (size_t)n) + 256;
+  return 2 * al256(sizeof(cxd) * (size_t)(m * n)) + al256(sizeof(cxd) * (size_t)(n + 1)) +
+         al256(sizeof(cxd) * (size_t)(((n + kNb - 1) / kNb) * kNb * kNb));
+}
+
+// QR of every site matrix (m ≥ n) in place, R to the descriptor's buffer.
+// One CTA per column (tn_qr_cols.cu) while a column's rows fit one CTA: a panel factored by one
+// CTA is bound by that SM's FP64 pipe, and a group of 16 is 16 of 152 (canonize, compress and norm
+// of 16 MPS of χ ≤ 72: 64 → 49 ms, of 24 of χ ≤ 512: 469 → 457 ms).  Blocked panels beyond.
+tn_status_t g_qr(tn_ctx* ctx, std::vector<QrD>& h, bool columns) {
   if (h.empty()) return TN_OK;
+  if (columns) {
+    std::vector<QrColsMat> mats;
+    for (auto& q : h) mats.push_back({q.A, q.A, q.R, q.adjoint ? q.n : q.m, (int)q.m, (int)q.n, q.adjoint});
+    if (ctx->ws_top + qr_cols_list_workspace(mats) > ctx->ws_cap)
+      return tn_set_error(ctx, TN_ECUDA, "group: workspace overrun (qr)");
+    return qr_cols_list(ctx, std::move(mats));
+  }
+  std::vector<CopyD> in, out;
+  for (auto& q : h) {
+    q.W = ws_take<cxd>(ctx, (size_t)(q.m * q.n));
+    q.Q = ws_take<cxd>(ctx, (size_t)(q.m * q.n));
+    q.tau = ws_take<cxd>(ctx, (size_t)(q.n + 1));
+    q.T = ws_take<cxd>(ctx, (size_t)(((q.n + kNb - 1) / kNb) * kNb * kNb));
+    if (q.adjoint) {
+      in.push_back({q.A, q.W, q.n, q.m, q.n, q.m, 1});
+      out.push_back({q.Q, q.A, q.m, q.n, q.m, q.n, 1});
+    } else {
+      in.push_back({q.A, q.W, q.m, q.m, q.m, q.n, 0});
+      out.push_back({q.Q, q.A, q.m, q.m, q.m, q.n, 0});
+    }
+  }
+  TN_RETURN_IF(ws_check(ctx));
+  TN_RETURN_IF(g_copy(ctx, in));
   QrD* d = nullptr;
   TN_RETURN_IF(upload(ctx, h, &d));
   int64_t mmax = 1, nmax = 1;
@@ -666,7 +709,7 @@ tn_status_t g_qr(tn_ctx* ctx, const std::vector<QrD>& h) {
     k_g_qr_apply<<<dim3(cdiv(nmax - j0, kSlab), B), 256, 0, ctx->stream>>>(d, j0, true);
     TN_LAUNCHED(ctx);
   }
-  return TN_OK;
+  return g_copy(ctx, out);
 }
 
 // the sweeps by grouped launches, one per round (rows > 512)
@@ -769,7 +812,6 @@ tn_status_t g_svd_left(tn_ctx* ctx, std::vector<JacD>& h, int* active, int* rota
   return TN_OK;
 }
 
-size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
 // descriptor tables of one step: at most 16 tables of ≤ 128 bytes per instance
 size_t table_bytes(size_t n) { return 16 * al256(128 * (n + 1)) + 65536; }
 
@@ -911,39 +953,32 @@ tn_status_t tn_group_canonize_compress_norm(tn_group* g, const int64_t* maxdim, 
       if (k <= g->L[b] - 1) ids.push_back(b);
     if (ids.empty()) continue;
     size_t need = table_bytes(ids.size());
+    int64_t rows = 0;
+    for (int b : ids) rows = std::max(rows, g->bond[b][k - 1] * d);
+    const bool columns = rows <= kQrColsMaxRows;
     for (int b : ids) {
       const int64_t m = g->bond[b][k - 1] * d, n = g->bond[b][k], n2 = d * g->bond[b][k + 1];
-      need += al256(sizeof(cxd) * (size_t)(m * n)) * 2 + al256(sizeof(cxd) * (size_t)(n * n)) +
-              al256(sizeof(cxd) * (size_t)(n + 1)) + al256(sizeof(cxd) * (size_t)(((n + kNb - 1) / kNb) * kNb * kNb)) +
-              al256(sizeof(cxd) * (size_t)(n * n2));
+      need += qr_need(m, n, columns) + al256(sizeof(cxd) * (size_t)(n * n)) + al256(sizeof(cxd) * (size_t)(n * n2));
     }
     TN_RETURN_IF(ws_reserve(ctx, need));
     std::vector<QrD> qr;
     std::vector<GemmD> mm;
-    std::vector<CopyD> cq, cb;
+    std::vector<CopyD> cb;
     for (int b : ids) {
       const int64_t m = g->bond[b][k - 1] * d, n = g->bond[b][k], n2 = d * g->bond[b][k + 1];
       if (m < n) return tn_set_error(ctx, TN_EUNSUPPORTED, "group canonize: site %d of instance %d is wide", k, b);
-      QrD q;
+      QrD q = {};
+      q.A = g->site[b][k];
       q.m = m;
       q.n = n;
-      q.W = ws_take<cxd>(ctx, (size_t)(m * n));
-      q.Q = ws_take<cxd>(ctx, (size_t)(m * n));
       q.R = ws_take<cxd>(ctx, (size_t)(n * n));
-      q.tau = ws_take<cxd>(ctx, (size_t)(n + 1));
-      q.T = ws_take<cxd>(ctx, (size_t)(((n + kNb - 1) / kNb) * kNb * kNb));
       cxd* tmp = ws_take<cxd>(ctx, (size_t)(n * n2));
       qr.push_back(q);
-      cq.push_back({g->site[b][k], q.W, m, m, m, n, 0});
       mm.push_back({q.R, g->site[b][k + 1], tmp, n, n2, n, n, n, n, 'N', 'N'});
       cb.push_back({tmp, g->site[b][k + 1], n, n, n, n2, 0});
     }
     TN_RETURN_IF(ws_check(ctx));
-    TN_RETURN_IF(g_copy(ctx, cq));
-    TN_RETURN_IF(g_qr(ctx, qr));
-    std::vector<CopyD> cqo;
-    for (size_t t = 0; t < ids.size(); ++t) cqo.push_back({qr[t].Q, g->site[ids[t]][k], qr[t].m, qr[t].m, qr[t].m, qr[t].n, 0});
-    TN_RETURN_IF(g_copy(ctx, cqo));
+    TN_RETURN_IF(g_qr(ctx, qr, columns));
     TN_RETURN_IF(g_gemm(ctx, mm));
     TN_RETURN_IF(g_copy(ctx, cb));
     g->steps_launched++;
@@ -955,43 +990,37 @@ tn_status_t tn_group_canonize_compress_norm(tn_group* g, const int64_t* maxdim, 
       if (g->L[b] - j >= 2) ids.push_back(b);
     if (ids.empty()) continue;
     size_t need = table_bytes(ids.size());
+    int64_t most = 0;
+    for (int b : ids) most = std::max(most, d * g->bond[b][g->L[b] - j]);
+    const bool columns = most <= kQrColsMaxRows;
     for (int b : ids) {
       const int i = g->L[b] - j;
       const int64_t rows = g->bond[b][i - 1], cols = d * g->bond[b][i], m0 = g->bond[b][i - 2] * d;
-      need += al256(sizeof(cxd) * (size_t)(rows * cols)) * 2 + al256(sizeof(cxd) * (size_t)(rows * rows)) +
-              al256(sizeof(cxd) * (size_t)(rows + 1)) +
-              al256(sizeof(cxd) * (size_t)(((rows + kNb - 1) / kNb) * kNb * kNb)) +
-              al256(sizeof(cxd) * (size_t)(m0 * rows));
+      need += qr_need(cols, rows, columns) + al256(sizeof(cxd) * (size_t)(rows * rows)) + al256(sizeof(cxd) * (size_t)(m0 * rows));
     }
     TN_RETURN_IF(ws_reserve(ctx, need));
     std::vector<QrD> qr;
-    std::vector<CopyD> ct, cback, cprev;
+    std::vector<CopyD> cprev;
     std::vector<GemmD> mm;
     for (int b : ids) {
       const int i = g->L[b] - j;
-      // A_i (χ_{i−1} × d χ_i); its adjoint (d χ_i × χ_{i−1}) is tall
+      // A_i (χ_{i−1} × d χ_i); its adjoint (d χ_i × χ_{i−1}) is tall: A_iᴴ = QR, A_i = Qᴴ
       const int64_t rows = g->bond[b][i - 1], cols = d * g->bond[b][i], m0 = g->bond[b][i - 2] * d;
       if (cols < rows) return tn_set_error(ctx, TN_EUNSUPPORTED, "group canonize: site %d of instance %d is tall", i, b);
-      QrD q;
+      QrD q = {};
+      q.A = g->site[b][i];
       q.m = cols;
       q.n = rows;
-      q.W = ws_take<cxd>(ctx, (size_t)(rows * cols));
-      q.Q = ws_take<cxd>(ctx, (size_t)(rows * cols));
+      q.adjoint = true;
       q.R = ws_take<cxd>(ctx, (size_t)(rows * rows));
-      q.tau = ws_take<cxd>(ctx, (size_t)(rows + 1));
-      q.T = ws_take<cxd>(ctx, (size_t)(((rows + kNb - 1) / kNb) * kNb * kNb));
       cxd* tmp = ws_take<cxd>(ctx, (size_t)(m0 * rows));
       qr.push_back(q);
-      ct.push_back({g->site[b][i], q.W, rows, cols, rows, cols, 1});     // W = A_iᴴ
-      cback.push_back({q.Q, g->site[b][i], cols, rows, cols, rows, 1});  // A_i = Qᴴ
       // A_{i−1} (m0 × χ_{i−1}) ← A_{i−1} Rᴴ
       mm.push_back({g->site[b][i - 1], q.R, tmp, m0, rows, rows, m0, rows, m0, 'N', 'C'});
       cprev.push_back({tmp, g->site[b][i - 1], m0, m0, m0, rows, 0});
     }
     TN_RETURN_IF(ws_check(ctx));
-    TN_RETURN_IF(g_copy(ctx, ct));
-    TN_RETURN_IF(g_qr(ctx, qr));
-    TN_RETURN_IF(g_copy(ctx, cback));
+    TN_RETURN_IF(g_qr(ctx, qr, columns));
     TN_RETURN_IF(g_gemm(ctx, mm));
     TN_RETURN_IF(g_copy(ctx, cprev));
     g->steps_launched++;

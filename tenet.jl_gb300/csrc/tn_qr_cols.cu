@@ -25,12 +25,14 @@
 // the sign opposite to Re x₁).  Every wait is bounded: a CTA whose wait ran out records an
 // error and leaves.
 #include <algorithm>
+#include <vector>
 
 #include "tn_internal.cuh"
 
 namespace {
 
 constexpr int kNT = 128;
+static_assert(kQrColsMaxRows == 4 * kNT);
 constexpr long long kSpinLimit = 1ll << 22;
 // A column or row far from its turn leaves the memory to the ones whose turn it is: asleep for
 // 1 µs between looks at a packet (a step is 2.3 µs) instead of 64 ns, 128 × 128 took 398 µs, not 443.
@@ -44,7 +46,8 @@ struct QMat {
   int64_t lda;
   int m, n, k;        // m × n: the factored matrix
   int rows;           // CTAs that form rows of Q (m or 0)
-  int adj;            // bit 0: op(A) = Aᴴ (A n × m); bit 1: Rᴴ (n × k, ld n) is stored for R
+  int adj;            // bit 0: op(A) = Aᴴ (A n × m); bit 1: Rᴴ (n × k, ld n) is stored for R;
+                      // bit 2: Qᴴ (k × m, ld k) is stored for Q
 };
 
 __device__ __forceinline__ void put(ulonglong2* p, double v) {
@@ -99,25 +102,44 @@ __device__ __forceinline__ double warp_sum2(double a, double b, int lane) {
   return keep;
 }
 
-// a batch of equal matrices: the first one and the strides to the next
+// a batch of equal matrices: the first one and the strides to the next; or a list of matrices
+// of falling n, whose columns are taken in the order 0 of all, 1 of all, …
 struct QBatch {
   QMat first;
   int64_t sA, sQ, sR, sBox;
+  const QMat* list;
+  const int* level;  // levels + 1: the columns before column c of the first matrix
+  int levels;
+  int* ticket;
 };
 
 template <int R>
 __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
-  QMat M = batch.first;
-  int b;
-  {
-    b = (int)blockIdx.x / (M.n + M.rows);
+  QMat M;
+  int index;
+  if (batch.list) {
+    __shared__ int s_t;
+    if (threadIdx.x == 0) s_t = atomicAdd(batch.ticket, 1);
+    __syncthreads();
+    const int t = s_t;
+    int lo = 0, hi = batch.levels;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      (batch.level[mid] <= t ? lo : hi) = mid;
+    }
+    index = lo;
+    M = batch.list[t - batch.level[lo]];
+  } else {
+    M = batch.first;
+    const int b = (int)blockIdx.x / (M.n + M.rows);
+    index = (int)blockIdx.x - b * (M.n + M.rows);
     M.A += b * batch.sA;
     if (M.Q) M.Q += b * batch.sQ;
     M.R += b * batch.sR;
     M.box += b * batch.sBox;
     if (M.perm) M.perm += b * M.n;
   }
-  const int m = M.m, k = M.k, index = (int)blockIdx.x - b * (M.n + M.rows);
+  const int m = M.m, k = M.k;
   const bool row = index >= M.n;         // a CTA that forms a row of Q
   const int col = row ? m + k : index;  // (rows wait for all reflectors)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = lane >> 4;
@@ -234,7 +256,11 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
 #pragma unroll
     for (int q = 0; q < R; ++q) {
       const int t = tid + q * kNT;
-      if (t < k) M.Q[(int64_t)t * m + index - M.n] = conjg(x[q]);
+      if (t >= k) continue;
+      if (M.adj & 4)
+        M.Q[(int64_t)(index - M.n) * k + t] = x[q];
+      else
+        M.Q[(int64_t)t * m + index - M.n] = conjg(x[q]);
     }
     return;
   }
@@ -302,7 +328,11 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
 #pragma unroll
   for (int q = 0; q < R; ++q) {
     const int t = tid + q * kNT;
-    if (t < m) M.Q[(int64_t)col * m + t] = x[q];
+    if (t >= m) continue;
+    if (M.adj & 4)
+      M.Q[(int64_t)t * k + col] = conjg(x[q]);
+    else
+      M.Q[(int64_t)col * m + t] = x[q];
   }
 }
 
@@ -323,7 +353,7 @@ size_t qr_cols_workspace(int64_t m, int64_t n, int64_t batch) {
 tn_status_t qr_cols_takes(tn_ctx* ctx, int64_t m, int64_t columns, bool* out) {
   static int per_sm[3] = {};
   *out = false;
-  if (m > 4 * kNT) return TN_OK;
+  if (m > kQrColsMaxRows) return TN_OK;
   int& p = per_sm[m <= kNT ? 0 : (m <= 2 * kNT ? 1 : 2)];
   int q = p;
   if (q == 0) {
@@ -337,20 +367,74 @@ tn_status_t qr_cols_takes(tn_ctx* ctx, int64_t m, int64_t columns, bool* out) {
 // thin QR of a batch of m × n matrices op(A)·Π (the caller asked qr_cols_takes with n·batch).
 // Q null: not formed.  perm (n per matrix): the column order Π, null for none.
 tn_status_t qr_cols_batch(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda, int64_t sA, cxd* Q, int64_t sQ,
-                          cxd* R, int64_t sR, int64_t batch, const int* perm, bool adj_in, bool adj_r) {
+                          cxd* R, int64_t sR, int64_t batch, const int* perm, bool adj_in, bool adj_r, bool adj_q) {
   const int64_t k = std::min(m, n);
   const size_t one = boxes_bytes(m, k);
   char* box = ws_take<char>(ctx, one * (size_t)batch);
   TN_CHECK_CUDA(ctx, cudaMemsetAsync(box, 0, one * (size_t)batch, ctx->stream));
   const int64_t rows = Q && (n + m) * batch <= 2 * (int64_t)ctx->num_sms ? m : 0;
   QBatch b = {QMat{A, Q, R, reinterpret_cast<ulonglong2*>(box), perm, lda, (int)m, (int)n, (int)k, (int)rows,
-                   (adj_in ? 1 : 0) + (adj_r ? 2 : 0)},
-              sA, sQ, sR, (int64_t)(one / sizeof(ulonglong2))};
+                   (adj_in ? 1 : 0) + (adj_r ? 2 : 0) + (adj_q ? 4 : 0)},
+              sA, sQ, sR, (int64_t)(one / sizeof(ulonglong2)), nullptr, nullptr, 0, nullptr};
   int* err = nullptr;
   TN_RETURN_IF(wait_error_word(ctx, &err));
   void* args[] = {&b, &err};
   TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel(kernel_for(m), dim3((unsigned)((n + rows) * batch)), dim3(kNT), args, 0,
                                                  ctx->stream));
+  TN_LAUNCHED(ctx);
+  return TN_OK;
+}
+
+size_t qr_cols_list_workspace(const std::vector<QrColsMat>& mats) {
+  size_t boxes = 256;
+  int64_t nmax = 0;
+  for (auto& q : mats) {
+    boxes += boxes_bytes(q.m, std::min(q.m, q.n));
+    nmax = std::max<int64_t>(nmax, q.n);
+  }
+  return ws_round(boxes) + ws_round(sizeof(QMat) * mats.size()) + ws_round(sizeof(int) * (size_t)(nmax + 1));
+}
+
+// thin QR of matrices of different sizes (rows ≤ kQrColsMaxRows) in one launch.  Their columns
+// need not be resident together: a CTA takes the next column of the order from a counter, so
+// whatever it waits for has been taken by a CTA that runs or has finished.  One column of every
+// matrix after the other keeps the matrices' chains running side by side.
+tn_status_t qr_cols_list(tn_ctx* ctx, std::vector<QrColsMat> mats) {
+  if (mats.empty()) return TN_OK;
+  std::stable_sort(mats.begin(), mats.end(), [](const QrColsMat& a, const QrColsMat& b) { return a.n > b.n; });
+  const int nmax = mats[0].n;
+  std::vector<QMat> list;
+  std::vector<int> level(nmax + 1, 0);
+  size_t boxes = 256;  // the counter
+  int64_t total = 0, mmax = 1;
+  for (auto& q : mats) {
+    boxes += boxes_bytes(q.m, std::min(q.m, q.n));
+    total += q.n;
+    mmax = std::max<int64_t>(mmax, q.m);
+  }
+  if (total > 0x7fffffffll) return tn_set_error(ctx, TN_EUNSUPPORTED, "qr: too many columns in a group");
+  char* box = ws_take<char>(ctx, boxes);
+  size_t at = 256;
+  for (auto& q : mats) {
+    const int k = std::min(q.m, q.n);
+    list.push_back(QMat{q.A, q.Q, q.R, reinterpret_cast<ulonglong2*>(box + at), nullptr, q.lda, q.m, q.n, k, 0,
+                        q.adjoint ? 5 : 0});
+    at += boxes_bytes(q.m, k);
+  }
+  for (int c = 0, live = (int)mats.size(); c < nmax; ++c) {
+    while (live > 0 && mats[live - 1].n <= c) --live;
+    level[c + 1] = level[c] + live;
+  }
+  QMat* d_list = ws_take<QMat>(ctx, list.size());
+  int* d_level = ws_take<int>(ctx, level.size());
+  TN_CHECK_CUDA(ctx, cudaMemcpyAsync(d_list, list.data(), sizeof(QMat) * list.size(), cudaMemcpyHostToDevice, ctx->stream));
+  TN_CHECK_CUDA(ctx, cudaMemcpyAsync(d_level, level.data(), sizeof(int) * level.size(), cudaMemcpyHostToDevice, ctx->stream));
+  TN_CHECK_CUDA(ctx, cudaMemsetAsync(box, 0, boxes, ctx->stream));
+  QBatch b = {QMat{}, 0, 0, 0, 0, d_list, d_level, nmax, reinterpret_cast<int*>(box)};
+  int* err = nullptr;
+  TN_RETURN_IF(wait_error_word(ctx, &err));
+  void* args[] = {&b, &err};
+  TN_CHECK_CUDA(ctx, cudaLaunchKernel(kernel_for(mmax), dim3((unsigned)total), dim3(kNT), args, 0, ctx->stream));
   TN_LAUNCHED(ctx);
   return TN_OK;
 }
