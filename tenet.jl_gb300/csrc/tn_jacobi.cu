@@ -1,4 +1,4 @@
-// K4c — persistent FP64 one-sided Jacobi: a column pair per CTA, columns handed from CTA to
+// K4 — persistent FP64 one-sided Jacobi: a column pair per CTA, columns handed from CTA to
 // CTA through flagged packets.
 //
 // What bounds it.  GB300 retires 2 DFMA per clock and SM (a warp's DFMA occupies its
@@ -8,20 +8,25 @@
 // rotation, columns out.  The chain here:
 //  * the columns stay in registers and travel as packets of two 64-bit words, each carrying
 //    32 data bits and the number of the round it is meant for: the receiver polls the data
-//    itself, so there is no fence, no separate flag and no barrier between rounds (one way
-//    555 clocks on the same die, 970 across, measured);
-//  * wᵢᴴwⱼ is reduced by a butterfly that carries Re in one half warp and Im in the other
-//    (5 DADD instead of 10), then across warps with one barrier per round; every warp forms
-//    the rotation itself from the same numbers;
-//  * the rotation's angle and phase come from FP32 (4 approximate MUFU operations instead of
-//    6 FP64 divisions and roots) and are made unitary to FP64 by one scaling (unit_rotation):
-//    the angle's 1e-7 relative error leaves 1e-7 of the coupling, which a later sweep
-//    removes (the stop test counts on it), while W, V and the inner products stay FP64;
+//    itself, so there is no fence, no separate flag and no barrier between rounds;
+//  * columns are held as w = √D·x (Pair): a rotation is 8 products per row, not 12, and needs
+//    neither the cosine nor a unitary correction on the chain; the new D follows its column as a
+//    packet of its own;
+//  * wᵢᴴwⱼ is added up in fixed point (fixed_warp_sum): integers take the place of 7 dependent
+//    DADDs; one barrier per round, after which every warp forms the rotation itself from the
+//    same numbers;
+//  * the tangent comes from FP32 (approximate MUFU operations instead of 6 FP64 divisions and
+//    roots); the rotation is unitary to FP64 for any tangent, whose 1e-7 relative error leaves
+//    1e-7 of the coupling, which a later sweep removes (the stop test counts on it);
 //  * V has CTAs of its own, which get each rotation as packets from the CTA that formed it, so
 //    its half of the FP64 work is off the chain and on other SMs;
 //  * the column norms (cached as unevaluated FP32 sums, updated by t|γ|, recomputed exactly in
-//    FP64 at the start of every sweep) travel with the columns; the stop test is one barrier among a matrix's CTAs per
-//    sweep, so the matrices of a batch converge independently.
+//    FP64 at the start of every sweep, when the scales are taken into the columns) travel with
+//    the columns; the stop test is one barrier among a matrix's CTAs per sweep, so the matrices of a
+//    batch converge independently.
+// A round of 64 to 128 rows is 1.9 µs (2.2 with 12 products, DADD sums and a corrected cosine), of
+// 256 rows 2.6 (3.1), 512 rows 5.8 (7.2); of 1.9 µs the hop is 0.85 (a look at packets in L2 takes
+// ~1000 clocks, 1.3 looks on average), the FP64 products 0.45, and the sums and the angle 0.5.
 // Every wait is bounded: a CTA that waited kSpinLimit polls records an error and leaves, and
 // so do, one limit later each, the CTAs that wait for it.
 #include <algorithm>
@@ -41,10 +46,10 @@ constexpr int kCtl = 4 + 2 * kSweepMax;
 struct Mat {
   cxd* W;             // m × n, dense
   cxd* V;             // n × n, dense, or null
-  double* nrm;        // n
-  ulonglong2* box;    // 2 × N × (2m + 1) packets
+  double* nrm;        // n: ‖wᵢ‖² at the start, Dᵢ at the end of a sweep
+  ulonglong2* box;    // 2 × N × (2m + 2) packets
   ulonglong2* vbox;   // 2 × N × 2n packets (with V)
-  ulonglong2* rot;    // (N − 1) × N/2 × 3 packets: the rotations of a sweep (with V)
+  ulonglong2* rot;    // (N − 1) × N/2 × 3 packets: the rotations of a sweep (with V), and N/2 × 2: the scales
   int* ctl;           // kCtl
   int m, n, N, cta0;  // cta0: the first CTA of this matrix
 };
@@ -121,27 +126,53 @@ __device__ __forceinline__ double widen(float f) {
   const int hi = (int)((b & 0x80000000u) | (((b >> 3) & 0x0fffffffu) + 0x38000000u));
   return (b & 0x7f800000u) ? __hiloint2double(hi, (int)(b << 29)) : 0.0;
 }
-// v · 2^s, truncated to float
-__device__ __forceinline__ float narrow(double v, int s) {
-  const int hi = __double2hiint(v), lo = __double2loint(v);
-  const int e = ((hi >> 20) & 0x7ff) + s - 896;
-  const unsigned m = ((unsigned)(hi & 0xfffff) << 3) | ((unsigned)lo >> 29);
-  const unsigned r = e <= 0 ? 0u : (e >= 255 ? 0x7f800000u : ((unsigned)e << 23) | m);
-  return __uint_as_float(r | (hi & 0x80000000));
-}
 // f · 2^s for a normal f whose result is normal
 __device__ __forceinline__ float shifted(float f, int s) { return __int_as_float(__float_as_int(f) + (s << 23)); }
 
-// (c, s) in FP32 with c² + |s|² = 1 + δ, |δ| ~ 1e-7, made unitary to FP64:
-// (1 + δ)^{-1/2} = 1 − δ/2 + 3δ²/8 + O(δ³), δ exact to one rounding each
-__device__ __forceinline__ void unit_rotation(float cf, float sxf, float syf, double& c, cxd& se) {
-  const double c0 = widen(cf), sx = widen(sxf), sy = widen(syf);
-  const double d = fma(sy, sy, fma(sx, sx, fma(c0, c0, -1.0)));
-  const double h = d * fma(0.375, d, -0.5);
-  c = fma(c0, h, c0);
-  se.x = fma(sx, h, sx);
-  se.y = fma(sy, h, sy);
+// Sums of FP64 values in fixed point: integer additions and the warp's redux take 4 to 30 clocks
+// where a DADD takes 64.  Every lane's value is cut to 55 bits below 2^(emax − 1022), emax the
+// largest exponent field of the warp, so a cut is at most 2⁻⁵⁵ of the largest value: less than
+// the rounding of an FP64 sum.  The parts of 24 bits add up without a carry between them.
+__device__ __forceinline__ unsigned exponent_field(double v) { return ((unsigned)__double2hiint(v) >> 20) & 0x7ff; }
+__device__ __forceinline__ long long fixed_warp_sum(double v, unsigned emax) {
+  const int hi = __double2hiint(v);
+  const unsigned e = exponent_field(v);
+  unsigned long long b = ((unsigned long long)((hi & 0xfffff) | 0x100000) << 34) | ((unsigned long long)(unsigned)__double2loint(v) << 2);
+  b = e ? b >> min(emax - e, 63u) : 0ull;
+  const long long sg = hi >> 31, f = ((long long)b ^ sg) - sg;
+  const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)f & 0xffffffu);
+  const unsigned mid = __reduce_add_sync(0xffffffffu, (unsigned)(f >> 24) & 0xffffffu);
+  const int top = __reduce_add_sync(0xffffffffu, (int)(f >> 48));
+  return ((long long)top << 48) + ((long long)mid << 24) + (long long)lo;
 }
+// |T| < 2⁶³ as a float
+__device__ __forceinline__ float fixed_to_float(long long T) {
+  const unsigned long long A = T < 0 ? (unsigned long long)-T : (unsigned long long)T;
+  const float f = fmaf((float)(unsigned)(A >> 32), 4294967296.f, (float)(unsigned)A);
+  return T < 0 ? -f : f;
+}
+// 1/x of a positive normal x: the hardware's approximation (20 bits or so) and one step of third
+// order, y ← y + y·e(1 + e) with e = 1 − x·y
+__device__ __forceinline__ double reciprocal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// √D = s·2^e for a normal D, s in FP32
+__device__ __forceinline__ void root_of(double D, float& s, int& e) {
+  const int hi = __double2hiint(D), ef = (hi >> 20) - 1023;
+  const float v = __int_as_float(((127 + (ef & 1)) << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)__double2loint(D) >> 29));
+  s = v * rsqrt_approx(v);
+  e = ef >> 1;
+}
+// 2^K, 0 below the normal range
+__device__ __forceinline__ float pow2(int K) { return K < -126 ? 0.f : __int_as_float((min(K, 127) + 127) << 23); }
 
 // a squared column norm relative to ‖W‖²_F as an unevaluated FP32 sum: FP64's 64-clock
 // additions stay off the chain
@@ -156,30 +187,39 @@ __device__ __forceinline__ Norm norm_add(Norm a, float d) {
   r.lo = lo - (r.hi - s);
   return r;
 }
-__device__ __forceinline__ void put_norm(ulonglong2* p, Norm v, unsigned flag) {
+__device__ __forceinline__ void put_words(ulonglong2* p, unsigned x, unsigned y, unsigned flag) {
   const unsigned long long f = (unsigned long long)flag << 32;
-  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(__float_as_uint(v.hi) | f),
-               "l"(__float_as_uint(v.lo) | f)
-               : "memory");
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(x | f), "l"(y | f) : "memory");
 }
 
-// x' = c·x − conj(se)·y, y' = se·x + c·y
-__device__ __forceinline__ void rotate(double c, cxd se, cxd& x, cxd& y) {
-  const cxd a = mkcx(fma(c, x.x, fma(-se.x, y.x, -se.y * y.y)), fma(c, x.y, fma(-se.x, y.y, se.y * y.x)));
-  const cxd b = mkcx(fma(c, y.x, fma(se.x, x.x, -se.y * x.y)), fma(c, y.y, fma(se.x, x.y, se.y * x.x)));
-  x = a;
-  y = b;
+// Columns are held as w = √D·x.  With a any complex number, q = Dx/Dy, b = q·a and
+// w = 1 + Re(ā b),   x ← x − ā y,  y ← y + b x,  D ← D/w
+// is a unitary rotation of the columns by the tangent a√q: 8 products per row instead of 12,
+// and no square root; the scales are off the chain of the columns.
+struct Pair {
+  double ax, ay, bx, by;
+};
+__device__ __forceinline__ cxd turned_x(const Pair& p, cxd x, cxd y) {
+  return mkcx(fma(-p.ax, y.x, fma(-p.ay, y.y, x.x)), fma(-p.ax, y.y, fma(p.ay, y.x, x.y)));
 }
-
-// the same, or with two threads per row only the output column of this one's side
+__device__ __forceinline__ cxd turned_y(const Pair& p, cxd x, cxd y) {
+  return mkcx(fma(p.bx, x.x, fma(-p.by, x.y, y.x)), fma(p.bx, x.y, fma(p.by, x.x, y.y)));
+}
+// with two threads per row only the output column of this one's side, by one expression
 template <bool SPLIT>
-__device__ __forceinline__ void rotate_side(double c, cxd se, cxd& x, cxd& y, int side) {
+__device__ __forceinline__ void rotate_side(const Pair& p, cxd& x, cxd& y, int side) {
   if (!SPLIT) {
-    rotate(c, se, x, y);
-  } else if (side == 0) {
-    x = mkcx(fma(c, x.x, fma(-se.x, y.x, -se.y * y.y)), fma(c, x.y, fma(-se.x, y.y, se.y * y.x)));
+    const cxd old = x;
+    x = turned_x(p, old, y);
+    y = turned_y(p, old, y);
   } else {
-    y = mkcx(fma(c, y.x, fma(se.x, x.x, -se.y * x.y)), fma(c, y.y, fma(se.x, x.y, se.y * x.x)));
+    const double c1 = side ? p.bx : -p.ax, c2 = side ? -p.by : -p.ay;
+    const cxd o = side ? y : x, z = side ? x : y;
+    const cxd v = mkcx(fma(c1, z.x, fma(c2, z.y, o.x)), fma(c1, z.y, fma(-c2, z.x, o.y)));
+    if (side)
+      y = v;
+    else
+      x = v;
   }
 }
 
@@ -219,41 +259,54 @@ __device__ __forceinline__ void v_role(const Mat& M, int k, bool v_given, int ma
       const ulonglong2* bi = M.vbox + ((int64_t)(flag & 1) * N + i) * colp;
       const ulonglong2* bj = M.vbox + ((int64_t)(flag & 1) * N + (two ? j : i)) * colp;
       const ulonglong2* br = M.rot + ((int64_t)r * pairs + k) * 3;
-      double c;
-      cxd se;
+      Pair p;
+      double fx = 1.0, fy = 1.0;
       long long spins = 0;
       bool ok;
       do {
         const ulonglong2 r0 = get_raw(br), r1 = get_raw(br + 1), r2 = get_raw(br + 2);
         ok = arrived(r0, flag + 1) && arrived(r1, flag + 1) && arrived(r2, flag + 1);
-        c = value_of(r0);
-        se = mkcx(value_of(r1), value_of(r2));
+        p.ax = widen(__uint_as_float((unsigned)r0.x));
+        p.ay = widen(__uint_as_float((unsigned)r0.y));
+        p.bx = value_of(r1);
+        p.by = value_of(r2);
       } while (!ok && ++spins < kSpinLimit);
+      if (r == 0 && flag > 0) {  // the scales are taken into the columns once a sweep
+        const ulonglong2* bs = M.rot + ((int64_t)(N - 1) * pairs) * 3 + 2 * k;
+        bool got;
+        do {
+          const ulonglong2 r0 = get_raw(bs), r1 = get_raw(bs + 1);
+          got = arrived(r0, flag + 1) && arrived(r1, flag + 1);
+          fx = value_of(r0);
+          fy = value_of(r1);
+        } while (!got && ++spins < kSpinLimit);
+        ok = ok && got;
+      }
       if (flag > 0) {
         constexpr int RC = R < 2 ? R : 2;
 #pragma unroll
         for (int q0 = 0; q0 < R; q0 += RC) {
           bool got;
           do {
-            ulonglong2 p[4 * RC];
+            ulonglong2 u[4 * RC];
             got = true;
 #pragma unroll
             for (int q = 0; q < RC; ++q) {
               const int t = row(q0 + q);
               if (t < n) {
-                p[4 * q] = get_raw(bi + t);
-                p[4 * q + 1] = get_raw(bi + n + t);
-                p[4 * q + 2] = get_raw(bj + t);
-                p[4 * q + 3] = get_raw(bj + n + t);
+                u[4 * q] = get_raw(bi + t);
+                u[4 * q + 1] = get_raw(bi + n + t);
+                u[4 * q + 2] = get_raw(bj + t);
+                u[4 * q + 3] = get_raw(bj + n + t);
               }
             }
 #pragma unroll
             for (int q = 0; q < RC; ++q)
               if (row(q0 + q) < n) {
-                got = got && arrived(p[4 * q], flag) && arrived(p[4 * q + 1], flag) && arrived(p[4 * q + 2], flag) &&
-                      arrived(p[4 * q + 3], flag);
-                x[q0 + q] = mkcx(value_of(p[4 * q]), value_of(p[4 * q + 1]));
-                y[q0 + q] = mkcx(value_of(p[4 * q + 2]), value_of(p[4 * q + 3]));
+                got = got && arrived(u[4 * q], flag) && arrived(u[4 * q + 1], flag) && arrived(u[4 * q + 2], flag) &&
+                      arrived(u[4 * q + 3], flag);
+                x[q0 + q] = mkcx(value_of(u[4 * q]), value_of(u[4 * q + 1]));
+                y[q0 + q] = mkcx(value_of(u[4 * q + 2]), value_of(u[4 * q + 3]));
               }
           } while (!got && ++spins < kSpinLimit);
           ok = ok && got;
@@ -267,9 +320,17 @@ __device__ __forceinline__ void v_role(const Mat& M, int k, bool v_given, int ma
       // read the packets that the column's next holder will overwrite
       if (SPLIT) __syncthreads();
       if (SPLIT ? s_vfail != 0 : !ok) return;
-      if (se.x != 0.0 || se.y != 0.0) {
+      if (r == 0 && flag > 0) {
 #pragma unroll
-        for (int q = 0; q < R; ++q) rotate_side<SPLIT>(c, se, x[q], y[q], side);
+        for (int q = 0; q < R; ++q) {
+          x[q] = mkcx(x[q].x * fx, x[q].y * fx);
+          y[q] = mkcx(y[q].x * fy, y[q].y * fy);
+        }
+      }
+      if (p.ax != 0.0 || p.ay != 0.0) {
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+          if (R == 1 || q * kNT + (tid & ~31) < n) rotate_side<SPLIT>(p, x[q], y[q], side);
       }
       const unsigned next = flag + 1;
       ulonglong2* oi = M.vbox + ((int64_t)(next & 1) * N + i) * colp;
@@ -292,12 +353,13 @@ __device__ __forceinline__ void v_role(const Mat& M, int k, bool v_given, int ma
     if (!mat_barrier(M.ctl, arrivals, err)) return;
     more = __ldcg(&M.ctl[4 + kSweepMax + sweep]) > 0 && __int_as_float(__ldcg(&M.ctl[4 + sweep])) > stop_ratio;
   }
+  const double fx = sqrt(__ldcg(&M.nrm[i])), fy = j < n ? sqrt(__ldcg(&M.nrm[j])) : 0.0;
 #pragma unroll
   for (int q = 0; q < R; ++q) {
     const int t = row(q);
     if (t >= n) continue;
-    if (!SPLIT || side == 0) M.V[(int64_t)i * n + t] = x[q];
-    if (j < n && (!SPLIT || side == 1)) M.V[(int64_t)j * n + t] = y[q];
+    if (!SPLIT || side == 0) M.V[(int64_t)i * n + t] = mkcx(x[q].x * fx, x[q].y * fx);
+    if (j < n && (!SPLIT || side == 1)) M.V[(int64_t)j * n + t] = mkcx(y[q].x * fy, y[q].y * fy);
   }
 }
 
@@ -324,8 +386,10 @@ __global__ void __launch_bounds__(kNT, 4)
   const int k = (int)blockIdx.x - M.cta0, ctas = M.V ? 2 * pairs : pairs;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = lane >> 4, side = SPLIT ? tid >> 6 : 0;
   __shared__ double red[2][4][2];
+  __shared__ __align__(16) long long fix[2][2][4];  // parity, Re or Im, warp
+  __shared__ __align__(16) int fix_e[2][2][4];
   __shared__ int s_fail;
-  const int64_t colp = 2 * (int64_t)m + 1;
+  const int64_t colp = 2 * (int64_t)m + 2;
   if (tid == 0) s_fail = 0;
   auto row = [&](int q) { return SPLIT ? tid & 63 : tid + q * kNT; };
 
@@ -339,8 +403,8 @@ __global__ void __launch_bounds__(kNT, 4)
     y[q] = (t < m && j < n) ? M.W[(int64_t)j * m + t] : mkcx(0.0, 0.0);
   }
   // Σ over the CTA of (a, b): lanes 0-15 get Σa, lanes 16-31 Σb.  SPLIT: the threads of side 0
-  // bring a, those of side 1 b.  One barrier; `between` runs before it.
-  auto block_sum2 = [&](double a, double b, auto between) -> double {
+  // bring a, those of side 1 b. One barrier.
+  auto block_sum2 = [&](double a, double b) -> double {
     if (SPLIT) {
       const double s = warp_sum(side ? b : a);
       if (lane == 0) red[buf][warp & 1][side] = s;
@@ -348,7 +412,6 @@ __global__ void __launch_bounds__(kNT, 4)
       const double s = warp_sum2(a, b, lane);
       if ((lane & 15) == 0) red[buf][warp][half] = s;
     }
-    between();
     __syncthreads();
     double v = red[buf][lane & (SPLIT ? 1 : 3)][half];
     v += __shfl_xor_sync(0xffffffffu, v, 1);
@@ -364,7 +427,7 @@ __global__ void __launch_bounds__(kNT, 4)
       a = fma(x[q].x, x[q].x, fma(x[q].y, x[q].y, a));
       b = fma(y[q].x, y[q].x, fma(y[q].y, y[q].y, b));
     }
-    const double v = block_sum2(a, b, [] {});
+    const double v = block_sum2(a, b);
     al = __shfl_sync(0xffffffffu, v, 0);
     be = __shfl_sync(0xffffffffu, v, 16);
   };
@@ -387,17 +450,41 @@ __global__ void __launch_bounds__(kNT, 4)
   constexpr double kEps = 2.220446049250313e-16;
   int ex = 0;
   frexp(fro, &ex);
-  ex = max(min(ex, 1000), -1000);
-  const double scale = ldexp(1.0, -ex);  // norms are kept relative to 2^ex ≈ ‖W‖²_F
+  ex = max(min(ex, 1000), -1000) >> 1;
+  // the columns are kept relative to 2^ex ≈ ‖W‖_F, their norms to its square
+  const double scale = ldexp(1.0, -2 * ex), scale1 = ldexp(1.0, -ex);
   const float floor2 = fmaxf((float)(fmax(kEps * kEps * fro, 1e-290) * scale), 1.2e-37f);
   auto as_norm = [&](double v) {
-    const double s = v * scale;
     Norm r;
-    r.hi = (float)s;
-    r.lo = (float)(s - (double)r.hi);
+    r.hi = (float)v;
+    r.lo = (float)(v - (double)r.hi);
     return r;
   };
-  Norm na = as_norm(al), nb = as_norm(be);
+  auto take_scales = [&](double fx, double fy) {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      x[q] = mkcx(x[q].x * fx, x[q].y * fx);
+      y[q] = mkcx(y[q].x * fy, y[q].y * fy);
+    }
+  };
+  take_scales(scale1, scale1);
+  Norm na = as_norm(al * scale), nb = as_norm(be * scale);
+  double Dx = 1.0, Dy = 1.0;
+  // The scales D/w that a round leaves, x's in lanes 0-15 of the last warp, y's in lanes 16-31.  With
+  // four rows per thread they are formed while the next round's first look at the packets is on its
+  // way (512 rows: 6.0 → 5.8 µs a round); with fewer they would arrive too late for their reader
+  // (64 rows: 1.92 → 2.02).
+  constexpr bool kScalesLater = R == 4;
+  Pair p = {0.0, 0.0, 0.0, 0.0};
+  bool turned = false, pending = false;
+  ulonglong2* dst = nullptr;
+  auto send_scales = [&](unsigned f) -> double {
+    double D = half ? Dy : Dx;
+    if (turned) D *= reciprocal(fma(p.ax, p.bx, fma(p.ay, p.by, 1.0)));
+    if (dst) put(dst, D, f);
+    pending = false;
+    return D;
+  };
 
   unsigned flag = 0;  // the round counter carried by the packets, over all sweeps
   int sweep = 0;
@@ -407,6 +494,21 @@ __global__ void __launch_bounds__(kNT, 4)
     int count = 0;
 #pragma unroll 1
     for (int r = 0; r < N - 1; ++r, ++flag) {
+      long long spins = 0;
+      const ulonglong2 *bD = nullptr, *bE = nullptr;
+      ulonglong2 d0, d1;
+      auto scales_in = [&] {
+        while (!(arrived(d0, flag) && arrived(d1, flag)) && ++spins < kSpinLimit) {
+          d0 = get_raw(bD);
+          d1 = get_raw(bE);
+        }
+        if (spins >= kSpinLimit) {
+          atomicExch(err, 1);
+          s_fail = 1;
+        }
+        Dx = value_of(d0);
+        Dy = value_of(d1);
+      };
       if (flag > 0) {
         circle_pair(N, r, k, i, j);
         const bool two = j < n;
@@ -415,40 +517,54 @@ __global__ void __launch_bounds__(kNT, 4)
         // (two rows of both columns at a time: more packets in flight cost the registers that
         // keep four CTAs of 512 rows on an SM)
         constexpr int RC = R < 2 ? R : 2;
-        long long spins = 0;
+        spins = 0;
         bool ok = true;
+        struct Look {
+          ulonglong2 p[4 * RC], a, b;
+        };
+        auto look = [&](Look& l, int q0) {
+#pragma unroll
+          for (int q = 0; q < RC; ++q) {
+            const int t = row(q0 + q);
+            if (t < m) {
+              l.p[4 * q] = get_raw(bi + t);
+              l.p[4 * q + 1] = get_raw(bi + m + t);
+              l.p[4 * q + 2] = get_raw(bj + t);
+              l.p[4 * q + 3] = get_raw(bj + m + t);
+            }
+          }
+          if (q0 == 0) {
+            l.a = get_raw(bi + 2 * m);
+            l.b = get_raw(bj + 2 * m);
+          }
+        };
+        auto take = [&](const Look& l, int q0) -> bool {
+          bool got = true;
+          if (q0 == 0) {
+            got = arrived(l.a, flag) && arrived(l.b, flag);
+            na.hi = __uint_as_float((unsigned)l.a.x);
+            na.lo = __uint_as_float((unsigned)l.a.y);
+            nb.hi = __uint_as_float((unsigned)l.b.x);
+            nb.lo = __uint_as_float((unsigned)l.b.y);
+          }
+#pragma unroll
+          for (int q = 0; q < RC; ++q)
+            if (row(q0 + q) < m) {
+              got = got && arrived(l.p[4 * q], flag) && arrived(l.p[4 * q + 1], flag) && arrived(l.p[4 * q + 2], flag) &&
+                    arrived(l.p[4 * q + 3], flag);
+              x[q0 + q] = mkcx(value_of(l.p[4 * q]), value_of(l.p[4 * q + 1]));
+              y[q0 + q] = mkcx(value_of(l.p[4 * q + 2]), value_of(l.p[4 * q + 3]));
+            }
+          return got;
+        };
 #pragma unroll
         for (int q0 = 0; q0 < R; q0 += RC) {
           bool got;
           do {
-            ulonglong2 p[4 * RC];
-#pragma unroll
-            for (int q = 0; q < RC; ++q) {
-              const int t = row(q0 + q);
-              if (t < m) {
-                p[4 * q] = get_raw(bi + t);
-                p[4 * q + 1] = get_raw(bi + m + t);
-                p[4 * q + 2] = get_raw(bj + t);
-                p[4 * q + 3] = get_raw(bj + m + t);
-              }
-            }
-            got = true;
-            if (q0 == 0) {
-              const ulonglong2 pa = get_raw(bi + 2 * m), pb = get_raw(bj + 2 * m);
-              got = arrived(pa, flag) && arrived(pb, flag);
-              na.hi = __uint_as_float((unsigned)pa.x);
-              na.lo = __uint_as_float((unsigned)pa.y);
-              nb.hi = __uint_as_float((unsigned)pb.x);
-              nb.lo = __uint_as_float((unsigned)pb.y);
-            }
-#pragma unroll
-            for (int q = 0; q < RC; ++q)
-              if (row(q0 + q) < m) {
-                got = got && arrived(p[4 * q], flag) && arrived(p[4 * q + 1], flag) && arrived(p[4 * q + 2], flag) &&
-                      arrived(p[4 * q + 3], flag);
-                x[q0 + q] = mkcx(value_of(p[4 * q]), value_of(p[4 * q + 1]));
-                y[q0 + q] = mkcx(value_of(p[4 * q + 2]), value_of(p[4 * q + 3]));
-              }
+            Look l;
+            look(l, q0);
+            if (kScalesLater && q0 == 0 && pending) send_scales(flag);
+            got = take(l, q0);
           } while (!got && ++spins < kSpinLimit);
           ok = ok && got;
         }
@@ -456,83 +572,148 @@ __global__ void __launch_bounds__(kNT, 4)
           atomicExch(err, 1);
           s_fail = 1;
         }
-        if (r == 0) {
+        // the scales follow their columns; they are looked for now and looked at before the barrier
+        bD = bi + 2 * m + 1;
+        bE = bj + 2 * m + 1;
+        d0 = get_raw(bD);
+        d1 = get_raw(bE);
+        if (r == 0) {  // once a sweep they are taken into the columns
+          scales_in();
+          const double fx = sqrt(Dx), fy = sqrt(Dy);
+          take_scales(fx, fy);
+          if (M.V && tid < 2) put(M.rot + ((int64_t)(N - 1) * pairs) * 3 + 2 * k + tid, tid ? fy : fx, flag + 1);
           exact_norms(al, be);
           na = as_norm(al);
           nb = as_norm(be);
+          Dx = Dy = 1.0;
         }
       }
       const bool two = j < n;
-      // γ = xᴴy
+      const unsigned next = flag + 1;
+      ulonglong2* oi = M.box + ((int64_t)(next & 1) * N + i) * colp;
+      ulonglong2* oj = M.box + ((int64_t)(next & 1) * N + j) * colp;
+      // what needs only the norms: the pair's scale 2^e ≈ √(αβ), 2^e/√(αβ) and (β − α)/√(αβ) (of no
+      // meaning unless live; without a branch they fit between the FP64 products that follow)
+      const bool live = two && na.hi > floor2 && nb.hi > floor2 && na.hi < 3e38f && nb.hi < 3e38f;
+      const int e = (((__float_as_int(na.hi) >> 23) + (__float_as_int(nb.hi) >> 23)) >> 1) - 127;
+      const float fa = shifted(na.hi, -e), fb = shifted(nb.hi, -e);
+      const float ra = rsqrt_approx(fa), rb = rsqrt_approx(fb), sa = fa * ra, sb = fb * rb, isab = ra * rb;
+      const float dif = ((nb.hi - na.hi) + (nb.lo - na.lo)) * shifted(1.f, -e) * isab;
+      // γ = xᴴy (of the columns as held)
       double gx = 0, gy = 0;
+      if (SPLIT) {
+        gx = gy = fma(x[0].x, side ? y[0].y : y[0].x, x[0].y * (side ? -y[0].x : y[0].y));
+      } else {
 #pragma unroll
-      for (int q = 0; q < R; ++q) {
-        if (!SPLIT || side == 0) gx = fma(x[q].x, y[q].x, fma(x[q].y, y[q].y, gx));
-        if (!SPLIT || side == 1) gy = fma(x[q].x, y[q].y, fma(-x[q].y, y[q].x, gy));
-      }
-      // what needs only the norms is formed while the partial sums settle: the pair's scale
-      // 2^e ≈ √(αβ), 2^e/√(αβ) and (β − α)/√(αβ)
-      const bool live = two && na.hi > floor2 && nb.hi > floor2;
-      int e = 0;
-      float sa = 1.f, sb = 1.f, isab = 1.f, dif = 0.f;
-      const double v = block_sum2(gx, gy, [&] {
-        if (live) {
-          e = (((__float_as_int(na.hi) >> 23) + (__float_as_int(nb.hi) >> 23)) >> 1) - 127;
-          const float a = shifted(na.hi, -e), b = shifted(nb.hi, -e);
-          const float ra = rsqrtf(a), rb = rsqrtf(b);
-          sa = a * ra;
-          sb = b * rb;
-          isab = ra * rb;
-          const float d = (nb.hi - na.hi) + (nb.lo - na.lo);
-          dif = d * shifted(1.f, -e) * isab;
+        for (int q = 0; q < R; ++q) {
+          if (R > 1 && q * kNT + warp * 32 >= m) continue;
+          gx = fma(x[q].x, y[q].x, fma(x[q].y, y[q].y, gx));
+          gy = fma(x[q].x, y[q].y, fma(-x[q].y, y[q].x, gy));
         }
-      });
-      if (s_fail) return;  // (set before the barrier by a thread whose wait ran out)
+      }
+      // (SPLIT: a warp has one of the two)
+      const unsigned we = __reduce_max_sync(0xffffffffu, max(exponent_field(gx), exponent_field(gy)));
+      if (SPLIT) {
+        const long long s = fixed_warp_sum(side ? gy : gx, we);
+        if (lane == 0) {
+          fix[buf][side][warp & 1] = s;
+          fix_e[buf][side][warp & 1] = (int)we;
+        }
+      } else {
+        const long long s0 = fixed_warp_sum(gx, we), s1 = fixed_warp_sum(gy, we);
+        if (lane == 0) {
+          fix[buf][0][warp] = s0;
+          fix[buf][1][warp] = s1;
+          fix_e[buf][0][warp] = fix_e[buf][1][warp] = (int)we;
+        }
+      }
+      if (flag > 0 && r > 0) scales_in();
+      __syncthreads();
+      // √D = s·2^se as floats for the angle
+      float sx, sy;
+      int ex_x, ex_y;
+      root_of(Dx, sx, ex_x);
+      root_of(Dy, sy, ex_y);
+      // (a ratio of scales beyond 2^±60 waits for the next sweep's columns of scale 1)
+      const float ratio = abs(ex_y - ex_x) > 60 ? 0.f : __fdividef(sy, sx) * pow2(ex_y - ex_x);
+      const double q = Dx * reciprocal(Dy);
+      long long total;
+      int E;
+      if (SPLIT) {
+        const int e0 = fix_e[buf][half][0], e1 = fix_e[buf][half][1];
+        E = max(e0, e1);
+        total = (fix[buf][half][0] >> min(E - e0, 63)) + (fix[buf][half][1] >> min(E - e1, 63));
+      } else {
+        const int4 ew = *reinterpret_cast<const int4*>(fix_e[buf][half]);
+        E = max(max(ew.x, ew.y), max(ew.z, ew.w));
+        total = ((fix[buf][half][0] >> min(E - ew.x, 63)) + (fix[buf][half][1] >> min(E - ew.y, 63))) +
+                ((fix[buf][half][2] >> min(E - ew.z, 63)) + (fix[buf][half][3] >> min(E - ew.w, 63)));
+      }
+      buf ^= 1;
       // ρ = γ/√(αβ)
-      const float rl = narrow(v, -ex - e) * isab;
+      const float rl = fixed_to_float(total) * (sx * sy * isab) * pow2(E - 1077 + ex_x + ex_y - e);
       const float rx = __shfl_sync(0xffffffffu, rl, 0), ry = __shfl_sync(0xffffffffu, rl, 16);
       const float rho2 = rx * rx + ry * ry;
       const bool apply = live && rho2 > tol2;
       if (live) worst = fmaxf(worst, rho2);
-      double c = 1.0;
-      cxd se = mkcx(0.0, 0.0);
+      p = {0.0, 0.0, 0.0, 0.0};
+      float axf = 0.f, ayf = 0.f;
       if (apply) {
         ++count;
         // t = sgn(ζ)/(|ζ| + √(1 + ζ²)), ζ = (β − α)/(2|γ|), without forming the quotient
-        const float irho = rsqrtf(rho2), rho = rho2 * irho;
+        const float irho = rsqrt_approx(rho2), rho = rho2 * irho;
         const float q2 = fmaf(dif, dif, 4.f * rho2);
-        const float t = copysignf(__fdividef(2.f * rho, fabsf(dif) + q2 * rsqrtf(q2)), dif);
-        const float cf = rsqrtf(fmaf(t, t, 1.f)), sf = cf * t * irho;
-        unit_rotation(cf, sf * rx, sf * ry, c, se);
+        float t = copysignf(__fdividef(2.f * rho, fabsf(dif) + q2 * rsqrt_approx(q2)), dif);
+        if (ratio == 0.f) t = 0.f;
+        const float g = t * irho * ratio;
+        axf = g * rx;
+        ayf = g * ry;
+        p.ax = widen(axf);
+        p.ay = widen(ayf);
+        if (!SPLIT || side) {
+          p.bx = p.ax * q;
+          p.by = p.ay * q;
+        }
+#pragma unroll
+        for (int u = 0; u < R; ++u)
+          if (R == 1 || u * kNT + warp * 32 < m) rotate_side<SPLIT>(p, x[u], y[u], side);
         // α − t|γ|, β + t|γ|
         const float tag = t * rho * (sa * shifted(1.f, e)) * sb;
         na = norm_add(na, -tag);
         nb = norm_add(nb, tag);
-#pragma unroll
-        for (int q = 0; q < R; ++q) rotate_side<SPLIT>(c, se, x[q], y[q], side);
       }
-      const unsigned next = flag + 1;
-      ulonglong2* oi = M.box + ((int64_t)(next & 1) * N + i) * colp;
-      ulonglong2* oj = M.box + ((int64_t)(next & 1) * N + j) * colp;
 #pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const int t = row(q);
+      for (int u = 0; u < R; ++u) {
+        const int t = row(u);
         if (t >= m) continue;
         if (!SPLIT || side == 0) {
-          put(oi + t, x[q].x, next);
-          put(oi + m + t, x[q].y, next);
+          put(oi + t, x[u].x, next);
+          put(oi + m + t, x[u].y, next);
         }
         if (two && (!SPLIT || side == 1)) {
-          put(oj + t, y[q].x, next);
-          put(oj + m + t, y[q].y, next);
+          put(oj + t, y[u].x, next);
+          put(oj + m + t, y[u].y, next);
         }
       }
-      if (tid == 0) put_norm(oi + 2 * m, na, next);
-      if (tid == 32 && two) put_norm(oj + 2 * m, nb, next);
-      if (M.V && tid >= 96 && tid < 99) {
-        const int w = tid - 96;
-        put(M.rot + ((int64_t)r * pairs + k) * 3 + w, w == 0 ? c : (w == 1 ? se.x : se.y), next);
+      if (warp == 3) {
+        turned = apply;
+        pending = true;
+        dst = (lane & 15) == 0 && (two || half == 0) ? (half ? oj : oi) + 2 * m + 1 : nullptr;
+        if (!kScalesLater || r == N - 2) {
+          const double D = send_scales(next);
+          if (dst && r == N - 2) M.nrm[half ? j : i] = D;
+        }
+      } else if (lane == 0 && warp < 2 && (two || warp == 0)) {
+        const Norm v = warp ? nb : na;
+        put_words((warp ? oj : oi) + 2 * m, __float_as_uint(v.hi), __float_as_uint(v.lo), next);
+      } else if (warp == 2 && M.V && lane < 3) {
+        ulonglong2* o = M.rot + ((int64_t)r * pairs + k) * 3 + lane;
+        if (lane == 0)
+          put_words(o, __float_as_uint(axf), __float_as_uint(ayf), next);
+        else
+          put(o, lane == 1 ? p.bx : p.by, next);
       }
+      if (s_fail) return;  // (set before the barrier by a thread whose wait ran out)
     }
     // stop test: a sweep whose largest ratio is ρ leaves ~ρ² for the next one
     if (tid == 0) {
@@ -544,6 +725,8 @@ __global__ void __launch_bounds__(kNT, 4)
     more = __ldcg(&M.ctl[4 + kSweepMax + sweep]) > 0 && __int_as_float(__ldcg(&M.ctl[4 + sweep])) > stop_ratio;
     ++sweep;
   }
+  const double back = ldexp(1.0, ex);
+  take_scales(sqrt(__ldcg(&M.nrm[i])) * back, j < n ? sqrt(__ldcg(&M.nrm[j])) * back : 0.0);
 #pragma unroll
   for (int q = 0; q < R; ++q) {
     const int t = row(q);
@@ -571,7 +754,7 @@ constexpr int64_t kMaxCtas = 152 * 6;
 // packets of a matrix: W's columns and norms, V's columns, the rotations of a sweep
 size_t packets(int64_t m, int64_t n, bool with_v) {
   const int64_t N = n + (n & 1);
-  return (size_t)(2 * N * (2 * m + 1) + (with_v ? 2 * N * 2 * n + (N - 1) * (N / 2) * 3 : 0));
+  return (size_t)(2 * N * (2 * m + 2) + (with_v ? 2 * N * 2 * n + (N - 1) * (N / 2) * 3 + N : 0));
 }
 
 }  // namespace
@@ -666,7 +849,7 @@ tn_status_t jacobi_pairs(tn_ctx* ctx, const std::vector<JacobiMat>& mats, bool v
       M.cta0 = cta;
       M.ctl = ctl + kCtl * q;
       M.box = box;
-      M.vbox = M.box + (size_t)2 * N * (2 * src.m + 1);
+      M.vbox = M.box + (size_t)2 * N * (2 * src.m + 2);
       M.rot = M.vbox + (size_t)2 * N * 2 * src.n;
       box += packets(src.m, src.n, with_v);
       for (int64_t c = 0; c < ctas_of(src); ++c) ho[cta++] = (int)q;

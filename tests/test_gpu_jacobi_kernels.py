@@ -65,6 +65,23 @@ def test_native_svd(ctx, m, n, batch):
     _check(A, *_svd(ctx, A, 0), 1e-13)
 
 
+@pytest.mark.parametrize("m,n", [(23, 23), (64, 2), (65, 3), (129, 22), (257, 23), (512, 8), (300, 300)])
+@pytest.mark.parametrize("kind", ["parallel", "repeated", "zero"])
+def test_large_rotations(ctx, m, n, kind):
+    """Columns that are almost one another, equal or zero: angles of 45° round after round, which the
+    columns' scales take up, and pairs that must be left alone."""
+    rng = np.random.default_rng(m * 1000 + n)
+    A = _gauss(rng, (m, n))
+    if kind == "parallel":
+        A = A[:, :1] * np.exp(2j * np.pi * rng.random(n)) + 1e-3 * A
+    elif kind == "repeated":
+        A = A[:, rng.integers(0, (n + 1) // 2, n)] * rng.choice([1, -1, 1j], n)
+    else:
+        A[:, rng.permutation(n)[: n // 2]] = 0
+    U, S, Vh = _svd(ctx, A[None], 0)
+    _check(A[None], U, S, Vh, 1e-13)
+
+
 @pytest.mark.parametrize("m,n,batch", [(128, 128, 1), (129, 128, 2), (200, 150, 1), (256, 255, 1), (385, 130, 3), (512, 512, 1)])
 def test_mixed_svd(ctx, m, n, batch):
     rng = np.random.default_rng(m * 1000 + n)
