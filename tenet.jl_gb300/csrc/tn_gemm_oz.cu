@@ -31,16 +31,25 @@
 // The only approximation is the dropped pairs (p + q ≥ S) and the digit remainders, of
 // relative size ~S·2^{1-bS} per product: S = 8, b = 7 gives ~52 bits, FP64-grade products.
 //
-// Kernel.  One CTA (6 warps) per 128×64 tile of the real 4M product, for one batch
-// instance.  Warp 4 lane 0 issues TMA loads: per K stage (64 BF16 = 128 bytes, 128-byte
-// swizzle) all S digit planes of the B tile into one of two B buffers, then the S planes
-// of the A tile through a 4-slot ring.  Warp 5 lane 0 issues tcgen05.mma (M=128, N=64,
-// K=16): for plane p of A it multiplies every resident B plane q < S − p into level
-// p + q (TMEM columns 64·(p+q)…).  Warps 0-3 then read the S level accumulators with
-// tcgen05.ld (warp w owns rows 32w…32w+31), combine them in int64, exchange Re/Im with
-// the neighbouring lane and write interleaved complex C.  Every mbarrier wait is
-// bounded: on timeout the kernel records an error word, skips the remaining work and
-// still releases its TMEM.
+// Kernel.  One persistent CTA (6 warps) per SM takes 128×64 tiles of the real 4M product of all
+// batch instances in turn.  Warp 4 lane 0 issues TMA loads: a K stage is 32 BF16 (64 bytes,
+// 64-byte swizzle) of all S digit planes of both tiles, two stages in shared memory.  Warp 5
+// lane 0 issues tcgen05.mma (M=128, K=16): plane p of A against every plane q < S − p of
+// B, into level p + q (TMEM columns 64·(p+q)…).  After that group plane p of A and plane S−1−p
+// of B are not needed again in this stage, so their place is given back to the producer group by
+// group, one stage ahead of its next use.  Warps 0-3 read the S level accumulators with
+// tcgen05.ld (warp w owns rows 32w…32w+31) into int64 sums in registers, give the accumulators
+// back to warp 5, and finish and write C while the next tile is multiplied.
+// Every mbarrier wait is bounded: on timeout the kernel records an error word, skips the
+// remaining work and still releases its TMEM.
+//
+// What bounds it: the operands' way into shared memory.  The S planes of B lie one after the
+// other and so do the levels, so up to four planes of B are one operand of N = 256: a tile of
+// k = 256 takes 35 thousand clocks of tensor pipe (a product per pair of planes, N = 64, took 81
+// clocks each, 90 thousand), its 1.5 MB of planes 53 thousand at the 29 bytes per clock and SM
+// that come from L2.  Reading the accumulators takes 12 thousand more; the rest of the epilogue (3
+// thousand; with 14 FP64 operations of 64 clocks per column 88 to 129) runs beside the next tile.
+// 16 products of 512 × 512 × 512: 1.97 → 0.77 ms, of it the operand preparation 0.54 → 0.24.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -51,15 +60,14 @@
 
 namespace {
 
-constexpr int OZ_BM = 128, OZ_BN = 64, OZ_BK = 64;  // tile 128×64, 64 BF16 (128 B) of K per stage
+constexpr int OZ_BM = 128, OZ_BN = 64, OZ_BK = 32;  // tile 128×64, 32 BF16 (64 B) of K per stage
 constexpr int OZ_MAX_S = 8;
-constexpr int OZ_A_RING = 4;
-constexpr int OZ_A_TILE = OZ_BM * OZ_BK * 2;  // 16 KB
-constexpr int OZ_B_TILE = OZ_BN * OZ_BK * 2;  // 8 KB
+constexpr int OZ_A_TILE = OZ_BM * OZ_BK * 2;  // 8 KB
+constexpr int OZ_B_TILE = OZ_BN * OZ_BK * 2;  // 4 KB
 constexpr int OZ_THREADS = 192;
 constexpr long long kOzSpin = 1ll << 24;
 
-inline int oz_smem_bytes(int S) { return OZ_A_RING * OZ_A_TILE + 2 * S * OZ_B_TILE + 1024 + 256; }
+inline int oz_smem_bytes(int S) { return 2 * S * (OZ_A_TILE + OZ_B_TILE) + 1024 + 512; }
 
 struct OzMaps {
   CUtensorMap a;  // digit planes of A'': (2k, 2m, S·batch), plane-major
@@ -72,6 +80,9 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -95,65 +106,69 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
       "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
-// shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart
+// shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups 512 B apart
 __device__ __forceinline__ uint64_t sdesc(const void* p) {
   const uint64_t addr = (uint64_t)smem_u32(p);
   uint64_t d = (addr & 0x3FFFFull) >> 4;
   d |= 1ull << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)(512 >> 4) << 32;
   d |= 1ull << 46;
-  d |= 2ull << 61;
+  d |= 4ull << 61;
   return d;
 }
-// instruction descriptor, kind::f16: D f32, A and B bf16, both K-major, N = 64, M = 128
-constexpr uint32_t kIdescBF16 =
-    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_BN >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
+// instruction descriptor, kind::f16: D f32, A and B bf16, both K-major, M = 128
+__device__ __forceinline__ uint32_t idesc_bf16(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
+}
 
-__device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t accum) {
+__device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
           dtmem),
-      "l"(a), "l"(b), "r"(kIdescBF16), "r"(accum)
+      "l"(a), "l"(b), "r"(idesc), "r"(accum)
       : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(taddr)
+      : "memory");
 }
 
-// grid: (tiles_m · tiles_n, batch); 192 threads
+// x · 2^e by an addition to the exponent (the FP64 pipe takes 64 clocks for a product), for x and
+// results that are 0 or normal numbers
+__device__ __forceinline__ double times_pow2(double x, int e) {
+  const int hi = __double2hiint(x);
+  return __hiloint2double((hi & 0x7ff00000) ? hi + (e << 20) : hi, __double2loint(x));
+}
+// the exponent of a power of two (1024 stands for what is none)
+__device__ __forceinline__ int exponent_of(double pow2) { return ((__double2hiint(pow2) >> 20) & 0x7ff) - 1023; }
+
+// grid: at most one CTA per SM; 192 threads
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     k_gemm_oz(const __grid_constant__ OzMaps maps, int S, int bits, int M2, int N, int K2, int batch, cxd* __restrict__ C,
               int64_t ldc, int64_t sC, const double* __restrict__ sig, const double* __restrict__ tau, cxd alpha,
-              cxd beta, int beta_zero, int m_complex, int* err) {
+              cxd beta, int m_complex, int* err) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base_u = smem_u32(smem_raw);
   unsigned char* smem = smem_raw + ((1024 - (base_u & 1023)) & 1023);
-  unsigned char* sA = smem;                               // OZ_A_RING tiles
-  unsigned char* sB = smem + OZ_A_RING * OZ_A_TILE;       // 2 buffers × S tiles
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sB + 2 * S * OZ_B_TILE);
-  uint64_t* a_full = bars;                  // [OZ_A_RING]
-  uint64_t* a_empty = bars + OZ_A_RING;     // [OZ_A_RING]
-  uint64_t* b_full = bars + 2 * OZ_A_RING;  // [2]
-  uint64_t* b_empty = b_full + 2;           // [2]
-  uint64_t* done = b_empty + 2;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+  unsigned char* sA = smem;                          // 2 stages × S planes
+  unsigned char* sB = smem + 2 * S * OZ_A_TILE;      // 2 stages × S planes
+  uint64_t* full = reinterpret_cast<uint64_t*>(sB + 2 * S * OZ_B_TILE);  // [2]
+  uint64_t* empty = full + 2;                                            // [2][OZ_MAX_S]
+  uint64_t* acc_full = empty + 2 * OZ_MAX_S;
+  uint64_t* acc_empty = acc_full + 1;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(acc_empty + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tiles_m = (M2 + OZ_BM - 1) / OZ_BM;
-  const int m0 = ((int)blockIdx.x % tiles_m) * OZ_BM, n0 = ((int)blockIdx.x / tiles_m) * OZ_BN;
-  const int bidx = (int)blockIdx.y;
+  const int tiles_m = (M2 + OZ_BM - 1) / OZ_BM, per = tiles_m * ((N + OZ_BN - 1) / OZ_BN);
+  const int64_t tiles = (int64_t)per * batch;
   const uint32_t tcols = S <= 4 ? 256u : 512u;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(tcols)
@@ -161,15 +176,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 32) {
-    for (int s = 0; s < OZ_A_RING; ++s) {
-      mbar_init(&a_full[s], 1);
-      mbar_init(&a_empty[s], 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&full[b], 1);
+      for (int p = 0; p < OZ_MAX_S; ++p) mbar_init(&empty[b * OZ_MAX_S + p], 1);
     }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&b_full[s], 1);
-      mbar_init(&b_empty[s], 1);
-    }
-    mbar_init(done, 1);
+    mbar_init(acc_full, 1);
+    mbar_init(acc_empty, 4);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -180,98 +192,142 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 
   if (warp == 4) {
     if (lane == 0) {
-      // producer: per K stage, the S planes of the B tile, then the S planes of the A tile
-      int ta = 0;
+      // producer: planes p of A and S − 1 − p of B as the stage before last gives their place back
+      long long g = 0;
       bool ok = true;
-      for (int ks = 0; ks < nks && ok; ++ks) {
-        const int kb = ks & 1;
-        if (ks >= 2 && !(ok = mbar_wait(&b_empty[kb], ((ks >> 1) & 1) ^ 1, err))) break;
-        mbar_expect_tx(&b_full[kb], (uint32_t)(S * OZ_B_TILE));
-        for (int q = 0; q < S; ++q)
-          tma_load_3d(sB + (kb * S + q) * OZ_B_TILE, &maps.b, &b_full[kb], ks * OZ_BK, n0, q * batch + bidx);
-        for (int p = 0; p < S; ++p, ++ta) {
-          const int slot = ta % OZ_A_RING;
-          if (ta >= OZ_A_RING && !(ok = mbar_wait(&a_empty[slot], ((ta / OZ_A_RING) & 1) ^ 1, err))) break;
-          mbar_expect_tx(&a_full[slot], (uint32_t)OZ_A_TILE);
-          tma_load_3d(sA + slot * OZ_A_TILE, &maps.a, &a_full[slot], ks * OZ_BK, m0, p * batch + bidx);
+      for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const int bidx = (int)(tile / per), w = (int)(tile % per), m0 = w % tiles_m * OZ_BM, n0 = w / tiles_m * OZ_BN;
+        for (int ks = 0; ks < nks && ok; ++ks, ++g) {
+          const int kb = (int)(g & 1);
+          const uint32_t parity = (uint32_t)((g >> 1) & 1) ^ 1;
+          for (int p = 0; p < S; ++p) {
+            if (g >= 2 && !(ok = mbar_wait(&empty[kb * OZ_MAX_S + p], parity, err))) break;
+            if (p == 0) mbar_expect_tx(&full[kb], (uint32_t)(S * (OZ_A_TILE + OZ_B_TILE)));
+            tma_load_3d(sA + (kb * S + p) * OZ_A_TILE, &maps.a, &full[kb], ks * OZ_BK, m0, p * batch + bidx);
+            const int q = S - 1 - p;
+            tma_load_3d(sB + (kb * S + q) * OZ_B_TILE, &maps.b, &full[kb], ks * OZ_BK, n0, q * batch + bidx);
+          }
         }
       }
     }
   } else if (warp == 5) {
     if (lane == 0) {
-      // MMA issuer: plane p of A against every resident plane q < S - p of B, level p + q
-      int ta = 0;
+      // MMA issuer: plane p of A against every plane q < S - p of B, level p + q
+      long long g = 0;
+      int it = 0;
       bool ok = true;
-      for (int ks = 0; ks < nks && ok; ++ks) {
-        const int kb = ks & 1;
-        if (!(ok = mbar_wait(&b_full[kb], (ks >> 1) & 1, err))) break;
+      for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++it) {
+        if (it > 0 && !(ok = mbar_wait(acc_empty, (uint32_t)(it - 1) & 1, err))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int p = 0; p < S; ++p, ++ta) {
-          const int slot = ta % OZ_A_RING;
-          if (!(ok = mbar_wait(&a_full[slot], (ta / OZ_A_RING) & 1, err))) break;
+        for (int ks = 0; ks < nks; ++ks, ++g) {
+          const int kb = (int)(g & 1);
+          if (!(ok = mbar_wait(&full[kb], (uint32_t)(g >> 1) & 1, err))) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint64_t a0 = sdesc(sA + slot * OZ_A_TILE);
-          for (int q = 0; q < S - p; ++q) {
-            const uint64_t b0 = sdesc(sB + (kb * S + q) * OZ_B_TILE);
-            const uint32_t d = tmem + (uint32_t)((p + q) * OZ_BN);
+          for (int p = 0; p < S; ++p) {
+            // the planes of B lie one after the other, and so do the levels: up to four planes are one
+            // operand of N = 256
+            const uint64_t a0 = sdesc(sA + (kb * S + p) * OZ_A_TILE), b0 = sdesc(sB + kb * S * OZ_B_TILE);
+            for (int q = 0; q < S - p; q += 4) {
+              const uint32_t idesc = idesc_bf16(OZ_BN * min(4, S - p - q));
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)  // 4 × (K = 16 BF16 = 32 bytes)
-              mma_bf16(d, a0 + (uint64_t)kk * 2, b0 + (uint64_t)kk * 2, (ks > 0 || p > 0 || kk > 0) ? 1u : 0u);
+              for (int kk = 0; kk < OZ_BK / 16; ++kk)  // K = 16 BF16 = 32 bytes
+                mma_bf16(tmem + (uint32_t)((p + q) * OZ_BN), a0 + (uint64_t)kk * 2,
+                         b0 + (uint64_t)(q * (OZ_B_TILE >> 4) + kk * 2), idesc, (ks > 0 || p > 0 || kk > 0) ? 1u : 0u);
+            }
+            mma_commit(&empty[kb * OZ_MAX_S + p]);
           }
-          mma_commit(&a_empty[slot]);
         }
-        mma_commit(&b_empty[kb]);
+        if (ok) mma_commit(acc_full);
       }
-      mma_commit(done);
     }
   } else {
     // epilogue: warps 0-3
-    const bool ok = mbar_wait(done, 0, err);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok) {
-      const int row = m0 + warp * 32 + lane;  // real row of the 4M product: 2i + (0 Re | 1 Im)
-      const int i = row >> 1;
-      const bool re_lane = (lane & 1) == 0;
-      // The levels are recombined exactly in int64 on the integer pipe (GB300's FP64 pipe
-      // is ~1/70 of its FP32 pipe, and an FP64 Horner step per level and output kept it
-      // busier than the tensor pipe): H = Σ_L acc_L · 2^{b(S−1−L)−D}, each acc_L an
-      // integer of magnitude ≤ 2^24 (exact in FP32), D = max(0, b(S−1) − 37) so that
-      // |H| < 2^62; the levels below 2^D are rounded to nearest (an error of at most
-      // S/2 units of 2^{D−b(S−1)} relative to acc_0, below 2^-60 of the largest term).
-      // One conversion to FP64 per output, then the scales σ_i τ_j 2^{4−2b+D−b(S−1)}.
-      const int D = bits * (S - 1) > 37 ? bits * (S - 1) - 37 : 0;
-      const double si =
-          (row < M2) ? ldexp(sig[(int64_t)bidx * m_complex + i], 4 - 2 * bits + D - bits * (S - 1)) : 0.0;
-      const bool alpha_one = alpha.x == 1.0 && alpha.y == 0.0;
-      cxd* Cb = C + (int64_t)bidx * sC;
+    // The levels are recombined exactly in int64 on the integer pipe (GB300's FP64 pipe
+    // is ~1/70 of its FP32 pipe): H = Σ_L acc_L · 2^{b(S−1−L)−D}, each acc_L an
+    // integer of magnitude ≤ 2^24 (exact in FP32), D = max(0, b(S−1) − 37) so that
+    // |H| < 2^62; the levels below 2^D are rounded to nearest (an error of at most
+    // S/2 units of 2^{D−b(S−1)} relative to acc_0, below 2^-60 of the largest term).
+    // The scales σ_i τ_j 2^{4−2b+D−b(S−1)} are powers of two: a lane writes its own component, and
+    // for alpha = ±1 and beta = 0 or 1 the only FP64 operation left is the sum with C.
+    const int D = bits * (S - 1) > 37 ? bits * (S - 1) - 37 : 0, shift = 4 - 2 * bits + D - bits * (S - 1);
+    const bool plain = alpha.y == 0.0 && (alpha.x == 1.0 || alpha.x == -1.0) && beta.y == 0.0 && (beta.x == 0.0 || beta.x == 1.0);
+    const bool beta_zero = beta.x == 0.0 && beta.y == 0.0;
+    int it = 0;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+      const int bidx = (int)(tile / per), wt = (int)(tile % per), m0 = wt % tiles_m * OZ_BM, n0 = wt / tiles_m * OZ_BN;
+      if (!mbar_wait(acc_full, (uint32_t)it & 1, err)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      long long h[OZ_BN];
+#pragma unroll
+      for (int j = 0; j < OZ_BN; ++j) h[j] = 0;
 #pragma unroll 1
-      for (int cb = 0; cb < OZ_BN; cb += 16) {
-        long long h[16];
-        float v[16];
+      for (int L = 0; L < S; ++L) {
+        const int sh = bits * (S - 1 - L) - D;
+        const int up = max(sh - 32, 0), mul = 1 << max(0, min(30, sh)), twice = sh == 31 ? 1 : 0;
+        const int rs = sh < 0 ? min(-sh, 31) : 0, half = sh < 0 ? 1 << (rs - 1) : 0;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) h[j] = 0;
-        for (int L = 0; L < S; ++L) {
-          tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(L * OZ_BN + cb), v);
-          const int sh = bits * (S - 1 - L) - D;
-          if (sh >= 0) {
+        for (int cb = 0; cb < OZ_BN; cb += 32) {
+          uint32_t v[32];
+          tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(L * OZ_BN + cb), v);
+          if (sh >= 32) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) h[j] += (long long)__float2int_rn(v[j]) * (1ll << sh);
+            for (int j = 0; j < 32; ++j)
+              h[cb + j] += (long long)((unsigned long long)(unsigned)(__float2int_rn(__uint_as_float(v[j])) << up) << 32);
+          } else if (sh >= 0) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              h[cb + j] += (long long)(__float2int_rn(__uint_as_float(v[j])) << twice) * (long long)mul;
           } else {
-            const long long half = 1ll << (-sh - 1);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) h[j] += ((long long)__float2int_rn(v[j]) + half) >> (-sh);
+            for (int j = 0; j < 32; ++j) h[cb + j] += (long long)((__float2int_rn(__uint_as_float(v[j])) + half) >> rs);
           }
         }
+      }
+      // the accumulators are read: the next tile's products may begin
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty);
+      const int row = m0 + warp * 32 + lane;  // real row of the 4M product: 2i + (0 Re | 1 Im)
+      const int i = row >> 1;
+      const bool live = row < M2;
+      cxd* Cb = C + (int64_t)bidx * sC;
+      const double si = live ? sig[(int64_t)bidx * m_complex + i] : 1.0;
+      const int ei = exponent_of(si);
+      // the tile's column scales: one exponent per lane and half
+      const double t0 = n0 + lane < N ? tau[(int64_t)bidx * N + n0 + lane] : 1.0;
+      const double t1 = n0 + 32 + lane < N ? tau[(int64_t)bidx * N + n0 + 32 + lane] : 1.0;
+      const int e0 = exponent_of(t0), e1 = exponent_of(t1);
+      double* Cr = reinterpret_cast<double*>(Cb + (int64_t)n0 * ldc) + row;
+      // (the code of the 64 columns is kept short: it runs once a tile, and its fetching would
+      // otherwise take longer than its execution)
+      const int base = ei + shift;
+      const int lowest = base + __reduce_min_sync(0xffffffffu, min(e0, e1)), highest = base + __reduce_max_sync(0xffffffffu, max(e0, e1));
+      // (|h| is 0 or between 1 and 2^62)
+      const bool normal = __all_sync(0xffffffffu, lowest > -1022 && highest < 960);
+      if (plain && normal) {
+        const unsigned flip = alpha.x < 0.0 ? 0x80000000u : 0u;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int col = n0 + cb + j;
-          const double x = (double)h[j];
-          const double y = __shfl_xor_sync(0xffffffffu, x, 1);
-          if (row < M2 && col < N && re_lane) {
-            const double s = si * tau[(int64_t)bidx * N + col];
-            const cxd c = mkcx(s * x, s * y);
-            cxd* dst = Cb + i + (int64_t)col * ldc;
-            cxd out = alpha_one ? c : alpha * c;
+        for (int c = 0; c < OZ_BN; c += 16) {
+          double old[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) old[j] = !beta_zero && live && n0 + c + j < N ? Cr[2 * (int64_t)(c + j) * ldc] : 0.0;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const int ej = __shfl_sync(0xffffffffu, c + j < 32 ? e0 : e1, (c + j) & 31);
+            const double x = times_pow2((double)h[c + j], base + ej);
+            const double y = __hiloint2double(__double2hiint(x) ^ flip, __double2loint(x));
+            if (live && n0 + c + j < N) Cr[2 * (int64_t)(c + j) * ldc] = beta_zero ? y : y + old[j];
+          }
+        }
+      } else {
+        // any alpha and beta, and scales whose products may not be normal numbers
+#pragma unroll
+        for (int j = 0; j < OZ_BN; ++j) {
+          const double tj = __shfl_sync(0xffffffffu, j < 32 ? t0 : t1, j & 31);
+          const double x = ldexp(si, shift) * tj * (double)h[j], y = __shfl_xor_sync(0xffffffffu, x, 1);
+          if (live && n0 + j < N && !(lane & 1)) {
+            cxd* dst = Cb + i + (int64_t)(n0 + j) * ldc;
+            cxd out = alpha * mkcx(x, y);
             if (!beta_zero) out = out + beta * *dst;
             *dst = out;
           }
@@ -300,41 +356,89 @@ __device__ __forceinline__ cxd view_at(const OpView& v, int64_t b, int64_t r, in
   return x;
 }
 
-// σ_r = the smallest power of two ≥ max_c max(|Re X̃(r,c)|, |Im X̃(r,c)|) (1 for a zero row);
-// one warp per row
-__global__ void k_oz_scales(OpView v, int64_t R, int64_t K, int64_t batch, double* __restrict__ out) {
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const int lane = threadIdx.x & 31;
-  for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w < R * batch; w += warps) {
-    const int64_t b = w / R, r = w % R;
-    double mx = 0.0;
-    for (int64_t c = lane; c < K; c += 32) {
-      const cxd x = view_at(v, b, r, c);
-      mx = fmax(mx, fmax(fabs(x.x), fabs(x.y)));
-    }
+// the larger of two |Re|, |Im| bit patterns (ordered like the values; a NaN counts as 0)
+__device__ __forceinline__ unsigned long long larger_abs(unsigned long long m, cxd x) {
+  const unsigned long long a = (unsigned long long)__double_as_longlong(fabs(x.x)), b = (unsigned long long)__double_as_longlong(fabs(x.y));
+  m = a > m && a <= 0x7ff0000000000000ull ? a : m;
+  return b > m && b <= 0x7ff0000000000000ull ? b : m;
+}
+__device__ __forceinline__ double scale_of(unsigned long long m) {
+  const double mx = __longlong_as_double((long long)m);
+  double s = 1.0;
+  if (mx > 0.0) {
+    int e;
+    const double f = frexp(mx, &e);  // mx = f·2^e, f ∈ [0.5, 1)
+    s = ldexp(1.0, f == 0.5 ? e - 1 : e);
+  }
+  return s;
+}
+
+// σ_r = the smallest power of two ≥ max_c max(|Re X̃(r,c)|, |Im X̃(r,c)|) (1 for a zero row).
+// Contiguous rows: 32 rows per block, a warp reads them side by side; otherwise one warp per row.
+__global__ void __launch_bounds__(256) k_oz_scales(OpView v, int64_t R, int64_t K, int64_t batch, double* __restrict__ out) {
+  __shared__ unsigned long long part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (v.r_contig) {
+    const int64_t blocks = (R + 31) / 32;
+    for (int64_t w = blockIdx.x; w < blocks * batch; w += gridDim.x) {
+      const int64_t b = w / blocks, r = w % blocks * 32 + lane;
+      unsigned long long mx = 0;
+      if (r < R)
+        for (int64_t c = warp; c < K; c += 8) mx = larger_abs(mx, view_at(v, b, r, c));
+      part[warp][lane] = mx;
+      __syncthreads();
+      if (warp == 0 && r < R) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) {
-      double s = 1.0;
-      if (mx > 0.0) {
-        int e;
-        const double f = frexp(mx, &e);  // mx = f·2^e, f ∈ [0.5, 1)
-        s = ldexp(1.0, f == 0.5 ? e - 1 : e);
+        for (int u = 1; u < 8; ++u) mx = part[u][lane] > mx ? part[u][lane] : mx;
+        out[b * R + r] = scale_of(mx);
       }
-      out[b * R + r] = s;
+      __syncthreads();
     }
+    return;
+  }
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + warp; w < R * batch; w += warps) {
+    const int64_t b = w / R, r = w % R;
+    unsigned long long mx = 0;
+    for (int64_t c = lane; c < K; c += 32) mx = larger_abs(mx, view_at(v, b, r, c));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long u = __shfl_xor_sync(0xffffffffu, mx, o);
+      mx = u > mx ? u : mx;
+    }
+    if (lane == 0) out[b * R + r] = scale_of(mx);
   }
 }
 
-__device__ __forceinline__ unsigned short bf16_bits(double d) {
-  return __bfloat16_as_ushort(__float2bfloat16_rn((float)d));  // |d| ≤ 128 integer: exact
+// v·2^ex rounded to the nearest integer (even on a tie), |v·2^ex| ≤ 2^62
+__device__ __forceinline__ long long fixed_of(double v, int ex) {
+  const long long bits = __double_as_longlong(v);
+  const int e = (int)((unsigned long long)bits >> 52) & 0x7ff, s = e - 1075 + ex;
+  if (e == 0 || e == 0x7ff) return v == 0.0 ? 0 : llrint(ldexp(v, ex));
+  const unsigned long long m = ((unsigned long long)bits & 0xfffffffffffffull) | 0x10000000000000ull;
+  unsigned long long q;
+  if (s >= 0) {
+    q = m << min(s, 10);
+  } else if (s < -54) {
+    q = 0;
+  } else {
+    const unsigned long long half = 1ull << (-s - 1), rem = m & (2 * half - 1);
+    q = m >> -s;
+    q += rem > half || (rem == half && (q & 1)) ? 1 : 0;
+  }
+  return bits < 0 ? -(long long)q : (long long)q;
 }
+// an integer of magnitude ≤ 2^22 as a float, by additions (its BF16 form is the upper half)
+__device__ __forceinline__ unsigned digit_bits(int d) { return __float_as_uint(__int_as_float(0x4B400000 + d) - 12582912.0f); }
 
 // digit planes of one operand.  a_form: A'' rows 2r (Re) / 2r+1 (Im) with columns
 // [Re | −Im] / [Im | Re]; otherwise B'' rows r with columns [Re | Im].  Planes are
 // stored plane-major: out[(p·batch + b)·rows'·pitch + row'·pitch + col].  32×32 tiles of
 // X̃ are staged through shared memory so that reads follow the source's contiguous index
-// and writes the contraction index.
+// and writes the contraction index, two entries per thread.  All arithmetic is on integers: an
+// entry becomes round(x·2^{bS−2}/σ) and its balanced base-2^b digits are peeled off from the bottom
+// (in FP64, with a conversion per digit, the FP64 pipe took 0.27 ms for 16 × 512² where the
+// planes' 200 MB take 0.05; now 0.12).
 __global__ void __launch_bounds__(256)
     k_oz_split(OpView v, int64_t R, int64_t K, int64_t batch, int S, int bits, bool a_form, const double* __restrict__ scale,
                int64_t pitch, unsigned short* __restrict__ out) {
@@ -353,46 +457,47 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   const int64_t rows_out = a_form ? 2 * R : R;
   const int64_t plane = rows_out * pitch;
-  for (int u = ty; u < 32; u += 8) {
-    const int64_t r = r0 + u, c = c0 + tx;
+  const long long half = 1ll << (bits - 1), mask = (1ll << bits) - 1;
+  const bool pairs = (K & 1) == 0;
+  for (int u = threadIdx.x >> 4; u < 32; u += 16) {
+    const int64_t r = r0 + u, c = c0 + 2 * (threadIdx.x & 15);
     if (r >= R || c >= K) continue;
-    const cxd x = tile[tx][u];
-    // The top digit is rint(x) in FP64; the remainder (|·| ≤ ½) becomes one integer of
-    // b·(S−1) fraction bits (≤ 2^55: exact in int64), whose balanced base-2^b digits are
-    // peeled off from the bottom with integer operations (the FP64 pipe is the scarce one
-    // on this part); the carry left after S−1 digits (−1, 0 or 1) goes to the top digit.
-    const double inv = ldexp(1.0 / scale[b * R + r], bits - 2);  // powers of two: exact
-    const double xr = x.x * inv, xi = x.y * inv;
-    const double tr = rint(xr), ti = rint(xi);
-    const double lo_scale = ldexp(1.0, bits * (S - 1));
-    long long Xr = llrint((xr - tr) * lo_scale), Xi = llrint((xi - ti) * lo_scale);
-    const long long half = 1ll << (bits - 1), mask = (1ll << bits) - 1;
-    int dr[OZ_MAX_S], di[OZ_MAX_S];
+    const int ex = bits * S - 2 - exponent_of(scale[b * R + r]);
+    long long X[4];  // Re, Im of entry c, Re, Im of entry c + 1 (0 beyond K: the tile's padding)
 #pragma unroll
-    for (int p = OZ_MAX_S - 1; p >= 1; --p) {
-      if (p < S) {
-        const long long lr = ((Xr + half) & mask) - half, li = ((Xi + half) & mask) - half;
-        Xr = (Xr - lr) >> bits;
-        Xi = (Xi - li) >> bits;
-        dr[p] = (int)lr;
-        di[p] = (int)li;
-      }
+    for (int z = 0; z < 2; ++z) {
+      const cxd x = tile[2 * (threadIdx.x & 15) + z][u];
+      X[2 * z] = fixed_of(x.x, ex);
+      X[2 * z + 1] = fixed_of(x.y, ex);
     }
-    dr[0] = (int)tr + (int)Xr;
-    di[0] = (int)ti + (int)Xi;
+    unsigned short* o = out + ((int64_t)(S - 1) * batch + b) * plane + (a_form ? 2 * r : r) * pitch + c;
+    for (int p = S - 1; p >= 0; --p, o -= (int64_t)batch * plane) {
+      unsigned f[4];
 #pragma unroll
-    for (int p = 0; p < OZ_MAX_S; ++p) {
-      if (p >= S) break;
-      unsigned short* o = out + ((int64_t)p * batch + b) * plane;
-      const double vr = (double)dr[p], vi = (double)di[p];
-      if (a_form) {
-        o[(2 * r) * pitch + c] = bf16_bits(vr);
-        o[(2 * r) * pitch + K + c] = bf16_bits(-vi);
-        o[(2 * r + 1) * pitch + c] = bf16_bits(vi);
-        o[(2 * r + 1) * pitch + K + c] = bf16_bits(vr);
+      for (int z = 0; z < 4; ++z) {
+        const long long d = p > 0 ? ((X[z] + half) & mask) - half : X[z];
+        X[z] = (X[z] - d) >> bits;
+        f[z] = digit_bits((int)d);
+      }
+      const unsigned re = __byte_perm(f[0], f[2], 0x7632), im = __byte_perm(f[1], f[3], 0x7632);
+      if (pairs) {
+        *reinterpret_cast<unsigned*>(o) = re;
+        *reinterpret_cast<unsigned*>(o + K) = a_form ? im ^ 0x80008000u : im;
+        if (a_form) {
+          *reinterpret_cast<unsigned*>(o + pitch) = im;
+          *reinterpret_cast<unsigned*>(o + pitch + K) = re;
+        }
       } else {
-        o[r * pitch + c] = bf16_bits(vr);
-        o[r * pitch + K + c] = bf16_bits(vi);
+        const int two = c + 1 < K ? 2 : 1;
+        for (int z = 0; z < two; ++z) {
+          const unsigned short dr = (unsigned short)(z ? re >> 16 : re), di = (unsigned short)(z ? im >> 16 : im);
+          o[z] = dr;
+          o[z + K] = a_form ? di ^ 0x8000 : di;
+          if (a_form) {
+            o[z + pitch] = di;
+            o[z + pitch + K] = dr;
+          }
+        }
       }
     }
   }
@@ -407,7 +512,7 @@ tn_status_t make_map3(tn_ctx* ctx, CUtensorMap* map, const void* base, int64_t K
   cuuint32_t box[3] = {(cuuint32_t)OZ_BK, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void*)base, dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return tn_set_error(ctx, TN_ECUDA, "cuTensorMapEncodeTiled (split GEMM) failed (%d)", (int)r);
   return TN_OK;
@@ -497,13 +602,13 @@ tn_status_t gemm_c64_split(tn_ctx* ctx, int S, char opa, char opb, int64_t m, in
   const OpView va = make_view(A, lda, sA, opa, true), vb = make_view(B, ldb, sB, opb, false);
   const int prep_slot = prof_begin(ctx);
   {
-    const int64_t rows = m * batch;
-    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + 7) / 8, (int64_t)ctx->num_sms * 16));
-    k_oz_scales<<<blocks, 256, 0, ctx->stream>>>(va, m, k, batch, sig);
+    auto scale_blocks = [&](const OpView& v, int64_t R) {
+      const int64_t want = v.r_contig ? (R + 31) / 32 * batch : (R * batch + 7) / 8;
+      return (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->num_sms * 16));
+    };
+    k_oz_scales<<<scale_blocks(va, m), 256, 0, ctx->stream>>>(va, m, k, batch, sig);
     TN_LAUNCHED(ctx);
-    const int64_t cols = n * batch;
-    const unsigned bb = (unsigned)std::max<int64_t>(1, std::min<int64_t>((cols + 7) / 8, (int64_t)ctx->num_sms * 16));
-    k_oz_scales<<<bb, 256, 0, ctx->stream>>>(vb, n, k, batch, tau);
+    k_oz_scales<<<scale_blocks(vb, n), 256, 0, ctx->stream>>>(vb, n, k, batch, tau);
     TN_LAUNCHED(ctx);
     k_oz_split<<<dim3(cdiv(m, 32), cdiv(k, 32), (unsigned)batch), 256, 0, ctx->stream>>>(va, m, k, batch, S, bits, true,
                                                                                        sig, pitch, dA);
@@ -525,8 +630,8 @@ tn_status_t gemm_c64_split(tn_ctx* ctx, int S, char opa, char opb, int64_t m, in
   TN_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_gemm_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const bool beta_zero = beta.x == 0.0 && beta.y == 0.0;
   const int slot = prof_begin(ctx);
-  k_gemm_oz<<<dim3((unsigned)tiles, (unsigned)batch), OZ_THREADS, smem, ctx->stream>>>(
-      maps, S, bits, (int)M2, (int)n, (int)K2, (int)batch, C, ldc, sC, sig, tau, alpha, beta, beta_zero ? 1 : 0, (int)m, err);
+  k_gemm_oz<<<(unsigned)std::min<int64_t>(tiles * batch, ctx->num_sms), OZ_THREADS, smem, ctx->stream>>>(
+      maps, S, bits, (int)M2, (int)n, (int)K2, (int)batch, C, ldc, sC, sig, tau, alpha, beta, (int)m, err);
   TN_LAUNCHED(ctx);
   if (slot >= 0)  // tensor-pipe flops of the S(S+1)/2 real products it issues; planes read once, C written
     prof_end(ctx, slot, TN_PROF_GEMM_SPLIT, 1, S * (S + 1) / 2 * 2.0 * M2 * n * K2 * batch,
