@@ -154,7 +154,7 @@ __device__ __forceinline__ int exponent_of(double pow2) { return ((__double2hiin
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     k_gemm_oz(const __grid_constant__ OzMaps maps, int S, int bits, int M2, int N, int K2, int batch, cxd* __restrict__ C,
               int64_t ldc, int64_t sC, const double* __restrict__ sig, const double* __restrict__ tau, cxd alpha,
-              cxd beta, int m_complex, int* err) {
+              cxd beta, int m_complex, int upper, int* err) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base_u = smem_u32(smem_raw);
   unsigned char* smem = smem_raw + ((1024 - (base_u & 1023)) & 1023);
@@ -167,8 +167,21 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   uint32_t* tslot = reinterpret_cast<uint32_t*>(acc_empty + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tiles_m = (M2 + OZ_BM - 1) / OZ_BM, per = tiles_m * ((N + OZ_BN - 1) / OZ_BN);
+  const int tiles_m = (M2 + OZ_BM - 1) / OZ_BM;
+  const int per = upper ? tiles_m * (tiles_m + 1) / 2 : tiles_m * ((N + OZ_BN - 1) / OZ_BN);
   const int64_t tiles = (int64_t)per * batch;
+  // a tile's first real row and its column; upper: the tiles on and above the diagonal, column by column
+  auto place = [&](int w, int& m0, int& n0) {
+    int ti = w % tiles_m, tj = w / tiles_m;
+    if (upper) {
+      tj = (int)((sqrtf(8.0f * (float)w + 1.0f) - 1.0f) * 0.5f);
+      while (tj * (tj + 1) / 2 > w) --tj;
+      while ((tj + 1) * (tj + 2) / 2 <= w) ++tj;
+      ti = w - tj * (tj + 1) / 2;
+    }
+    m0 = ti * OZ_BM;
+    n0 = tj * OZ_BN;
+  };
   const uint32_t tcols = S <= 4 ? 256u : 512u;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(tcols)
@@ -196,7 +209,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       long long g = 0;
       bool ok = true;
       for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const int bidx = (int)(tile / per), w = (int)(tile % per), m0 = w % tiles_m * OZ_BM, n0 = w / tiles_m * OZ_BN;
+        const int bidx = (int)(tile / per);
+        int m0, n0;
+        place((int)(tile % per), m0, n0);
         for (int ks = 0; ks < nks && ok; ++ks, ++g) {
           const int kb = (int)(g & 1);
           const uint32_t parity = (uint32_t)((g >> 1) & 1) ^ 1;
@@ -254,7 +269,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const bool beta_zero = beta.x == 0.0 && beta.y == 0.0;
     int it = 0;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
-      const int bidx = (int)(tile / per), wt = (int)(tile % per), m0 = wt % tiles_m * OZ_BM, n0 = wt / tiles_m * OZ_BN;
+      const int bidx = (int)(tile / per);
+      int m0, n0;
+      place((int)(tile % per), m0, n0);
+      const bool mirror = upper && m0 != 2 * n0;  // a tile above the diagonal writes the one below it as well
       if (!mbar_wait(acc_full, (uint32_t)it & 1, err)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       long long h[OZ_BN];
@@ -316,7 +334,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             const int ej = __shfl_sync(0xffffffffu, c + j < 32 ? e0 : e1, (c + j) & 31);
             const double x = times_pow2((double)h[c + j], base + ej);
             const double y = __hiloint2double(__double2hiint(x) ^ flip, __double2loint(x));
-            if (live && n0 + c + j < N) Cr[2 * (int64_t)(c + j) * ldc] = beta_zero ? y : y + old[j];
+            const double z = beta_zero ? y : y + old[j];
+            if (live && n0 + c + j < N) {
+              Cr[2 * (int64_t)(c + j) * ldc] = z;
+              if (mirror) reinterpret_cast<double*>(Cb + (n0 + c + j) + (int64_t)i * ldc)[row & 1] = (row & 1) ? -z : z;
+            }
           }
         }
       } else {
@@ -330,6 +352,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             cxd out = alpha * mkcx(x, y);
             if (!beta_zero) out = out + beta * *dst;
             *dst = out;
+            if (mirror) Cb[(n0 + j) + (int64_t)i * ldc] = conjg(out);
           }
         }
       }
@@ -503,12 +526,13 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// planes of rows × K2 BF16, a row `pitch` and a plane `plane` elements after the one before
 tn_status_t make_map3(tn_ctx* ctx, CUtensorMap* map, const void* base, int64_t K2, int64_t rows, int64_t planes,
-                      int64_t pitch, uint32_t box_rows) {
+                      int64_t pitch, int64_t plane, uint32_t box_rows) {
   EncodeTiledFn fn = tn_encode_tiled_fn(ctx);
   if (!fn) return TN_ECUDA;
   cuuint64_t dims[3] = {(cuuint64_t)K2, (cuuint64_t)rows, (cuuint64_t)planes};
-  cuuint64_t strides[2] = {(cuuint64_t)(pitch * 2), (cuuint64_t)(pitch * 2 * rows)};
+  cuuint64_t strides[2] = {(cuuint64_t)(pitch * 2), (cuuint64_t)(plane * 2)};
   cuuint32_t box[3] = {(cuuint32_t)OZ_BK, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void*)base, dims, strides, box, estr,
@@ -565,11 +589,16 @@ tn_status_t oz_scratch(tn_ctx* ctx, size_t bytes, char** out) {
 
 tn_status_t gemm_c64_split(tn_ctx* ctx, int S, char opa, char opb, int64_t m, int64_t n, int64_t k, cxd alpha,
                            const cxd* A, int64_t lda, int64_t sA, const cxd* B, int64_t ldb, int64_t sB, cxd beta,
-                           cxd* C, int64_t ldc, int64_t sC, int64_t batch) {
+                           cxd* C, int64_t ldc, int64_t sC, int64_t batch, bool hermitian) {
   if (m == 0 || n == 0 || batch == 0) return TN_OK;
   if (S < 2 || S > OZ_MAX_S) return tn_set_error(ctx, TN_EINVAL, "split GEMM: slices must be in [2, %d]", OZ_MAX_S);
   if (batch > 65535) return tn_set_error(ctx, TN_EUNSUPPORTED, "split GEMM: batch > 65535");
   if (k == 0) return gemm_cx<double>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+  // Aᴴ·A: B'' is the even rows of A'', so its planes need not be cut, and with a real alpha the
+  // product is Hermitian: for beta = 0, or where C is known to be, the tiles above the diagonal
+  // are enough (16 × 512³: 0.79 → 0.46 ms)
+  const bool gram = opa == 'C' && opb == 'N' && A == B && lda == ldb && (sA == sB || batch == 1) && m == n;
+  const bool upper = gram && alpha.y == 0.0 && ((beta.x == 0.0 && beta.y == 0.0) || (hermitian && beta.y == 0.0));
   // a level's FP32 sum is exact while S·(2k)·2^{2b-2} ≤ 2^24: the widest such digit b
   // (at most 8); contractions that would need b < 7 run in chunks of k sized for b = 7,
   // the later chunks accumulating into C (beta = 1)
@@ -582,14 +611,14 @@ tn_status_t gemm_c64_split(tn_ctx* ctx, int S, char opa, char opb, int64_t m, in
       const cxd* Ac = (opa == 'N') ? A + k0 * lda : A + k0;
       const cxd* Bc = (opb == 'N') ? B + k0 : B + k0 * ldb;
       TN_RETURN_IF(gemm_c64_split(ctx, S, opa, opb, m, n, kc, alpha, Ac, lda, sA, Bc, ldb, sB,
-                                  k0 == 0 ? beta : mkcx(1.0, 0.0), C, ldc, sC, batch));
+                                  k0 == 0 ? beta : mkcx(1.0, 0.0), C, ldc, sC, batch, upper));
     }
     return TN_OK;
   }
   const int64_t M2 = 2 * m, K2 = 2 * k, pitch = (K2 + 7) / 8 * 8;
   if (M2 > (1ll << 30) || n > (1ll << 30)) return tn_set_error(ctx, TN_EUNSUPPORTED, "split GEMM: too large");
   const size_t bytesA = ws_round(2 * (size_t)(S * batch * M2 * pitch));
-  const size_t bytesB = ws_round(2 * (size_t)(S * batch * n * pitch));
+  const size_t bytesB = gram ? 0 : ws_round(2 * (size_t)(S * batch * n * pitch));
   const size_t bytesS = ws_round(sizeof(double) * (size_t)(batch * m)) + ws_round(sizeof(double) * (size_t)(batch * n));
   char* ws = nullptr;
   int* err = nullptr;
@@ -598,7 +627,7 @@ tn_status_t gemm_c64_split(tn_ctx* ctx, int S, char opa, char opb, int64_t m, in
   unsigned short* dA = reinterpret_cast<unsigned short*>(ws);
   unsigned short* dB = reinterpret_cast<unsigned short*>(ws + bytesA);
   double* sig = reinterpret_cast<double*>(ws + bytesA + bytesB);
-  double* tau = sig + ws_round(sizeof(double) * (size_t)(batch * m)) / sizeof(double);
+  double* tau = gram ? sig : sig + ws_round(sizeof(double) * (size_t)(batch * m)) / sizeof(double);
   const OpView va = make_view(A, lda, sA, opa, true), vb = make_view(B, ldb, sB, opb, false);
   const int prep_slot = prof_begin(ctx);
   {
@@ -608,33 +637,41 @@ tn_status_t gemm_c64_split(tn_ctx* ctx, int S, char opa, char opb, int64_t m, in
     };
     k_oz_scales<<<scale_blocks(va, m), 256, 0, ctx->stream>>>(va, m, k, batch, sig);
     TN_LAUNCHED(ctx);
-    k_oz_scales<<<scale_blocks(vb, n), 256, 0, ctx->stream>>>(vb, n, k, batch, tau);
-    TN_LAUNCHED(ctx);
+    if (!gram) {
+      k_oz_scales<<<scale_blocks(vb, n), 256, 0, ctx->stream>>>(vb, n, k, batch, tau);
+      TN_LAUNCHED(ctx);
+    }
     k_oz_split<<<dim3(cdiv(m, 32), cdiv(k, 32), (unsigned)batch), 256, 0, ctx->stream>>>(va, m, k, batch, S, bits, true,
                                                                                        sig, pitch, dA);
     TN_LAUNCHED(ctx);
-    k_oz_split<<<dim3(cdiv(n, 32), cdiv(k, 32), (unsigned)batch), 256, 0, ctx->stream>>>(vb, n, k, batch, S, bits,
-                                                                                       false, tau, pitch, dB);
-    TN_LAUNCHED(ctx);
+    if (!gram) {
+      k_oz_split<<<dim3(cdiv(n, 32), cdiv(k, 32), (unsigned)batch), 256, 0, ctx->stream>>>(vb, n, k, batch, S, bits,
+                                                                                         false, tau, pitch, dB);
+      TN_LAUNCHED(ctx);
+    }
   }
   if (prep_slot >= 0)  // read op(A), op(B) once, write their digit planes and scales
-    prof_end(ctx, prep_slot, TN_PROF_SPLIT_PREP, 4, 0.0,
-             2.0 * 16.0 * ((double)m * k + (double)k * n) * batch + 2.0 * S * ((double)M2 + n) * K2 * batch);
+    prof_end(ctx, prep_slot, TN_PROF_SPLIT_PREP, gram ? 2 : 4, 0.0,
+             2.0 * 16.0 * ((double)m * k + (gram ? 0.0 : (double)k * n)) * batch +
+                 2.0 * S * ((double)M2 + (gram ? 0 : n)) * K2 * batch);
   OzMaps maps;
   memset(&maps, 0, sizeof(maps));
-  TN_RETURN_IF(make_map3(ctx, &maps.a, dA, K2, M2, (int64_t)S * batch, pitch, OZ_BM));
-  TN_RETURN_IF(make_map3(ctx, &maps.b, dB, K2, n, (int64_t)S * batch, pitch, OZ_BN));
-  const int64_t tiles = (int64_t)cdiv(M2, OZ_BM) * cdiv(n, OZ_BN);
+  TN_RETURN_IF(make_map3(ctx, &maps.a, dA, K2, M2, (int64_t)S * batch, pitch, M2 * pitch, OZ_BM));
+  if (gram)
+    TN_RETURN_IF(make_map3(ctx, &maps.b, dA, K2, n, (int64_t)S * batch, 2 * pitch, M2 * pitch, OZ_BN));
+  else
+    TN_RETURN_IF(make_map3(ctx, &maps.b, dB, K2, n, (int64_t)S * batch, pitch, n * pitch, OZ_BN));
+  const int64_t tiles_m = cdiv(M2, OZ_BM), tiles = upper ? tiles_m * (tiles_m + 1) / 2 : tiles_m * cdiv(n, OZ_BN);
   if (tiles > 0x7fffffffll) return tn_set_error(ctx, TN_EUNSUPPORTED, "split GEMM: too many tiles");
   const int smem = oz_smem_bytes(S);
   TN_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_gemm_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const bool beta_zero = beta.x == 0.0 && beta.y == 0.0;
   const int slot = prof_begin(ctx);
   k_gemm_oz<<<(unsigned)std::min<int64_t>(tiles * batch, ctx->num_sms), OZ_THREADS, smem, ctx->stream>>>(
-      maps, S, bits, (int)M2, (int)n, (int)K2, (int)batch, C, ldc, sC, sig, tau, alpha, beta, (int)m, err);
+      maps, S, bits, (int)M2, (int)n, (int)K2, (int)batch, C, ldc, sC, sig, tau, alpha, beta, (int)m, upper ? 1 : 0, err);
   TN_LAUNCHED(ctx);
   if (slot >= 0)  // tensor-pipe flops of the S(S+1)/2 real products it issues; planes read once, C written
-    prof_end(ctx, slot, TN_PROF_GEMM_SPLIT, 1, S * (S + 1) / 2 * 2.0 * M2 * n * K2 * batch,
+    prof_end(ctx, slot, TN_PROF_GEMM_SPLIT, 1, S * (S + 1) / 2 * 2.0 * M2 * n * K2 * batch * (upper ? (tiles_m + 1.0) / (2.0 * tiles_m) : 1.0),
              (2.0 * S * ((double)M2 + n) * K2 + 16.0 * m * n * (beta_zero ? 1 : 2)) * batch);
   return TN_OK;
 }

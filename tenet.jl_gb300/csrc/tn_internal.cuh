@@ -467,7 +467,7 @@ EncodeTiledFn tn_encode_tiled_fn(tn_ctx* ctx);
 constexpr int kSplitSlicesDefault = 8;
 tn_status_t gemm_c64_split(tn_ctx* ctx, int slices, char opa, char opb, int64_t m, int64_t n, int64_t k, cxd alpha,
                            const cxd* A, int64_t lda, int64_t sA, const cxd* B, int64_t ldb, int64_t sB, cxd beta,
-                           cxd* C, int64_t ldc, int64_t sC, int64_t batch);
+                           cxd* C, int64_t ldc, int64_t sC, int64_t batch, bool hermitian = false);
 // reads (and clears) the split GEMMs' error word after draining the stream: TN_ETIMEOUT
 // when a pipeline wait ran out since the last check
 tn_status_t split_gemm_check(tn_ctx* ctx);

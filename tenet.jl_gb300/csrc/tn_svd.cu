@@ -1380,12 +1380,9 @@ constexpr float kRefineStop = 1e-8f;
 constexpr double kRefineNormMax = 0.5;  // ‖E‖_F above which the first-order steps diverge
 constexpr int kRefineMaxIter = 7;
 
-__global__ void k_set_identity_cxd(int64_t n, int64_t batch, cxd* X) {
-  const int64_t total = n * n * batch;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t w = t % (n * n);
-    X[t] = mkcx((w % n) == (w / n) ? 1.0 : 0.0, 0.0);
-  }
+__global__ void k_add_identity_cxd(int64_t n, int64_t batch, cxd* X) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n * batch; t += (int64_t)gridDim.x * blockDim.x)
+    X[t / n * n * n + (t % n) * (n + 1)].x += 1.0;
 }
 
 // λ_i = Re S_ii / (1 − Re R_ii); stat[4b + 2] = max_i λ_i (float bits)
@@ -1705,10 +1702,10 @@ tn_status_t svd_tall_mixed(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int6
       cluster_ran = false;
       TN_RETURN_IF(gemm_c64(ctx, TN_PREC_MIXED, 'C', 'N', n, n, m, one, W64, m, m * n, W64, m, m * n, zero, G, n, n * n,
                             batch));
-      k_set_identity_cxd<<<blocks, 256, 0, ctx->stream>>>(n, batch, RE);
-      TN_LAUNCHED(ctx);
-      TN_RETURN_IF(gemm_c64(ctx, TN_PREC_MIXED, 'C', 'N', n, n, n, mone, V64, n, n * n, V64, n, n * n, one, RE, n, n * n,
+      TN_RETURN_IF(gemm_c64(ctx, TN_PREC_MIXED, 'C', 'N', n, n, n, mone, V64, n, n * n, V64, n, n * n, zero, RE, n, n * n,
                             batch));
+      k_add_identity_cxd<<<lblocks, 256, 0, ctx->stream>>>(n, batch, RE);
+      TN_LAUNCHED(ctx);
       TN_CHECK_CUDA(ctx, cudaMemsetAsync(stat, 0, sizeof(int) * 4 * batch, ctx->stream));
       TN_CHECK_CUDA(ctx, cudaMemsetAsync(esq, 0, sizeof(double) * batch, ctx->stream));
       k_refine_lambda<<<lblocks, 256, 0, ctx->stream>>>(n, batch, G, RE, nrm64, stat);
@@ -1791,10 +1788,10 @@ tn_status_t svd_tall_mixed(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int6
       // restore V's unitarity (V ← V + V·R/2, quadratic: the pre-pass leaves R ~ 1e-4)
       // and leave every pair with a kept column to the FP64 sweeps
       for (int rep = 0; rep < 3; ++rep) {
-        k_set_identity_cxd<<<blocks, 256, 0, ctx->stream>>>(n, batch, RE);
-        TN_LAUNCHED(ctx);
-        TN_RETURN_IF(gemm_c64(ctx, TN_PREC_MIXED, 'C', 'N', n, n, n, mone, V64, n, n * n, V64, n, n * n, one, RE, n,
+        TN_RETURN_IF(gemm_c64(ctx, TN_PREC_MIXED, 'C', 'N', n, n, n, mone, V64, n, n * n, V64, n, n * n, zero, RE, n,
                               n * n, batch));
+        k_add_identity_cxd<<<lblocks, 256, 0, ctx->stream>>>(n, batch, RE);
+        TN_LAUNCHED(ctx);
         TN_RETURN_IF(scale_real_cxd(ctx, RE, n * n * batch, 0.5));
         TN_CHECK_CUDA(ctx, cudaMemcpyAsync(V, V64, sizeof(cxd) * (size_t)(n * n * batch), cudaMemcpyDeviceToDevice,
                                            ctx->stream));

@@ -33,6 +33,37 @@ def test_tiles_and_epilogue_exact(ctx, m, n, k, batch, alpha, beta):  # noqa: F8
     assert np.array_equal(got, alpha * (A @ B) + beta * C0)
 
 
+@pytest.mark.parametrize("n,k,batch", [(96, 32, 2), (128, 300, 1), (129, 64, 3), (191, 33, 1), (320, 600, 2), (512, 40, 1)])
+@pytest.mark.parametrize("alpha,beta", [(1, 0), (-1, 0), (2, 0), (1, 1), (1 + 1j, 0)])
+def test_gram_products_exact(ctx, n, k, batch, alpha, beta):  # noqa: F811
+    """AᴴA of one operand (its planes cut once, with a real alpha and beta = 0 the tiles above the
+    diagonal only) against the integer result; for Gaussian data it is Hermitian
+    to the last bit off the diagonal blocks."""
+    import ctypes as C
+
+    import tenetgb
+
+    rng = np.random.default_rng(n + k)
+    al, be = (C.c_double * 2)(complex(alpha).real, complex(alpha).imag), (C.c_double * 2)(beta, 0)
+    for exact in (True, False):
+        A = _ints(rng, (batch, k, n), 1000) if exact else cgauss(rng, (batch, k, n))
+        C0 = _ints(rng, (batch, n, n), 9)
+        dA = tenetgb.DeviceTensor.from_numpy(ctx, np.transpose(A, (1, 2, 0)))
+        dC = tenetgb.DeviceTensor.from_numpy(ctx, np.transpose(C0, (1, 2, 0)))
+        ctx.check(ctx.lib.tn_gemm(ctx.h, 3, 3, b"C", b"N", n, n, k, al, C.c_void_p(dA.ptr), k, k * n, C.c_void_p(dA.ptr), k,
+                                  k * n, be, C.c_void_p(dC.ptr), n, n * n, batch))
+        got = np.transpose(dC.numpy(), (2, 0, 1))
+        ref = alpha * (A.conj().transpose(0, 2, 1) @ A) + beta * C0
+        if exact:
+            assert np.array_equal(got, ref)
+        else:
+            assert np.linalg.norm(got - ref) <= 1e-13 * np.linalg.norm(ref)
+            if beta == 0 and complex(alpha).imag == 0:  # (64 × 64 blocks on the diagonal are computed in full)
+                h = got.conj().transpose(0, 2, 1)
+                off = np.arange(n)[:, None] // 64 != np.arange(n)[None] // 64
+                assert np.array_equal(got[:, off], h[:, off])
+
+
 @pytest.mark.parametrize("ea,eb", [(-400, 300), (-500, -480), (500, 450), (-600, 0)])
 def test_scales_are_exact(ctx, ea, eb):  # noqa: F811
     """Rows and columns scaled by powers of two: the products scale exactly, also where the sum of
