@@ -20,9 +20,12 @@
 //    one M = 128, N = 64 product gives hi·hi and lo·hi, and G = HH + LH + LHᵀ.  Each 128 rows
 //    have their own accumulator; they are added in FP32.
 //  * W·J, V·J: per 128 rows A (rows × 64 real columns) hi and lo against the 64 × 64 real form
-//    of J: lo·hi + hi·lo + hi·hi into one accumulator.
+//    of J: hi·[hi | lo] as one product of N = 128 and lo·hi, added in FP32 (products of N = 64
+//    take the tensor pipe nearly as long as those of N = 128).
 // One 64 KB operand buffer, which between the products also holds G and J, leaves room for two
 // CTAs per SM: one's rotations run under the other's products and memory traffic.
+// A round of 16 matrices of n = 512 takes 44 µs (47 with J's hi and lo parts as products of their
+// own); of a CTA's 73 thousand clocks the products of W and V take 35, the rotations 21, G 15.
 // Error: ~1e-6 of ‖wᵢ‖‖wⱼ‖ in G, below the pre-pass's rotation threshold (4√m·2⁻²³, 1e-5 at
 // m = 512); what it leaves is removed by the FP64 stage that follows every pre-pass.
 #include <cuda.h>
@@ -62,11 +65,12 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr) {
   d |= 2ull << 61;
   return d;
 }
-// D f32, A and B tf32, both K-major, M = 128, N = 64
+// D f32, A and B tf32, both K-major, M = 128, N = 64 or 128
 constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t accum) {
+constexpr uint32_t kIdesc128 = kIdesc + ((uint32_t)(64 >> 3) << 17);
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t accum, uint32_t idesc = kIdesc) {
   asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-               "l"(a), "l"(b), "r"(kIdesc), "r"(accum)
+               "l"(a), "l"(b), "r"(idesc), "r"(accum)
                : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -106,6 +110,12 @@ __device__ __forceinline__ void pair_of(int N, int r, int k, int& i, int& j) {
   }
 }
 
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 struct Rot {
   float c, sx, sy, monitor;
   int apply;
@@ -118,17 +128,17 @@ __device__ __forceinline__ Rot rotation(float al, float be, float gx, float gy, 
   Rot R = {1.f, 0.f, 0.f, 0.f, 0};
   const float fl = fmaxf(negl, 1e-32f);
   if (!(al > fl) || !(be > fl)) return R;
-  const float ra = rsqrtf(al), rb = rsqrtf(be);
+  const float ra = rsqrt_approx(al), rb = rsqrt_approx(be);
   const float px = gx * ra * rb, py = gy * ra * rb;
   const float rho2 = fmaf(px, px, py * py);
   if (!(rho2 > 0.f)) return R;
-  const float irho = rsqrtf(rho2), rho = rho2 * irho;
+  const float irho = rsqrt_approx(rho2), rho = rho2 * irho;
   R.monitor = rho;
   if (!(rho > tol)) return R;
   const float d = (be - al) * ra * rb, q = fmaf(d, d, 4.f * rho2);
-  const float t = copysignf(__fdividef(2.f * rho, fabsf(d) + q * rsqrtf(q)), d);
+  const float t = copysignf(__fdividef(2.f * rho, fabsf(d) + q * rsqrt_approx(q)), d);
   if (!(fabsf(t) > 0.f)) return R;
-  float c = rsqrtf(fmaf(t, t, 1.f));
+  float c = rsqrt_approx(fmaf(t, t, 1.f));
   const float s = c * t * irho;
   float sx = s * px, sy = s * py;
   const float e = -0.5f * fmaf(sy, sy, fmaf(sx, sx, fmaf(c, c, -1.f)));
@@ -170,7 +180,7 @@ __global__ void __launch_bounds__(kNT, 2)
     S.tail[tid] = (tail && c < n) ? tail[b * n + c] : 0;
   }
   const int CHm = (m + 127) / 128, CHn = (n + 127) / 128;  // chunks of 128 rows of W, of V (n ≤ m)
-  const uint32_t tcols = CHm == 1 ? 64 : (CHm == 2 ? 128 : 256);
+  const uint32_t tcols = CHm <= 2 ? 128 : 256;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.tslot)), "r"(tcols)
                  : "memory");
@@ -277,6 +287,7 @@ __global__ void __launch_bounds__(kNT, 2)
   // one barrier per round, G alternating between two copies ----
   const float negl = 1.1920929e-7f * 1.1920929e-7f * nrm[n * nmat + b];
   const int rounds = R == 0 ? kC - 1 : 16;
+  const unsigned there = __ballot_sync(0xffffffffu, S.col[lane] >= 0), tails = __ballot_sync(0xffffffffu, S.tail[lane] != 0);
   float worst = 0.f;
   int mine = 0, cur = 0;
 #pragma unroll 1
@@ -291,12 +302,13 @@ __global__ void __launch_bounds__(kNT, 2)
       pi = k;
       pj = 16 + ((k + r) & 15);
     }
-    if (S.col[pi] >= 0 && S.col[pj] >= 0 && !(S.tail[pi] && S.tail[pj])) {
+    const bool ti = (tails >> pi) & 1, tj = (tails >> pj) & 1;
+    if (((there >> pi) & (there >> pj) & 1) && !(ti && tj)) {
       const float al = G[cur][pi][pi].x, be = G[cur][pj][pj].x;
       const float2 g = G[cur][pi][pj];
       rt = rotation(al, be, g.x, g.y, tol, negl);
-      if (S.tail[pi] != S.tail[pj] && al > 0.f && be > 0.f) {
-        const float ak = S.tail[pi] ? be : al, at = S.tail[pi] ? al : be;
+      if (ti != tj && al > 0.f && be > 0.f) {
+        const float ak = ti ? be : al, at = ti ? al : be;
         rt.monitor *= at / ak;
         if (!(rt.monitor > tol)) {
           rt.apply = 0;
@@ -365,15 +377,15 @@ __global__ void __launch_bounds__(kNT, 2)
   __syncthreads();
   if (S.cnt > 0) {
     load(Wb, m, 0);
-    // ---- J in its real 64 × 64 form, B[n][k]: hi tiles (k < 32, k ≥ 32), then lo tiles ----
+    // ---- J in its real 64 × 64 form, B[n][k]: k < 32 and k ≥ 32, of each the hi parts of all n, then lo ----
     for (int e = tid; e < 64 * 64; e += kNT) {
       const int k = e & 63, nn = e >> 6;
       const float2 q = Q[k & 31][nn & 31];
       const float v = (k < 32) == (nn < 32) ? q.x : (nn < 32 ? -q.y : q.y);
       const float h = tf32_hi(v);
-      const uint32_t at = (uint32_t)(k >> 5) * 8192 + tile_at(nn, k & 31);
+      const uint32_t at = (uint32_t)(k >> 5) * 16384 + tile_at(nn, k & 31);
       *reinterpret_cast<float*>(bj + at) = h;
-      *reinterpret_cast<float*>(bj + 16384 + at) = v - h;
+      *reinterpret_cast<float*>(bj + 8192 + at) = v - h;
     }
     __syncthreads();  // Q's place becomes the operand buffer again
     // X ← X·J, 128 rows at a time: W, then V
@@ -397,19 +409,14 @@ __global__ void __launch_bounds__(kNT, 2)
       }
       publish();
       if (tid == 0) {
-        const uint32_t d = tmem + (uint32_t)(ch * 64);
-        uint32_t acc = 0;
-#pragma unroll 1
-        for (int pass = 0; pass < 3; ++pass) {  // lo·hi, hi·lo, hi·hi
 #pragma unroll
-          for (int kt = 0; kt < 2; ++kt) {
-            const uint64_t a = sdesc(smem_u32(buf + (pass == 0 ? 32768 : 0) + kt * 16384));
-            const uint64_t q = sdesc(smem_u32(bj + (pass == 1 ? 16384 : 0) + kt * 8192));
+        for (int kt = 0; kt < 2; ++kt) {
+          const uint64_t h = sdesc(smem_u32(buf + kt * 16384)), l = sdesc(smem_u32(buf + 32768 + kt * 16384));
+          const uint64_t q = sdesc(smem_u32(bj + kt * 16384));
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              mma(d, a + 2 * kk, q + 2 * kk, acc);
-              acc = 1;
-            }
+          for (int kk = 0; kk < 4; ++kk) {
+            mma(tmem, h + 2 * kk, q + 2 * kk, (kt > 0 || kk > 0) ? 1u : 0u, kIdesc128);  // hi·hi | hi·lo
+            mma(tmem, l + 2 * kk, q + 2 * kk, 1u);                                        // lo·hi
           }
         }
         mma_commit(&S.bar);
@@ -424,9 +431,15 @@ __global__ void __launch_bounds__(kNT, 2)
       finish();
       cxf* X = is_v ? Vb : Wb;
       const int rows = is_v ? n : m, row = ch * 128 + rloc;
-      float re[16], im[16];
-      tmem_ld16(tmem + tlane + (uint32_t)(ch * 64 + hf * 16), re);
-      tmem_ld16(tmem + tlane + (uint32_t)(ch * 64 + 32 + hf * 16), im);
+      float re[16], im[16], lo[16];
+      tmem_ld16(tmem + tlane + (uint32_t)(hf * 16), re);
+      tmem_ld16(tmem + tlane + (uint32_t)(64 + hf * 16), lo);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) re[j] += lo[j];
+      tmem_ld16(tmem + tlane + (uint32_t)(32 + hf * 16), im);
+      tmem_ld16(tmem + tlane + (uint32_t)(96 + hf * 16), lo);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) im[j] += lo[j];
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int col = S.col[hf * 16 + j];
