@@ -20,6 +20,7 @@ CASES = [
     ("axbyc", (64, 9, 32, 2, 20), "xyuv", (9, 2, 5, 7), "xy"),      # three runs of rows: permuted copy
     ("abxcy", (40, 30, 5, 33, 7), "uyvx", (6, 7, 9, 5), "xy"),      # b's legs interleaved
     ("axb", (300, 130, 150), "xu", (130, 33), "x"),
+    ("axb", (200, 300, 200), "xu", (300, 56), "x"),                 # k over more than one table of offsets
     ("abx", (200, 210, 1), "xu", (1, 40), "x"),                     # k = 1
     ("xab", (4, 128, 304), "ux", (32, 4), "x"),                     # exactly the smallest columns
     ("ayxb", (129, 8, 8, 310), "xyu", (8, 8, 64), "xy"),            # K order differs between a and b
