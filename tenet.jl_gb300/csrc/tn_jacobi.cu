@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "tn_fixed_sum.cuh"
 #include "tn_internal.cuh"
 
 namespace {
@@ -129,28 +130,6 @@ __device__ __forceinline__ double widen(float f) {
 // f · 2^s for a normal f whose result is normal
 __device__ __forceinline__ float shifted(float f, int s) { return __int_as_float(__float_as_int(f) + (s << 23)); }
 
-// Sums of FP64 values in fixed point: integer additions and the warp's redux take 4 to 30 clocks
-// where a DADD takes 64.  Every lane's value is cut to 55 bits below 2^(emax − 1022), emax the
-// largest exponent field of the warp, so a cut is at most 2⁻⁵⁵ of the largest value: less than
-// the rounding of an FP64 sum.  The parts of 24 bits add up without a carry between them.
-__device__ __forceinline__ unsigned exponent_field(double v) { return ((unsigned)__double2hiint(v) >> 20) & 0x7ff; }
-__device__ __forceinline__ long long fixed_warp_sum(double v, unsigned emax) {
-  const int hi = __double2hiint(v);
-  const unsigned e = exponent_field(v);
-  unsigned long long b = ((unsigned long long)((hi & 0xfffff) | 0x100000) << 34) | ((unsigned long long)(unsigned)__double2loint(v) << 2);
-  b = e ? b >> min(emax - e, 63u) : 0ull;
-  const long long sg = hi >> 31, f = ((long long)b ^ sg) - sg;
-  const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)f & 0xffffffu);
-  const unsigned mid = __reduce_add_sync(0xffffffffu, (unsigned)(f >> 24) & 0xffffffu);
-  const int top = __reduce_add_sync(0xffffffffu, (int)(f >> 48));
-  return ((long long)top << 48) + ((long long)mid << 24) + (long long)lo;
-}
-// |T| < 2⁶³ as a float
-__device__ __forceinline__ float fixed_to_float(long long T) {
-  const unsigned long long A = T < 0 ? (unsigned long long)-T : (unsigned long long)T;
-  const float f = fmaf((float)(unsigned)(A >> 32), 4294967296.f, (float)(unsigned)A);
-  return T < 0 ? -f : f;
-}
 // 1/x of a positive normal x: the hardware's approximation (20 bits or so) and one step of third
 // order, y ← y + y·e(1 + e) with e = 1 − x·y
 __device__ __forceinline__ double reciprocal(double x) {
@@ -644,10 +623,7 @@ __global__ void __launch_bounds__(kNT, 4)
         E = max(e0, e1);
         total = (fix[buf][half][0] >> min(E - e0, 63)) + (fix[buf][half][1] >> min(E - e1, 63));
       } else {
-        const int4 ew = *reinterpret_cast<const int4*>(fix_e[buf][half]);
-        E = max(max(ew.x, ew.y), max(ew.z, ew.w));
-        total = ((fix[buf][half][0] >> min(E - ew.x, 63)) + (fix[buf][half][1] >> min(E - ew.y, 63))) +
-                ((fix[buf][half][2] >> min(E - ew.z, 63)) + (fix[buf][half][3] >> min(E - ew.w, 63)));
+        total = fixed_sum4(fix[buf][half], fix_e[buf][half], E);
       }
       buf ^= 1;
       // ρ = γ/√(αβ)

@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "tn_fixed_sum.cuh"
 #include "tn_internal.cuh"
 
 namespace {
@@ -92,16 +93,6 @@ __device__ __forceinline__ double reciprocal(double x) {
   return fma(y, fma(e, e, e), y);
 }
 
-// Σ over the warp of (a, b): lanes 0-15 end with Σa, lanes 16-31 with Σb
-__device__ __forceinline__ double warp_sum2(double a, double b, int lane) {
-  double keep = (lane & 16) ? b : a;
-  const double send = (lane & 16) ? a : b;
-  keep += __shfl_xor_sync(0xffffffffu, send, 16);
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) keep += __shfl_xor_sync(0xffffffffu, keep, o);
-  return keep;
-}
-
 // a batch of equal matrices: the first one and the strides to the next; or a list of matrices
 // of falling n, whose columns are taken in the order 0 of all, 1 of all, …
 struct QBatch {
@@ -144,7 +135,8 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
   const int col = row ? m + k : index;  // (rows wait for all reflectors)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = lane >> 4;
   const int64_t stride = 2 * (int64_t)m + 4;
-  __shared__ double red[2][4][2];
+  __shared__ __align__(16) long long fix[2][2][4];  // parity, Re or Im, warp: partial sums in fixed point
+  __shared__ __align__(16) int fix_e[2][4];
   __shared__ double s_row[2][2];  // this column's entry in the pivot row
   __shared__ int s_fail;
   if (tid == 0) s_fail = 0;
@@ -205,8 +197,15 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
         s_row[buf][1] = x[q].y;
       }
     }
-    const double s = warp_sum2(wx, wy, lane);
-    if ((lane & 15) == 0) red[buf][warp][half] = s;
+    {
+      const unsigned e = __reduce_max_sync(0xffffffffu, max(exponent_field(wx), exponent_field(wy)));
+      const long long s0 = fixed_warp_sum(wx, e), s1 = fixed_warp_sum(wy, e);
+      if (lane == 0) {
+        fix[buf][0][warp] = s0;
+        fix[buf][1][warp] = s1;
+        fix_e[buf][warp] = (int)e;
+      }
+    }
     const bool far = adj && col > j + 8;
     while (!(arrived(p0) && arrived(p1)) && ++spins < kSpinLimit) {
       if (far) __nanosleep(kFarSleep);
@@ -221,9 +220,9 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     }
     __syncthreads();
     if (s_fail) return false;
-    double d = red[buf][lane & 3][half];
-    d += __shfl_xor_sync(0xffffffffu, d, 1);
-    d += __shfl_xor_sync(0xffffffffu, d, 2);
+    int E;
+    const long long total = fixed_sum4(fix[buf][half], fix_e[buf], E);
+    const double d = fixed_value(total, E);
     const double ux = value_of(p0), uy = value_of(p1);
     // w = uᴴx + conj(u₁)·x_j, f = κ'·w (κ' = conj(κ) for Hᴴ): Re in lanes 0-15, Im in 16-31
     const double cx_ = s_row[buf][0], cy_ = s_row[buf][1];
@@ -284,12 +283,20 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
         s_row[buf][1] = x[q].y;
       }
     }
-    s2 = warp_sum(s2);
-    if (lane == 0) red[buf][warp][0] = s2;
+    {
+      const unsigned e = __reduce_max_sync(0xffffffffu, exponent_field(s2));
+      const long long s0 = fixed_warp_sum(s2, e);
+      if (lane == 0) {
+        fix[buf][0][warp] = s0;
+        fix_e[buf][warp] = (int)e;
+      }
+    }
     __syncthreads();
-    s2 = red[buf][lane & 3][0];
-    s2 += __shfl_xor_sync(0xffffffffu, s2, 1);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, 2);
+    {
+      int E;
+      const long long total = fixed_sum4(fix[buf][0], fix_e[buf], E);
+      s2 = fixed_value(total, E);
+    }
     const double ax = s_row[buf][0], ay = s_row[buf][1];
     buf ^= 1;
     double beta = ax, ux = 0, uy = 0, kx = 0, ky = 0;

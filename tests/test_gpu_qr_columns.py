@@ -81,3 +81,17 @@ def test_columns_qr_of_special_matrices(ctx, scale):
     A = scale * np.stack([zero, twice, g.real + 0j, np.triu(g)])
     Q, R = _qr(ctx, A)
     _check(A, Q, R, lapack=False)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("m,n", [(60, 24), (200, 40)])
+def test_columns_qr_non_finite(ctx, bad, m, n):
+    """A column that is not finite spoils its own part of R, and Q from there on, and no column of R
+    before it (Q's earlier columns follow all reflectors where its rows are formed)."""
+    rng = np.random.default_rng(6)
+    A = rng.standard_normal((1, m, n)) + 1j * rng.standard_normal((1, m, n))
+    clean = A.copy()
+    A[0, m // 2, 7] = bad
+    Q, R = _qr(ctx, A)
+    assert np.abs(R[0][:, :7] - np.linalg.qr(clean[0])[1][:, :7]).max() <= 1e-9
+    assert not np.isfinite(R[0][:8, 7]).all() and not np.isfinite(Q[0][:, 8:]).any()
