@@ -91,7 +91,7 @@ const char* tn_version(void);
  * time (ms) and the algorithmic flops and bytes.  Classes: 0 Jacobi sweeps FP32, 1 Jacobi
  * sweeps FP64, 2 complex FP64 GEMM, 3 split-BF16 tensor-core GEMM (flops = the BF16
  * tensor-pipe products it issues), 4 its digit-plane preparation, 5 Householder QR,
- * 6 cooperative small-matrix Jacobi.  Enabling (or disabling) resets the totals. */
+ * 6 column-pair Jacobi (a whole iteration per launch).  Enabling (or disabling) resets the totals. */
 tn_status_t tn_profile_enable(tn_ctx* ctx, int32_t enable);
 tn_status_t tn_profile_read(tn_ctx* ctx, int32_t cls, int64_t* launches, double* ms, double* flops,
                             double* bytes);

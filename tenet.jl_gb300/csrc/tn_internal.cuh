@@ -243,7 +243,7 @@ enum {
   TN_PROF_GEMM_SPLIT = 3,   // split-BF16 tensor-core GEMM kernel (k_gemm_oz)
   TN_PROF_SPLIT_PREP = 4,   // its digit-plane preparation
   TN_PROF_QR = 5,           // blocked Householder QR (panel + block reflector)
-  TN_PROF_JACOBI_COOP = 6,  // cooperative small-matrix Jacobi (whole iteration)
+  TN_PROF_JACOBI_COOP = 6,  // column-pair Jacobi, a whole iteration per launch
   TN_PROF_NCLASS = 7
 };
 int prof_begin(tn_ctx* ctx);
