@@ -20,8 +20,9 @@
 //    one M = 128, N = 64 product gives hi·hi and lo·hi, and G = HH + LH + LHᵀ.  Each 128 rows
 //    have their own accumulator; they are added in FP32.
 //  * W·J, V·J: per 128 rows A (rows × 64 real columns) hi and lo against the 64 × 64 real form
-//    of J: hi·[hi | lo] as one product of N = 128 and lo·hi, added in FP32 (products of N = 64
-//    take the tensor pipe nearly as long as those of N = 128).
+//    of J: hi·[hi | lo] and lo·[hi | lo] as products of N = 128, the halves added in FP32 (products of
+//    N = 64 take the tensor pipe nearly as long).  All products into an accumulator have one
+//    shape: only those are executed in the order of issue.
 // One 64 KB operand buffer, which between the products also holds G and J, leaves room for two
 // CTAs per SM: one's rotations run under the other's products and memory traffic.
 // A round of 16 matrices of n = 512 takes 44 µs (47 with J's hi and lo parts as products of their
@@ -131,7 +132,7 @@ __device__ __forceinline__ Rot rotation(float al, float be, float gx, float gy, 
   const float ra = rsqrt_approx(al), rb = rsqrt_approx(be);
   const float px = gx * ra * rb, py = gy * ra * rb;
   const float rho2 = fmaf(px, px, py * py);
-  if (!(rho2 > 0.f)) return R;
+  if (!(rho2 > 1.2e-38f)) return R;  // (below: no normal number, and nothing the threshold would see)
   const float irho = rsqrt_approx(rho2), rho = rho2 * irho;
   R.monitor = rho;
   if (!(rho > tol)) return R;
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(kNT, 2)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
             mma(tmem, h + 2 * kk, q + 2 * kk, (kt > 0 || kk > 0) ? 1u : 0u, kIdesc128);  // hi·hi | hi·lo
-            mma(tmem, l + 2 * kk, q + 2 * kk, 1u);                                        // lo·hi
+            mma(tmem, l + 2 * kk, q + 2 * kk, 1u, kIdesc128);                             // lo·hi | lo·lo
           }
         }
         mma_commit(&S.bar);

@@ -89,6 +89,16 @@ def test_mixed_svd(ctx, m, n, batch):
     _check(A, *_svd(ctx, A, 1), 1e-12)
 
 
+@pytest.mark.parametrize("m,n", [(128, 128), (256, 200), (512, 512)])
+@pytest.mark.parametrize("coupling", [0.0, 1e-15, 1e-20, 1e-22, 1e-25, 1e-40])
+def test_mixed_svd_of_nearly_orthogonal_columns(ctx, m, n, coupling):
+    """Couplings whose squares are no normal FP32 numbers must not turn into rotations."""
+    rng = np.random.default_rng(m + n)
+    A = coupling * _gauss(rng, (m, n))
+    A[np.arange(n), rng.permutation(n)] += np.linspace(1.0, 2.0, n) * np.exp(2j * np.pi * rng.random(n))
+    _check(A[None], *_svd(ctx, A[None], 1), 1e-12)
+
+
 @pytest.mark.parametrize("m,n", [(32, 32), (100, 40)])
 @pytest.mark.parametrize("scale", [1.0, 1e-130, 1e130])
 def test_columns_of_different_scale(ctx, m, n, scale):
