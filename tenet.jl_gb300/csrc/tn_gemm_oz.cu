@@ -35,7 +35,7 @@
 // batch instances in turn.  Warp 4 lane 0 issues TMA loads: a K stage is 32 BF16 (64 bytes,
 // 64-byte swizzle) of all S digit planes of both tiles, two stages in shared memory.  Warp 5
 // lane 0 issues tcgen05.mma (M=128, K=16): plane p of A against every plane q < S − p of
-// B, into level p + q (TMEM columns 64·(p+q)…).  After that group plane p of A and plane S−1−p
+// B, into level p + q (TMEM columns 64·(p+q)…).  After that group plane p of A and plane 7−p
 // of B are not needed again in this stage, so their place is given back to the producer group by
 // group, one stage ahead of its next use.  Warps 0-3 read the S level accumulators with
 // tcgen05.ld (warp w owns rows 32w…32w+31) into int64 sums in registers, give the accumulators
@@ -44,12 +44,12 @@
 // remaining work and still releases its TMEM.
 //
 // What bounds it: the operands' way into shared memory.  The S planes of B lie one after the
-// other and so do the levels, so up to four planes of B are one operand of N = 256: a tile of
-// k = 256 takes 35 thousand clocks of tensor pipe (a product per pair of planes, N = 64, took 81
+// other and so do the levels, so four planes of B are one operand of N = 256: a tile of
+// k = 256 takes 47 thousand clocks of tensor pipe (a product per pair of planes, N = 64, took 81
 // clocks each, 90 thousand), its 1.5 MB of planes 53 thousand at the 29 bytes per clock and SM
 // that come from L2.  Reading the accumulators takes 12 thousand more; the rest of the epilogue (3
 // thousand; with 14 FP64 operations of 64 clocks per column 88 to 129) runs beside the next tile.
-// 16 products of 512 × 512 × 512: 1.97 → 0.77 ms, of it the operand preparation 0.54 → 0.24.
+// 16 products of 512 × 512 × 512: 1.97 → 0.86 ms, of it the operand preparation 0.54 → 0.24.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -62,12 +62,15 @@ namespace {
 
 constexpr int OZ_BM = 128, OZ_BN = 64, OZ_BK = 32;  // tile 128×64, 32 BF16 (64 B) of K per stage
 constexpr int OZ_MAX_S = 8;
+constexpr int OZ_WIN = 4;  // levels of one accumulator, planes of B in one product (N = 256)
 constexpr int OZ_A_TILE = OZ_BM * OZ_BK * 2;  // 8 KB
 constexpr int OZ_B_TILE = OZ_BN * OZ_BK * 2;  // 4 KB
 constexpr int OZ_THREADS = 192;
 constexpr long long kOzSpin = 1ll << 24;
 
-inline int oz_smem_bytes(int S) { return 2 * S * (OZ_A_TILE + OZ_B_TILE) + 1024 + 512; }
+// planes of B that a stage has room for: three of zeros, then a multiple of OZ_WIN
+__host__ __device__ inline int oz_b_planes(int S) { return OZ_WIN - 1 + (S <= OZ_WIN ? OZ_WIN : 2 * OZ_WIN); }
+inline int oz_smem_bytes(int S) { return 2 * (S * OZ_A_TILE + oz_b_planes(S) * OZ_B_TILE) + 1024 + 512; }
 
 struct OzMaps {
   CUtensorMap a;  // digit planes of A'': (2k, 2m, S·batch), plane-major
@@ -116,16 +119,15 @@ __device__ __forceinline__ uint64_t sdesc(const void* p) {
   d |= 4ull << 61;
   return d;
 }
-// instruction descriptor, kind::f16: D f32, A and B bf16, both K-major, M = 128
-__device__ __forceinline__ uint32_t idesc_bf16(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
-}
+// instruction descriptor, kind::f16: D f32, A and B bf16, both K-major, M = 128, N = 256
+constexpr uint32_t kIdescBF16 =
+    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_WIN * OZ_BN >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
 
-__device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+__device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t accum) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
           dtmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accum)
+      "l"(a), "l"(b), "r"(kIdescBF16), "r"(accum)
       : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -159,8 +161,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   const uint32_t base_u = smem_u32(smem_raw);
   unsigned char* smem = smem_raw + ((1024 - (base_u & 1023)) & 1023);
   unsigned char* sA = smem;                          // 2 stages × S planes
-  unsigned char* sB = smem + 2 * S * OZ_A_TILE;      // 2 stages × S planes
-  uint64_t* full = reinterpret_cast<uint64_t*>(sB + 2 * S * OZ_B_TILE);  // [2]
+  const int b_planes = oz_b_planes(S), SB = b_planes - (OZ_WIN - 1);
+  unsigned char* sZ = smem + 2 * S * OZ_A_TILE;      // 2 stages × (3 planes of zeros and SB of B)
+  unsigned char* sB = sZ + (OZ_WIN - 1) * OZ_B_TILE;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sZ + 2 * b_planes * OZ_B_TILE);  // [2]
   uint64_t* empty = full + 2;                                            // [2][OZ_MAX_S]
   uint64_t* acc_full = empty + 2 * OZ_MAX_S;
   uint64_t* acc_empty = acc_full + 1;
@@ -197,6 +201,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     mbar_init(acc_empty, 4);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  for (int t = tid; t < 2 * b_planes * (OZ_B_TILE / 16); t += OZ_THREADS)  // (also what no plane is loaded to)
+    reinterpret_cast<uint4*>(sZ)[t] = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -205,7 +212,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 
   if (warp == 4) {
     if (lane == 0) {
-      // producer: planes p of A and S − 1 − p of B as the stage before last gives their place back
+      // producer: planes p of A and SB − 1 − p of B as the stage before last gives their place back
       long long g = 0;
       bool ok = true;
       for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
@@ -219,8 +226,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             if (g >= 2 && !(ok = mbar_wait(&empty[kb * OZ_MAX_S + p], parity, err))) break;
             if (p == 0) mbar_expect_tx(&full[kb], (uint32_t)(S * (OZ_A_TILE + OZ_B_TILE)));
             tma_load_3d(sA + (kb * S + p) * OZ_A_TILE, &maps.a, &full[kb], ks * OZ_BK, m0, p * batch + bidx);
-            const int q = S - 1 - p;
-            tma_load_3d(sB + (kb * S + q) * OZ_B_TILE, &maps.b, &full[kb], ks * OZ_BK, n0, q * batch + bidx);
+            // (after group p plane SB − 1 − p is done with, after the last group all of them)
+            for (int q = min(S - 1, SB - 1 - p); q >= (p == S - 1 ? 0 : SB - 1 - p); --q)
+              tma_load_3d(sB + (kb * b_planes + q) * OZ_B_TILE, &maps.b, &full[kb], ks * OZ_BK, n0, q * batch + bidx);
           }
         }
       }
@@ -239,15 +247,16 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           if (!(ok = mbar_wait(&full[kb], (uint32_t)(g >> 1) & 1, err))) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           for (int p = 0; p < S; ++p) {
-            // the planes of B lie one after the other, and so do the levels: up to four planes are one
-            // operand of N = 256
-            const uint64_t a0 = sdesc(sA + (kb * S + p) * OZ_A_TILE), b0 = sdesc(sB + kb * S * OZ_B_TILE);
-            for (int q = 0; q < S - p; q += 4) {
-              const uint32_t idesc = idesc_bf16(OZ_BN * min(4, S - p - q));
+            // The planes of B lie one after the other, and so do the levels: four planes are one operand
+            // of N = 256 for the levels 0 … 3 or 4 … 7, planes before the first are zeros.  (All
+            // products into an accumulator have one shape: only those are executed in the order
+            // of issue.)
+            const uint64_t a0 = sdesc(sA + (kb * S + p) * OZ_A_TILE), b0 = sdesc(sB + kb * b_planes * OZ_B_TILE);
+            for (int w = p < OZ_WIN ? 0 : OZ_WIN; w < SB; w += OZ_WIN) {
 #pragma unroll
               for (int kk = 0; kk < OZ_BK / 16; ++kk)  // K = 16 BF16 = 32 bytes
-                mma_bf16(tmem + (uint32_t)((p + q) * OZ_BN), a0 + (uint64_t)kk * 2,
-                         b0 + (uint64_t)(q * (OZ_B_TILE >> 4) + kk * 2), idesc, (ks > 0 || p > 0 || kk > 0) ? 1u : 0u);
+                mma_bf16(tmem + (uint32_t)(w * OZ_BN), a0 + (uint64_t)kk * 2,
+                         b0 + (uint64_t)((int64_t)(w - p) * (OZ_B_TILE >> 4) + kk * 2), (ks > 0 || p > 0 || kk > 0) ? 1u : 0u);
             }
             mma_commit(&empty[kb * OZ_MAX_S + p]);
           }
@@ -596,7 +605,7 @@ tn_status_t gemm_c64_split(tn_ctx* ctx, int S, char opa, char opb, int64_t m, in
   if (k == 0) return gemm_cx<double>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
   // Aᴴ·A: B'' is the even rows of A'', so its planes need not be cut, and with a real alpha the
   // product is Hermitian: for beta = 0, or where C is known to be, the tiles above the diagonal
-  // are enough (16 × 512³: 0.79 → 0.46 ms)
+  // are enough (16 × 512³: 0.87 → 0.51 ms)
   const bool gram = opa == 'C' && opb == 'N' && A == B && lda == ldb && (sA == sB || batch == 1) && m == n;
   const bool upper = gram && alpha.y == 0.0 && ((beta.x == 0.0 && beta.y == 0.0) || (hermitian && beta.y == 0.0));
   // a level's FP32 sum is exact while S·(2k)·2^{2b-2} ≤ 2^24: the widest such digit b
