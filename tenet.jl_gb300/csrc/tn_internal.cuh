@@ -377,6 +377,8 @@ template <typename T>
 tn_status_t qr_cx(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>* A, int64_t lda, int64_t sA,
                   cx<T>* Q, int64_t sQ, cx<T>* R, int64_t sR, int64_t batch);
 
+tn_status_t lq_in_place(tn_ctx* ctx, int64_t m, int64_t n, cxd* A, int64_t sA, cxd* R, int64_t sR, int64_t batch, bool* done);
+
 // thin QR with one CTA per column (tn_qr_cols.cu): of op(A)·Π, Q m × k (ld m) or null, R k × n
 // (ld k) or its adjoint (ld n)
 size_t qr_cols_workspace(int64_t m, int64_t n, int64_t batch);

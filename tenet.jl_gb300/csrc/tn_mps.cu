@@ -156,8 +156,12 @@ tn_status_t gauge_left(tn_mps* p, int i, bool svd_lambda) {
   cxd* Q = ws_take<cxd>(ctx, (size_t)(B * m * n));
   cxd* R = ws_take<cxd>(ctx, (size_t)(B * k * n));
   cxd* tmp = ws_take<cxd>(ctx, (size_t)(B * rows_b * k));
-  TN_RETURN_IF(transpose_cx<double>(ctx, n, m, p->site[i], n, p->cap[i], Mh, m, m * n, B, true));
-  if (svd_lambda) {
+  bool in_place = false;
+  if (!svd_lambda) TN_RETURN_IF(lq_in_place(ctx, m, n, p->site[i], p->cap[i], R, k * n, B, &in_place));
+  if (!in_place) TN_RETURN_IF(transpose_cx<double>(ctx, n, m, p->site[i], n, p->cap[i], Mh, m, m * n, B, true));
+  if (in_place) {
+    // site i is Qᴴ already
+  } else if (svd_lambda) {
     TN_RETURN_IF(ensure_lam(p, k));
     TN_RETURN_IF(svd_any(ctx, TN_C64, p->prec, m, n, Mh, m, m * n, Q, m * n, p->lam, p->lam_cap, R, k * n, B));
     p->lam_len = k;
@@ -165,7 +169,7 @@ tn_status_t gauge_left(tn_mps* p, int i, bool svd_lambda) {
     TN_RETURN_IF(qr_cx<double>(ctx, m, n, Mh, m, m * n, Q, m * n, R, k * n, B));
   }
   // new site i = Qᴴ (k × d χ_r)
-  TN_RETURN_IF(transpose_cx<double>(ctx, m, k, Q, m, m * n, p->site[i], k, p->cap[i], B, true));
+  if (!in_place) TN_RETURN_IF(transpose_cx<double>(ctx, m, k, Q, m, m * n, p->site[i], k, p->cap[i], B, true));
   // site i-1 ← B · Rᴴ
   TN_RETURN_IF(gemm_c64(ctx, p->prec, 'N', 'C', rows_b, k, n, kOne, p->site[i - 1], rows_b, p->cap[i - 1], R, k, k * n,
                         kZero, tmp, rows_b, rows_b * k, B));

@@ -345,6 +345,36 @@ static tn_status_t qr_takes_columns(tn_ctx* ctx, int64_t m, int64_t n, const cxd
   return qr_cols_takes(ctx, m, n * batch, out);
 }
 
+// the tuning table's key of a shape
+static void qr_tuning_key(char* key, size_t bytes, size_t elem, int64_t m, int64_t n, int64_t batch) {
+  const int bb = batch <= 1 ? 1 : batch <= 4 ? 4 : batch <= 16 ? 16 : 64;
+  snprintf(key, bytes, "qr%zu:%lld:%lld:%d", elem, (long long)m, (long long)n, bb);
+}
+static void qr_columns_profile(tn_ctx* ctx, int slot, int64_t m, int64_t n, int64_t batch) {
+  const double kk = (double)std::min(m, n), f = 4.0 * (2.0 * m * kk * kk - 2.0 / 3.0 * kk * kk * kk);
+  if (slot >= 0)
+    prof_end(ctx, slot, TN_PROF_QR, 1, 2.0 * f * batch, sizeof(cxd) * ((double)m * n + (double)m * kk + kk * n) * batch);
+}
+
+// Aᴴ = Q·R of a batch of n × m matrices (m ≥ n, dense) with Qᴴ in A's place and R n × n, where the
+// column kernel takes the shape (done): neither the adjoint nor its way back is a pass over memory
+tn_status_t lq_in_place(tn_ctx* ctx, int64_t m, int64_t n, cxd* A, int64_t sA, cxd* R, int64_t sR, int64_t batch, bool* done) {
+  *done = false;
+  if (m < n || n == 0 || batch == 0) return TN_OK;
+  char key[96];
+  qr_tuning_key(key, sizeof(key), sizeof(double), m, n, batch);
+  if (ctx->tuning.find(key) != ctx->tuning.end()) return TN_OK;
+  if (batch > 1 && (sA < m * n || sR < n * n)) return TN_OK;
+  if (ranges_meet(R, sizeof(cxd) * (size_t)((batch - 1) * sR + n * n), A, sizeof(cxd) * (size_t)((batch - 1) * sA + m * n)))
+    return TN_OK;
+  TN_RETURN_IF(qr_cols_takes(ctx, m, n * batch, done));
+  if (!*done) return TN_OK;
+  const int slot = prof_begin(ctx);
+  TN_RETURN_IF(qr_cols_batch(ctx, m, n, A, n, sA, A, sA, R, sR, batch, nullptr, true, false, true));
+  qr_columns_profile(ctx, slot, m, n, batch);
+  return TN_OK;
+}
+
 // Panel width and slab width come from the context's tuning table, keyed by the shape
 // (m, n and a batch bucket).  With autotuning on, the first call of an unseen shape
 // times every candidate (panel 4/8/16/32 that fits shared memory × slab 1/2/4) with
@@ -359,9 +389,8 @@ tn_status_t qr_cx(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>* A, int64_t lda
   if (sizeof(cx<T>) * (size_t)m * 1 > kPanelSmemMax)
     return tn_set_error(ctx, TN_EUNSUPPORTED, "qr: m=%lld too large for the panel kernel", (long long)m);
   const int64_t npan_max = (k + nb_max - 1) / nb_max;
-  const int bb = batch <= 1 ? 1 : batch <= 4 ? 4 : batch <= 16 ? 16 : 64;
   char key[96];
-  snprintf(key, sizeof(key), "qr%zu:%lld:%lld:%d", sizeof(T), (long long)m, (long long)n, bb);
+  qr_tuning_key(key, sizeof(key), sizeof(T), m, n, batch);
   auto it = ctx->tuning.find(key);
   const double kk = (double)k, f = 4.0 * (2.0 * m * kk * kk - 2.0 / 3.0 * kk * kk * kk);
   if constexpr (sizeof(T) == 8) {
@@ -371,9 +400,7 @@ tn_status_t qr_cx(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>* A, int64_t lda
     if (columns) {
       const int slot = prof_begin(ctx);
       TN_RETURN_IF(qr_cols_batch(ctx, m, n, A, lda, sA, Q, sQ, R, sR, batch));
-      if (slot >= 0)
-        prof_end(ctx, slot, TN_PROF_QR, 1, 2.0 * f * batch,
-                 sizeof(cx<T>) * ((double)m * n + (double)m * k + (double)k * n) * batch);
+      qr_columns_profile(ctx, slot, m, n, batch);
       return TN_OK;
     }
   }
