@@ -195,18 +195,17 @@ _PIPE = {"jacobi_fp32": ("fp32_tflops", "fp32_cuda_cores"), "jacobi_fp64": ("fp6
          "gemm_fp64": ("fp64_tflops", "fp64_cuda_cores"), "gemm_split_bf16": ("bf16_tflops", "tensor"),
          "split_prep": (None, "hbm"), "qr": ("fp64_tflops", "fp64_cuda_cores"),
          "jacobi_coop": ("fp64_tflops", "fp64_cuda_cores")}
-_KERNEL = {"jacobi_fp32": "k_jacobi_block_f32 (FP32 block rounds)", "jacobi_fp64": "k_jacobi_step_reg<double>",
-           "gemm_fp64": "k_gemm_cx<double>", "gemm_split_bf16": "k_gemm_oz (tcgen05 kind::f16)",
-           "split_prep": "k_oz_scales + k_oz_split", "qr": "k_qr_panel + k_apply_block_reflector",
-           "jacobi_coop": "k_jacobi_coop<double>"}
+_KERNEL = {"jacobi_fp32": "k_jacobi_block_tc (block rounds, tcgen05 kind::tf32)", "jacobi_fp64": "k_jacobi_step_reg<double>",
+           "gemm_fp64": "k_gemm_fine<double> / k_gemm_cx<double>", "gemm_split_bf16": "k_gemm_oz (tcgen05 kind::f16)",
+           "split_prep": "k_oz_scales + k_oz_split", "qr": "k_qr_cols, k_qr_panel + k_apply_block_reflector",
+           "jacobi_coop": "k_jacobi_pairs"}
 
 
 # what ncu shows bounds each class beyond the two roofs (profiles/ summaries)
-_LIMIT = {"jacobi_fp32": "instruction issue (ncu: 56-61 % of issue slots busy, one 512-thread CTA per SM); DRAM "
-                         "traffic is half the algorithmic bytes (the rest hits L2)",
-          "gemm_split_bf16": "N = 64 tiles (TMEM holds 8 levels x 64 columns): tensor subpipe 64 % busy yields 0.21 "
-                             "of peak; one CTA per SM, epilogue not overlapped",
-          "qr": "the FP64 pipe (one panel CTA per matrix between block-reflector updates)"}
+_LIMIT = {"jacobi_fp32": "the chain of a block pair's products and rotations (two CTAs per SM, one under the other)",
+          "gemm_split_bf16": "the digit planes' way from L2 into shared memory (29 bytes per clock and SM)",
+          "qr": "the FP64 pipe (batches of 16), the chain of one step per column (single matrices)",
+          "jacobi_coop": "the chain of one round; the FP64 pipe from two CTAs per SM"}
 
 
 def kernel_rooflines(prof, peaks):
@@ -1080,7 +1079,7 @@ def run_dmrg(args):
     launches = ctx.launches() - launches0
     ms = float(np.mean(times))
     stats = tenetgb.dmrg_last_stats(ctx)
-    # dominant kernel: the pair SVD (k_jacobi_coop, one launch per 256×256 split).
+    # dominant kernel: the pair SVD (k_jacobi_pairs, one launch per 256×256 split).
     # Algorithmic flops per launch = sweeps × 255 rounds × 128 pairs × (8m + 24m), m = 256
     # (no right vectors), the sweeps averaged over the call's splits; time per launch =
     # the splits' device time (CUDA events) ÷ the local updates
@@ -1089,7 +1088,7 @@ def run_dmrg(args):
     split_ms = stats["split_ms"] / max(1, stats["updates"])
     peak = ctx.pipe_peak("fp64")
     achieved = flops / (split_ms * 1e-3) / 1e12
-    roofline = {"bound": "fp64_cuda_cores", "kernel": "k_jacobi_coop<double> (FP64 pipe; latency-bound rounds)",
+    roofline = {"bound": "fp64_cuda_cores", "kernel": "k_jacobi_pairs (FP64 pipe; latency-bound rounds)",
                 "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
                 "peak_source": "FP64 FMA rate of the CUDA cores measured in this run (tn_pipe_peak)",
                 "flops_per_launch": flops, "sweeps_per_split": sweeps_per_split, "launch_avg_ms": split_ms,
