@@ -203,7 +203,7 @@ _KERNEL = {"jacobi_fp32": "k_jacobi_block_tc (block rounds, tcgen05 kind::tf32)"
 
 # what ncu shows bounds each class beyond the two roofs (profiles/ summaries)
 _LIMIT = {"jacobi_fp32": "the chain of a block pair's products and rotations (two CTAs per SM, one under the other)",
-          "gemm_split_bf16": "the digit planes' way from L2 into shared memory (29 bytes per clock and SM)",
+          "gemm_split_bf16": "the tensor pipe, and reading the accumulators between tiles",
           "qr": "the FP64 pipe (batches of 16), the chain of one step per column (single matrices)",
           "jacobi_coop": "the chain of one round; the FP64 pipe from two CTAs per SM"}
 

@@ -34,22 +34,22 @@
 // Kernel.  One persistent CTA (6 warps) per SM takes 128×64 tiles of the real 4M product of all
 // batch instances in turn.  Warp 4 lane 0 issues TMA loads: a K stage is 32 BF16 (64 bytes,
 // 64-byte swizzle) of all S digit planes of both tiles, two stages in shared memory.  Warp 5
-// lane 0 issues tcgen05.mma (M=128, K=16): plane p of A against every plane q < S − p of
-// B, into level p + q (TMEM columns 64·(p+q)…).  After that group plane p of A and plane 7−p
-// of B are not needed again in this stage, so their place is given back to the producer group by
-// group, one stage ahead of its next use.  Warps 0-3 read the S level accumulators with
+// lane 0 issues tcgen05.mma (M=128, N=256, K=16): plane p of A against four planes of B at a time,
+// every plane q < S − p into level p + q (TMEM columns 64·(p+q)…).  After plane 3 of A, the first four
+// of A and the last four of B are not needed again in this stage, and their place goes back to the
+// producer one stage ahead of its next use.  Warps 0-3 read the S level accumulators with
 // tcgen05.ld (warp w owns rows 32w…32w+31) into int64 sums in registers, give the accumulators
 // back to warp 5, and finish and write C while the next tile is multiplied.
 // Every mbarrier wait is bounded: on timeout the kernel records an error word, skips the
 // remaining work and still releases its TMEM.
 //
-// What bounds it: the operands' way into shared memory.  The S planes of B lie one after the
-// other and so do the levels, so four planes of B are one operand of N = 256: a tile of
-// k = 256 takes 47 thousand clocks of tensor pipe (a product per pair of planes, N = 64, took 81
-// clocks each, 90 thousand), its 1.5 MB of planes 53 thousand at the 29 bytes per clock and SM
-// that come from L2.  Reading the accumulators takes 12 thousand more; the rest of the epilogue (3
-// thousand; with 14 FP64 operations of 64 clocks per column 88 to 129) runs beside the next tile.
-// 16 products of 512 × 512 × 512: 1.97 → 0.86 ms, of it the operand preparation 0.54 → 0.24.
+// What bounds it: the tensor pipe.  The S planes of B lie one after the other and so do the
+// levels, so four planes of B are one operand of N = 256: a tile of k = 256 takes 47 thousand clocks of
+// tensor pipe (a product per pair of planes, N = 64, took 81 clocks each, 90 thousand).  Its planes come
+// four to a TMA load; one load each, 16 a stage, took 53 thousand clocks to issue and complete.
+// Reading the accumulators takes 12 thousand more; the rest of the epilogue (3 thousand; with 14
+// FP64 operations of 64 clocks per column 88 to 129) runs beside the next tile.
+// 16 products of 512 × 512 × 512: 1.97 → 0.77 ms, of it the operand preparation 0.54 → 0.24.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -68,13 +68,15 @@ constexpr int OZ_B_TILE = OZ_BN * OZ_BK * 2;  // 4 KB
 constexpr int OZ_THREADS = 192;
 constexpr long long kOzSpin = 1ll << 24;
 
-// planes of B that a stage has room for: three of zeros, then a multiple of OZ_WIN
-__host__ __device__ inline int oz_b_planes(int S) { return OZ_WIN - 1 + (S <= OZ_WIN ? OZ_WIN : 2 * OZ_WIN); }
-inline int oz_smem_bytes(int S) { return 2 * (S * OZ_A_TILE + oz_b_planes(S) * OZ_B_TILE) + 1024 + 512; }
+// planes that a stage has room for: a multiple of OZ_WIN, those beyond S are filled with zeros
+__host__ __device__ inline int oz_planes(int S) { return S <= OZ_WIN ? OZ_WIN : 2 * OZ_WIN; }
+inline int oz_smem_bytes(int S) {  // (three planes of zeros before B's)
+  return 2 * (oz_planes(S) * OZ_A_TILE + (oz_planes(S) + OZ_WIN - 1) * OZ_B_TILE) + 1024 + 512;
+}
 
 struct OzMaps {
-  CUtensorMap a;  // digit planes of A'': (2k, 2m, S·batch), plane-major
-  CUtensorMap b;  // digit planes of B'': (2k, n, S·batch)
+  CUtensorMap a;  // digit planes of A'': (2k, 2m, batch, S)
+  CUtensorMap b;  // digit planes of B'': (2k, n, batch, S)
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -102,11 +104,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   atomicExch(err, 1);
   return false;
 }
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z, int w) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::
           "r"(smem_u32(dst)),
-      "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+      "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
       : "memory");
 }
 // shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups 512 B apart
@@ -160,13 +162,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base_u = smem_u32(smem_raw);
   unsigned char* smem = smem_raw + ((1024 - (base_u & 1023)) & 1023);
-  unsigned char* sA = smem;                          // 2 stages × S planes
-  const int b_planes = oz_b_planes(S), SB = b_planes - (OZ_WIN - 1);
-  unsigned char* sZ = smem + 2 * S * OZ_A_TILE;      // 2 stages × (3 planes of zeros and SB of B)
+  unsigned char* sA = smem;                          // 2 stages × SP planes
+  const int SP = oz_planes(S), b_planes = SP + OZ_WIN - 1;
+  unsigned char* sZ = smem + 2 * SP * OZ_A_TILE;     // 2 stages × (3 planes of zeros and SP of B)
   unsigned char* sB = sZ + (OZ_WIN - 1) * OZ_B_TILE;
   uint64_t* full = reinterpret_cast<uint64_t*>(sZ + 2 * b_planes * OZ_B_TILE);  // [2]
-  uint64_t* empty = full + 2;                                            // [2][OZ_MAX_S]
-  uint64_t* acc_full = empty + 2 * OZ_MAX_S;
+  uint64_t* empty = full + 2;                                            // [2][2]
+  uint64_t* acc_full = empty + 4;
   uint64_t* acc_empty = acc_full + 1;
   uint32_t* tslot = reinterpret_cast<uint32_t*>(acc_empty + 1);
 
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   if (tid == 32) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&full[b], 1);
-      for (int p = 0; p < OZ_MAX_S; ++p) mbar_init(&empty[b * OZ_MAX_S + p], 1);
+      for (int p = 0; p < 2; ++p) mbar_init(&empty[b * 2 + p], 1);
     }
     mbar_init(acc_full, 1);
     mbar_init(acc_empty, 4);
@@ -212,7 +214,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 
   if (warp == 4) {
     if (lane == 0) {
-      // producer: planes p of A and SB − 1 − p of B as the stage before last gives their place back
+      // producer: four planes of A from the first and of B from the last, as the stage before last
+      // gives their place back
       long long g = 0;
       bool ok = true;
       for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
@@ -222,13 +225,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         for (int ks = 0; ks < nks && ok; ++ks, ++g) {
           const int kb = (int)(g & 1);
           const uint32_t parity = (uint32_t)((g >> 1) & 1) ^ 1;
-          for (int p = 0; p < S; ++p) {
-            if (g >= 2 && !(ok = mbar_wait(&empty[kb * OZ_MAX_S + p], parity, err))) break;
-            if (p == 0) mbar_expect_tx(&full[kb], (uint32_t)(S * (OZ_A_TILE + OZ_B_TILE)));
-            tma_load_3d(sA + (kb * S + p) * OZ_A_TILE, &maps.a, &full[kb], ks * OZ_BK, m0, p * batch + bidx);
-            // (after group p plane SB − 1 − p is done with, after the last group all of them)
-            for (int q = min(S - 1, SB - 1 - p); q >= (p == S - 1 ? 0 : SB - 1 - p); --q)
-              tma_load_3d(sB + (kb * b_planes + q) * OZ_B_TILE, &maps.b, &full[kb], ks * OZ_BK, n0, q * batch + bidx);
+          for (int p = 0; p < SP / OZ_WIN; ++p) {
+            if (g >= 2 && !(ok = mbar_wait(&empty[kb * 2 + p], parity, err))) break;
+            if (p == 0) mbar_expect_tx(&full[kb], (uint32_t)(SP * (OZ_A_TILE + OZ_B_TILE)));
+            tma_load_4d(sA + (kb * SP + p * OZ_WIN) * OZ_A_TILE, &maps.a, &full[kb], ks * OZ_BK, m0, bidx, p * OZ_WIN);
+            const int q = SP - (p + 1) * OZ_WIN;
+            tma_load_4d(sB + (kb * b_planes + q) * OZ_B_TILE, &maps.b, &full[kb], ks * OZ_BK, n0, bidx, q);
           }
         }
       }
@@ -251,14 +253,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             // of N = 256 for the levels 0 … 3 or 4 … 7, planes before the first are zeros.  (All
             // products into an accumulator have one shape: only those are executed in the order
             // of issue.)
-            const uint64_t a0 = sdesc(sA + (kb * S + p) * OZ_A_TILE), b0 = sdesc(sB + kb * b_planes * OZ_B_TILE);
-            for (int w = p < OZ_WIN ? 0 : OZ_WIN; w < SB; w += OZ_WIN) {
+            const uint64_t a0 = sdesc(sA + (kb * SP + p) * OZ_A_TILE), b0 = sdesc(sB + kb * b_planes * OZ_B_TILE);
+            for (int w = p < OZ_WIN ? 0 : OZ_WIN; w < SP; w += OZ_WIN) {
 #pragma unroll
               for (int kk = 0; kk < OZ_BK / 16; ++kk)  // K = 16 BF16 = 32 bytes
                 mma_bf16(tmem + (uint32_t)(w * OZ_BN), a0 + (uint64_t)kk * 2,
                          b0 + (uint64_t)((int64_t)(w - p) * (OZ_B_TILE >> 4) + kk * 2), (ks > 0 || p > 0 || kk > 0) ? 1u : 0u);
             }
-            mma_commit(&empty[kb * OZ_MAX_S + p]);
+            // (planes 0 … 3 of A and the last four of B are done with after group 3)
+            if (p % OZ_WIN == OZ_WIN - 1 || p == S - 1) mma_commit(&empty[kb * 2 + p / OZ_WIN]);
           }
         }
         if (ok) mma_commit(acc_full);
@@ -535,16 +538,17 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// planes of rows × K2 BF16, a row `pitch` and a plane `plane` elements after the one before
-tn_status_t make_map3(tn_ctx* ctx, CUtensorMap* map, const void* base, int64_t K2, int64_t rows, int64_t planes,
-                      int64_t pitch, int64_t plane, uint32_t box_rows) {
+// planes of rows × K2 BF16 per instance: a row `pitch` and an instance `matrix` elements after the one
+// before, the planes batch instances apart; a box is `box_rows` rows of 64 bytes of OZ_WIN planes
+tn_status_t make_map4(tn_ctx* ctx, CUtensorMap* map, const void* base, int64_t K2, int64_t rows, int64_t batch, int64_t planes,
+                      int64_t pitch, int64_t matrix, uint32_t box_rows) {
   EncodeTiledFn fn = tn_encode_tiled_fn(ctx);
   if (!fn) return TN_ECUDA;
-  cuuint64_t dims[3] = {(cuuint64_t)K2, (cuuint64_t)rows, (cuuint64_t)planes};
-  cuuint64_t strides[2] = {(cuuint64_t)(pitch * 2), (cuuint64_t)(plane * 2)};
-  cuuint32_t box[3] = {(cuuint32_t)OZ_BK, box_rows, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void*)base, dims, strides, box, estr,
+  cuuint64_t dims[4] = {(cuuint64_t)K2, (cuuint64_t)rows, (cuuint64_t)batch, (cuuint64_t)planes};
+  cuuint64_t strides[3] = {(cuuint64_t)(pitch * 2), (cuuint64_t)(matrix * 2), (cuuint64_t)(matrix * 2 * batch)};
+  cuuint32_t box[4] = {(cuuint32_t)OZ_BK, box_rows, 1, (cuuint32_t)OZ_WIN};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)base, dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return tn_set_error(ctx, TN_ECUDA, "cuTensorMapEncodeTiled (split GEMM) failed (%d)", (int)r);
@@ -605,7 +609,7 @@ tn_status_t gemm_c64_split(tn_ctx* ctx, int S, char opa, char opb, int64_t m, in
   if (k == 0) return gemm_cx<double>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
   // Aᴴ·A: B'' is the even rows of A'', so its planes need not be cut, and with a real alpha the
   // product is Hermitian: for beta = 0, or where C is known to be, the tiles above the diagonal
-  // are enough (16 × 512³: 0.87 → 0.51 ms)
+  // are enough (16 × 512³: 0.78 → 0.46 ms)
   const bool gram = opa == 'C' && opb == 'N' && A == B && lda == ldb && (sA == sB || batch == 1) && m == n;
   const bool upper = gram && alpha.y == 0.0 && ((beta.x == 0.0 && beta.y == 0.0) || (hermitian && beta.y == 0.0));
   // a level's FP32 sum is exact while S·(2k)·2^{2b-2} ≤ 2^24: the widest such digit b
@@ -665,11 +669,11 @@ tn_status_t gemm_c64_split(tn_ctx* ctx, int S, char opa, char opb, int64_t m, in
                  2.0 * S * ((double)M2 + (gram ? 0 : n)) * K2 * batch);
   OzMaps maps;
   memset(&maps, 0, sizeof(maps));
-  TN_RETURN_IF(make_map3(ctx, &maps.a, dA, K2, M2, (int64_t)S * batch, pitch, M2 * pitch, OZ_BM));
+  TN_RETURN_IF(make_map4(ctx, &maps.a, dA, K2, M2, batch, S, pitch, M2 * pitch, OZ_BM));
   if (gram)
-    TN_RETURN_IF(make_map3(ctx, &maps.b, dA, K2, n, (int64_t)S * batch, 2 * pitch, M2 * pitch, OZ_BN));
+    TN_RETURN_IF(make_map4(ctx, &maps.b, dA, K2, n, batch, S, 2 * pitch, M2 * pitch, OZ_BN));
   else
-    TN_RETURN_IF(make_map3(ctx, &maps.b, dB, K2, n, (int64_t)S * batch, pitch, n * pitch, OZ_BN));
+    TN_RETURN_IF(make_map4(ctx, &maps.b, dB, K2, n, batch, S, pitch, n * pitch, OZ_BN));
   const int64_t tiles_m = cdiv(M2, OZ_BM), tiles = upper ? tiles_m * (tiles_m + 1) / 2 : tiles_m * cdiv(n, OZ_BN);
   if (tiles > 0x7fffffffll) return tn_set_error(ctx, TN_EUNSUPPORTED, "split GEMM: too many tiles");
   const int smem = oz_smem_bytes(S);
