@@ -208,8 +208,9 @@ __global__ void __launch_bounds__(kOrthThreads)
 // One warp, lane k on row k.  A rotation is a chain of FP64 operations of 64 clocks and was two
 // divisions and two roots of 580 clocks and 12 operations for every row; here the rows are side
 // by side, the tangent comes from the hardware's approximate root and quotient (some 18 bits:
-// what the angle leaves, a later sweep removes) and c = (1 + t²)^(-1/2) from the approximation and a
-// step of third order, y ← y + y·e(1/2 + 3e/8) with e = 1 − (1 + t²)y².  41 → 24 µs for three vectors.
+// what the angle leaves, a later sweep removes) and only c = (1 + t²)^(-1/2) is a root to full
+// precision.  41 → 24 µs for three vectors with c approximated too, which a sweep does not show (L = 24,
+// χ = 32: 60.6 ms with CUDA's root).
 __device__ void sym_eig(int n, double (*A)[kLzMax + 1], double (*Z)[kLzMax + 1], int lane) {
   if (lane < n)
     for (int j = 0; j < n; ++j) Z[lane][j] = lane == j ? 1.0 : 0.0;
@@ -230,15 +231,12 @@ __device__ void sym_eig(int n, double (*A)[kLzMax + 1], double (*Z)[kLzMax + 1],
         const double d = A[q][q] - A[p][p], h = fma(d, d, 4.0 * apq * apq);
         double t, c;
         if (h > 1e-280 && h < 1e280) {
-          double r, y;
+          double r;
           asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(h));
           const double den = fma(h, r, fabs(d));
           asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(den));
           t = (d >= 0.0 ? 2.0 : -2.0) * apq * r;
-          const double w = fma(t, t, 1.0);
-          asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(w));
-          const double e = fma(-w * y, y, 1.0);
-          c = fma(y * e, fma(0.375, e, 0.5), y);
+          c = rsqrt(fma(t, t, 1.0));
         } else {
           const double tau = d / (2.0 * apq);
           t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));

@@ -34,6 +34,7 @@
 
 #include "tn_fixed_sum.cuh"
 #include "tn_internal.cuh"
+#include "tn_newton.cuh"
 
 namespace {
 
@@ -130,14 +131,6 @@ __device__ __forceinline__ double widen(float f) {
 // f · 2^s for a normal f whose result is normal
 __device__ __forceinline__ float shifted(float f, int s) { return __int_as_float(__float_as_int(f) + (s << 23)); }
 
-// 1/x of a positive normal x: the hardware's approximation (20 bits or so) and one step of third
-// order, y ← y + y·e(1 + e) with e = 1 − x·y
-__device__ __forceinline__ double reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
 __device__ __forceinline__ float rsqrt_approx(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -461,7 +454,7 @@ __global__ void __launch_bounds__(kNT, 4)
   ulonglong2* dst = nullptr;
   auto send_scales = [&](unsigned f) -> double {
     double D = half ? Dy : Dx;
-    if (turned) D *= reciprocal(fma(p.ax, p.bx, fma(p.ay, p.by, 1.0)));
+    if (turned) D *= newton_reciprocal(fma(p.ax, p.bx, fma(p.ay, p.by, 1.0)));
     if (dst) put(dst, D, f);
     pending = false;
     return D;
@@ -617,7 +610,7 @@ __global__ void __launch_bounds__(kNT, 4)
       root_of(Dy, sy, ex_y);
       // (a ratio of scales beyond 2^±60 waits for the next sweep's columns of scale 1)
       const float ratio = abs(ex_y - ex_x) > 60 ? 0.f : __fdividef(sy, sx) * pow2(ex_y - ex_x);
-      const double q = Dx * reciprocal(Dy);
+      const double q = Dx * newton_reciprocal(Dy);
       long long total;
       int E;
       if (SPLIT) {

@@ -29,6 +29,7 @@
 
 #include "tn_fixed_sum.cuh"
 #include "tn_internal.cuh"
+#include "tn_newton.cuh"
 
 namespace {
 
@@ -66,32 +67,10 @@ __device__ __forceinline__ double value_of(ulonglong2 v) {
   return __longlong_as_double((long long)((v.x & 0xffffffffull) | (v.y << 32)));
 }
 
-// ‖x‖ = √n2, 1/‖x‖ and, by reciprocal(), 1/|u₁|²: the hardware's approximations (some 20 bits)
-// and one step of third order, y ← y + y·e(1/2 + 3e/8) with e = 1 − n2·y² and
-// y ← y + y·e(1 + e) with e = 1 − x·y, which leaves an error of order e³.  They are in the chain
-// of every step; CUDA's rsqrt and divide, of up to 600 clocks each, take the arguments outside
-// the range where the approximations are normal numbers.
-constexpr double kNormLo = 1e-280, kNormHi = 1e280;
-__device__ __forceinline__ void norm_of(double n2, double* nrm, double* inv) {
-  if (n2 > kNormLo && n2 < kNormHi) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(n2));
-    const double t = n2 * y, e = fma(-t, y, 1.0), p = fma(0.375, e, 0.5);
-    *nrm = fma(t * e, p, t);
-    *inv = fma(y * e, p, y);
-  } else {
-    const double rs = rsqrt(n2), r = n2 * rs;
-    *nrm = fma(fma(-r, r, n2), 0.5 * rs, r);
-    *inv = rs;
-  }
-}
-__device__ __forceinline__ double reciprocal(double x) {
-  if (!(x > kNormLo && x < kNormHi)) return 1.0 / x;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
+// ‖x‖² between these: ‖x‖ and 1/(‖x‖·|u₁|²), |u₁| ≤ 2‖x‖, by Newton's iteration.  They are in the chain of
+// every step; CUDA's rsqrt and divide, of up to 600 clocks each, take what lies outside.
+// One reciprocal in place of 1/‖x‖ and 1/|u₁|²: 31 QRs of bond 64 5.07 → 4.97 ms.
+constexpr double kNormLo = 1e-180, kNormHi = 1e180;
 
 // a batch of equal matrices: the first one and the strides to the next; or a list of matrices
 // of falling n, whose columns are taken in the order 0 of all, 1 of all, …
@@ -303,15 +282,29 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     if (!(s2 == 0.0 && ay == 0.0)) {
       // β = −sgn(Re α)·‖x‖, u₁ = α − β, conj(κ) = −1/(β·u₁) = −(conj(u₁)/|u₁|²)/β
       const double n2 = fma(ax, ax, fma(ay, ay, s2));
-      double nrm, rs;
-      norm_of(n2, &nrm, &rs);
+      const bool newton = n2 > kNormLo && n2 < kNormHi;
+      double nrm, rs = 0.0;
+      if (newton) {
+        nrm = newton_root(n2);
+      } else {
+        rs = rsqrt(n2);
+        nrm = n2 * rs;
+        nrm = fma(fma(-nrm, nrm, n2), 0.5 * rs, nrm);
+      }
       beta = ax >= 0.0 ? -nrm : nrm;
       ux = ax - beta;
       uy = ay;
       if (tid < 2) put(b + 2 * m + tid, tid == 0 ? ux : uy);  // κ follows
-      const double inv2 = reciprocal(fma(ux, ux, uy * uy)), invb = ax >= 0.0 ? rs : -rs;
-      kx = (ux * inv2) * invb;
-      ky = (-uy * inv2) * invb;
+      const double uu = fma(ux, ux, uy * uy);
+      if (newton) {
+        const double q = newton_reciprocal(nrm * uu);
+        kx = (ax >= 0.0 ? ux : -ux) * q;
+        ky = (ax >= 0.0 ? -uy : uy) * q;
+      } else {
+        const double inv2 = 1.0 / uu, invb = ax >= 0.0 ? rs : -rs;
+        kx = (ux * inv2) * invb;
+        ky = (-uy * inv2) * invb;
+      }
     } else if (tid < 2) {
       put(b + 2 * m + tid, 0.0);
     }

@@ -95,3 +95,22 @@ def test_columns_qr_non_finite(ctx, bad, m, n):
     Q, R = _qr(ctx, A)
     assert np.abs(R[0][:, :7] - np.linalg.qr(clean[0])[1][:, :7]).max() <= 1e-9
     assert not np.isfinite(R[0][:8, 7]).all() and not np.isfinite(Q[0][:, 8:]).any()
+
+
+def test_columns_qr_norms_and_reflectors_to_rounding(ctx):
+    """Single columns of three entries from 1e-130 to 1e130, on both sides of where Newton's iteration
+    forms the norm and the reflector's scale: R = ∓‖a‖ and Q = a/R.
+
+    With u = 1.1e-16: ‖a‖² is off by 3u, its root by 3u/2 and its own rounding, so R by 4u relative.
+    An entry of Q is κ·u·conj(u₁), at most 2 in modulus, from a handful of such roundings: 16u.
+    """
+    rng = np.random.default_rng(7)
+    n = 500
+    g = rng.standard_normal((n, 3, 1)) + 1j * rng.standard_normal((n, 3, 1))
+    A = g * 10.0 ** np.concatenate([rng.uniform(-130, 130, n - 100), rng.uniform(-91, -89, 50), rng.uniform(89, 91, 50)])[:, None, None]
+    Q, R = _qr(ctx, A)
+    wide = A[:, :, 0].astype(np.clongdouble)
+    r = -np.sign(wide[:, 0].real) * np.sqrt((wide.real**2 + wide.imag**2).sum(axis=1))
+    u = 2.0**-53
+    assert np.abs(R[:, 0, 0] / r - 1).max() <= 4 * u
+    assert np.abs(Q[:, :, 0] - wide / r[:, None]).max() <= 16 * u
