@@ -385,7 +385,7 @@ size_t qr_cols_workspace(int64_t m, int64_t n, int64_t batch);
 tn_status_t qr_cols_takes(tn_ctx* ctx, int64_t m, int64_t columns, bool* out);
 tn_status_t qr_cols_batch(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda, int64_t sA, cxd* Q, int64_t sQ,
                           cxd* R, int64_t sR, int64_t batch, const int* perm = nullptr, bool adj_in = false,
-                          bool adj_r = false, bool adj_q = false);
+                          bool adj_r = false, bool adj_q = false, const int* expo = nullptr);
 // the same for matrices of different sizes, m ≥ n, m ≤ kQrColsMaxRows: QR of A (m × n, lda), or
 // (adjoint) of Aᴴ with A n × m and Qᴴ stored (ld n).  Q may be A if lda is Q's.
 constexpr int64_t kQrColsMaxRows = 512;

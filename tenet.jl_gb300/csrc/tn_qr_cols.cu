@@ -24,6 +24,9 @@
 // Reflectors and signs are LAPACK's (H = I − τ v vᴴ, v₁ = 1, τ v vᴴ = κ u uᴴ, R_jj real with
 // the sign opposite to Re x₁).  Every wait is bounded: a CTA whose wait ran out records an
 // error and leaves.
+// A column whose ‖x‖² leaves the range in which squares and their inverses are normal numbers is
+// taken in units of its largest entry: u₁ and κ are sent in those units, with the exponent as u₁'s
+// flag, and the receivers bring the entries, sent already, to them (kUnits).
 #include <algorithm>
 #include <vector>
 
@@ -45,6 +48,7 @@ struct QMat {
   cxd *Q, *R;       // Q m × k (ld m), R k × n (ld k)
   ulonglong2* box;  // k reflectors × (2m + 4) packets
   const int* perm;  // column c of the factored matrix is column perm[c] of op(A); null: c
+  const int* expo;  // A is read in units of 2^expo (one of each matrix); null: as it is
   int64_t lda;
   int m, n, k;        // m × n: the factored matrix
   int rows;           // CTAs that form rows of Q (m or 0)
@@ -52,8 +56,8 @@ struct QMat {
                       // bit 2: Qᴴ (k × m, ld k) is stored for Q
 };
 
-__device__ __forceinline__ void put(ulonglong2* p, double v) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v), f = 1ull << 32;
+__device__ __forceinline__ void put(ulonglong2* p, double v, unsigned flag = 1) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v), f = (unsigned long long)flag << 32;
   asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"((b & 0xffffffffull) | f), "l"((b >> 32) | f)
                : "memory");
 }
@@ -67,10 +71,86 @@ __device__ __forceinline__ double value_of(ulonglong2 v) {
   return __longlong_as_double((long long)((v.x & 0xffffffffull) | (v.y << 32)));
 }
 
-// ‖x‖² between these: ‖x‖ and 1/(‖x‖·|u₁|²), |u₁| ≤ 2‖x‖, by Newton's iteration.  They are in the chain of
-// every step; CUDA's rsqrt and divide, of up to 600 clocks each, take what lies outside.
-// One reciprocal in place of 1/‖x‖ and 1/|u₁|²: 31 QRs of bond 64 5.07 → 4.97 ms.
-constexpr double kNormLo = 1e-180, kNormHi = 1e180;
+// ‖x‖² between these: ‖x‖ and 1/(‖x‖·|u₁|²), |u₁| ≤ 2‖x‖, by Newton's iteration, as they are in the chain of
+// every step (CUDA's rsqrt and divide take up to 600 clocks each).  One reciprocal in place of 1/‖x‖
+// and 1/|u₁|²: 31 QRs of bond 64 5.07 → 4.97 ms.  What lies outside is brought into the range by a
+// power of two first: u₁'s flag is then kUnits + e with the entries in units of 2^e, 1 otherwise.
+// (compared as exponent fields: 2^±600, integers beside FP64 comparisons of 64 clocks)
+constexpr int kNormLo = 1023 - 600, kNormHi = 1023 + 600;
+constexpr int kUnits = 4096;
+// v · 2^k, |k| ≤ 1074, by two factors that are normal numbers
+__device__ __forceinline__ double times_pow2(double v, int k) {
+  const int h = k >> 1;
+  return v * __hiloint2double((1023 + h) << 20, 0) * __hiloint2double((1023 + k - h) << 20, 0);
+}
+__device__ __forceinline__ cxd times_pow2(cxd v, int k) { return mkcx(times_pow2(v.x, k), times_pow2(v.y, k)); }
+__device__ __forceinline__ bool is_zero(double v) { return (((unsigned)__double2hiint(v) << 1) | (unsigned)__double2loint(v)) == 0; }
+
+__device__ __forceinline__ double block_sum(double v, long long* part, int* exps) {  // one barrier
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned e = __reduce_max_sync(0xffffffffu, exponent_field(v));
+  const long long s = fixed_warp_sum(v, e);
+  if (lane == 0) {
+    part[warp] = s;
+    exps[warp] = (int)e;
+  }
+  __syncthreads();
+  int E;
+  const long long total = fixed_sum4(part, exps, E);
+  return fixed_value(total, E);
+}
+
+// β = −sgn(Re α)·‖x‖, u₁ = α − β, conj(κ) = −1/(β·u₁) = −(conj(u₁)/|u₁|²)/β from α = (ax, ay), s2 = ‖x‖² − |α|²
+// and n2 = ‖x‖²: the scalar packets p, unless ‖x‖² is out of range.  Returns β
+__device__ __forceinline__ double send_scalars(ulonglong2* p, double ax, double ay, double s2, double n2, unsigned flag, bool out) {
+  const int tid = threadIdx.x;
+  const bool none = is_zero(s2) && is_zero(ay);  // H = I
+  // (signs are turned and zeros found as bits: an FP64 operation is 64 clocks of the chain; 31 QRs of
+  // bond 64 5.08 → 4.72 ms)
+  const int flip = __double2hiint(ax) < 0 && !is_zero(ax) ? 0 : (int)0x80000000;
+  const double nrm = newton_root(n2), refl = __hiloint2double(__double2hiint(nrm) ^ flip, __double2loint(nrm));
+  const double d = ax - refl, ux = none ? 0.0 : d, uy = ay;
+  if (tid < 2 && !out) put(p + tid, tid == 0 ? ux : uy, flag);  // κ follows
+  const double r = newton_reciprocal(nrm * fma(d, d, uy * uy));
+  const double q = none ? 0.0 : __hiloint2double(__double2hiint(r) ^ (~flip & (int)0x80000000), __double2loint(r));
+  if (tid < 2 && !out) put(p + 2 + tid, (tid == 0 ? ux : -uy) * q);
+  return none ? ax : refl;
+}
+
+// the same for a column x (rows tid + q·kNT) whose ‖x‖² is out of range, in units of its largest
+// entry.  A function of its own, called behind the chain's code: in its place before the root it made 31
+// QRs of bond 64 take 5.23 ms, here 5.08
+__device__ __noinline__ double send_in_units(const cxd* x, int R, int col, int m, double ax, double ay, ulonglong2* p,
+                                             long long* part, int* exps, int* tops) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the largest entry's high word; 1 where only low words are left
+  unsigned top = 0;
+  for (int q = 0; q < R; ++q) {
+    const int t = tid + q * kNT;
+    if (t < col || t >= m) continue;
+    const unsigned hx = (unsigned)__double2hiint(x[q].x) & 0x7fffffffu, hy = (unsigned)__double2hiint(x[q].y) & 0x7fffffffu;
+    top = max(top, max(max(hx, hy), (__double2loint(x[q].x) | __double2loint(x[q].y)) != 0 ? 1u : 0u));
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  __syncthreads();
+  if (lane == 0) tops[warp] = (int)top;
+  __syncthreads();
+  top = (unsigned)max(max(tops[0], tops[1]), max(tops[2], tops[3]));
+  // (zeros, and what is not finite, stay as they are)
+  const int e = top == 0 || top >= 0x7ff00000u ? 0 : top < 0x100000u ? -1060 : (int)(top >> 20) - 1023;
+  double s2 = 0;
+  for (int q = 0; q < R; ++q) {
+    const int t = tid + q * kNT;
+    if (t <= col || t >= m) continue;
+    const cxd v = times_pow2(x[q], -e);
+    s2 = fma(v.x, v.x, fma(v.y, v.y, s2));
+  }
+  s2 = block_sum(s2, part, exps);
+  __syncthreads();
+  ax = times_pow2(ax, -e);
+  ay = times_pow2(ay, -e);
+  return times_pow2(send_scalars(p, ax, ay, s2, fma(ax, ax, fma(ay, ay, s2)), (unsigned)(kUnits + e), false), e);
+}
 
 // a batch of equal matrices: the first one and the strides to the next; or a list of matrices
 // of falling n, whose columns are taken in the order 0 of all, 1 of all, …
@@ -108,6 +188,7 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     M.R += b * batch.sR;
     M.box += b * batch.sBox;
     if (M.perm) M.perm += b * M.n;
+    if (M.expo) M.expo += b;
   }
   const int m = M.m, k = M.k;
   const bool row = index >= M.n;         // a CTA that forms a row of Q
@@ -117,8 +198,10 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
   __shared__ __align__(16) long long fix[2][2][4];  // parity, Re or Im, warp: partial sums in fixed point
   __shared__ __align__(16) int fix_e[2][4];
   __shared__ double s_row[2][2];  // this column's entry in the pivot row
-  __shared__ int s_fail;
-  if (tid == 0) s_fail = 0;
+  // whether a wait ran out, and the flag of a reflector that came in units (0: none did); looked at
+  // together behind the one barrier of a step, of either parity
+  __shared__ __align__(8) int2 s_state[2];
+  if (tid < 2) s_state[tid] = make_int2(0, 0);
   cxd x[R];
   const int64_t src = row ? 0 : (M.perm ? M.perm[col] : col);
 #pragma unroll
@@ -126,6 +209,11 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     const int64_t t = tid + q * kNT;
     x[q] = mkcx(row && t == index - M.n ? 1.0 : 0.0, 0.0);
     if (!row && t < m) x[q] = (M.adj & 1) ? conjg(M.A[src + t * M.lda]) : M.A[src * M.lda + t];
+  }
+  if (!row && M.expo && *M.expo != 0) {
+    const int e = -*M.expo;
+#pragma unroll
+    for (int q = 0; q < R; ++q) x[q] = times_pow2(x[q], e);
   }
   int buf = 0;
   // whether a warp's 32 rows of group q meet the reflector's, j … m − 1: what lies outside is zeros, and
@@ -165,40 +253,51 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
       }
       if (!ok && adj && col > j + 8) __nanosleep(kFarSleep);
     } while (!ok && ++spins < kSpinLimit);
-    double wx = 0, wy = 0;
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      if (!warp_row(q, j)) continue;
-      wx = fma(u[q].x, x[q].x, fma(u[q].y, x[q].y, wx));
-      wy = fma(u[q].x, x[q].y, fma(-u[q].y, x[q].x, wy));
-      if (tid + q * kNT == j) {
-        s_row[buf][0] = x[q].x;
-        s_row[buf][1] = x[q].y;
-      }
-    }
-    {
-      const unsigned e = __reduce_max_sync(0xffffffffu, max(exponent_field(wx), exponent_field(wy)));
-      const long long s0 = fixed_warp_sum(wx, e), s1 = fixed_warp_sum(wy, e);
-      if (lane == 0) {
-        fix[buf][0][warp] = s0;
-        fix[buf][1][warp] = s1;
-        fix_e[buf][warp] = (int)e;
-      }
-    }
     const bool far = adj && col > j + 8;
-    while (!(arrived(p0) && arrived(p1)) && ++spins < kSpinLimit) {
-      if (far) __nanosleep(kFarSleep);
-      p0 = get_raw(b + 2 * m);
-      p1 = get_raw(b + 2 * m + 1);
-      p2 = get_raw(b + 2 * m + 2);
-      p3 = get_raw(b + 2 * m + 3);
+    // (a second time round for a reflector in units)
+    for (bool again = false;; again = true) {
+      double wx = 0, wy = 0;
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        if (!warp_row(q, j)) continue;
+        wx = fma(u[q].x, x[q].x, fma(u[q].y, x[q].y, wx));
+        wy = fma(u[q].x, x[q].y, fma(-u[q].y, x[q].x, wy));
+        if (tid + q * kNT == j) {
+          s_row[buf][0] = x[q].x;
+          s_row[buf][1] = x[q].y;
+        }
+      }
+      {
+        const unsigned e = __reduce_max_sync(0xffffffffu, max(exponent_field(wx), exponent_field(wy)));
+        const long long s0 = fixed_warp_sum(wx, e), s1 = fixed_warp_sum(wy, e);
+        if (lane == 0) {
+          fix[buf][0][warp] = s0;
+          fix[buf][1][warp] = s1;
+          fix_e[buf][warp] = (int)e;
+        }
+      }
+      while (!(arrived(p0) && arrived(p1)) && ++spins < kSpinLimit) {
+        if (far) __nanosleep(kFarSleep);
+        p0 = get_raw(b + 2 * m);
+        p1 = get_raw(b + 2 * m + 1);
+        p2 = get_raw(b + 2 * m + 2);
+        p3 = get_raw(b + 2 * m + 3);
+      }
+      if (spins >= kSpinLimit) {
+        atomicExch(err, 1);
+        s_state[0].x = s_state[1].x = 1;
+      }
+      if ((unsigned)(p0.x >> 32) > 1 && !again) s_state[buf].y = (int)(unsigned)(p0.x >> 32);
+      __syncthreads();
+      const int2 state = s_state[buf];
+      if ((state.x | state.y) == 0) break;
+      if (state.x) return false;
+      // u₁ and κ are in units of 2^e: the other entries, and their products, in the same
+#pragma unroll
+      for (int q = 0; q < R; ++q) u[q] = times_pow2(u[q], kUnits - state.y);
+      __syncthreads();
+      if (tid == 0) s_state[buf].y = 0;
     }
-    if (spins >= kSpinLimit) {
-      atomicExch(err, 1);
-      s_fail = 1;
-    }
-    __syncthreads();
-    if (s_fail) return false;
     int E;
     const long long total = fixed_sum4(fix[buf][half], fix_e[buf], E);
     const double d = fixed_value(total, E);
@@ -212,7 +311,7 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
     }
     if (spins >= kSpinLimit) {  // (seen after the next reflector's barrier)
       atomicExch(err, 1);
-      s_fail = 1;
+      s_state[0].x = s_state[1].x = 1;
     }
     const double kx = value_of(p2), ky = adj ? value_of(p3) : -value_of(p3);
     const double wo = __shfl_xor_sync(0xffffffffu, w, 16);
@@ -262,53 +361,19 @@ __global__ void __launch_bounds__(kNT, 4) k_qr_cols(QBatch batch, int* err) {
         s_row[buf][1] = x[q].y;
       }
     }
-    {
-      const unsigned e = __reduce_max_sync(0xffffffffu, exponent_field(s2));
-      const long long s0 = fixed_warp_sum(s2, e);
-      if (lane == 0) {
-        fix[buf][0][warp] = s0;
-        fix_e[buf][warp] = (int)e;
-      }
-    }
-    __syncthreads();
-    {
-      int E;
-      const long long total = fixed_sum4(fix[buf][0], fix_e[buf], E);
-      s2 = fixed_value(total, E);
-    }
+    s2 = block_sum(s2, fix[buf][0], fix_e[buf]);
     const double ax = s_row[buf][0], ay = s_row[buf][1];
     buf ^= 1;
-    double beta = ax, ux = 0, uy = 0, kx = 0, ky = 0;
-    if (!(s2 == 0.0 && ay == 0.0)) {
-      // β = −sgn(Re α)·‖x‖, u₁ = α − β, conj(κ) = −1/(β·u₁) = −(conj(u₁)/|u₁|²)/β
-      const double n2 = fma(ax, ax, fma(ay, ay, s2));
-      const bool newton = n2 > kNormLo && n2 < kNormHi;
-      double nrm, rs = 0.0;
-      if (newton) {
-        nrm = newton_root(n2);
-      } else {
-        rs = rsqrt(n2);
-        nrm = n2 * rs;
-        nrm = fma(fma(-nrm, nrm, n2), 0.5 * rs, nrm);
-      }
-      beta = ax >= 0.0 ? -nrm : nrm;
-      ux = ax - beta;
-      uy = ay;
-      if (tid < 2) put(b + 2 * m + tid, tid == 0 ? ux : uy);  // κ follows
-      const double uu = fma(ux, ux, uy * uy);
-      if (newton) {
-        const double q = newton_reciprocal(nrm * uu);
-        kx = (ax >= 0.0 ? ux : -ux) * q;
-        ky = (ax >= 0.0 ? -uy : uy) * q;
-      } else {
-        const double inv2 = 1.0 / uu, invb = ax >= 0.0 ? rs : -rs;
-        kx = (ux * inv2) * invb;
-        ky = (-uy * inv2) * invb;
-      }
-    } else if (tid < 2) {
-      put(b + 2 * m + tid, 0.0);
+    const double n2 = fma(ax, ax, fma(ay, ay, s2));
+    const int n2_field = __double2hiint(n2) >> 20;
+    const bool out = n2_field < kNormLo || n2_field > kNormHi;
+    double beta = send_scalars(b + 2 * m, ax, ay, s2, n2, 1, out);
+    if (out) {
+      cxd y[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) y[q] = x[q];
+      beta = send_in_units(y, R, col, m, ax, ay, b + 2 * m, fix[buf][0], fix_e[buf], fix_e[buf ^ 1]);
     }
-    if (tid < 2) put(b + 2 * m + 2 + tid, tid == 0 ? kx : ky);
 #pragma unroll
     for (int q = 0; q < R; ++q)
       if (tid + q * kNT == col) x[q] = mkcx(beta, 0.0);
@@ -368,15 +433,17 @@ tn_status_t qr_cols_takes(tn_ctx* ctx, int64_t m, int64_t columns, bool* out) {
 }
 
 // thin QR of a batch of m × n matrices op(A)·Π (the caller asked qr_cols_takes with n·batch).
-// Q null: not formed.  perm (n per matrix): the column order Π, null for none.
+// Q null: not formed.  perm (n per matrix): the column order Π, null for none.  expo (one per
+// matrix): A is read, and R is left, in units of 2^expo.
 tn_status_t qr_cols_batch(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda, int64_t sA, cxd* Q, int64_t sQ,
-                          cxd* R, int64_t sR, int64_t batch, const int* perm, bool adj_in, bool adj_r, bool adj_q) {
+                          cxd* R, int64_t sR, int64_t batch, const int* perm, bool adj_in, bool adj_r, bool adj_q,
+                          const int* expo) {
   const int64_t k = std::min(m, n);
   const size_t one = boxes_bytes(m, k);
   char* box = ws_take<char>(ctx, one * (size_t)batch);
   TN_CHECK_CUDA(ctx, cudaMemsetAsync(box, 0, one * (size_t)batch, ctx->stream));
   const int64_t rows = Q && (n + m) * batch <= 2 * (int64_t)ctx->num_sms ? m : 0;
-  QBatch b = {QMat{A, Q, R, reinterpret_cast<ulonglong2*>(box), perm, lda, (int)m, (int)n, (int)k, (int)rows,
+  QBatch b = {QMat{A, Q, R, reinterpret_cast<ulonglong2*>(box), perm, expo, lda, (int)m, (int)n, (int)k, (int)rows,
                    (adj_in ? 1 : 0) + (adj_r ? 2 : 0) + (adj_q ? 4 : 0)},
               sA, sQ, sR, (int64_t)(one / sizeof(ulonglong2)), nullptr, nullptr, 0, nullptr};
   int* err = nullptr;
@@ -420,7 +487,7 @@ tn_status_t qr_cols_list(tn_ctx* ctx, std::vector<QrColsMat> mats) {
   size_t at = 256;
   for (auto& q : mats) {
     const int k = std::min(q.m, q.n);
-    list.push_back(QMat{q.A, q.Q, q.R, reinterpret_cast<ulonglong2*>(box + at), nullptr, q.lda, q.m, q.n, k, 0,
+    list.push_back(QMat{q.A, q.Q, q.R, reinterpret_cast<ulonglong2*>(box + at), nullptr, nullptr, q.lda, q.m, q.n, k, 0,
                         q.adjoint ? 5 : 0});
     at += boxes_bytes(q.m, k);
   }
