@@ -145,8 +145,10 @@ extern "C" tn_status_t tn_contract(tn_ctx* ctx, tn_dtype_t dtype, tn_precision_t
   const bool perm_c = !is_identity(pc);
   // ComplexF32 products with tall outputs read their operands in place where the modes fuse into
   // two runs each (a boundary tensor absorbing the next site of a lattice), without a permuted
-  // copy
-  if (dtype == TN_C32 && h == 1 && !perm_c) {
+  // copy.  An output over an operand needs the copies
+  const bool over_operand = ranges_meet(c->data, es * (size_t)(m * n * h), a->data, es * (size_t)(m * k * h)) ||
+                            ranges_meet(c->data, es * (size_t)(m * n * h), b->data, es * (size_t)(k * n * h));
+  if (dtype == TN_C32 && h == 1 && !perm_c && !over_operand) {
     GemmView va, vb;
     va.conj = vb.conj = false;
     const bool views =

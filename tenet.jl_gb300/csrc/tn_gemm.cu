@@ -452,7 +452,16 @@ tn_status_t gemm_any(tn_ctx* ctx, tn_dtype_t dtype, tn_precision_t prec, char op
     const size_t es = dtype == TN_C32 ? 8 : 4;
     const size_t top = ctx->ws_top;
     const GemmView va = matrix_view(opa, lda), vb = matrix_view(opb, ldb);
-    if (dtype == TN_C32 && tc_gemm_tall_fits(ctx, m, n, k, va)) {
+    // (read in place: C over an operand of its product is left to the general path, which copies)
+    const size_t na = es * (size_t)(opa == 'N' ? (k - 1) * lda + m : (m - 1) * lda + k),
+                 nb = es * (size_t)(opb == 'N' ? (n - 1) * ldb + k : (k - 1) * ldb + n), nc = es * (size_t)((n - 1) * ldc + m);
+    bool apart = true;
+    for (int64_t b = 0; b < batch && apart; ++b) {
+      const char *a = (const char*)A + es * (size_t)(b * strideA), *x = (const char*)B + es * (size_t)(b * strideB),
+                 *c = (const char*)C + es * (size_t)(b * strideC);
+      apart = !ranges_meet(c, nc, a, na) && !ranges_meet(c, nc, x, nb);
+    }
+    if (dtype == TN_C32 && apart && tc_gemm_tall_fits(ctx, m, n, k, va)) {
       for (int64_t b = 0; b < batch; ++b)
         TN_RETURN_IF(tc_gemm_tall(ctx, passes, m, n, k, (float)alpha[0], (const cxf*)A + b * strideA, va,
                                   (const cxf*)B + b * strideB, vb, (float)beta[0], (cxf*)C + b * strideC, ldc));

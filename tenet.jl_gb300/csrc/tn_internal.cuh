@@ -315,6 +315,12 @@ inline size_t dtype_size(tn_dtype_t t) {
 }
 inline bool dtype_complex(tn_dtype_t t) { return t == TN_C32 || t == TN_C64; }
 
+// whether [a, a + na) and [b, b + nb) share bytes
+inline bool ranges_meet(const void* a, size_t na, const void* b, size_t nb) {
+  const char *x = (const char*)a, *y = (const char*)b;
+  return x < y + nb && y < x + na;
+}
+
 inline unsigned cdiv(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b); }
 
 // ---------------------------------------------------------------------------------

@@ -318,12 +318,6 @@ tn_status_t qr_run(tn_ctx* ctx, int nb, int slab, int64_t m, int64_t n, const cx
 
 }  // namespace
 
-// Whether [a, a + na) and [b, b + nb) share bytes
-static bool ranges_meet(const void* a, size_t na, const void* b, size_t nb) {
-  const char *x = (const char*)a, *y = (const char*)b;
-  return x < y + nb && y < x + na;
-}
-
 // Which kernel: one CTA per column (tn_qr_cols.cu) while all columns of all matrices are
 // resident at once, the blocked panels below beyond that (rows > 512, or batches that fill
 // the FP64 pipe with panels of different matrices) and for shapes whose launch configuration
