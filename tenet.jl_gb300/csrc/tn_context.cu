@@ -122,7 +122,12 @@ tn_status_t wait_error_check(tn_ctx* ctx) {
   volatile int* w = reinterpret_cast<int*>(static_cast<char*>(ctx->pinned) + kPinnedBytes) - 1;
   if (*w == 0) return TN_OK;
   *w = 0;
-  return tn_set_error(ctx, TN_ETIMEOUT, "a wait between the blocks of a factorisation exceeded its limit");
+  return tn_set_error(ctx, TN_ETIMEOUT, "a bounded wait inside a kernel (QR, SVD or tensor-pipe product) exceeded its limit");
+}
+
+tn_status_t read_back_sync(tn_ctx* ctx) {
+  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  return wait_error_check(ctx);
 }
 
 tn_status_t ws_reserve(tn_ctx* ctx, size_t bytes) {
@@ -246,8 +251,7 @@ void* tn_get_stream(tn_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 
 tn_status_t tn_sync(tn_ctx* ctx) {
   if (!ctx) return TN_EINVAL;
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return wait_error_check(ctx);
+  return read_back_sync(ctx);
 }
 
 tn_status_t tn_alloc(tn_ctx* ctx, size_t bytes, void** dptr) {
@@ -273,8 +277,7 @@ tn_status_t tn_memcpy_d2h(tn_ctx* ctx, void* dst, const void* src, size_t bytes)
   if (!ctx) return TN_EINVAL;
   TN_ARG(ctx, dst && src, "tn_memcpy_d2h: null pointer");
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return wait_error_check(ctx);
+  return read_back_sync(ctx);
 }
 
 tn_status_t tn_memcpy_d2d(tn_ctx* ctx, void* dst, const void* src, size_t bytes) {

@@ -714,7 +714,7 @@ tn_status_t form_pair(Dmrg& D, int j) {
 tn_status_t read_energies(Dmrg& D, double* h) {
   std::vector<LzState> hs(D.B);
   TN_CHECK_CUDA(D.ctx, cudaMemcpyAsync(hs.data(), D.st, sizeof(LzState) * D.B, cudaMemcpyDeviceToHost, D.ctx->stream));
-  TN_CHECK_CUDA(D.ctx, cudaStreamSynchronize(D.ctx->stream));
+  TN_RETURN_IF(read_back_sync(D.ctx));
   for (int b = 0; b < D.B; ++b) h[b] = hs[b].theta;
   return TN_OK;
 }
@@ -880,8 +880,7 @@ tn_status_t run(Dmrg& D, const void* const* h_mpo, int mpo_count, int nsweeps, d
     else
       TN_RETURN_IF(read_energies(D, h_energy));
   }
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return TN_OK;
+  return read_back_sync(ctx);
 }
 
 }  // namespace

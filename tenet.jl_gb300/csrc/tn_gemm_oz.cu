@@ -708,7 +708,7 @@ tn_status_t split_gemm_check(tn_ctx* ctx) {
   if (!ctx->oz_err) return TN_OK;
   int* hp = reinterpret_cast<int*>(ctx->pinned);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(hp, ctx->oz_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(read_back_sync(ctx));
   if (hp[0]) {
     TN_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->oz_err, 0, sizeof(int), ctx->stream));
     return tn_set_error(ctx, TN_ETIMEOUT, "split GEMM: a pipeline wait timed out");

@@ -920,8 +920,7 @@ tn_status_t tn_group_get_site(const tn_group* g, int32_t b, int32_t i, void* h_d
   if (!g || !h_data || b < 0 || b >= g->B || i < 1 || i > g->L[b]) return tn_set_error(g ? g->ctx : nullptr, TN_EINVAL, "tn_group_get_site: bad arguments");
   const int64_t e = g->bond[b][i - 1] * g->d * g->bond[b][i];
   TN_CHECK_CUDA(g->ctx, cudaMemcpyAsync(h_data, g->site[b][i], sizeof(cxd) * e, cudaMemcpyDeviceToHost, g->ctx->stream));
-  TN_CHECK_CUDA(g->ctx, cudaStreamSynchronize(g->ctx->stream));
-  return TN_OK;
+  return read_back_sync(g->ctx);
 }
 
 tn_status_t tn_group_bond_dims(const tn_group* g, int32_t b, int64_t* h_bonds) {
@@ -1100,7 +1099,7 @@ tn_status_t tn_group_canonize_compress_norm(tn_group* g, const int64_t* maxdim, 
         TN_CHECK_CUDA(ctx, cudaMemcpyAsync(g->lambda[b].data(), jd[t].S, sizeof(double) * jd[t].r, cudaMemcpyDeviceToHost,
                                            ctx->stream));
       }
-      TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+      TN_RETURN_IF(read_back_sync(ctx));
       for (int t : last) {
         const int b = ids[t];
         double s2 = 0;
@@ -1110,7 +1109,7 @@ tn_status_t tn_group_canonize_compress_norm(tn_group* g, const int64_t* maxdim, 
     }
     g->steps_launched++;
   }
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  TN_RETURN_IF(read_back_sync(ctx));
   g->compressed = true;
   if (h_norms) memcpy(h_norms, norms.data(), sizeof(double) * B);
   return TN_OK;

@@ -226,9 +226,12 @@ struct tn_ctx {
 };
 // a word of page-locked host memory that kernels of this context set when a bounded wait ran
 // out (kernels whose callers do not synchronise); wait_error_check reports and clears it.
-// It is looked at by every workspace reservation and every read-back to the host.
+// It is looked at by every workspace reservation and, through read_back_sync, before results
+// copied to the host are handed out.
 tn_status_t wait_error_word(tn_ctx* ctx, int** out);
 tn_status_t wait_error_check(tn_ctx* ctx);
+// drains the context's stream, then wait_error_check
+tn_status_t read_back_sync(tn_ctx* ctx);
 void ctx_release(tn_ctx* ctx);  // frees the context (called when refs drop to 0)
 
 // ---------------------------------------------------------------------------------

@@ -482,8 +482,7 @@ tn_status_t overlap_impl(const tn_mps* a, const tn_mps* b, double* h_out) {
   }
   TN_CHECK_CUDA(ctx, cudaMemcpy2DAsync(h_out, sizeof(cxd), F, env * sizeof(cxd), sizeof(cxd), B, cudaMemcpyDeviceToHost,
                                        ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  TN_RETURN_IF(wait_error_check(ctx));
+  TN_RETURN_IF(read_back_sync(ctx));
   return TN_OK;
 }
 
@@ -688,8 +687,7 @@ tn_status_t tn_mps_get_instance_site(const tn_mps* p, int32_t b, int32_t i, void
   TN_ARG(ctx, h != nullptr, "tn_mps_get_site: null output");
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h, p->site[i] + (size_t)b * p->cap[i], sizeof(cxd) * sz(p, i),
                                      cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  TN_RETURN_IF(wait_error_check(ctx));
+  TN_RETURN_IF(read_back_sync(ctx));
   return TN_OK;
 }
 
@@ -717,8 +715,7 @@ tn_status_t tn_mps_get_instance_sites(const tn_mps* p, int32_t b, void* const* h
   for (int i = 1; i <= p->L; ++i)
     TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h[i - 1], p->site[i] + (size_t)b * p->cap[i], sizeof(cxd) * sz(p, i),
                                        cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  TN_RETURN_IF(wait_error_check(ctx));
+  TN_RETURN_IF(read_back_sync(ctx));
   return TN_OK;
 }
 
@@ -768,7 +765,7 @@ tn_status_t tn_mps_get_lambda(const tn_mps* p, double* h, int64_t* len) {
   if (h && p->lam_len > 0) {
     TN_CHECK_CUDA(ctx, cudaMemcpy2DAsync(h, sizeof(double) * p->lam_len, p->lam, sizeof(double) * p->lam_cap,
                                          sizeof(double) * p->lam_len, p->B, cudaMemcpyDeviceToHost, ctx->stream));
-    TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    TN_RETURN_IF(read_back_sync(ctx));
   }
   return TN_OK;
 }
@@ -930,8 +927,7 @@ tn_status_t tn_mps_amplitude(const tn_mps* p, const void* h_vectors, double* h_o
   }
   TN_CHECK_CUDA(ctx, cudaMemcpy2DAsync(h_out, sizeof(cxd), e, ve * sizeof(cxd), sizeof(cxd), B, cudaMemcpyDeviceToHost,
                                        ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  TN_RETURN_IF(wait_error_check(ctx));
+  TN_RETURN_IF(read_back_sync(ctx));
   return TN_OK;
 }
 
@@ -1043,8 +1039,7 @@ tn_status_t tn_mps_sample(tn_mps* p, int32_t instance, int64_t nshots, const dou
     TN_LAUNCHED(ctx);
   }
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h_out, O, sizeof(int32_t) * nshots * L, cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  TN_RETURN_IF(wait_error_check(ctx));
+  TN_RETURN_IF(read_back_sync(ctx));
   return TN_OK;
 }
 
@@ -1220,9 +1215,8 @@ tn_status_t evolve_mpo_zipup(tn_mps* p, const std::vector<const cxd*>& hW, const
     TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // W0 came from pageable host memory
   }
   for (int i = 1; i < L; ++i) p->cap_bond[i] = std::max(p->cap_bond[i], p->bond[i]);
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   p->lam_len = 0;  // the reference leaves the form as it was set before the sweep
-  return TN_OK;
+  return read_back_sync(ctx);
 }
 
 }  // namespace
@@ -1280,10 +1274,14 @@ tn_status_t tn_mps_save(const tn_mps* p, const char* path) {
     for (int i = 1; i <= p->L && ok; ++i) {
       buf.resize((size_t)sz(p, i));
       if (cudaMemcpyAsync(buf.data(), p->site[i] + (size_t)b * p->cap[i], sizeof(cxd) * buf.size(),
-                          cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
-          cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+                          cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess) {
         fclose(f);
         return tn_set_error(ctx, TN_ECUDA, "tn_mps_save: device read failed");
+      }
+      const tn_status_t st = read_back_sync(ctx);
+      if (st != TN_OK) {
+        fclose(f);
+        return st;
       }
       ok = fwrite(buf.data(), sizeof(cxd), buf.size(), f) == buf.size();
     }
@@ -1292,9 +1290,10 @@ tn_status_t tn_mps_save(const tn_mps* p, const char* path) {
     for (int b = 0; b < p->B; ++b)
       cudaMemcpyAsync(lam.data() + (size_t)b * lam_len, p->lam + (size_t)b * p->lam_cap, sizeof(double) * lam_len,
                       cudaMemcpyDeviceToHost, ctx->stream);
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+    const tn_status_t st = read_back_sync(ctx);
+    if (st != TN_OK) {
       fclose(f);
-      return tn_set_error(ctx, TN_ECUDA, "tn_mps_save: device read failed");
+      return st;
     }
     ok = fwrite(lam.data(), sizeof(double), lam.size(), f) == lam.size();
   }

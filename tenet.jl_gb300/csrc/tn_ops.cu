@@ -197,8 +197,7 @@ tn_status_t sumsq(tn_ctx* ctx, int64_t n, const E* x, double* h_out) {
   TN_LAUNCHED(ctx);
   double* hp = reinterpret_cast<double*>(ctx->pinned);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(hp, partial + nb, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  TN_RETURN_IF(wait_error_check(ctx));
+  TN_RETURN_IF(read_back_sync(ctx));
   *h_out = hp[0];
   return TN_OK;
 }
@@ -214,8 +213,7 @@ tn_status_t rank_select_batched(tn_ctx* ctx, double* S, int64_t k, int64_t sS, i
   TN_LAUNCHED(ctx);
   int* hp = reinterpret_cast<int*>(ctx->pinned);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(hp, flags, sizeof(int) * batch, cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  TN_RETURN_IF(wait_error_check(ctx));
+  TN_RETURN_IF(read_back_sync(ctx));
   int64_t r = 0;
   bool uneven = false;
   for (int64_t b = 0; b < batch; ++b) {
@@ -435,8 +433,7 @@ tn_status_t norms_batched(tn_ctx* ctx, bool complex_data, int64_t n, const void*
     k_sumsq_real_batched<<<(unsigned)batch, 512, 0, ctx->stream>>>(n, (const double*)x, sx, d);
   TN_LAUNCHED(ctx);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h_out, d, sizeof(double) * batch, cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  TN_RETURN_IF(wait_error_check(ctx));
+  TN_RETURN_IF(read_back_sync(ctx));
   for (int64_t b = 0; b < batch; ++b) h_out[b] = sqrt(h_out[b]);
   return TN_OK;
 }
@@ -480,8 +477,7 @@ tn_status_t zdotc_batched(tn_ctx* ctx, int64_t n, const cxd* x, int64_t sx, cons
   k_zdotc_batched<<<(unsigned)batch, 512, 0, ctx->stream>>>(n, (const double2*)x, sx, (const double2*)y, sy, d);
   TN_LAUNCHED(ctx);
   TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h_out, d, 2 * sizeof(double) * batch, cudaMemcpyDeviceToHost, ctx->stream));
-  TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  TN_RETURN_IF(wait_error_check(ctx));
+  TN_RETURN_IF(read_back_sync(ctx));
   return TN_OK;
 }
 

@@ -1104,7 +1104,7 @@ static tn_status_t jacobi_core(tn_ctx* ctx, int64_t m, int64_t n, cx<T>* W, cx<T
       ctx->launches += rounds + 2;  // norm refresh, ‖A‖_F, the rounds
       TN_CHECK_CUDA(ctx, cudaMemcpyAsync(h_rot.data(), rotated, sizeof(int) * 2 * batch, cudaMemcpyDeviceToHost,
                                          ctx->stream));
-      TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+      TN_RETURN_IF(read_back_sync(ctx));
       if (sweeps < (int)(sizeof(ctx->sweep_rotations) / sizeof(int))) {
         // the matrix with the largest off-diagonal ratio among those still active
         int64_t worst = 0;
