@@ -70,9 +70,10 @@ tn_status_t tn_destroy(tn_ctx* ctx);
 tn_status_t tn_set_stream(tn_ctx* ctx, void* stream);
 void* tn_get_stream(tn_ctx* ctx);
 tn_status_t tn_sync(tn_ctx* ctx);
-/* tn_free waits for the device and keeps the block for later allocations of the context (up to
- * 4 GiB of freed blocks; given back to the driver before an allocation would fail or exceed
- * the budget, and with the context; not counted by tn_hbm_in_use) */
+/* tn_free waits for the context's stream and keeps the block for later allocations of the context (up
+ * to 4 GiB of freed blocks; given back to the driver before an allocation would fail or exceed
+ * the budget, and with the context; not counted by tn_hbm_in_use).  A block is handed out again
+ * only after the whole device has drained, so other streams may still be using it when it is freed. */
 tn_status_t tn_alloc(tn_ctx* ctx, size_t bytes, void** dptr);
 tn_status_t tn_free(tn_ctx* ctx, void* dptr);
 tn_status_t tn_memcpy_h2d(tn_ctx* ctx, void* d_dst, const void* h_src, size_t bytes);

@@ -163,11 +163,10 @@ struct tn_ctx {
   size_t budget = 0;  // 0 = unlimited
   size_t in_use = 0;
   std::unordered_map<void*, size_t> allocs;  // live blocks: bytes asked for
-  // Freed blocks kept for the next allocation of about their size (cudaMalloc and cudaFree of
-  // a 128 MB result take 0.3 ms, as long as the product that fills it): capacity → block, the
-  // oldest given back to the driver beyond kPoolBytes, all of them before an allocation
-  // would fail or exceed the budget, and with the context.  A block enters only after the
-  // device has drained (as cudaFree waits for it), so no stream still uses it.
+  // freed blocks kept for the next allocation of their size (tn_context.cu): size → block; the
+  // oldest are given back to the driver beyond a limit, all of them before an allocation would fail
+  // or exceed the budget, and with the context.  What was released before `drained` is in use by
+  // no stream
   struct pool_block {
     void* p;
     uint64_t age;
@@ -175,7 +174,8 @@ struct tn_ctx {
   std::multimap<size_t, pool_block> pool;
   std::unordered_map<void*, size_t> capacity;  // of every block from the driver, live or pooled
   size_t pool_bytes = 0;
-  uint64_t pool_age = 0;
+  uint64_t pool_age = 0, drained = 0;
+  void* drain_block = nullptr;
   int64_t launches = 0;
   // instantiated CUDA graphs (e.g. one Jacobi sweep), keyed by shape + buffer addresses
   std::unordered_map<std::string, cudaGraphExec_t> graphs;
