@@ -22,13 +22,20 @@ tn_status_t tn_set_error(tn_ctx* ctx, tn_status_t st, const char* fmt, ...) {
 
 namespace {
 
-// Freed blocks kept for the next allocation of about their size: cudaMalloc and cudaFree of a 128 MB
+// Freed blocks kept for the next allocation of their size: cudaMalloc and cudaFree of a 128 MB
 // result take 0.15 ms, as long as the product that fills it.  A block may still be in use by a stream
 // that the context does not know of, so it is handed out again only after the device has drained.
 constexpr size_t kPoolBytes = size_t(4) << 30;  // most bytes kept
 // Undrained blocks of one size at which an allocation drains the device rather than take new memory: a
 // drain is 9 µs, and one call in four (of 128 MB results) to thirty-two (of small ones) pays for it
 constexpr size_t kDrainCount = 32, kDrainBytes = size_t(512) << 20;
+
+// the size in which a request is allocated, so that blocks fit each other: the driver's own granularity
+// (pages of 2 MiB, and pieces of them), so no memory is held that the request would not take
+size_t block_size(size_t bytes) {
+  const size_t unit = bytes >= (size_t(2) << 20) ? size_t(2) << 20 : 512;
+  return (bytes + unit - 1) / unit * unit;
+}
 
 cudaError_t driver_free(tn_ctx* ctx, void* p) {
   const cudaError_t e = cudaFree(p);
@@ -68,14 +75,11 @@ cudaError_t pool_shrink(tn_ctx* ctx, size_t keep) {
   return cudaSuccess;
 }
 
-// a pooled block that holds `bytes` with at most a quarter to spare and that no stream uses any
-// more, or null
-void* pool_take(tn_ctx* ctx, size_t bytes) {
+// a pooled block of this size that no stream uses any more, or null
+void* pool_take(tn_ctx* ctx, size_t size) {
   if (ctx->budget && ctx->in_use + ctx->pool_bytes > ctx->budget) return nullptr;
-  const auto fit = ctx->pool.lower_bound(bytes);
-  if (fit == ctx->pool.end() || fit->first > bytes + bytes / 4 + 4096) return nullptr;
-  const size_t size = fit->first;
   const auto range = ctx->pool.equal_range(size);  // (in the order of their release)
+  if (range.first == range.second) return nullptr;
   if (range.first->second.age >= ctx->drained) {
     const size_t count = (size_t)std::distance(range.first, range.second);
     if (!ctx->budget && count < kDrainCount && count * size < kDrainBytes) return nullptr;
@@ -94,22 +98,23 @@ tn_status_t tn_dev_alloc(tn_ctx* ctx, size_t bytes, void** p) {
   if (ctx->budget && ctx->in_use + bytes > ctx->budget)
     return tn_set_error(ctx, TN_ENOMEM, "HBM budget exceeded: %zu in use + %zu > %zu",
                         ctx->in_use, bytes, ctx->budget);
-  *p = pool_take(ctx, bytes);
+  const size_t size = block_size(bytes);
+  *p = pool_take(ctx, size);
   if (!*p) {
     if (ctx->budget && ctx->in_use + ctx->pool_bytes + bytes > ctx->budget)
       TN_CHECK_CUDA(ctx, pool_shrink(ctx, ctx->budget - ctx->in_use - bytes));
-    cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = cudaMalloc(p, size);
     if (e != cudaSuccess && !ctx->pool.empty()) {
       cudaGetLastError();
       TN_CHECK_CUDA(ctx, pool_shrink(ctx, 0));
-      e = cudaMalloc(p, bytes);
+      e = cudaMalloc(p, size);
     }
     if (e != cudaSuccess) {
       cudaGetLastError();
       return tn_set_error(ctx, TN_ENOMEM, "cudaMalloc(%zu) failed: %s", bytes,
                           cudaGetErrorString(e));
     }
-    ctx->capacity[*p] = bytes;
+    ctx->capacity[*p] = size;
   }
   ctx->allocs[*p] = bytes;
   ctx->in_use += bytes;

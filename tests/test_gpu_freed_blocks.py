@@ -1,5 +1,5 @@
 """Freed blocks that a context keeps: not handed out while any stream may use them, whatever another
-thread captures meanwhile."""
+thread captures meanwhile, and never beyond the HBM budget."""
 
 import threading
 
@@ -77,3 +77,49 @@ def test_freed_while_another_thread_captures():
     assert (x == 2).all()
     # (a tensor's free that failed would have been swallowed: nothing may be left over)
     assert ctx.hbm_in_use() == 0
+
+
+def _held(before):
+    import torch
+
+    return before - torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("sizes", [(80, 64, 36), (90, 75, 25), (40, 33, 67)])
+def test_budget_holds_over_reused_blocks(sizes):
+    """A block freed, one up to a quarter smaller taken, then what the budget leaves: the memory held is
+    within it, up to the driver's pages of 2 MiB, and nothing within it is refused."""
+    import tenetgb
+    import torch
+
+    MB = 1 << 20
+    ctx = tenetgb.Context(0)
+    warm = ctx.alloc(256)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    ctx.set_hbm_budget(100 * MB + 256)
+    first, second, third = (s * MB for s in sizes)
+    ctx.free(ctx.alloc(first))
+    assert _held(before) <= 100 * MB + 8 * MB
+    p, q = ctx.alloc(second), ctx.alloc(third)
+    assert ctx.hbm_in_use() == second + third + 256
+    assert _held(before) <= 100 * MB + 8 * MB
+    with pytest.raises(Exception, match="budget"):
+        ctx.alloc(1)
+    ctx.free(p)
+    ctx.free(q)
+    ctx.free(warm)
+
+
+def test_budget_set_over_kept_blocks():
+    import tenetgb
+    import torch
+
+    MB = 1 << 20
+    ctx = tenetgb.Context(0)
+    ctx.alloc(256)
+    before = torch.cuda.mem_get_info()[0]
+    for p in [ctx.alloc(s * MB) for s in (50, 60, 70)]:
+        ctx.free(p)
+    ctx.set_hbm_budget(100 * MB)
+    assert _held(before) <= 100 * MB + 8 * MB
