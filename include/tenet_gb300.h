@@ -72,10 +72,12 @@ void* tn_get_stream(tn_ctx* ctx);
 tn_status_t tn_sync(tn_ctx* ctx);
 /* tn_free waits for the context's stream and keeps the block for later allocations of the context (up
  * to 4 GiB of freed blocks; given back to the driver before an allocation would fail or exceed
- * the budget, and with the context; not counted by tn_hbm_in_use).  A block is handed out again
+ * the budget, by tn_release_cached, and with the context; not counted by tn_hbm_in_use).  A block is handed out again
  * only after the whole device has drained, so other streams may still be using it when it is freed. */
 tn_status_t tn_alloc(tn_ctx* ctx, size_t bytes, void** dptr);
 tn_status_t tn_free(tn_ctx* ctx, void* dptr);
+/* gives all kept blocks back to the driver, for other users of the device's memory */
+tn_status_t tn_release_cached(tn_ctx* ctx);
 tn_status_t tn_memcpy_h2d(tn_ctx* ctx, void* d_dst, const void* h_src, size_t bytes);
 tn_status_t tn_memcpy_d2h(tn_ctx* ctx, void* h_dst, const void* d_src, size_t bytes);
 tn_status_t tn_memcpy_d2d(tn_ctx* ctx, void* d_dst, const void* d_src, size_t bytes);

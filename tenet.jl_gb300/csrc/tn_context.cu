@@ -303,6 +303,12 @@ tn_status_t tn_free(tn_ctx* ctx, void* dptr) {
   return tn_dev_free(ctx, dptr);
 }
 
+tn_status_t tn_release_cached(tn_ctx* ctx) {
+  if (!ctx) return TN_EINVAL;
+  TN_CHECK_CUDA(ctx, pool_shrink(ctx, 0));
+  return TN_OK;
+}
+
 tn_status_t tn_memcpy_h2d(tn_ctx* ctx, void* dst, const void* src, size_t bytes) {
   if (!ctx) return TN_EINVAL;
   TN_ARG(ctx, dst && src, "tn_memcpy_h2d: null pointer");

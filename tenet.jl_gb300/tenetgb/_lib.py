@@ -78,6 +78,7 @@ SIGNATURES = {
     "tn_memcpy_d2h": (_st, [_vp, _vp, _vp, _sz]),
     "tn_memcpy_d2d": (_st, [_vp, _vp, _vp, _sz]),
     "tn_set_hbm_budget": (_st, [_vp, _sz]),
+    "tn_release_cached": (_st, [_vp]),
     "tn_hbm_in_use": (_st, [_vp, C.POINTER(_sz)]),
     "tn_kernel_launches": (_st, [_vp, _pi64]),
     "tn_last_error_string": (C.c_char_p, [_vp]),

@@ -92,6 +92,10 @@ class Context:
         if ptr:
             self.check(self.lib.tn_free(self.h, C.c_void_p(ptr)))
 
+    def release_cached(self):
+        """Give the freed blocks that the context keeps back to the driver."""
+        self.check(self.lib.tn_release_cached(self.h))
+
     def h2d(self, dst, arr):
         arr = np.asarray(arr)
         self.check(self.lib.tn_memcpy_h2d(self.h, C.c_void_p(dst), arr.ctypes.data_as(C.c_void_p), arr.nbytes))

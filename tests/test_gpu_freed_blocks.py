@@ -123,3 +123,18 @@ def test_budget_set_over_kept_blocks():
         ctx.free(p)
     ctx.set_hbm_budget(100 * MB)
     assert _held(before) <= 100 * MB + 8 * MB
+
+
+def test_release_cached():
+    import tenetgb
+    import torch
+
+    MB = 1 << 20
+    ctx = tenetgb.Context(0)
+    ctx.alloc(256)
+    before = torch.cuda.mem_get_info()[0]
+    for p in [ctx.alloc(s * MB) for s in (50, 60, 70)]:
+        ctx.free(p)
+    ctx.release_cached()
+    assert _held(before) <= 8 * MB and ctx.hbm_in_use() == 256
+    ctx.free(ctx.alloc(60 * MB))
