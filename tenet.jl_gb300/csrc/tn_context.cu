@@ -167,10 +167,13 @@ tn_status_t read_back_sync(tn_ctx* ctx) {
   return wait_error_check(ctx);
 }
 
-tn_status_t ws_reserve(tn_ctx* ctx, size_t bytes) {
+tn_status_t ws_reserve(tn_ctx* ctx, size_t bytes, size_t spare) {
   ctx->ws_top = 0;
   TN_RETURN_IF(wait_error_check(ctx));
   if (bytes <= ctx->ws_cap) return TN_OK;
+  auto with_margin = [](size_t b) { return b + b / 4 + (1 << 20); };
+  // (without the spare part it holds what the budget would refuse to grow)
+  if (bytes - spare <= ctx->ws_cap && ctx->budget && ctx->in_use - ctx->ws_cap + with_margin(bytes) > ctx->budget) return TN_OK;
   // growth: the stream must be idle before the old arena is released
   TN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   // (the cached graphs point into the arena; the profiler's events do not and stay)
@@ -179,9 +182,14 @@ tn_status_t ws_reserve(tn_ctx* ctx, size_t bytes) {
   if (ctx->ws) TN_RETURN_IF(tn_dev_free(ctx, ctx->ws));
   ctx->ws = nullptr;
   ctx->ws_cap = 0;
-  size_t cap = bytes + bytes / 4 + (1 << 20);
+  size_t cap = with_margin(bytes);
   void* p = nullptr;
-  TN_RETURN_IF(tn_dev_alloc(ctx, cap, &p));
+  tn_status_t st = tn_dev_alloc(ctx, cap, &p);
+  if (st == TN_ENOMEM && spare > 0) {
+    cap = with_margin(bytes - spare);
+    st = tn_dev_alloc(ctx, cap, &p);
+  }
+  TN_RETURN_IF(st);
   ctx->ws = (char*)p;
   ctx->ws_cap = cap;
   return TN_OK;

@@ -630,7 +630,7 @@ tn_status_t split_pair_impl(Dmrg& D, int j, bool absorb_right) {
   const int64_t keep = std::min(D.maxdim, k);
   const cxd* theta = D.V;
   if (absorb_right && m >= n) {
-    TN_RETURN_IF(ws_reserve(ctx, svd_left_workspace(p->prec, m, n, D.B)));
+    TN_RETURN_IF(ws_reserve(ctx, svd_left_workspace(p->prec, m, n, D.B), svd_spare(TN_C64, p->prec, m, n, D.B)));
     TN_RETURN_IF(svd_left(ctx, p->prec, m, n, theta, m, D.sV, D.U, D.Nmax, D.S, D.Nmax, D.B, keep));
     k_inv_norm<<<D.B, 256, 0, ctx->stream>>>((int)keep, D.S, D.Nmax, D.inv);
     TN_LAUNCHED(ctx);
@@ -643,7 +643,7 @@ tn_status_t split_pair_impl(Dmrg& D, int j, bool absorb_right) {
   } else if (!absorb_right && n >= m) {
     // θᴴ (n × m) into the x0 buffer (θ itself stays in slot 0)
     TN_RETURN_IF(transpose_cx<double>(ctx, m, n, theta, m, D.sV, D.x0, n, D.Nmax, D.B, true));
-    TN_RETURN_IF(ws_reserve(ctx, svd_left_workspace(p->prec, n, m, D.B)));
+    TN_RETURN_IF(ws_reserve(ctx, svd_left_workspace(p->prec, n, m, D.B), svd_spare(TN_C64, p->prec, n, m, D.B)));
     TN_RETURN_IF(svd_left(ctx, p->prec, n, m, D.x0, n, D.Nmax, D.U, D.Nmax, D.S, D.Nmax, D.B, keep));
     k_inv_norm<<<D.B, 256, 0, ctx->stream>>>((int)keep, D.S, D.Nmax, D.inv);
     TN_LAUNCHED(ctx);
@@ -655,7 +655,7 @@ tn_status_t split_pair_impl(Dmrg& D, int j, bool absorb_right) {
                                  (int64_t)p->cap[j], D.B));
     TN_RETURN_IF(scale_inst(D, p->site[j], (int64_t)p->cap[j], m * keep));
   } else {
-    TN_RETURN_IF(ws_reserve(ctx, svd_any_workspace(TN_C64, p->prec, m, n, D.B)));
+    TN_RETURN_IF(ws_reserve(ctx, svd_any_workspace(TN_C64, p->prec, m, n, D.B), svd_spare(TN_C64, p->prec, m, n, D.B)));
     TN_RETURN_IF(svd_any(ctx, TN_C64, p->prec, m, n, theta, m, D.sV, D.U, D.Nmax, D.S, D.Nmax, D.Vh, D.Nmax, D.B));
     k_inv_norm<<<D.B, 256, 0, ctx->stream>>>((int)keep, D.S, D.Nmax, D.inv);
     TN_LAUNCHED(ctx);

@@ -775,10 +775,11 @@ tn_status_t g_sweeps_by_rounds(tn_ctx* ctx, const std::vector<JacD>& h, JacD* d,
 tn_status_t g_svd_left(tn_ctx* ctx, std::vector<JacD>& h, int* active, int* rotated) {
   if (h.empty()) return TN_OK;
   const int P = (int)h.size();
-  int64_t mmax = 1, Nmax = 2;
+  int64_t mmax = 1, n_most = 1, Nmax = 2;
   for (auto& j : h) {
     j.N = (int)(j.n + (j.n & 1));
     mmax = std::max(mmax, j.m);
+    n_most = std::max(n_most, j.n);
     Nmax = std::max<int64_t>(Nmax, j.N);
   }
   if (mmax > 4096) return tn_set_error(ctx, TN_EUNSUPPORTED, "group svd: more than 4096 rows");
@@ -786,7 +787,7 @@ tn_status_t g_svd_left(tn_ctx* ctx, std::vector<JacD>& h, int* active, int* rota
   TN_RETURN_IF(upload(ctx, h, &d));
   int64_t resident = 0;
   TN_RETURN_IF(jacobi_pairs_resident(ctx, mmax, &resident));
-  if (mmax <= 512 && Nmax / 2 <= resident) {
+  if (mmax <= 512 && Nmax / 2 <= resident && jacobi_pairs_workspace(mmax, n_most, P, false) <= ws_room(ctx)) {
     std::vector<JacobiMat> mats;
     for (auto& j : h) mats.push_back({j.W, nullptr, j.nrm, (int)j.m, (int)j.n});
     // like sizes together: a launch lasts as long as its slowest matrix
@@ -1038,7 +1039,8 @@ tn_status_t tn_group_canonize_compress_norm(tn_group* g, const int64_t* maxdim, 
       mmax = std::max(mmax, g->bond[b][k - 1] * d);
       nmax = std::max(nmax, g->bond[b][k]);
     }
-    if (mmax <= 512) need += jacobi_pairs_workspace(mmax, nmax, P, false);
+    const size_t pairs = mmax <= 512 ? jacobi_pairs_workspace(mmax, nmax, P, false) : 0;
+    need += pairs;
     for (int b : ids) {
       const int64_t m = g->bond[b][k - 1] * d, n = g->bond[b][k], n2 = d * g->bond[b][k + 1];
       const int64_t r = std::min<int64_t>(maxdim[b], std::min(m, n));
@@ -1046,7 +1048,7 @@ tn_status_t tn_group_canonize_compress_norm(tn_group* g, const int64_t* maxdim, 
               al256(sizeof(double) * (size_t)(n + 1)) + al256(sizeof(double) * (size_t)n) + al256(sizeof(int) * (size_t)n) +
               al256(sizeof(cxd) * (size_t)(r * n)) + al256(sizeof(cxd) * (size_t)(r * n2));
     }
-    TN_RETURN_IF(ws_reserve(ctx, need));
+    TN_RETURN_IF(ws_reserve(ctx, need, pairs));
     int* active = ws_take<int>(ctx, (size_t)P + 1);
     int* rotated = ws_take<int>(ctx, (size_t)(2 * P + 2));
     std::vector<JacD> jd;

@@ -287,8 +287,10 @@ tn_status_t tn_set_error(tn_ctx* ctx, tn_status_t st, const char* fmt, ...);
 tn_status_t tn_dev_alloc(tn_ctx* ctx, size_t bytes, void** p);
 tn_status_t tn_dev_free(tn_ctx* ctx, void* p);
 
-// workspace: reserve (may reallocate: only between operations), then take
-tn_status_t ws_reserve(tn_ctx* ctx, size_t bytes);
+// workspace: reserve (may reallocate: only between operations), then take.  `spare` of the bytes are for
+// faster kernels that look at ws_room first: they are left out where the memory does not reach
+tn_status_t ws_reserve(tn_ctx* ctx, size_t bytes, size_t spare = 0);
+inline size_t ws_room(const tn_ctx* ctx) { return ctx->ws_cap - ctx->ws_top; }
 inline size_t ws_round(size_t b) { return (b + 255) & ~size_t(255); }
 // a take beyond the reserved arena is a bug in the caller's size computation: stop the
 // process on the host (after the stream has drained, so no kernel is left in flight)
@@ -442,6 +444,9 @@ size_t svd_mixed_workspace(int64_t m, int64_t n, int64_t batch);
 tn_status_t svd_tall_mixed(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda,
                            int64_t sA, cxd* U, int64_t sU, double* S, int64_t sS, cxd* V,
                            int64_t sV, int64_t batch, int64_t keep);
+
+// the part of svd_any_workspace and svd_left_workspace that the kernels can do without (ws_reserve)
+size_t svd_spare(tn_dtype_t dt, tn_precision_t prec, int64_t m, int64_t n, int64_t batch);
 
 // left vectors + values only (m >= n): U m×n, S n (no V accumulation on large matrices).
 // keep > 0: a truncation to at most `keep` values follows (the mixed path then skips the

@@ -788,6 +788,7 @@ tn_status_t jacobi_pairs(tn_ctx* ctx, const std::vector<JacobiMat>& mats, bool v
     first = last;
   }
   starts.push_back(mats.size());
+  const size_t top = ctx->ws_top;
   char* zeroed = ws_take<char>(ctx, zero_bytes);
   char* table = ws_take<char>(ctx, table_bytes);
   std::vector<char> host;
@@ -862,5 +863,6 @@ tn_status_t jacobi_pairs(tn_ctx* ctx, const std::vector<JacobiMat>& mats, bool v
     if (slot >= 0) prof_end(ctx, slot, TN_PROF_JACOBI_COOP, 1, flops, 0.0);
     if (h_ctl[kCtl * count]) return tn_set_error(ctx, TN_ETIMEOUT, "svd: a wait of the Jacobi rounds exceeded its limit");
   }
+  ctx->ws_top = top;
   return TN_OK;
 }

@@ -130,7 +130,8 @@ extern "C" tn_status_t tn_tensor_svd_thin(tn_ctx* ctx, tn_dtype_t dtype, tn_prec
   const size_t es = dtype_size(dtype);
   TN_RETURN_IF(ws_reserve(ctx, ws_round(es * (size_t)(m * n)) + ws_round(es * (size_t)(m * k)) +
                                    ws_round(es * (size_t)(k * n)) + ws_round(sizeof(double) * (size_t)k) +
-                                   svd_any_workspace(dtype, prec, m, n, 1)));
+                                   svd_any_workspace(dtype, prec, m, n, 1),
+                          svd_spare(dtype, prec, m, n, 1)));
   const void* M = nullptr;
   TN_RETURN_IF(matricise(ctx, dtype, A, perm, &M));
   char* Uw = ws_take<char>(ctx, es * (size_t)(m * k));

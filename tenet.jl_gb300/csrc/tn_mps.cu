@@ -120,7 +120,7 @@ tn_status_t gauge_right(tn_mps* p, int i, bool svd_lambda) {
     need += ws_round(sizeof(cxd) * (size_t)(B * m * k)) + svd_any_workspace(TN_C64, p->prec, m, n, B);
   else
     need += qr_workspace<double>(m, n, B);
-  TN_RETURN_IF(ws_reserve(ctx, need));
+  TN_RETURN_IF(ws_reserve(ctx, need, svd_lambda ? svd_spare(TN_C64, p->prec, m, n, B) : 0));
   cxd* R = ws_take<cxd>(ctx, (size_t)(B * k * n));
   cxd* tmp = ws_take<cxd>(ctx, (size_t)(B * k * nbc));
   if (svd_lambda) {
@@ -151,7 +151,7 @@ tn_status_t gauge_left(tn_mps* p, int i, bool svd_lambda) {
   size_t need = 2 * ws_round(sizeof(cxd) * (size_t)(B * m * n)) + ws_round(sizeof(cxd) * (size_t)(B * k * n)) +
                 ws_round(sizeof(cxd) * (size_t)(B * rows_b * k));
   need += svd_lambda ? svd_any_workspace(TN_C64, p->prec, m, n, B) : qr_workspace<double>(m, n, B);
-  TN_RETURN_IF(ws_reserve(ctx, need));
+  TN_RETURN_IF(ws_reserve(ctx, need, svd_lambda ? svd_spare(TN_C64, p->prec, m, n, B) : 0));
   cxd* Mh = ws_take<cxd>(ctx, (size_t)(B * m * n));
   cxd* Q = ws_take<cxd>(ctx, (size_t)(B * m * n));
   cxd* R = ws_take<cxd>(ctx, (size_t)(B * k * n));
@@ -322,7 +322,7 @@ tn_status_t simple_update_core(tn_ctx* ctx, tn_precision_t prec, int64_t chl, in
   size_t need = 2 * ws_round(sizeof(cxd) * (size_t)(batch * m * n)) + ws_round(sizeof(cxd) * (size_t)(batch * m * k)) +
                 ws_round(sizeof(double) * (size_t)(batch * k)) + ws_round(sizeof(cxd) * (size_t)(batch * k * n)) +
                 svd_ws;
-  TN_RETURN_IF(ws_reserve(ctx, need));
+  TN_RETURN_IF(ws_reserve(ctx, need, svd_spare(TN_C64, prec, m, n, batch)));
   cxd* th0 = ws_take<cxd>(ctx, (size_t)(batch * m * n));
   cxd* th = ws_take<cxd>(ctx, (size_t)(batch * m * n));
   cxd* U = ws_take<cxd>(ctx, (size_t)(batch * m * k));
@@ -1148,7 +1148,7 @@ tn_status_t evolve_mpo_zipup(tn_mps* p, const std::vector<const cxd*>& hW, const
                       5 * ws_round(sizeof(cxd) * (size_t)(big * B)) + ws_round(sizeof(cxd) * (size_t)(rows * kk * B)) +
                       ws_round(sizeof(double) * (size_t)(kk * B)) + ws_round(sizeof(cxd) * (size_t)(kk * cols * B)) +
                       svd_any_workspace(TN_C64, p->prec, rows, cols, B);
-  TN_RETURN_IF(ws_reserve(ctx, need));
+  TN_RETURN_IF(ws_reserve(ctx, need, svd_spare(TN_C64, p->prec, rows, cols, B)));
   cxd* W0 = ws_take<cxd>(ctx, (size_t)(wm * d * d * wm));
   cxd* W1 = ws_take<cxd>(ctx, (size_t)(wm * d * d * wm));
   cxd* R = ws_take<cxd>(ctx, (size_t)(big * B));
@@ -1202,7 +1202,9 @@ tn_status_t evolve_mpo_zipup(tn_mps* p, const std::vector<const cxd*>& hW, const
       break;
     }
     const int64_t kmin = std::min(m, n);
+    const size_t top = ctx->ws_top;
     TN_RETURN_IF(svd_any(ctx, TN_C64, p->prec, m, n, Tm, m, m * n, U, m * kmin, S, kmin, Vh, kmin * n, B));
+    ctx->ws_top = top;  // (its scratch is the next site's)
     int64_t rk = 0;
     TN_RETURN_IF(rank_select_batched(ctx, S, kmin, kmin, B, maxdim, threshold, &rk, nullptr));
     // site i = U[:, :rk] as (k, o, rk);  R = diag(S[:rk]) Vh[:rk, :] as (rk, r, b)

@@ -862,11 +862,20 @@ __global__ void k_unorder_rows(int64_t n, const cxd* __restrict__ in, int64_t sI
 
 }  // namespace
 
-// beside W, V and the sweeps' own: Q, two n × n matrices, the QR's reflectors, keys and order
+// beside W, V and the sweeps' own: Q, two n × n matrices, the QR's reflectors, keys and order (nothing
+// for more columns than the chip can hold CTAs of the QR)
 static size_t svd_ordered_workspace(int64_t m, int64_t n, int64_t batch) {
+  if (n * batch > 16 * 160) return 0;
   return ws_round(sizeof(cxd) * (size_t)(m * n * batch)) + 2 * ws_round(sizeof(cxd) * (size_t)(n * n * batch)) +
          qr_cols_workspace(m, n, batch) + 2 * ws_round(sizeof(int) * (size_t)(m * batch)) +
          ws_round(sizeof(int) * (size_t)batch);
+}
+
+// (without it the sweeps run by launches per round, or in one CTA's shared memory)
+size_t svd_spare(tn_dtype_t dt, tn_precision_t prec, int64_t m, int64_t n, int64_t batch) {
+  if (m < n) std::swap(m, n);
+  if (dt != TN_C64 || !jacobi_pairs_fits(m, n)) return 0;
+  return jacobi_pairs_workspace(m, n, batch, true) + (prec == TN_PREC_MIXED ? 0 : svd_ordered_workspace(m, n, batch));
 }
 
 template <typename T>
@@ -874,9 +883,7 @@ size_t svd_workspace(int64_t m, int64_t n, int64_t batch) {
   return ws_round(sizeof(cx<T>) * (size_t)(m * n * batch)) + ws_round(sizeof(cx<T>) * (size_t)(n * n * batch)) +
          ws_round(sizeof(int) * (size_t)(n * batch)) + ws_round(sizeof(int) * (size_t)(batch + 1)) +
          ws_round(sizeof(int) * (size_t)(2 * batch + 2)) + ws_round(sizeof(T) * (size_t)((n + 1) * batch)) +
-         (sizeof(T) == 8 && jacobi_pairs_fits(m, n)
-              ? jacobi_pairs_workspace(m, n, batch, true) + svd_ordered_workspace(m, n, batch)
-              : 0);
+         (sizeof(T) == 8 ? svd_spare(TN_C64, TN_PREC_NATIVE, m, n, batch) : 0);
 }
 template size_t svd_workspace<double>(int64_t, int64_t, int64_t);
 template size_t svd_workspace<float>(int64_t, int64_t, int64_t);
@@ -956,7 +963,7 @@ static tn_status_t launch_step(tn_ctx* ctx, int64_t m, int64_t n, int N, int r, 
 // that they fill the chip twice over with one SM each.
 static tn_status_t jacobi_takes_pairs(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch, bool with_v, bool* out) {
   *out = false;
-  if (!jacobi_pairs_fits(m, n) || n < kPairsMinN) return TN_OK;
+  if (!jacobi_pairs_fits(m, n) || n < kPairsMinN || jacobi_pairs_workspace(m, n, batch, with_v) > ws_room(ctx)) return TN_OK;
   int64_t resident = 0;
   TN_RETURN_IF(jacobi_pairs_resident(ctx, m, &resident));
   if ((n + 1) / 2 * (with_v ? 2 : 1) > resident) return TN_OK;
@@ -1198,7 +1205,7 @@ constexpr int64_t kOrderedMinN = 24;  // below this the QR costs more than the s
 
 static tn_status_t svd_takes_ordered(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch, bool with_v, bool* out) {
   *out = false;
-  if (n < kOrderedMinN) return TN_OK;
+  if (n < kOrderedMinN || svd_ordered_workspace(m, n, batch) + jacobi_pairs_workspace(m, n, batch, true) > ws_room(ctx)) return TN_OK;
   bool pairs = false;
   TN_RETURN_IF(jacobi_takes_pairs(ctx, m, n, batch, with_v || m > n, &pairs));
   if (pairs) TN_RETURN_IF(qr_cols_takes(ctx, m, n * batch, out));
@@ -1211,6 +1218,7 @@ static tn_status_t svd_ordered(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, 
                                int* order, double* nrm, int* sweeps_out, bool* noconv) {
   const unsigned gy = (unsigned)batch;
   const bool from_left = Vo || m > n;  // A·Π = Q·R; otherwise Aᴴ·Π = Q·R (A square)
+  const size_t top = ctx->ws_top;
   cxd* Q = ws_take<cxd>(ctx, (size_t)(m * n * batch));
   cxd* Y = ws_take<cxd>(ctx, (size_t)(n * n * batch));
   cxd* Vg = ws_take<cxd>(ctx, (size_t)(n * n * batch));
@@ -1237,6 +1245,7 @@ static tn_status_t svd_ordered(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, 
   if (!from_left) {
     k_unorder_rows<<<dim3(blocks, gy), 256, 0, ctx->stream>>>(n, Y, n * n, perm, U, sU, false);
     TN_LAUNCHED(ctx);
+    ctx->ws_top = top;
     return TN_OK;
   }
   TN_RETURN_IF(gemm_cx<double>(ctx, 'N', 'N', m, n, n, mkcx(1.0, 0.0), Q, m, m * n, Vg, n, n * n, mkcx(0.0, 0.0), U, m, sU,
@@ -1245,6 +1254,7 @@ static tn_status_t svd_ordered(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, 
     k_unorder_rows<<<dim3(blocks, gy), 256, 0, ctx->stream>>>(n, Y, n * n, perm, Vo, sVo, vh);
     TN_LAUNCHED(ctx);
   }
+  ctx->ws_top = top;
   return TN_OK;
 }
 
@@ -1630,8 +1640,7 @@ size_t svd_mixed_workspace(int64_t m, int64_t n, int64_t batch) {
   s += ws_round((size_t)(n * batch));                     // tail flags
   s += ws_round(sizeof(cxd) * (size_t)(n * n * batch));  // R / E of the refinement
   s += ws_round((size_t)(n * batch)) + ws_round(sizeof(int) * (size_t)(5 * batch + 4));  // cluster marks, stats
-  if (jacobi_pairs_fits(m, n)) s += jacobi_pairs_workspace(m, n, batch, true);
-  return s;
+  return s + svd_spare(TN_C64, TN_PREC_MIXED, m, n, batch);
 }
 
 tn_status_t svd_tall_mixed(tn_ctx* ctx, int64_t m, int64_t n, const cxd* A, int64_t lda, int64_t sA, cxd* U,
@@ -2201,6 +2210,6 @@ extern "C" tn_status_t tn_svd_thin(tn_ctx* ctx, tn_dtype_t dtype, tn_precision_t
   TN_ARG(ctx, lda >= (m > 1 ? m : 1), "tn_svd_thin: lda < m");
   TN_ARG(ctx, (m == 0 || n == 0 || batch == 0) || (A && U && S && Vh), "tn_svd_thin: null pointer");
   TN_ARG(ctx, dtype == TN_C64 || dtype == TN_C32, "tn_svd_thin: only C64 and C32 are implemented");
-  TN_RETURN_IF(ws_reserve(ctx, svd_any_workspace(dtype, prec, m, n, batch)));
+  TN_RETURN_IF(ws_reserve(ctx, svd_any_workspace(dtype, prec, m, n, batch), svd_spare(dtype, prec, m, n, batch)));
   return svd_any(ctx, dtype, prec, m, n, A, lda, strideA, U, strideU, S, strideS, Vh, strideVh, batch);
 }
