@@ -103,7 +103,9 @@ tn_status_t tn_profile_read(tn_ctx* ctx, int32_t cls, int64_t* launches, double*
  * kernels) */
 tn_status_t tn_pipe_peak(tn_ctx* ctx, int32_t which, double* tflops);
 /* autotuner: with enable != 0 the first call of an unseen shape bucket times the
- * candidate launch configurations (QR panel and slab widths) and records the fastest.
+ * candidate launch configurations (QR panel and slab widths) and records the fastest.  The
+ * table is for the blocked QR: matrices that the kernel with one CTA per column takes (FP64, m <= 512,
+ * n·batch up to a few hundred) have no entry, and one loaded for them changes nothing.
  * tn_tuning_dump writes the table as text ("key v1 v2" lines; *needed = bytes incl. the
  * terminator); tn_tuning_load reads such text back (a tuning cache file; QR entries hold a
  * panel width in 1, 2, 4, …, 32 and a slab width in 1, 2, 4, anything else is TN_EINVAL). */

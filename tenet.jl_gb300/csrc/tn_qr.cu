@@ -320,10 +320,11 @@ tn_status_t qr_run(tn_ctx* ctx, int nb, int slab, int64_t m, int64_t n, const cx
 
 // Which kernel: one CTA per column (tn_qr_cols.cu) while all columns of all matrices are
 // resident at once, the blocked panels below beyond that (rows > 512, or batches that fill
-// the FP64 pipe with panels of different matrices) and for shapes whose launch configuration
-// the caller set (tn_tuning_load).  Measured, one matrix, blocked /
-// columns, µs: 64×64 630 / 174, 128×128 1420 / 394, 256×256 3345 / 1158, 512×256 5728 / 1510,
-// 512×512 9634 / 4000.
+// the FP64 pipe with panels of different matrices).  Measured, µs, blocked at the best of its
+// panel widths / columns: one matrix 64×64 594 / 135, 128×128 1347 / 299, 256×256 3328 / 975,
+// 512×256 5394 / 1364, 512×512 9312 / 3073; as many as are resident 150 of 8×4 40 / 27, 32 of 16×16
+// 141 / 65, 8 of 64×64 617 / 237, 4 of 128×128 1399 / 521, 4 of 512×128 3157 / 1141.  The tuning table
+// and the autotuner are for the blocked panels' own widths.
 // A column's CTA reads it before anything is written only if no other CTA's output lies
 // there, so Q or R over A is left to the blocked kernel (which factors a copy) unless Q is
 // exactly A.
@@ -355,9 +356,6 @@ static void qr_columns_profile(tn_ctx* ctx, int slot, int64_t m, int64_t n, int6
 tn_status_t lq_in_place(tn_ctx* ctx, int64_t m, int64_t n, cxd* A, int64_t sA, cxd* R, int64_t sR, int64_t batch, bool* done) {
   *done = false;
   if (m < n || n == 0 || batch == 0) return TN_OK;
-  char key[96];
-  qr_tuning_key(key, sizeof(key), sizeof(double), m, n, batch);
-  if (ctx->tuning.find(key) != ctx->tuning.end()) return TN_OK;
   if (batch > 1 && (sA < m * n || sR < n * n)) return TN_OK;
   if (ranges_meet(R, sizeof(cxd) * (size_t)((batch - 1) * sR + n * n), A, sizeof(cxd) * (size_t)((batch - 1) * sA + m * n)))
     return TN_OK;
@@ -389,8 +387,7 @@ tn_status_t qr_cx(tn_ctx* ctx, int64_t m, int64_t n, const cx<T>* A, int64_t lda
   const double kk = (double)k, f = 4.0 * (2.0 * m * kk * kk - 2.0 / 3.0 * kk * kk * kk);
   if constexpr (sizeof(T) == 8) {
     bool columns = false;
-    if (it == ctx->tuning.end())
-      TN_RETURN_IF(qr_takes_columns(ctx, m, n, A, lda, sA, Q, sQ, R, sR, batch, &columns));
+    TN_RETURN_IF(qr_takes_columns(ctx, m, n, A, lda, sA, Q, sQ, R, sR, batch, &columns));
     if (columns) {
       const int slot = prof_begin(ctx);
       TN_RETURN_IF(qr_cols_batch(ctx, m, n, A, lda, sA, Q, sQ, R, sR, batch));
