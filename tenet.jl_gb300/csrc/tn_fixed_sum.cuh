@@ -4,10 +4,13 @@
 
 #include <cuda_runtime.h>
 
-// Every lane's value is cut to 55 bits below 2^(emax − 1022), emax the largest exponent field of
-// the warp, so a cut is at most 2⁻⁵⁵ of the largest value: less than the rounding of an FP64 sum.
-// The parts of 24 bits add up without a carry between them.  The sum is in units of
-// 2^(emax − 1077); four warps' sums aligned to a common exponent fit in 63 bits.
+// Every lane's value is cut towards zero to 55 bits below 2^(emax − 1022), emax the largest exponent
+// field of the warp.  A unit is 2^(emax − 1077), the largest value at least 2^(emax − 1023): a cut is less
+// than 2⁻⁵⁴ of it, and the 31 others' cuts of a warp less than 31·2⁻⁵⁴ (a value within a factor of 4
+// of the largest is not cut at all).  An FP64 tree's five roundings are 2⁻⁵³ of the partial sums each: less
+// where one value outweighs the rest, more where the values are alike.  Values below FP64's normal
+// range count as zero.  The parts of 24 bits add up without a carry between them; four warps' sums
+// aligned to a common exponent fit in 63 bits.
 __device__ __forceinline__ unsigned exponent_field(double v) { return ((unsigned)__double2hiint(v) >> 20) & 0x7ff; }
 __device__ __forceinline__ long long fixed_warp_sum(double v, unsigned emax) {
   const int hi = __double2hiint(v);
