@@ -339,8 +339,8 @@ __device__ __forceinline__ void v_role(const Mat& M, int k, bool v_given, int ma
 // threads per row, one for each output column, so that all four schedulers have work.
 template <int R, bool SPLIT>
 __global__ void __launch_bounds__(kNT, 4)
-    k_jacobi_pairs(const Mat* __restrict__ mats, const int* __restrict__ owner, bool v_given, int max_sweeps, int first,
-                   int* err) {
+    k_jacobi_pairs(const Mat* __restrict__ mats, const int* __restrict__ owner, bool v_given, double tol_rel, int max_sweeps,
+                   int first, int* err) {
   static_assert(!SPLIT || R == 1, "two threads per row cover 64 rows");
   // (block `first` is CTA 0, and so on around)
   const int cta = (int)blockIdx.x >= first ? (int)blockIdx.x - first : (int)(blockIdx.x + gridDim.x) - first;
@@ -352,7 +352,9 @@ __global__ void __launch_bounds__(kNT, 4)
   // 1e-7 of it), is below rounding
   constexpr float kTwoU = 2.220446e-16f;
   const float tol2 = kTwoU * kTwoU;
-  constexpr float stop_ratio = 1e-9f;
+  // (1e-9 for every m that this kernel takes; as a constant the 512-row kernel came out 0.6 % slower,
+  // 78.4 → 78.9 ms of two 512 × 512 SVDs and a TEBD layer around them)
+  const float stop_ratio = (float)fmin(sqrt(tol_rel * sqrt((double)(m > 1 ? m : 1)) * 0.1), 1e-9);
   if (cta - M.cta0 >= pairs) {
     v_role<R, SPLIT>(M, cta - M.cta0 - pairs, v_given, max_sweeps, stop_ratio, err);
     return;
@@ -830,13 +832,14 @@ tn_status_t jacobi_pairs(tn_ctx* ctx, const std::vector<JacobiMat>& mats, bool v
     TN_CHECK_CUDA(ctx, cudaMemcpyAsync(table, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream));
     const Mat* dm = reinterpret_cast<const Mat*>(table);
     const int* down = reinterpret_cast<const int*>(table + owner_at);
+    double tol_rel = 4.0 * 2.220446049250313e-16;
     // One matrix with V on slightly more CTAs than SMs: the blocks beyond one per SM share the SMs of
     // the first ones, so those are given to V, which has time to spare, as long as W's
     // CTAs then have an SM each (200 × 200: 3.2 → 3.0 µs a round).  Where blocks really lie only
     // matters for the time.
     const int64_t extra = g - ctx->num_sms;
     int turn = with_v && count == 1 && extra > 0 && extra + g / 2 <= ctx->num_sms ? (int)extra : 0;
-    void* args[] = {&dm, &down, &v_given, &max_sweeps, &turn, &err};
+    void* args[] = {&dm, &down, &v_given, &tol_rel, &max_sweeps, &turn, &err};
     const int slot = prof_begin(ctx);
     TN_CHECK_CUDA(ctx, cudaLaunchCooperativeKernel(kernel_for(mmax), dim3((unsigned)g), dim3(kNT), args, 0, ctx->stream));
     TN_LAUNCHED(ctx);
