@@ -22,6 +22,7 @@
 // t = sgn(ζ)/(|ζ|+√(1+ζ²)), c = 1/√(1+t²), s = c·t:
 //   w_i' = c·w_i − s·e^{−iφ}·w_j,   w_j' = s·e^{iφ}·w_i + c·w_j.
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "tn_internal.cuh"
@@ -960,7 +961,12 @@ static tn_status_t launch_step(tn_ctx* ctx, int64_t m, int64_t n, int N, int r, 
 // Which FP64 kernel a batch takes (no truncation flags): the persistent column-pair kernel
 // spreads every matrix over n/2 SMs; one CTA per matrix in shared memory is left for matrices
 // of a few columns, where the launch is the time, and for batches of so many small matrices
-// that they fill the chip twice over with one SM each.
+// that they fill the chip twice over with one SM each.  With V (twice the CTAs) it is left a fuller
+// wave of one matrix per SM already: the pairs take as long at a fraction of the wave that grows
+// with the matrix.  Measured, µs, shared memory / pairs: 8×8 ×64 281 / 207, ×128 281 / 367, ×303 438 / 754;
+// 16×16 ×64 1215 / 712, ×128 1243 / 1418; 32×32 ×64 4801 / 2895, ×128 4634 / 5423, ×200 9125 / 8764, ×303
+// 9122 / 12696; 64×64 ×128 25726 / 25818, ×200 50243 / 39984, ×303 51699 / 60060; 128×64 ×128 30875 / 26600.
+// (At 32 columns the shared-memory kernel goes from 128 to 512 threads.)
 static tn_status_t jacobi_takes_pairs(tn_ctx* ctx, int64_t m, int64_t n, int64_t batch, bool with_v, bool* out) {
   *out = false;
   if (!jacobi_pairs_fits(m, n) || n < kPairsMinN || jacobi_pairs_workspace(m, n, batch, with_v) > ws_room(ctx)) return TN_OK;
@@ -969,6 +975,12 @@ static tn_status_t jacobi_takes_pairs(tn_ctx* ctx, int64_t m, int64_t n, int64_t
   if ((n + 1) / 2 * (with_v ? 2 : 1) > resident) return TN_OK;
   const bool in_smem = sizeof(cxd) * (size_t)(m * n + n * n) <= kSmemMax && n <= 256;
   *out = !(in_smem && (n + 1) / 2 * batch > 2 * resident && batch >= 2 * ctx->num_sms);
+  if (*out && in_smem && with_v) {
+    const int64_t waves = (batch + ctx->num_sms - 1) / ctx->num_sms;
+    const double size = std::log2((double)(m * n));
+    const double part = n >= 32 ? 0.70 + 0.0625 * (size - 10.0) : 0.47 + 0.055 * (size - 6.0) + 0.15 / (double)waves;
+    *out = (double)batch < part * (double)(waves * ctx->num_sms);
+  }
   return TN_OK;
 }
 
