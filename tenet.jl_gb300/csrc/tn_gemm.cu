@@ -240,14 +240,41 @@ __global__ void __launch_bounds__(kFineThreads)
   }
 }
 
+// K split over a cluster while the 8-wide column tiles leave SMs idle and a rank keeps a
+// whole stage: a function of n and k only (see the kernel)
+int fine_ranks(int64_t n, int64_t k, int64_t sms) {
+  int CS = 1;
+  while (CS < 8 && (int64_t)cdiv(n, 8) * CS * 2 <= sms && k >= (int64_t)kFineBK * CS * 2) CS *= 2;
+  return CS;
+}
+
+// Whether FP64 products of these sizes take less time in k_gemm_fine, which spends a whole stage of
+// 32 on what is left of k and 16 accumulators' sums per output and rank (some 16 of k; 36 and 22 with
+// the tiles of one and two rows): both times in outputs·k of one SM, 2 clocks of its FP64 pipe each.
+// 2000 products of every size from 1 to 20000: of 400 in which k_gemm_fine was up to 5 times slower
+// 12 are left, by at most 9 %.  Measured, µs, register tiles / fine: 64×1000×1 ×200 814 / 4213,
+// 2000×64×4 12.6 / 49.7, 20000×64×4 114 / 431, 2000×128×200 ×16 5643 / 9065, 64×128×200 ×200 2466 / 3636;
+// 256×256×512 ×1 1.4 times faster fine.
+bool fine_pays(int64_t m, int64_t n, int64_t k, int64_t batch, int64_t bm, int64_t bn, int64_t sms) {
+  int64_t tm = 32, tn = 32;  // the register tile that would serve
+  if (m <= 8 && n >= 64)
+    tm = 8;
+  else if (m <= 16 && n >= 64)
+    tm = 16;
+  else if ((int64_t)cdiv(m, 64) * cdiv(n, 64) * batch >= sms)
+    tm = tn = 64;
+  const double tiles = (double)cdiv((int64_t)cdiv(m, tm) * cdiv(n, tn) * batch, sms) * (double)(tm * tn);
+  const int CS = fine_ranks(n, k, sms);
+  const double stages = (double)cdiv(k, kFineBK), sums = bm == 1 ? 36 : bm == 2 ? 22 : 16;
+  const double fine = (double)cdiv((int64_t)cdiv(m, bm) * cdiv(n, bn) * batch * CS, sms) * (double)(bm * bn);
+  return fine * (kFineBK * stages / CS + sums) + 900 < tiles * 0.95 * 8.0 * (double)cdiv(k, 8);
+}
+
 template <typename T, int BM, int BN>
 tn_status_t launch_fine(tn_ctx* ctx, char opa, char opb, int64_t m, int64_t n, int64_t k, cx<T> alpha, const cx<T>* A,
                         int64_t lda, int64_t sA, const cx<T>* B, int64_t ldb, int64_t sB, cx<T> beta, cx<T>* C,
                         int64_t ldc, int64_t sC, int64_t batch) {
-  // K split over a cluster while the 8-wide column tiles leave SMs idle and a rank keeps a
-  // whole stage: a function of n and k only (see the kernel)
-  int CS = 1;
-  while (CS < 8 && (int64_t)cdiv(n, 8) * CS * 2 <= ctx->num_sms && k >= (int64_t)kFineBK * CS * 2) CS *= 2;
+  const int CS = fine_ranks(n, k, ctx->num_sms);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cdiv(m, BM) * (unsigned)CS, cdiv(n, BN), (unsigned)(batch < 65535 ? batch : 65535));
   cfg.blockDim = dim3(kFineThreads);
@@ -299,8 +326,9 @@ tn_status_t gemm_cx(tn_ctx* ctx, char opa, char opb, int64_t m, int64_t n, int64
   const int64_t bm = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : 8, bn = bm < 8 ? 16 : 8;
   const int64_t tiles_f = (int64_t)cdiv(m, bm) * cdiv(n, bn) * batch;
   const bool fits = cdiv(n, bn) <= 65535u && (int64_t)cdiv(m, bm) * 8 <= 0x7fffffff;
-  const bool fine = sizeof(T) == 8 ? cdiv(tiles64, sms) * 4096.0 > cdiv(tiles_f, sms) * (double)(bm * bn) * 1.05
-                                   : 4 * tiles32 <= sms;
+  bool fine = sizeof(T) == 8 ? cdiv(tiles64, sms) * 4096.0 > cdiv(tiles_f, sms) * (double)(bm * bn) * 1.05
+                             : 4 * tiles32 <= sms;
+  if (sizeof(T) == 8 && fine) fine = fine_pays(m, n, k, batch, bm, bn, sms);
   if (fine && fits) {
     if (bm == 1)
       return launch_fine<T, 1, 16>(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
