@@ -980,6 +980,18 @@ static tn_status_t jacobi_takes_pairs(tn_ctx* ctx, int64_t m, int64_t n, int64_t
     const double size = std::log2((double)(m * n));
     const double part = n >= 32 ? 0.70 + 0.0625 * (size - 10.0) : 0.47 + 0.055 * (size - 6.0) + 0.15 / (double)waves;
     *out = (double)batch < part * (double)(waves * ctx->num_sms);
+  } else if (*out && with_v && m > 256) {
+    // Four rows per thread, and more matrices than one launch holds: µs of a round over all of them, by
+    // one launch after the other of up to `resident` CTAs, and by one launch per round (four CTAs of a
+    // pair each to an SM).  Measured, ms, pairs / rounds: 300×150 ×8 23.9 / 21.6, ×40 118.7 / 93.0; 300×300 ×5 76.5 /
+    // 88.3, ×16 223.9 / 204.9; 400×400 ×2 65.5 / 76.2, ×5 161.5 / 149.8; 260×60 ×16 7.57 / 6.77; 512×256 ×5
+    // 55.6 / 60.7; 512×512 ×3 157 / 191
+    const int64_t each = n + (n & 1), per = resident / each, rest = batch % per, ctas = batch * ((n + 1) / 2);
+    auto launch = [&](int64_t c) { return 5.3 + (double)c * (0.0018 + 1.4e-5 * (double)n); };
+    const double by_pairs = (double)(batch / per) * launch(per * each) + (rest > 0 ? launch(rest * each) : 0.0);
+    const double waves = std::ceil((double)ctas / (4.0 * ctx->num_sms));
+    const double by_rounds = (6.0 + 0.01 * (double)n) * (0.4 + 0.6 * waves) + (double)ctas * (24.0 * (double)m + 30.0 * (double)n) * 1e-6;
+    *out = by_pairs < by_rounds;
   }
   return TN_OK;
 }
