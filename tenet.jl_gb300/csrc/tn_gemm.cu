@@ -251,8 +251,8 @@ int fine_ranks(int64_t n, int64_t k, int64_t sms) {
 // Whether FP64 products of these sizes take less time in k_gemm_fine, which spends a whole stage of
 // 32 on what is left of k and 16 accumulators' sums per output and rank (some 16 of k; 36 and 22 with
 // the tiles of one and two rows): both times in outputs·k of one SM, 2 clocks of its FP64 pipe each.
-// 2000 products of every size from 1 to 20000: of 400 in which k_gemm_fine was up to 5 times slower
-// 12 are left, by at most 9 %.  Measured, µs, register tiles / fine: 64×1000×1 ×200 814 / 4213,
+// 3000 products of sizes from 1 to 20000: of 880 in which k_gemm_fine was slower by more than 6 %, up to
+// 5 times, 12 are left, and the sum of all is 0.1 % above that of the faster kernel of each.  Measured, µs, register tiles / fine: 64×1000×1 ×200 814 / 4213,
 // 2000×64×4 12.6 / 49.7, 20000×64×4 114 / 431, 2000×128×200 ×16 5643 / 9065, 64×128×200 ×200 2466 / 3636;
 // 256×256×512 ×1 1.4 times faster fine.
 bool fine_pays(int64_t m, int64_t n, int64_t k, int64_t batch, int64_t bm, int64_t bn, int64_t sms) {
@@ -263,11 +263,13 @@ bool fine_pays(int64_t m, int64_t n, int64_t k, int64_t batch, int64_t bm, int64
     tm = 16;
   else if ((int64_t)cdiv(m, 64) * cdiv(n, 64) * batch >= sms)
     tm = tn = 64;
-  const double tiles = (double)cdiv((int64_t)cdiv(m, tm) * cdiv(n, tn) * batch, sms) * (double)(tm * tn);
+  // (in 0.95 of k, rounded up to the 8 that are staged together; 0.97 of it in a single wave of 32×32 tiles)
+  const int64_t waves = cdiv((int64_t)cdiv(m, tm) * cdiv(n, tn) * batch, sms);
+  const double spent = (tm == 32 && waves == 1 && k > 24 ? 0.97 : 0.95) * 8.0 * (double)cdiv(k, 8);
   const int CS = fine_ranks(n, k, sms);
   const double stages = (double)cdiv(k, kFineBK), sums = bm == 1 ? 36 : bm == 2 ? 22 : 16;
   const double fine = (double)cdiv((int64_t)cdiv(m, bm) * cdiv(n, bn) * batch * CS, sms) * (double)(bm * bn);
-  return fine * (kFineBK * stages / CS + sums) + 900 < tiles * 0.95 * 8.0 * (double)cdiv(k, 8);
+  return fine * (kFineBK * stages / CS + sums) + 900 < (double)(waves * tm * tn) * spent;
 }
 
 template <typename T, int BM, int BN>
