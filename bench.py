@@ -185,13 +185,14 @@ def pipe_peaks(ctx):
         hbm, bf16, src = mp["hbm_gbs"], mp["bf16_tflops"], "MEASURED_PEAKS.json"
     else:
         hbm, bf16, src = 6800.0, 1900.0, "fallback (6.8 TB/s, 1.9 PFLOP/s bf16)"
-    return {"hbm_gbs": hbm, "bf16_tflops": bf16, "fp32_tflops": ctx.pipe_peak("fp32"),
+    return {"hbm_gbs": hbm, "bf16_tflops": bf16, "tf32_tflops": bf16 / 2, "fp32_tflops": ctx.pipe_peak("fp32"),
             "fp64_tflops": ctx.pipe_peak("fp64"),
-            "source": f"HBM and BF16: {src} (measured); FP32 / FP64 CUDA-core FMA rate: measured in this run"}
+            "source": f"HBM and BF16: {src} (measured), TF32 half the BF16 rate; FP32 / FP64 CUDA-core FMA rate: measured in this run"}
 
 
-# per profiled class: the pipe whose peak bounds its arithmetic
-_PIPE = {"jacobi_fp32": ("fp32_tflops", "fp32_cuda_cores"), "jacobi_fp64": ("fp64_tflops", "fp64_cuda_cores"),
+# per profiled class: the pipe that does its arithmetic (the FP32 sweeps' flops are the rotations'
+# own, not those of the products that the tensor pipe forms them from)
+_PIPE = {"jacobi_fp32": ("tf32_tflops", "tensor"), "jacobi_fp64": ("fp64_tflops", "fp64_cuda_cores"),
          "gemm_fp64": ("fp64_tflops", "fp64_cuda_cores"), "gemm_split_bf16": ("bf16_tflops", "tensor"),
          "split_prep": (None, "hbm"), "qr": ("fp64_tflops", "fp64_cuda_cores"),
          "jacobi_coop": ("fp64_tflops", "fp64_cuda_cores")}

@@ -860,7 +860,8 @@ tn_status_t jacobi_pairs(tn_ctx* ctx, const std::vector<JacobiMat>& mats, bool v
         }
       }
       const double mm = hm[q].m, nn = hm[q].n;
-      flops += h[1] * nn * (nn - 1) / 2 * (32.0 * mm + (with_v ? 24.0 * nn : 0.0));
+      // a pair's row: 8 operations of wᵢᴴwⱼ, 16 of the scaled rotation of W [16 of V's]
+      flops += h[1] * nn * (nn - 1) / 2 * (24.0 * mm + (with_v ? 16.0 * nn : 0.0));
     }
     if (slot >= 0) prof_end(ctx, slot, TN_PROF_JACOBI_COOP, 1, flops, 0.0);
     if (h_ctl[kCtl * count]) return tn_set_error(ctx, TN_ETIMEOUT, "svd: a wait of the Jacobi rounds exceeded its limit");

@@ -19,7 +19,7 @@
 //    column q of Q = H₀…H_{k−1}, which needs reflectors q…0 only, is formed by its column's CTA
 //    as soon as column q is done, with half the products.
 //  * u₁ is sent before κ, so that the receivers' wᴴ = uᴴc is complete when κ arrives.
-// A step takes 2.3 µs with a column per SM: a packet's 0.4 µs, two reductions of 0.4 µs, the
+// A step takes 2.0 µs with a column per SM: a packet's 0.4 µs, two reductions of 0.4 µs, the
 // scalars of 0.5 µs and the updates, in FP64 operations of 64 clocks' latency each.
 // Reflectors and signs are LAPACK's (H = I − τ v vᴴ, v₁ = 1, τ v vᴴ = κ u uᴴ, R_jj real with
 // the sign opposite to Re x₁).  Every wait is bounded: a CTA whose wait ran out records an
@@ -40,7 +40,8 @@ constexpr int kNT = 128;
 static_assert(kQrColsMaxRows == 4 * kNT);
 constexpr long long kSpinLimit = 1ll << 22;
 // A column or row far from its turn leaves the memory to the ones whose turn it is: asleep for
-// 1 µs between looks at a packet (a step is 2.3 µs) instead of 64 ns, 128 × 128 took 398 µs, not 443.
+// 1 µs between looks at a packet (a step is 2 µs) instead of 64 ns, 128 × 128 took 398 µs, not 443 (299
+// now).
 constexpr unsigned kFarSleep = 1000;
 
 struct QMat {
