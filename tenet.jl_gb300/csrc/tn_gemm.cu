@@ -252,9 +252,9 @@ int fine_ranks(int64_t n, int64_t k, int64_t sms) {
 // 32 on what is left of k and 16 accumulators' sums per output and rank (some 16 of k; 36 and 22 with
 // the tiles of one and two rows): both times in outputs·k of one SM, 2 clocks of its FP64 pipe each.
 // 3000 products of sizes from 1 to 20000: of 880 in which k_gemm_fine was slower by more than 6 %, up to
-// 5 times, 12 are left, and the sum of all is 0.1 % above that of the faster kernel of each.  Measured, µs, register tiles / fine: 64×1000×1 ×200 814 / 4213,
-// 2000×64×4 12.6 / 49.7, 20000×64×4 114 / 431, 2000×128×200 ×16 5643 / 9065, 64×128×200 ×200 2466 / 3636;
-// 256×256×512 ×1 1.4 times faster fine.
+// 5 times, 12 are left, and the sum of all is 0.1 % above that of the faster kernel of each.  Measured,
+// µs, register tiles / fine: 64×1000×1 ×200 814 / 4213, 2000×64×4 12.6 / 49.7, 20000×64×4 114 / 431,
+// 2000×128×200 ×16 5643 / 9065, 64×128×200 ×200 2466 / 3636; 256×256×512 ×1 1.4 times faster fine.
 bool fine_pays(int64_t m, int64_t n, int64_t k, int64_t batch, int64_t bm, int64_t bn, int64_t sms) {
   int64_t tm = 32, tn = 32;  // the register tile that would serve
   if (m <= 8 && n >= 64)

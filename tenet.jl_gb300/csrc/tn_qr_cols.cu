@@ -40,7 +40,7 @@ constexpr int kNT = 128;
 static_assert(kQrColsMaxRows == 4 * kNT);
 constexpr long long kSpinLimit = 1ll << 22;
 // A column or row far from its turn leaves the memory to the ones whose turn it is: asleep for
-// 1 µs between looks at a packet (a step is 2 µs) instead of 64 ns, 128 × 128 took 398 µs, not 443 (299
+// 1 µs between looks at a packet (a step is 2 µs) instead of 64 ns, 128 × 128 took 398 µs, not 443 (299 by
 // now).
 constexpr unsigned kFarSleep = 1000;
 
